@@ -1,20 +1,27 @@
 // clip_engine.cuh -- warp-cooperative exact clipping of tets against unit cells.
 //
-// A batch of up to 32 (tet, cell) pairs is clipped by the whole warp at once.
-// Every lane holds one piece (a tet, 12 FP32 coordinates in the cell frame)
-// in registers.  Each step a lane either
-//   * drops its piece (entirely outside a cell face it has not yet passed),
-//   * finishes it (inside all six faces): its 6x volume is added, as exact
-//     64-bit fixed point, to the accumulator of the pair it came from, or
-//   * at the last cell face it crosses, adds the inside fraction of its
-//     volume (from the edge parameters alone, no cut points), or
-//   * splits it by a cell face it crosses (of those, one with the fewest of
-//     its vertices inside: next_face) into 1 or 3 inside pieces, keeps one
-//     and pushes the others onto a per-warp shared-memory pool;
-// then idle lanes pop pieces from the pool (last in, first out).  All lanes
-// run the same split code every step, so a pair whose tet crosses several
-// faces (up to 3^6 pieces) spreads over the warp instead of serialising one
-// lane.  No per-thread stack: nothing spills to local memory.
+// The (tet, cell) pairs a CTA has listed are clipped by its warps, a lane per
+// piece (a tet, 12 FP32 coordinates in the cell frame), in three kinds of
+// steps, each with the same instructions on every lane:
+//   * a build step turns 32 listed pairs into pieces, which go to the warp's
+//     shared-memory pool, or to its last-face list if they cross one cell face;
+//   * a split step takes up to 32 pieces from the pool (last in, first out)
+//     and splits each by a cell face it crosses (of those, one with the fewest
+//     of its vertices inside: next_face) into 1 or 3 inside pieces.  A child
+//     outside a face is dropped; one inside all of them adds its 6x volume, as
+//     exact 64-bit fixed point, to the accumulator of the pair it came from;
+//     one that crosses a single face goes to the last-face list with its
+//     volume; only the others go back to the pool;
+//   * a last-face step sums the inside parts of up to 32 listed pieces: their
+//     volumes times the inside fractions (from the edge parameters alone, no
+//     cut points).
+// A pair whose tet crosses several faces (up to 3^6 pieces) so spreads over
+// the warp instead of serialising one lane.  No per-thread stack: nothing
+// spills to local memory.  One loop whose step did all of it, each lane in its
+// own branch, had run ~640 instructions a step; the three kinds run ~290, 800
+// and 110, the 800 once for the pieces of 2.6 such steps.  With the selects
+// free of branches (bit_sel), octree leaves of a 192^3 lattice: 1.78e10 ->
+// 1.43e10 warp instructions with 21.9 -> 26.0 of 32 lanes.
 //
 // The split keeps every piece positively oriented: the vertices are permuted
 // (an even permutation) so that the k inside vertices come first, then the
@@ -33,13 +40,19 @@ static const uint8_t h_split_perm[16] = ADECO_SPLIT_PERM;
 static const int8_t h_split_kin[16] = ADECO_SPLIT_KIN;
 
 // The tables are read with lane-dependent masks, which a constant-memory load
-// serialises per distinct address; the entries are therefore taken from two
-// 64-bit immediates (the permutation, a byte per mask) and from the popcount
-// (the inside count) -- the same values as ADECO_SPLIT_PERM / ADECO_SPLIT_KIN.
+// serialises per distinct address; the entries are therefore taken from
+// immediates (the permutation: a byte per mask, picked by a byte permute) and
+// from the popcount (the inside count) -- the same values as
+// ADECO_SPLIT_PERM / ADECO_SPLIT_KIN.
 ADECO_HD inline int split_perm(int m)
 {
+#ifdef __CUDA_ARCH__
+    const unsigned lo = __byte_perm(0xe4b1e4e4u, 0xe4c9d2d2u, m & 7), hi = __byte_perm(0xb1879c63u, 0xe436784eu, m & 7);
+    return (int)(((m & 8) ? hi : lo) & 0xffu);
+#else
     const unsigned long long w = (m & 8) ? 0xe436784eb1879c63ull : 0xe4c9d2d2e4b1e4e4ull;
     return (int)((w >> ((m & 7) * 8)) & 0xffu);
+#endif
 }
 ADECO_HD inline int split_kin(int m)
 {
@@ -56,110 +69,109 @@ ADECO_HD inline float sel4(int i, float a, float b, float c, float d)
 }
 ADECO_HD inline float sel3(int i, float x, float y, float z) { return i == 0 ? x : (i == 1 ? y : z); }
 
-// 6 inside bits of a point: bit 2a = (x_a > 0), bit 2a+1 = (x_a < 1)
-ADECO_HD inline int face_bits(float x, float y, float z)
+// A select by a bit mask (all ones: a, zero: b), one logic instruction.  Where
+// an expression selects among many candidates the compiler turns ternaries
+// into branches (the cut of a piece: 33 branch instructions of 224, and most
+// of its time); the mask form has none.
+ADECO_HD inline unsigned bit_mask(bool c) { return c ? 0xffffffffu : 0u; }
+ADECO_HD inline float bit_sel(unsigned m, float a, float b)
 {
-    return (int)(x > 0.f) | ((int)(x < 1.f) << 1) | ((int)(y > 0.f) << 2) | ((int)(y < 1.f) << 3) |
-           ((int)(z > 0.f) << 4) | ((int)(z < 1.f) << 5);
+#ifdef __CUDA_ARCH__
+    unsigned r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xCA;" : "=r"(r) : "r"(m), "r"(__float_as_uint(a)), "r"(__float_as_uint(b)));
+    return __uint_as_float(r);
+#else
+    return m ? a : b;
+#endif
 }
 
-// The cut of piece p by face f (mask: its vertices inside, 0 < mask < 15;
-// k of them), shared by a split and a last-face fraction: the vertices
-// permuted to A B C D, inside first by an even permutation (the orientation
-// is kept), the four cut edges' end points -- k=1: AB AC AD AD; k=2: AC AD
-// BC BD; k=3: AD BD CD CD -- and on each edge the reciprocal r of its extent
-// along the face's axis and the face's parameter t from the inside end.
-struct Cut {
-    float A[3], B[3], C[3], D[3];
-    float i[4][3], o[4][3];
-    float t[4], r[4];
-    int k;
-};
+// x limited to [0, 1]
+ADECO_HD inline float sat01(float x)
+{
+#ifdef __CUDA_ARCH__
+    return __saturatef(x);
+#else
+    return fminf(fmaxf(x, 0.f), 1.f);
+#endif
+}
 
-ADECO_HD inline void cut_piece(const float p[12], int mask, int f, Cut &c)
+// 6 inside bits of a point: bit 2a = (x_a > 0), bit 2a+1 = (x_a < 1).  On the
+// device from the sign bits of 0 - x and x - 1 (exact signs; a zero result is
+// +0, a NaN has sign 0), shifted in one by one: half on the FMA pipe, where
+// six compares and selects all go to the ALU pipe, the busiest one.
+ADECO_HD inline int face_bits(float x, float y, float z)
+{
+#ifdef __CUDA_ARCH__
+    unsigned b = __float_as_uint(__fsub_rn(z, 1.f)) >> 31;
+    b = __funnelshift_l(__float_as_uint(__fsub_rn(0.f, z)), b, 1);
+    b = __funnelshift_l(__float_as_uint(__fsub_rn(y, 1.f)), b, 1);
+    b = __funnelshift_l(__float_as_uint(__fsub_rn(0.f, y)), b, 1);
+    b = __funnelshift_l(__float_as_uint(__fsub_rn(x, 1.f)), b, 1);
+    return (int)__funnelshift_l(__float_as_uint(__fsub_rn(0.f, x)), b, 1);
+#else
+    return (int)(x > 0.f) | ((int)(x < 1.f) << 1) | ((int)(y > 0.f) << 2) | ((int)(y < 1.f) << 3) |
+           ((int)(z > 0.f) << 4) | ((int)(z < 1.f) << 5);
+#endif
+}
+
+// The cut of a piece by face f, its vertices permuted to A B C D, the k
+// inside ones first by an even permutation (the orientation is kept): the cut
+// points E0..E3 of the four cut edges -- k=1: AB AC AD AD; k=2: AC AD BC BD;
+// k=3: AD BD CD CD -- snapped onto the face.
+ADECO_HD inline void cut_points(const float A[3], const float B[3], const float C[3], const float D[3], int k, int f,
+                                float E[4][3])
 {
     const int axis = f >> 1;
     const float plane = (f & 1) ? 1.f : 0.f;
-    const int pm = split_perm(mask), k = split_kin(mask);
-    c.k = k;
-    const int ia = pm & 3, ib = (pm >> 2) & 3, ic = (pm >> 4) & 3, id = (pm >> 6) & 3;
+    const unsigned k1 = bit_mask(k == 1), k2 = bit_mask(k == 2), k3 = bit_mask(k == 3);
+    const unsigned a[3] = {bit_mask(axis == 0), bit_mask(axis == 1), bit_mask(axis == 2)};
+    float in[4][3], out[4][3];
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
-        c.A[x] = sel4(ia, p[x], p[3 + x], p[6 + x], p[9 + x]);
-        c.B[x] = sel4(ib, p[x], p[3 + x], p[6 + x], p[9 + x]);
-        c.C[x] = sel4(ic, p[x], p[3 + x], p[6 + x], p[9 + x]);
-        c.D[x] = sel4(id, p[x], p[3 + x], p[6 + x], p[9 + x]);
-        c.i[0][x] = c.A[x];
-        c.o[0][x] = (k == 1) ? c.B[x] : ((k == 2) ? c.C[x] : c.D[x]);
-        c.i[1][x] = (k == 3) ? c.B[x] : c.A[x];
-        c.o[1][x] = (k == 1) ? c.C[x] : c.D[x];
-        c.i[2][x] = (k == 1) ? c.A[x] : ((k == 2) ? c.B[x] : c.C[x]);
-        c.o[2][x] = (k == 2) ? c.C[x] : c.D[x];
-        c.i[3][x] = (k == 2) ? c.B[x] : ((k == 3) ? c.C[x] : c.A[x]);
-        c.o[3][x] = c.D[x];
+        in[0][x] = A[x];
+        out[0][x] = bit_sel(k1, B[x], bit_sel(k2, C[x], D[x]));
+        in[1][x] = bit_sel(k3, B[x], A[x]);
+        out[1][x] = bit_sel(k1, C[x], D[x]);
+        in[2][x] = bit_sel(k1, A[x], bit_sel(k2, B[x], C[x]));
+        out[2][x] = bit_sel(k2, C[x], D[x]);
+        in[3][x] = bit_sel(k2, B[x], bit_sel(k3, C[x], A[x]));
+        out[3][x] = D[x];
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        const float din = sel3(axis, c.i[e][0], c.i[e][1], c.i[e][2]);
-        const float dout = sel3(axis, c.o[e][0], c.o[e][1], c.o[e][2]);
-        c.r[e] = rcp_nr(dout - din);  // |dout - din| > 0 on a crossing edge
-        c.t[e] = fminf(fmaxf((plane - din) * c.r[e], 0.f), 1.f);
+        const float din = bit_sel(a[0], in[e][0], bit_sel(a[1], in[e][1], in[e][2]));
+        const float dout = bit_sel(a[0], out[e][0], bit_sel(a[1], out[e][1], out[e][2]));
+        const float t = sat01((plane - din) * rcp_nr(dout - din));  // |dout - din| > 0 on a crossing edge
+#pragma unroll
+        for (int x = 0; x < 3; ++x) E[e][x] = bit_sel(a[x], plane, fmaf(t, out[e][x] - in[e][x], in[e][x]));
     }
 }
 
-// Inside part of a cut piece as n = 1 or 3 positively oriented pieces
-// c0..c2, from the cut points E0..E3 of the cut's edges (snapped onto the
-// face):
+// Inside part of a cut piece as 1 or 3 positively oriented pieces, child
+// 0..2:
 //   k = 1: (A, Xab, Xac, Xad)
 //   k = 2: (A, B, Xbc, Xbd) (A, Xbc, Xac, Xbd) (A, Xac, Xad, Xbd)
 //   k = 3: (A, B, C, Xcd)  (A, B, Xcd, Xbd) (A, Xbd, Xcd, Xad)
-// written as one code path: the children's vertices picked by k.
-ADECO_HD inline int split_cut(const Cut &c, int f, float c0[12], float c1[12], float c2[12])
+// child_vertex picks vertex 1..3 of a child (vertex 0 is A) among the values
+// of B, C and the cut points: coordinates, or any other 32-bit words of them.
+ADECO_HD inline float child_vertex(int child, int v, unsigned k1, unsigned k2, float B, float C, const float E[4])
 {
-    const int axis = f >> 1;
-    const float plane = (f & 1) ? 1.f : 0.f;
-    float E[4][3];
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-#pragma unroll
-        for (int x = 0; x < 3; ++x)
-            E[e][x] = (x == axis) ? plane : fmaf(c.t[e], c.o[e][x] - c.i[e][x], c.i[e][x]);
-    // k=1: E0=Xab E1=Xac E2=Xad | k=2: E0=Xac E1=Xad E2=Xbc E3=Xbd | k=3: E0=Xad E1=Xbd E2=Xcd
-    const bool k1 = (c.k == 1), k2 = (c.k == 2);
-#pragma unroll
-    for (int x = 0; x < 3; ++x) {
-        c0[x] = c.A[x];
-        c0[3 + x] = k1 ? E[0][x] : c.B[x];
-        c0[6 + x] = k1 ? E[1][x] : (k2 ? E[2][x] : c.C[x]);
-        c0[9 + x] = k1 ? E[2][x] : (k2 ? E[3][x] : E[2][x]);
-        c1[x] = c.A[x];
-        c1[3 + x] = k2 ? E[2][x] : c.B[x];
-        c1[6 + x] = k2 ? E[0][x] : E[2][x];
-        c1[9 + x] = k2 ? E[3][x] : E[1][x];
-        c2[x] = c.A[x];
-        c2[3 + x] = k2 ? E[0][x] : E[1][x];
-        c2[6 + x] = k2 ? E[1][x] : E[2][x];
-        c2[9 + x] = k2 ? E[3][x] : E[0][x];
-    }
-    return k1 ? 1 : 3;
+    if (child == 0) return v == 1 ? bit_sel(k1, E[0], B)
+                                  : (v == 2 ? bit_sel(k1, E[1], bit_sel(k2, E[2], C)) : bit_sel(k2, E[3], E[2]));
+    if (child == 1) return v == 1 ? bit_sel(k2, E[2], B) : (v == 2 ? bit_sel(k2, E[0], E[2]) : bit_sel(k2, E[3], E[1]));
+    return v == 1 ? bit_sel(k2, E[0], E[1]) : (v == 2 ? bit_sel(k2, E[1], E[2]) : bit_sel(k2, E[3], E[0]));
 }
 
-// The fraction of a cut piece inside the face (its last crossed face), from
-// the edge parameters alone: t from the cut, u = 1 - t taken as (x_o -
-// plane) r so both keep their relative precision (side_fraction's formulas,
-// on the same edges).
-ADECO_HD inline float cut_fraction(const Cut &c, int f)
+ADECO_HD inline void split_child(int child, unsigned k1, unsigned k2, const float A[3], const float B[3],
+                                 const float C[3], const float E[4][3], float p[12])
 {
-    const int axis = f >> 1;
-    const float plane = (f & 1) ? 1.f : 0.f;
-    float u[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-        u[e] = fminf(fmaxf((sel3(axis, c.o[e][0], c.o[e][1], c.o[e][2]) - plane) * c.r[e], 0.f), 1.f);
-    const float *t = c.t;
-    if (c.k == 1) return t[0] * t[1] * t[2];
-    if (c.k == 2) return fmaf(t[2], t[3], t[0] * (t[3] * u[2] + t[1] * u[3]));
-    return fmaf(u[0], fmaf(u[1], t[2], t[1]), t[0]);
+    for (int x = 0; x < 3; ++x) {
+        const float e[4] = {E[0][x], E[1][x], E[2][x], E[3][x]};
+        p[x] = A[x];
+#pragma unroll
+        for (int v = 1; v < 4; ++v) p[3 * v + x] = child_vertex(child, v, k1, k2, B[x], C[x], e);
+    }
 }
 
 // Fraction of piece p inside face f (mask = 4-bit inside flags, 0 < mask <
@@ -177,26 +189,26 @@ ADECO_HD inline float cut_fraction(const Cut &c, int f)
 ADECO_HD inline float side_fraction(float x0, float x1, float x2, float x3, int mask, float plane)
 {
     const int pm = split_perm(mask), k = split_kin(mask);
+    const bool k1 = k == 1, k2 = k == 2, k3 = k == 3;
     const float a = sel4(pm & 3, x0, x1, x2, x3), b = sel4((pm >> 2) & 3, x0, x1, x2, x3);
     const float c = sel4((pm >> 4) & 3, x0, x1, x2, x3), d = sel4((pm >> 6) & 3, x0, x1, x2, x3);
-    // edges as in cut_piece: k=1: AB AC AD; k=2: AC AD BC BD; k=3: AD BD CD
-    const float i0 = a, o0 = (k == 1) ? b : ((k == 2) ? c : d);
-    const float i1 = (k == 3) ? b : a, o1 = (k == 1) ? c : d;
-    const float i2 = (k == 1) ? a : ((k == 2) ? b : c), o2 = (k == 2) ? c : d;
-    const float i3 = b, o3 = d;
+    // edges as in cut_points: k=1: AB AC AD; k=2: AC AD BC BD; k=3: AD BD CD
+    const float in[4] = {a, k3 ? b : a, k1 ? a : (k2 ? b : c), b};
+    const float out[4] = {k1 ? b : (k2 ? c : d), k1 ? c : d, k2 ? c : d, d};
     float t[4], u[4];
-    const float in[4] = {i0, i1, i2, i3}, out[4] = {o0, o1, o2, o3};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         // an unbiased reciprocal (rcp_nr): an approximate one biases the
         // fractions of all pairs the same way and shows in the total mass
         const float r = rcp_nr(out[e] - in[e]);
-        t[e] = fminf(fmaxf((plane - in[e]) * r, 0.f), 1.f);
-        u[e] = fminf(fmaxf((out[e] - plane) * r, 0.f), 1.f);
+        t[e] = sat01((plane - in[e]) * r);
+        u[e] = sat01((out[e] - plane) * r);
     }
-    if (k == 1) return t[0] * t[1] * t[2];
-    if (k == 2) return fmaf(t[2], t[3], t[0] * (t[3] * u[2] + t[1] * u[3]));
-    return fmaf(u[0], fmaf(u[1], t[2], t[1]), t[0]);
+    // all three formulas and a select: a branch by k runs them one after the other anyway
+    const float f1 = t[0] * t[1] * t[2];
+    const float f2 = fmaf(t[2], t[3], t[0] * (t[3] * u[2] + t[1] * u[3]));
+    const float f3 = fmaf(u[0], fmaf(u[1], t[2], t[1]), t[0]);
+    return k1 ? f1 : (k2 ? f2 : f3);
 }
 
 // 6x volume of the unit cube's part where G(u) = G0 + n.u > 0 (G0 a
@@ -283,23 +295,20 @@ ADECO_HD inline int next_face(int b0, int b1, int b2, int b3, int done, int &fac
 {
     const int all_in = b0 & b1 & b2 & b3, any_in = b0 | b1 | b2 | b3;
     const int relevant = 63 & ~done;
-    if ((~any_in) & relevant) return 0;  // entirely outside a remaining face
-    const int next = (~all_in) & relevant;
-    if (!next) return 1;
+    const int next = (~all_in) & relevant;  // crossed, or entirely outside
     // per crossed face 1..3 vertices inside: odd -> 1 or 3, `two` -> at least 2
     const int odd = b0 ^ b1 ^ b2 ^ b3;
     const int two = (b0 & b1) | (b2 & b3) | ((b0 | b1) & (b2 | b3));
-    int pick = next & odd & ~two;   // one vertex inside
-    if (!pick) pick = next & ~odd;  // two inside
-    if (!pick) pick = next;         // three inside
+    const int one_in = next & odd & ~two, two_in = next & ~odd;
+    const int pick = (one_in ? one_in : (two_in ? two_in : next)) | (next ? 0 : 1);
 #ifdef __CUDA_ARCH__
-    face = __ffs(pick) - 1;
+    face = 31 - __clz(pick & -pick);
 #else
     face = __builtin_ctz(pick);
 #endif
     mask = ((b0 >> face) & 1) | (((b1 >> face) & 1) << 1) | (((b2 >> face) & 1) << 2) | (((b3 >> face) & 1) << 3);
     last = (next & (next - 1)) == 0;
-    return 2;
+    return (~any_in & relevant) ? 0 : (next ? 2 : 1);
 }
 
 // ---------------------------------------------------- barycentric clipping
@@ -493,6 +502,18 @@ ADECO_HD inline int piece_step(const float p[12], int done, int &face, int &mask
                      face_bits(p[9], p[10], p[11]), done, face, mask, last);
 }
 
+// 6x volume, in fixed point, of a piece that needs no further split: inside
+// every remaining face, or the part inside the last crossed one (last).
+ADECO_HD inline long long leaf_volume(const float p[12], bool last, int f, int mask)
+{
+    const int axis = f >> 1;
+    float v = piece_vol6(p);
+    if (last)
+        v *= side_fraction(sel3(axis, p[0], p[1], p[2]), sel3(axis, p[3], p[4], p[5]), sel3(axis, p[6], p[7], p[8]),
+                           sel3(axis, p[9], p[10], p[11]), mask, (f & 1) ? 1.f : 0.f);
+    return vol_fixed(v);
+}
+
 // Serial clipping of one piece whose faces in `done0` are done (used when the
 // warp pool is full): depth-first over the same splits and last-face fractions, so the
 // fixed-point sum is the warp engine's.
@@ -521,30 +542,27 @@ long long clip_piece_serial(const float p0[12], int done0)
         const int code = piece_step(p, sdone[sp], face, mask, last);
         if (code == 0) continue;
         if (code == 1) {
-            acc += vol_fixed(piece_vol6(p));
+            acc += leaf_volume(p, false, face, mask);
             continue;
         }
-        Cut cut;
-        cut_piece(p, mask, face, cut);
         if (last) {
-            acc += vol_fixed(piece_vol6(p) * cut_fraction(cut, face));
+            acc += leaf_volume(p, true, face, mask);
             continue;
         }
-        float c0[12], c1[12], c2[12];
-        const int n = split_cut(cut, face, c0, c1, c2);
+        const int pm = split_perm(mask), k = split_kin(mask);
+        float V[4][3], E[4][3];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int x = 0; x < 3; ++x) V[q][x] = sel4((pm >> (2 * q)) & 3, p[x], p[3 + x], p[6 + x], p[9 + x]);
+        cut_points(V[0], V[1], V[2], V[3], k, face, E);
+        const int n = k == 1 ? 1 : 3;
         if (sp + 3 > kDepth) continue;  // cannot happen (depth <= 2*5 + 3)
         const int d = sdone[sp] | (1 << face);
 #pragma unroll
-        for (int x = 0; x < 12; ++x) stk[sp][x] = c0[x];
-        sdone[sp] = d;
-        ++sp;
-        if (n == 3) {
-#pragma unroll
-            for (int x = 0; x < 12; ++x) stk[sp][x] = c1[x];
-            sdone[sp] = d;
-            ++sp;
-#pragma unroll
-            for (int x = 0; x < 12; ++x) stk[sp][x] = c2[x];
+        for (int c = 0; c < 3; ++c) {
+            if (c >= n) continue;
+            split_child(c, bit_mask(k == 1), bit_mask(k == 2), V[0], V[1], V[2], E, stk[sp]);
             sdone[sp] = d;
             ++sp;
         }
@@ -553,138 +571,244 @@ long long clip_piece_serial(const float p0[12], int done0)
 }
 
 #ifdef __CUDACC__
-constexpr int kPool = 56;    // pieces per warp pool (2 CTAs of 8 warps fit in an SM's shared memory)
-constexpr int kPairs = 128;  // partial pairs per warp list
+constexpr int kPool = 72;    // pieces per warp pool (2 CTAs of 8 warps fit in an SM's shared memory)
+constexpr int kLast = 88;    // pieces at their last crossed face per warp
+constexpr int kPairs = 1024;  // partial pairs a CTA lists
+
+static_assert(kPool >= 32 + 3 && kLast >= 32 + 3, "one split step fits a full pool and list");
 
 struct WarpPool {
-    float4 v[kPool][3];       // a piece's 12 coordinates per slot: 48 bytes, moved as three 16-byte words
-    uint32_t meta[kPool];     // owner | faces done << 8
-    long long vacc[kPairs];   // 6x volume of each listed pair, fixed point 2^kVolShift
+    float v[12][kPool];         // the pieces' coordinates, a row per coordinate: a lane's four vertices come in
+                                // any order by their addresses, without a bank conflict
+    uint32_t flags[kPool];      // the vertices' inside flags, 6 bits each
+    uint16_t owner[kPool];      // the piece's pair
+    float last[5][kLast];       // pieces at their last face: 6x volume, the vertices' coordinate along its axis
+    uint32_t last_meta[kLast];  // inside mask | upper face << 4 | owner << 8
 };
 
-// Clip the warp's list of np partial pairs: an idle lane takes a piece from
-// the pool (last in, first out) or, when the pool is empty, the next pair of
-// the list (build(j, p) writes its tet in cell coordinates).  Each step a
-// lane makes at most one split: at the piece's last crossed face the
-// children are summed in place, otherwise one child is kept and the others
-// pushed.  On return pool.vacc[0..np) hold the pairs' 6x volumes.
+// The partial pairs a CTA has listed and their 6x volumes.
+struct PairList {
+    int n;      // pairs listed
+    int next;   // first pair no warp has taken
+    uint32_t cell[kPairs];  // the pair's cell (the caller's encoding)
+    uint8_t tet[kPairs];    //   and its tet
+    uint32_t vlo[kPairs], vhi[kPairs];  // fixed point 2^kVolShift
+
+    __device__ __forceinline__ long long volume(int j) const
+    {
+        return (long long)(((unsigned long long)vhi[j] << 32) | vlo[j]);
+    }
+    // 64-bit add as two 32-bit shared-memory additions, the carry taken from
+    // the first one's result (a 64-bit shared-memory atomic is a
+    // compare-and-swap loop, which lanes of the same pair repeat)
+    __device__ __forceinline__ void add(int j, long long v)
+    {
+        const unsigned lo = (unsigned)v;
+        const unsigned old = atomicAdd(&vlo[j], lo);
+        atomicAdd(&vhi[j], (unsigned)((unsigned long long)v >> 32) + (unsigned)(old + lo < old));
+    }
+    __device__ __forceinline__ void set(int j, long long v)
+    {
+        vlo[j] = (uint32_t)v;
+        vhi[j] = (uint32_t)((unsigned long long)v >> 32);
+    }
+};
+
+__device__ __forceinline__ void put_last(WarpPool &pool, int slot, const float p[12], float v6, int f, int mask, int owner)
+{
+    const unsigned ax = bit_mask(f < 2), ay = bit_mask(f < 4);
+    pool.last[0][slot] = v6;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) pool.last[1 + q][slot] = bit_sel(ax, p[3 * q], bit_sel(ay, p[3 * q + 1], p[3 * q + 2]));
+    pool.last_meta[slot] = (uint32_t)(mask | ((f & 1) << 4) | (owner << 8));
+}
+
+// Clip the CTA's np listed pairs (build(j, p) writes pair j's tet in cell
+// coordinates); every warp takes pairs from the list until none is left.  When
+// all warps are through, list.volume(j) of j < np are the pairs' 6x volumes.
 template <typename Build>
-__device__ __forceinline__ void clip_pairs(WarpPool &pool, int np, Build build, unsigned &fallbacks)
+__device__ __forceinline__ void clip_pairs(WarpPool &pool, PairList &list, int np, Build build, unsigned &fallbacks)
 {
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1;
-    for (int j = lane; j < np; j += 32) pool.vacc[j] = 0;
-    __syncwarp();
-    bool valid = false;
-    float p[12];
-    int owner = 0, done = 0;  // the piece's pair and its faces done (one bit per face)
-    int top = 0, next = 0;
+    int top = 0, nlast = 0;
+    bool more_pairs = np > 0;
     for (;;) {
-        // refill idle lanes
-        const unsigned need = __ballot_sync(0xffffffffu, !valid);
-        const int rank = __popc(need & lt), nneed = __popc(need);
-        if (!valid) {
-            if (rank < top) {
-                const int idx = top - 1 - rank;
-#pragma unroll
-                for (int w = 0; w < 3; ++w) {
-                    const float4 q = pool.v[idx][w];
-                    p[4 * w] = q.x;
-                    p[4 * w + 1] = q.y;
-                    p[4 * w + 2] = q.z;
-                    p[4 * w + 3] = q.w;
-                }
-                const uint32_t m = pool.meta[idx];
-                owner = (int)(m & 0xff);
-                done = (int)(m >> 8);
-                valid = true;
-            } else {
-                const int j = next + rank - top;
-                if (j < np) {
-                    build(j, p);
-                    owner = j;
-                    done = 0;
-                    valid = true;
-                }
+        if (nlast >= 32 || (nlast && !top && !more_pairs)) {
+            // the inside parts of up to 32 pieces at their last face
+            const int n = min(nlast, 32), idx = nlast - 1 - lane;
+            if (lane < n) {
+                const uint32_t m = pool.last_meta[idx];
+                const float frac = side_fraction(pool.last[1][idx], pool.last[2][idx], pool.last[3][idx],
+                                                 pool.last[4][idx], m & 15, (m & 16) ? 1.f : 0.f);
+                list.add((int)(m >> 8), vol_fixed(pool.last[0][idx] * frac));
             }
+            nlast -= n;
+            __syncwarp();
+            continue;
         }
-        const int from_pool = nneed < top ? nneed : top;
-        top -= from_pool;
-        next = min(np, next + (nneed - from_pool));
-        const unsigned held = __ballot_sync(0xffffffffu, valid);
-        if (!held) break;
-        __syncwarp();  // the pool slots just read may be written by this step's pushes
-        // one step.  A lane about to split into three reserves room in the
-        // pool for its two extra children first: in lane order, as many as
-        // fit.  A lane whose children do not fit keeps its piece and steps
-        // again next round, while the other lanes finish pieces and idle lanes
-        // drain the pool.  Only when every lane holds a piece and none can
-        // move does one lane clip its piece alone (serially, with a local
-        // stack): letting every pushing lane of a full pool do that had put
-        // most of the fine-grid time into one-lane serial clipping.
-        int f = 0, mask = 0, code = 0;
-        bool last = false;
-        if (valid) code = piece_step(p, done, f, mask, last);
-        const bool split = valid && code == 2 && !last;
-        const bool push = split && split_kin(mask) != 1;  // two children to push
-        const unsigned pushing = __ballot_sync(0xffffffffu, push);
-        const int fit = (kPool - top) >> 1;  // pushing lanes whose children fit
-        const int prank = __popc(pushing & lt);
-        const bool defer = push && prank >= fit;
-        const int nfit = min(__popc(pushing), fit);
-        const bool stuck = held == 0xffffffffu && pushing == 0xffffffffu && fit == 0;
-        if (valid && !defer) {
+        if (top < 32 && more_pairs) {
+            // build step
+            int nb = min(32, min(kPool - top, kLast - nlast)), j = 0;
+            if (lane == 0) j = atomicAdd(&list.next, nb);
+            j = __shfl_sync(0xffffffffu, j, 0);
+            more_pairs = j + nb < np;
+            nb = min(nb, np - j);  // may be <= 0
+            j += lane;
+            bool push = false, last = false;
+            float p[12];
+            uint32_t flags = 0;
+            int f = 0, mask = 0;
             long long v = 0;
-            // the cut is shared by the lanes that split and the lanes at
-            // their last crossed face, so the warp runs it once per step
-            float frac = 1.f;
-            Cut cut;
-            if (code == 2) cut_piece(p, mask, f, cut);
-            if (split) {
-                float c0[12], c1[12], c2[12];
-                split_cut(cut, f, c0, c1, c2);
-#pragma unroll
-                for (int x = 0; x < 12; ++x) p[x] = c0[x];
-                done |= 1 << f;
-                if (push) {
-                    // second children in one block, third children in the
-                    // next: consecutive pushing lanes write slots 48 bytes
-                    // apart, which spreads a quarter-warp's 16-byte words
-                    // over all banks
-                    const int s1 = top + prank, s2 = top + nfit + prank;
-                    const uint32_t m = (uint32_t)owner | ((uint32_t)done << 8);
-#pragma unroll
-                    for (int w = 0; w < 3; ++w) {
-                        pool.v[s1][w] = make_float4(c1[4 * w], c1[4 * w + 1], c1[4 * w + 2], c1[4 * w + 3]);
-                        pool.v[s2][w] = make_float4(c2[4 * w], c2[4 * w + 1], c2[4 * w + 2], c2[4 * w + 3]);
-                    }
-                    pool.meta[s1] = m;
-                    pool.meta[s2] = m;
-                }
-            } else {
-                // finished, or at its last crossed face: the inside part
-                // needs no more clipping, so its volume is added here
-                if (code == 2) frac = cut_fraction(cut, f);
-                if (code != 0) v = vol_fixed(piece_vol6(p) * frac);
-                valid = false;
+            if (lane < nb) {
+                build(j, p);
+                const int b0 = face_bits(p[0], p[1], p[2]), b1 = face_bits(p[3], p[4], p[5]),
+                          b2 = face_bits(p[6], p[7], p[8]), b3 = face_bits(p[9], p[10], p[11]);
+                flags = (uint32_t)(b0 | (b1 << 6) | (b2 << 12) | (b3 << 18));
+                const int code = next_face(b0, b1, b2, b3, 0, f, mask, last);
+                push = code == 2 && !last;
+                last = code == 2 && last;
+                if (code == 1) v = vol_fixed(piece_vol6(p));
+                list.set(j, v);
             }
-            if (v) atomicAdd(reinterpret_cast<unsigned long long *>(&pool.vacc[owner]), (unsigned long long)v);
-        } else if (stuck && lane == 0) {
-            // a copy made here: handing p itself to the out-of-line routine
-            // takes its address, and p then lives in local memory, stored
-            // there on every step although this branch almost never runs
-            float q[12];
+            const unsigned pushing = __ballot_sync(0xffffffffu, push), lasts = __ballot_sync(0xffffffffu, last);
+            if (push) {
+                const int slot = top + __popc(pushing & lt);
 #pragma unroll
-            for (int x = 0; x < 12; ++x) q[x] = p[x];
-            const long long acc = clip_piece_serial(q, done);
-            atomicAdd(reinterpret_cast<unsigned long long *>(&pool.vacc[owner]), (unsigned long long)acc);
-            valid = false;
-            ++fallbacks;
+                for (int x = 0; x < 12; ++x) pool.v[x][slot] = p[x];
+                pool.flags[slot] = flags;
+                pool.owner[slot] = (uint16_t)j;
+            }
+            if (last) put_last(pool, nlast + __popc(lasts & lt), p, piece_vol6(p), f, mask, j);
+            top += __popc(pushing);
+            nlast += __popc(lasts);
+            __syncwarp();
+            continue;
         }
-        top += 2 * nfit;
+        if (!top) break;
+        // split step: lane l takes slot top - 1 - l
+        const int n = min(top, 32), idx = top - 1 - lane;
+        int owner = 0;
+        int code[3] = {0, 0, 0};  // per child: 0 dropped, 1 inside, 2 at its last face, 3 to split further
+        uint32_t cflags[3];
+        int cnext[3];
+        float A[3], B[3], C[3], E[4][3];
+        unsigned k1 = 0, k2 = 0;
+        if (lane < n) {
+            // A done face has all four flags 0, which no other face of a pool
+            // piece can have (the piece would lie outside it): no done set is kept.
+            const uint32_t m = pool.flags[idx];
+            owner = pool.owner[idx];
+            const int done = 63 & ~(int)(m | (m >> 6) | (m >> 12) | (m >> 18));
+            int f, mask;
+            bool last;
+            next_face(m & 63, (m >> 6) & 63, (m >> 12) & 63, (m >> 18) & 63, done, f, mask, last);
+            const int pm = split_perm(mask), k = split_kin(mask);
+            const int ia = pm & 3, ib = (pm >> 2) & 3, ic = (pm >> 4) & 3, id = (pm >> 6) & 3;
+            float D[3];
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                A[x] = pool.v[3 * ia + x][idx];
+                B[x] = pool.v[3 * ib + x][idx];
+                C[x] = pool.v[3 * ic + x][idx];
+                D[x] = pool.v[3 * id + x][idx];
+            }
+            cut_points(A, B, C, D, k, f, E);
+            k1 = bit_mask(k == 1);
+            k2 = bit_mask(k == 2);
+            const int keep = 63 & ~(done | (1 << f));
+            const int bA = (int)(m >> (6 * ia)) & keep;
+            const float bB = __int_as_float((int)(m >> (6 * ib)) & keep), bC = __int_as_float((int)(m >> (6 * ic)) & keep);
+            float bE[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) bE[e] = __int_as_float(face_bits(E[e][0], E[e][1], E[e][2]) & keep);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const int b1 = __float_as_int(child_vertex(c, 1, k1, k2, bB, bC, bE)),
+                          b2 = __float_as_int(child_vertex(c, 2, k1, k2, bB, bC, bE)),
+                          b3 = __float_as_int(child_vertex(c, 3, k1, k2, bB, bC, bE));
+                cflags[c] = (uint32_t)(bA | (b1 << 6) | (b2 << 12) | (b3 << 18));
+                cnext[c] = keep & ~(bA & b1 & b2 & b3);  // crossed, or entirely outside
+                const bool out = (keep & ~(bA | b1 | b2 | b3)) != 0 || (c > 0 && k1);
+                code[c] = out ? 0 : (cnext[c] == 0 ? 1 : ((cnext[c] & (cnext[c] - 1)) == 0 ? 2 : 3));
+            }
+        }
+        unsigned sm[3], lm[3];  // the lanes whose child c goes to the pool / to the last-face list
+        int ns = 0, nl = 0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            sm[c] = __ballot_sync(0xffffffffu, code[c] == 3);
+            lm[c] = __ballot_sync(0xffffffffu, code[c] == 2);
+            ns += __popc(sm[c]);
+            nl += __popc(lm[c]);
+        }
+        // When the children do not all fit, the first lanes for which they do
+        // commit their step; the pieces of the others, the lower slots, stay
+        // where they are.  Only when not even one step fits is a piece clipped
+        // serially, with a local stack.
+        int commit = n;
+        if (top - n + ns > kPool || nlast + nl > kLast) {
+            int s_incl = 0, l_incl = 0;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                s_incl += __popc(sm[c] & (lt << 1 | 1));
+                l_incl += __popc(lm[c] & (lt << 1 | 1));
+            }
+            const unsigned bad =
+                __ballot_sync(0xffffffffu, lane < n && (top - (lane + 1) + s_incl > kPool || nlast + l_incl > kLast));
+            if (bad) commit = __ffs(bad) - 1;
+            const unsigned cm = commit < 32 ? (1u << commit) - 1 : 0xffffffffu;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                sm[c] &= cm;
+                lm[c] &= cm;
+            }
+            if (commit == 0) {
+                if (lane == 0) {
+                    float q[12];
+#pragma unroll
+                    for (int x = 0; x < 12; ++x) q[x] = pool.v[x][idx];
+                    const uint32_t m = pool.flags[idx];
+                    list.add(owner, clip_piece_serial(q, 63 & ~(int)(m | (m >> 6) | (m >> 12) | (m >> 18))));
+                    ++fallbacks;
+                }
+                --top;
+                __syncwarp();
+                continue;
+            }
+        }
+        top -= commit;
+        __syncwarp();  // every lane has read its slot
+        long long v = 0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if (lane < commit && code[c]) {
+                float ch[12];
+                split_child(c, k1, k2, A, B, C, E, ch);
+                if (code[c] == 3) {
+                    const int slot = top + __popc(sm[c] & lt);
+#pragma unroll
+                    for (int x = 0; x < 12; ++x) pool.v[x][slot] = ch[x];
+                    pool.flags[slot] = cflags[c];
+                    pool.owner[slot] = (uint16_t)owner;
+                } else {
+                    const float v6 = piece_vol6(ch);
+                    if (code[c] == 1) {
+                        v += vol_fixed(v6);
+                    } else {
+                        const int f = 31 - __clz(cnext[c]);
+                        const uint32_t t = cflags[c] >> f;
+                        const int mask = (int)((t & 1) | ((t >> 5) & 2) | ((t >> 10) & 4) | ((t >> 15) & 8));
+                        put_last(pool, nlast + __popc(lm[c] & lt), ch, v6, f, mask, owner);
+                    }
+                }
+            }
+            top += __popc(sm[c]);
+            nlast += __popc(lm[c]);
+        }
+        if (v) list.add(owner, v);
         __syncwarp();
     }
-    __syncwarp();
 }
 
 // ------------------------------------------- barycentric warp engine

@@ -6,10 +6,18 @@
 // (7^3 lattice cubes: a meta-cell of a resident lattice, or a sub-block of a
 // reference-format patch).  A CTA stages the block's vertices in shared
 // memory, culls its cubes against the grid box, and deposits the surviving
-// tets with one warp per 32 tets: the tets' candidate (tet, cell) pairs are
-// flattened across the warp, classified with per-tet plane bounds, easy
-// cells are scattered at once and partial cells go through a per-warp
-// shared-memory queue so that 32 lanes always clip together.
+// tets 256 at a time, in phases that all its warps run together:
+//   set-up     each warp builds the table entries of 32 tets, a lane each;
+//   classify   the tets' candidate (tet, cell) pairs are flattened over the
+//              CTA and classified with per-tet plane bounds; easy cells are
+//              scattered at once, partial ones listed;
+//   clip       the listed pairs are clipped by the warps' clip engines;
+//   deposit    the listed pairs' masses are scattered.
+// Together, because the code of all the phases is larger than the SM's
+// instruction cache: with each warp in a phase of its own (a warp taking 32
+// tets through all of them) a third of the issue slots waited for
+// instructions (no_instruction 2.9 stall cycles an issue; 0.25 in phases).
+// And the pairs are the CTA's, so no warp waits for one that holds more.
 //
 // Mass is accumulated as 64-bit fixed point (2^shift units per mass unit)
 // with integer atomics: the sum is exact and independent of the order in
@@ -31,7 +39,8 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxVerts = 512;   // 8^3
 constexpr int kMaxCubes = 343;   // 7^3
-constexpr int kQueue = kPairs;  // partial pairs listed per warp before clipping
+constexpr int kWave = kThreads;       // tets set up together
+constexpr int kQueue = kPairs / kWarps;  // partial pairs listed per warp before clipping, at the most
 
 struct Item {
     long long base;  // vertex index of the block origin (lattice) or of the patch origin + offset
@@ -55,7 +64,7 @@ struct DepositParams {
     int *counter;                     // persistent work counter
     unsigned long long *stats;        // kNumStats counters or nullptr
     int *error;                       // device error flag (bit 0: tet too large, bit 2: route list full,
-                                      // bit 3: a work-sharing wait timed out)
+                                      // bit 3: a bounded wait timed out)
     // ill-conditioned tets, deposited by a second launch (route_fp64_kernel):
     // entries item << 16 | (cube slot * 6 + tet), count in *route_count
     unsigned long long *route;
@@ -63,10 +72,7 @@ struct DepositParams {
     unsigned long long route_cap;
     // launch-shape and batching parameters (set by the host, tunable)
     int per_cta_items;   // items a CTA takes before it exits (0: persistent, until the queue is empty)
-    int share_chunk;     // work sharing: candidate pairs per chunk (zoom grids)
-    int clip_batch;      // partial pairs a warp lists before its engine clips them (64..kQueue)
-    unsigned help_spins; // work sharing: sleeps a helper looks for open slots before leaving
-    unsigned close_spins;  // work sharing: sleeps an owner waits for its helpers (then error bit 3)
+    int clip_batch;      // partial pairs listed per warp before they are clipped (64..kQueue)
 };
 
 enum Stat : int {
@@ -81,23 +87,38 @@ enum Stat : int {
     kNumStats = 8
 };
 
-// Per-warp table of up to 32 tets (structure of arrays in shared memory).
-// Two CTAs of 8 warps fill an SM's shared memory to within a few hundred
-// bytes, so the fields are as narrow as their ranges allow.
-struct WarpTets {
-    float q[12][32];     // vertices in the tet's anchor-cell frame (cell units), rounded
-    float qlo[12][32];   // rounding remainders: q + qlo carries the vertex to ~44 bits
-    float n[4][3][32];   // inward face normals
-    float d[4][32];      // plane offsets n . (face centroid): inside <=> n.x - d > 0
-    float dlo[4][32];    //   and their remainders (d + dlo: ~44 bits)
-    float tol[32];       // FP32 error bound of the plane tests (largest face)
-    float bmin[3][32];   // tet AABB in the anchor frame
-    float bmax[3][32];
-    float f6[32];        // mass per unit of 6x clipped volume (tet mass / |6V| in cell units)
-    uint16_t lo[3][32];  // anchor cell (first candidate cell) in grid indices (dims <= 4096)
-    uint16_t ex[3][32];  // candidate extents (cells per axis)
-    int scan[33];        // exclusive prefix of candidate counts
+// What the classification needs of N tets (structure of arrays in shared
+// memory, the fields as narrow as their ranges allow).
+template <int N>
+struct TetPlanes {
+    float n[4][3][N];   // inward face normals
+    float d[4][N];      // plane offsets n . (face centroid): inside <=> n.x - d > 0
+    float tol[N];       // FP32 error bound of the plane tests (largest face)
+    float bmin[3][N];   // tet AABB in the anchor frame
+    float bmax[3][N];
+    float f6[N];        // mass per unit of 6x clipped volume (tet mass / |6V| in cell units)
+    uint16_t lo[3][N];  // anchor cell (first candidate cell) in grid indices (dims <= 4096)
+    uint16_t ex[3][N];  // candidate extents (cells per axis)
 };
+
+// The vertices of up to 32 tets in their anchor cells' frames (cell units).
+struct TetVertices {
+    float q[12][32];    // rounded
+    float qlo[12][32];  // rounding remainders: q + qlo carries the vertex to ~44 bits
+};
+
+// A table with everything in it, the exact plane offsets' remainders too
+// (d + dlo: ~44 bits), which setup_tet<true> stores.  The kernels form the
+// vertices and the exact offsets again for the pairs that need them.
+struct WarpTets : TetPlanes<32>, TetVertices {
+    float dlo[4][32];
+};
+
+ADECO_HD inline void tet_coord(const WarpTets &W, const GridDesc &, int s, int v, int x, float &hi, float &lo)
+{
+    hi = W.q[3 * v + x][s];
+    lo = W.qlo[3 * v + x][s];
+}
 
 // Tets whose conditioning kappa = (longest edge)^3 / |6V| exceeds this take
 // the FP64 route: FP32 vertices in the cell frame carry ~2^-24 * kappa
@@ -105,16 +126,9 @@ struct WarpTets {
 // miss the 1e-5 per-cell bar.  Lattice tets sit near kappa = 5.2.
 constexpr float kKappaFp64 = 32.f;
 
-// Work sharing inside an item: default pairs per chunk, and the default
-// bounds of its waits (a helper looking for work gives up; an owner waiting
-// for its helpers sets error bit 3 -- the value 8 -- and goes on).
-constexpr int kChunk = 512;
-constexpr unsigned kHelpSpins = 1u << 14;
-constexpr unsigned kCloseSpins = 1u << 26;
-
 // Waits, sleeping `ns` between looks, until *count is 0, at most `limit`
-// looks; false if the limit ran out first.  Every spin-wait of the deposit
-// kernels goes through here, so that none can wait forever.
+// looks; false if the limit ran out first.  A spin-wait in a kernel goes
+// through here, so that none can wait forever (the deposit kernels have none).
 __device__ __forceinline__ bool wait_zero_bounded(const int *count, unsigned limit, unsigned ns)
 {
     for (unsigned spin = 0; *(volatile const int *)count != 0; ++spin) {
@@ -124,25 +138,39 @@ __device__ __forceinline__ bool wait_zero_bounded(const int *count, unsigned lim
     return true;
 }
 
+// The staged vertex block and the wave's tets.
+struct WaveTets : TetPlanes<kWave> {
+    float gh[3][kMaxVerts];  // grid-frame coordinates of the staged vertices, hi
+    float gl[3][kMaxVerts];  //   and lo parts
+    ushort4 vid[kWave];      // the tets' vertices, ordered by the orientation rule
+};
+
+// Vertex coordinate of a wave's tet in its anchor cell's frame: formed again
+// from the staged vertex with the operations of the set-up.
+__device__ __forceinline__ void tet_coord(const WaveTets &W, const GridDesc &g, int s, int v, int x, float &hi, float &lo)
+{
+    const ushort4 id = W.vid[s];
+    const int i = v == 0 ? id.x : (v == 1 ? id.y : (v == 2 ? id.z : id.w));
+    shift_frame(W.gh[x][i], W.gl[x][i], W.lo[x][s], g.drcell[x], hi, lo);
+}
+
 struct SharedMixed {
-    float4 vert[kMaxVerts];
-    float gh[3][kMaxVerts];   // grid-frame coordinates of the staged vertices, hi
-    float gl[3][kMaxVerts];   //   and lo parts
-    uint16_t cubes[kMaxCubes + 1];
+    WaveTets wt;
+    uint2 range[kMaxVerts];   // the staged vertices' candidate cells and box flags (vertex_range)
+    alignas(16) int src_off[6][4];        // the six tets' corners: offsets in the source from a cube's first vertex
+    alignas(8) uint16_t vert_off[6][4];  //   and among the staged vertices
+    uint16_t cubes[kMaxCubes + 1];  // the live cubes' first staged vertices
     int n_cubes;
     int item;
-    int next_group;
     GridDesc g;
-    WarpTets wt[kWarps];
-    uint32_t queue[kWarps][kQueue];
-    WarpPool pool[kWarps];
-    // work sharing inside an item: slot w = warp w's current group
-    int slot_total[kWarps];  // its candidate pairs
-    int slot_next[kWarps];   // first pair not yet taken
-    int slot_busy[kWarps];   // helpers inside the slot
-    int slot_open[kWarps];   // 1 while helpers may join
-    int groups_set;  // groups of the item set up (published or kept private)
+    int scan[kWave];     // pairs of the warp's tets before this one
+    int warp_pairs[kWarps];
+    int cursor;          // first candidate pair of the wave not yet taken
+    int wide;            // a tet of the wave has more than 1024 candidate cells along an axis
+    PairList list;
+    WarpPool pool[kWarps];  // the set-up's TetVertices use the same memory
 };
+static_assert(sizeof(TetVertices) <= sizeof(WarpPool), "the set-up's vertices share the pool");
 
 __device__ __forceinline__ void stat_add(unsigned long long *stats, int which, unsigned long long v)
 {
@@ -159,78 +187,84 @@ __device__ __forceinline__ void warp_stat(unsigned long long *stats, int which, 
 }
 
 // ---------------------------------------------------------------- staging
-__device__ __forceinline__ void stage_block(const DepositParams &P, const Item &it, float4 *vert, int vx, int vy,
-                                            int vz, float (*gh)[kMaxVerts] = nullptr,
-                                            float (*gl)[kMaxVerts] = nullptr)
+// What the candidate range of a tet needs of each vertex, once per vertex
+// instead of once per tet (2058 tets share 512 vertices, and the six FP32
+// divisions of candidate_range were a fifth of the set-up): per axis twice
+// the floor of (x - gmin) / delta, x limited to the grid box, plus one where
+// it is no whole number.  The word grows with x, so a tet's first and last
+// candidate cells (candidate_range) come from the least and the greatest word
+// of its vertices.  x: axes 0 | 1 << 16; y: axis 2 | flags << 16.
+constexpr uint32_t kBelowMax = 0x7u << 16, kAboveMin = 0x38u << 16;    // x < gmax, gmin < x, a bit per axis
+constexpr uint32_t kCullBox = 0xfc0u << 16, kPadVertex = 0x1000u << 16;  // the same two for the cull box; padding
+
+__device__ __forceinline__ uint2 vertex_range(const float p[3], const GridDesc &g, bool pad)
 {
-    const GridDesc *gd = P.grids + it.grid;
+    uint32_t w[3], flags = pad ? kPadVertex : 0u;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float x = p[a];
+        const float lim = (x < g.gmin[a]) ? g.gmin[a] : x;
+        const float q = div_rn(sub_rn((lim < g.gmax[a]) ? lim : g.gmax[a], g.gmin[a]), g.delta[a]);
+        const int lo = (int)floorf(q), hi = (int)ceilf(q);
+        w[a] = (uint32_t)(2 * max(0, min(lo, 8191)) + (hi > lo));
+        flags |= ((x < g.gmax[a] ? 1u : 0u) | (g.gmin[a] < x ? 8u : 0u) | (x < g.cull_max[a] ? 64u : 0u) |
+                  (g.cull_min[a] < x ? 512u : 0u)) << (16 + a);
+    }
+    return make_uint2(w[0] | (w[1] << 16), w[2] | flags);
+}
+
+// position of source vertex gi (the w of a lattice vertex is not used)
+__device__ __forceinline__ float3 load_vertex(const DepositParams &P, long long gi)
+{
+    if (P.src_kind == SRC_LATTICE_F4) {
+        const float4 q = __ldg(reinterpret_cast<const float4 *>(P.src) + gi);
+        return make_float3(q.x, q.y, q.z);
+    }
+    const float *s = reinterpret_cast<const float *>(P.src) + 3 * gi;
+    return make_float3(__ldg(s), __ldg(s + 1), __ldg(s + 2));
+}
+
+// vertex v < 512 of a block vx vertices wide (<= 8) -> v / vx, exact
+__device__ __forceinline__ int small_div(int v, int vx) { return (int)((unsigned)(v * (65536 / vx + 1)) >> 16); }
+
+__device__ __forceinline__ void stage_block(const DepositParams &P, const Item &it, const GridDesc &g, SharedMixed &S,
+                                            int vx, int vy, int vz)
+{
     const int nvt = vx * vy * vz;
     for (int v = threadIdx.x; v < nvt; v += blockDim.x) {
-        const int i = v % vx, r = v / vx, j = r % vy, k = r / vy;
-        const long long gi = it.base + i + P.stride_y * j + P.stride_z * k;
-        float4 p;
-        if (P.src_kind == SRC_LATTICE_F4) {
-            p = __ldg(reinterpret_cast<const float4 *>(P.src) + gi);
-            p.w = 0.f;
-        } else {
-            const float *s = reinterpret_cast<const float *>(P.src) + 3 * gi;
-            p = make_float4(__ldg(s), __ldg(s + 1), __ldg(s + 2), 0.f);
-            if (P.pad_check) {
-                // the reference's padding test on the float inputs
-                const float sum = __fadd_rn(__fadd_rn(fabsf(__fsub_rn(p.x, 666.f)), fabsf(__fsub_rn(p.y, 666.f))),
-                                            fabsf(__fsub_rn(p.z, 666.f)));
-                if ((double)sum < 1.E-03) p.w = 1.f;
-            }
+        const int r = small_div(v, vx), i = v - r * vx, k = small_div(r, vy), j = r - k * vy;
+        const float3 q = load_vertex(P, it.base + i + P.stride_y * j + P.stride_z * k);
+        const float p[3] = {q.x, q.y, q.z};
+        bool pad = false;
+        if (P.pad_check) {
+            // the reference's padding test on the float inputs
+            const float sum = __fadd_rn(__fadd_rn(fabsf(__fsub_rn(p[0], 666.f)), fabsf(__fsub_rn(p[1], 666.f))),
+                                        fabsf(__fsub_rn(p[2], 666.f)));
+            pad = (double)sum < 1.E-03;
         }
-        vert[v] = p;
-        if (gh) {
-            grid_frame(p.x, __ldg(&gd->gmin[0]), __ldg(&gd->scale_hi[0]), __ldg(&gd->scale_lo[0]), gh[0][v], gl[0][v]);
-            grid_frame(p.y, __ldg(&gd->gmin[1]), __ldg(&gd->scale_hi[1]), __ldg(&gd->scale_lo[1]), gh[1][v], gl[1][v]);
-            grid_frame(p.z, __ldg(&gd->gmin[2]), __ldg(&gd->scale_hi[2]), __ldg(&gd->scale_lo[2]), gh[2][v], gl[2][v]);
-        }
+        S.range[v] = vertex_range(p, g, pad);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) grid_frame(p[a], g.gmin[a], g.scale_hi[a], g.scale_lo[a], S.wt.gh[a][v], S.wt.gl[a][v]);
+    }
+    if (threadIdx.x < 24) {
+        const int t = threadIdx.x >> 2, q = threadIdx.x & 3;
+        const int3 o = corner_offset(P.order, tet_conn(t, q));
+        S.vert_off[t][q] = (uint16_t)(o.x + vx * (o.y + vy * o.z));
+        S.src_off[t][q] = (int)(o.x + P.stride_y * o.y + P.stride_z * o.z);
     }
 }
 
-// cube (ci,cj,ck) of the staged block: alive if no padding vertex and its AABB
-// strictly overlaps the grid box
-__device__ __forceinline__ bool cube_alive(const float4 *vert, int vx, int vy, int ci, int cj, int ck,
-                                           const GridDesc &g)
+// cube whose first staged vertex is v0: alive if no padding vertex and its
+// AABB strictly overlaps the grid box (the tile's widened box)
+__device__ __forceinline__ bool cube_alive(const SharedMixed &S, int v0, int vx, int vy)
 {
-    float mn[3] = {3.4e38f, 3.4e38f, 3.4e38f}, mx[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
-    bool pad = false;
+    uint32_t f = 0;
 #pragma unroll
-    for (int s = 0; s < 8; ++s) {
-        const float4 p = vert[(ci + (s & 1)) + vx * ((cj + ((s >> 1) & 1)) + vy * (ck + (s >> 2)))];
-        pad |= (p.w != 0.f);
-        mn[0] = fminf(mn[0], p.x); mx[0] = fmaxf(mx[0], p.x);
-        mn[1] = fminf(mn[1], p.y); mx[1] = fmaxf(mx[1], p.y);
-        mn[2] = fminf(mn[2], p.z); mx[2] = fmaxf(mx[2], p.z);
-    }
-    if (pad) return false;
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-        if (!(mn[a] < g.cull_max[a] && g.cull_min[a] < mx[a])) return false;
-    return true;
-}
-
-__device__ __forceinline__ void load_tet(const float4 *vert, int vx, int vy, int cube_local_idx, int t, int order,
-                                         int cvx, int cvy, float3 v[4], int *vid = nullptr)
-{
-    const int ci = cube_local_idx % cvx, r = cube_local_idx / cvx, cj = r % cvy, ck = r / cvy;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int3 o = corner_offset(order, tet_conn(t, q));
-        const int id = (ci + o.x) + vx * ((cj + o.y) + vy * (ck + o.z));
-        const float4 p = vert[id];
-        v[q] = make_float3(p.x, p.y, p.z);
-        if (vid) vid[q] = id;
-    }
+    for (int s = 0; s < 8; ++s) f |= S.range[v0 + (s & 1) + vx * (((s >> 1) & 1) + vy * (s >> 2))].y;
+    return (f & (kCullBox | kPadVertex)) == kCullBox;
 }
 
 // ------------------------------------------------------ per-tet set-up
-// Build one tet (bit-exact orientation rule and candidate range), then its
-// FP64 anchor-frame geometry, rounded once to FP32.  Returns the candidate
-// pair count (0 if the tet is skipped).
 // Candidate pairs of one tet are limited to kMaxPairsPerTet so that the
 // per-warp flattened pair index fits 32 bits and a queue entry (5-bit slot,
 // 27-bit local index); a larger tet sets the error flag and is skipped.
@@ -255,146 +289,168 @@ ADECO_HD inline F2 plane_offset(const float qa[3], const float la[3], const floa
     return {d_hi, (fmaf(-d_hi, 3.f, dd.hi) + dd.lo) * kThird};
 }
 
+// Entry t of table W from the grid-frame coordinates of a tet's vertices,
+// ordered by the orientation rule (frame(q, a, hi, lo): vertex q, axis a), and
+// its candidate cells as vertex_range words (mn / mx: the least and the
+// greatest of its vertices); its vertices in the anchor frame go to Q's entry
+// `lane`.  Returns the candidate pair count (0 if the tet is skipped).
+//
+// The loops over axes, cofactors and faces are not unrolled: code size (the
+// instruction cache holds about 32 KB: a loop of that size issues at 0.87 of
+// the peak, one of 48 KB at 0.5).
+//
 // kExactD: store each face's exact plane offset (d, dlo: the one-face closed
 // form reads them).  Otherwise only an FP32 d for the classification, whose
 // error band covers its rounding; the closed form then forms the exact
-// offset itself (plane_offset from the stored vertices) for the few pairs
-// that take it.  Octree leaves at the benchmark's cell sizes send almost no
-// pair to the closed form, and the double-float offsets had been ~40% of the
-// set-up; zoom grids, fine against the tets, send many.
-template <bool kExactD = true>
-ADECO_HD inline int setup_tet(const float3 vin[4], const float ghin[4][3], const float glin[4][3], const GridDesc &g,
-                              WarpTets &W, int lane, int *error, bool *fp64_route)
+// offset itself (plane_offset from the stored vertices) for the pairs that
+// take it: the double-float offsets had been ~40% of the set-up.
+template <bool kExactD, class Table, class Frame>
+ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc &g, TetVertices &Q, int lane, Table &W,
+                                int t, int *error, bool *fp64_route)
 {
-    *fp64_route = false;
-    float3 v[4] = {vin[0], vin[1], vin[2], vin[3]};
-    const float v6 = vol6_exact(v[0], v[1], v[2], v[3]);
-    const int sgn = vol6_sign_ref(v6);
-    int lo[3], hi[3];
-    if (!candidate_range(v, g, lo, hi)) return 0;
-    if (sgn == 0) return 0;
-    if (!tile_clamp(g, lo, hi)) return 0;
-    {
-        const long long cnt0 = (long long)(hi[0] - lo[0] + 1) * (hi[1] - lo[1] + 1) * (hi[2] - lo[2] + 1);
-        if (cnt0 > kMaxPairsPerTet) {
-#ifdef __CUDA_ARCH__
-            if (error) atomicOr(error, 1);
-#else
-            if (error) *error |= 1;
-#endif
-            return 0;
-        }
-    }
-    // orientation rule on the vertex order: swap 0 <-> 3 when negative
-    const bool swap03 = sgn < 0;  // selects, not an index: an indexed vertex array would live in local memory
-    // Tight range: of the candidate cells [lo, hi], only those whose box
-    // [c r, c r + 1] (grid frame) meets the tet's AABB can receive mass (the
-    // rest fail the AABB test).  Bounds widened by the FP32 rounding of the
-    // grid-frame coordinates; the frame is then anchored at the first cell.
-    float qf[4][3], ql[4][3];
-#pragma unroll
+    long long cnt0 = 1;
+    unsigned cnt = 1;
+    float R = 0.f;
+#pragma unroll 1
     for (int a = 0; a < 3; ++a) {
-        const float g0 = ghin[0][a], g1 = ghin[1][a], g2 = ghin[2][a], g3 = ghin[3][a];
-        const float bmn = fminf(fminf(g0, g1), fminf(g2, g3)), bmx = fmaxf(fmaxf(g0, g1), fmaxf(g2, g3));
+        const int top = g.dims - 1;
+        const int wlo = (int)((a == 2 ? mn.y : (mn.x >> (16 * a))) & 0xffffu),
+                  whi = (int)((a == 2 ? mx.y : (mx.x >> (16 * a))) & 0xffffu);
+        int lo = wlo >> 1, hi = (whi + 1) >> 1;
+        lo = lo > top ? top : lo;
+        hi = hi > top ? top : hi;
+        lo = lo < g.tile_lo[a] ? g.tile_lo[a] : lo;
+        hi = hi > g.tile_hi[a] ? g.tile_hi[a] : hi;
+        cnt0 = hi < lo ? 0 : cnt0 * (hi - lo + 1);
+        // Tight range: of the candidate cells [lo, hi], only those whose box
+        // [c r, c r + 1] (grid frame) meets the tet's AABB can receive mass (the
+        // rest fail the AABB test).  Bounds widened by the FP32 rounding of the
+        // grid-frame coordinates; the frame is then anchored at the first cell.
+        float h[4], l[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) frame(q, a, h[q], l[q]);
+        const float bmn = fminf(fminf(h[0], h[1]), fminf(h[2], h[3])), bmx = fmaxf(fmaxf(h[0], h[1]), fmaxf(h[2], h[3]));
         const float ir = g.inv_rcell_f[a];
         const float m0 = 4e-7f * (fabsf(bmn) + 2.f), m1 = 4e-7f * (fabsf(bmx) + 2.f);
-        const int c0 = max(lo[a], (int)floorf((bmn - 1.f) * ir - m0) + 1);
-        const int c1 = min(hi[a], (int)ceilf(bmx * ir + m1) - 1);
-        if (c1 < c0) return 0;
-        lo[a] = c0;
-        hi[a] = c1;
+        const int u0 = (int)floorf((bmn - 1.f) * ir - m0) + 1, u1 = (int)ceilf(bmx * ir + m1) - 1;
+        const int c0 = lo > u0 ? lo : u0, c1 = hi < u1 ? hi : u1;
+        const int ex = c1 - c0 + 1;
+        cnt = ex > 0 ? cnt * (unsigned)ex : 0u;
+        float qf[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const int src = (q == 0) ? 0 : ((q == 3) ? 3 : q);  // the vertex before the orientation swap
-            const float h = (q == 0 || q == 3) ? (swap03 ? ghin[3 - src][a] : ghin[src][a]) : ghin[q][a];
-            const float l = (q == 0 || q == 3) ? (swap03 ? glin[3 - src][a] : glin[src][a]) : glin[q][a];
-            shift_frame(h, l, c0, g.drcell[a], qf[q][a], ql[q][a]);
+            float lq;
+            shift_frame(h[q], l[q], c0, g.drcell[a], qf[q], lq);
+            Q.q[3 * q + a][lane] = qf[q];
+            Q.qlo[3 * q + a][lane] = lq;
+            R = fmaxf(R, fabsf(qf[q]));
         }
+        R = fmaxf(R, (float)(ex - 1) + 1.f);
+        W.bmin[a][t] = fminf(fminf(qf[0], qf[1]), fminf(qf[2], qf[3]));
+        W.bmax[a][t] = fmaxf(fmaxf(qf[0], qf[1]), fmaxf(qf[2], qf[3]));
+        W.lo[a][t] = (uint16_t)c0;
+        W.ex[a][t] = (uint16_t)ex;
     }
+    if (cnt0 > kMaxPairsPerTet) {
+#ifdef __CUDA_ARCH__
+        if (error) atomicOr(error, 1);
+#else
+        if (error) *error |= 1;
+#endif
+        return 0;
+    }
+    if (cnt0 <= 0 || cnt == 0) return 0;
     // |6 V| in the anchor frame from the FP32 pairs, in double-float (the
     // tet's volume normaliser): edge vectors from vertex 3, then the triple
-    // product with TwoProd / TwoSum
-    F2 e[3][3];
-#pragma unroll
-    for (int q = 0; q < 3; ++q)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) e[q][a] = f2_add(F2{qf[q][a], ql[q][a]}, F2{-qf[3][a], -ql[3][a]});
-    const F2 cx = f2_add(f2_mul(e[1][1], e[2][2]), f2_neg(f2_mul(e[1][2], e[2][1])));
-    const F2 cy = f2_add(f2_mul(e[1][2], e[2][0]), f2_neg(f2_mul(e[1][0], e[2][2])));
-    const F2 cz = f2_add(f2_mul(e[1][0], e[2][1]), f2_neg(f2_mul(e[1][1], e[2][0])));
-    F2 w6 = f2_add(f2_add(f2_mul(e[0][0], cx), f2_mul(e[0][1], cy)), f2_mul(e[0][2], cz));
+    // product with TwoProd / TwoSum, a cofactor of the first edge at a time
+    F2 w6 = {0.f, 0.f};
+#pragma unroll 1
+    for (int a = 0; a < 3; ++a) {
+        const int b = a == 2 ? 0 : a + 1, c = a == 0 ? 2 : a - 1;
+        auto edge = [&](int q, int x) {
+            return f2_add(F2{Q.q[3 * q + x][lane], Q.qlo[3 * q + x][lane]}, F2{-Q.q[9 + x][lane], -Q.qlo[9 + x][lane]});
+        };
+        const F2 cof = f2_add(f2_mul(edge(1, b), edge(2, c)), f2_neg(f2_mul(edge(1, c), edge(2, b))));
+        w6 = f2_add(w6, f2_mul(edge(0, a), cof));
+    }
     if (w6.hi < 0.f) w6 = f2_neg(w6);
     const float vq6 = w6.hi;
-    const float f6 = f2_div_to_f(F2{g.mf_hi, g.mf_lo}, w6);  // mass per unit of 6x volume
+    W.f6[t] = f2_div_to_f(F2{g.mf_hi, g.mf_lo}, w6);  // mass per unit of 6x volume
     // planes from the FP32 vertices: inward normals (outward ones negated:
     // faces (0,1,2) (0,2,3) (0,3,1) (1,3,2)); each plane's offset is taken
     // through the face's centroid, so that the FP32 rounding of the normal
     // only turns the plane about the centroid (the one-face closed form
     // relies on it)
-    const int fa[4] = {0, 0, 0, 1}, fb[4] = {2, 3, 1, 2}, fc[4] = {1, 2, 3, 3};
-    float R = 0.f;
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) R = fmaxf(R, fabsf(qf[q][a]));
-    R = fmaxf(R, (float)max(max(hi[0] - lo[0], hi[1] - lo[1]), hi[2] - lo[2]) + 1.f);
-    float tolmax = 0.f;
-#pragma unroll
+    float tolmax = 0.f, L2 = 0.f;
+#pragma unroll 1
     for (int f = 0; f < 4; ++f) {
+        const int fa = f == 3, fb = (0x2312 >> (12 - 4 * f)) & 3, fc = (0x1233 >> (12 - 4 * f)) & 3;
+        float A[3], B[3], C[3], e1[3], e2[3];
+        float s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            A[x] = Q.q[3 * fa + x][lane];
+            B[x] = Q.q[3 * fb + x][lane];
+            C[x] = Q.q[3 * fc + x][lane];
+            e1[x] = B[x] - A[x];
+            e2[x] = C[x] - A[x];
+            const float e3 = C[x] - B[x];
+            s1 = fmaf(e1[x], e1[x], s1);
+            s2 = fmaf(e2[x], e2[x], s2);
+            s3 = fmaf(e3, e3, s3);
+        }
+        L2 = fmaxf(L2, fmaxf(s1, fmaxf(s2, s3)));
         // n_in = (vb - va) x (vc - va) with the outward order reversed
-        const float e1x = qf[fb[f]][0] - qf[fa[f]][0], e1y = qf[fb[f]][1] - qf[fa[f]][1],
-                    e1z = qf[fb[f]][2] - qf[fa[f]][2];
-        const float e2x = qf[fc[f]][0] - qf[fa[f]][0], e2y = qf[fc[f]][1] - qf[fa[f]][1],
-                    e2z = qf[fc[f]][2] - qf[fa[f]][2];
-        const float nx = e1y * e2z - e1z * e2y, ny = e1z * e2x - e1x * e2z, nz = e1x * e2y - e1y * e2x;
-        const float nn[3] = {nx, ny, nz};
-        W.n[f][0][lane] = nx;
-        W.n[f][1][lane] = ny;
-        W.n[f][2][lane] = nz;
-        if (kExactD) {
-            const F2 d = plane_offset(qf[fa[f]], ql[fa[f]], qf[fb[f]], ql[fb[f]], qf[fc[f]], ql[fc[f]], nn);
-            W.d[f][lane] = d.hi;
-            W.dlo[f][lane] = d.lo;
+        const float nn[3] = {e1[1] * e2[2] - e1[2] * e2[1], e1[2] * e2[0] - e1[0] * e2[2], e1[0] * e2[1] - e1[1] * e2[0]};
+#pragma unroll
+        for (int x = 0; x < 3; ++x) W.n[f][x][t] = nn[x];
+        if constexpr (kExactD) {
+            float la[3], lb[3], lc[3];
+            for (int x = 0; x < 3; ++x) {
+                la[x] = Q.qlo[3 * fa + x][lane];
+                lb[x] = Q.qlo[3 * fb + x][lane];
+                lc[x] = Q.qlo[3 * fc + x][lane];
+            }
+            const F2 d = plane_offset(A, la, B, lb, C, lc, nn);
+            W.d[f][t] = d.hi;
+            W.dlo[f][t] = d.lo;
         } else {
             constexpr float kThird = 1.f / 3.f;
-            W.d[f][lane] = (nx * (qf[fa[f]][0] + qf[fb[f]][0] + qf[fc[f]][0]) +
-                            ny * (qf[fa[f]][1] + qf[fb[f]][1] + qf[fc[f]][1]) +
-                            nz * (qf[fa[f]][2] + qf[fb[f]][2] + qf[fc[f]][2])) * kThird;
+            W.d[f][t] = (nn[0] * (A[0] + B[0] + C[0]) + nn[1] * (A[1] + B[1] + C[1]) + nn[2] * (A[2] + B[2] + C[2])) * kThird;
         }
-        const float L1 = fmaxf(fmaxf(fabsf(e1x), fabsf(e1y)), fabsf(e1z));
-        const float L2 = fmaxf(fmaxf(fabsf(e2x), fabsf(e2y)), fabsf(e2z));
+        const float L1 = fmaxf(fmaxf(fabsf(e1[0]), fabsf(e1[1])), fabsf(e1[2]));
+        const float M1 = fmaxf(fmaxf(fabsf(e2[0]), fabsf(e2[1])), fabsf(e2[2]));
         // generous bound on the FP32 rounding of n.x - d (|x| <= R + 1)
-        tolmax = fmaxf(tolmax, 1.0e-5f * L1 * L2 * (R + 1.f));
+        tolmax = fmaxf(tolmax, 1.0e-5f * L1 * M1 * (R + 1.f));
     }
-    W.tol[lane] = tolmax;
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            W.q[3 * q + a][lane] = qf[q][a];
-            W.qlo[3 * q + a][lane] = ql[q][a];
-        }
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        W.bmin[a][lane] = fminf(fminf(qf[0][a], qf[1][a]), fminf(qf[2][a], qf[3][a]));
-        W.bmax[a][lane] = fmaxf(fmaxf(qf[0][a], qf[1][a]), fmaxf(qf[2][a], qf[3][a]));
-        W.lo[a][lane] = (uint16_t)lo[a];
-        W.ex[a][lane] = (uint16_t)(hi[a] - lo[a] + 1);
-    }
-    W.f6[lane] = f6;
-    // conditioning: longest edge cubed over |6V|, both in cell units
-    float L2 = 0.f;
-#pragma unroll
-    for (int a0 = 0; a0 < 4; ++a0)
-#pragma unroll
-        for (int b0 = a0 + 1; b0 < 4; ++b0) {
-            const float dx = qf[a0][0] - qf[b0][0], dy = qf[a0][1] - qf[b0][1], dz = qf[a0][2] - qf[b0][2];
-            L2 = fmaxf(L2, dx * dx + dy * dy + dz * dz);
-        }
-    // L^3 <= kappa |6V| squared (both sides non-negative): no square root;
-    // NaN or an overflow routes the tet
+    W.tol[t] = tolmax;
+    // conditioning: longest edge cubed over |6V|, both in cell units.  L^3 <=
+    // kappa |6V| squared (both sides non-negative): no square root; NaN or an
+    // overflow routes the tet
     *fp64_route = !(L2 * L2 * L2 <= (kKappaFp64 * kKappaFp64) * (vq6 * vq6));
-    return (hi[0] - lo[0] + 1) * (hi[1] - lo[1] + 1) * (hi[2] - lo[2] + 1);
+    return (int)cnt;
+}
+
+// One tet from its positions (bit-exact orientation rule and candidate range)
+// and their grid-frame coordinates.
+template <bool kExactD = true, class Table>
+ADECO_HD inline int setup_tet(const float3 v[4], const float gh[4][3], const float gl[4][3], const GridDesc &g,
+                              Table &W, int lane, int *error, bool *fp64_route)
+{
+    *fp64_route = false;
+    const int sgn = vol6_sign_ref(vol6_exact(v[0], v[1], v[2], v[3]));
+    int lo[3], hi[3];
+    if (!candidate_range(v, g, lo, hi) || sgn == 0) return 0;
+    const uint2 mn = make_uint2((uint32_t)(2 * lo[0] | (2 * lo[1]) << 16), (uint32_t)(2 * lo[2]));
+    const uint2 mx = make_uint2((uint32_t)(2 * hi[0] | (2 * hi[1]) << 16), (uint32_t)(2 * hi[2]));
+    return setup_frame<kExactD>(
+        mn, mx,
+        [&](int q, int a, float &h, float &l) {
+            const int v_ = (sgn < 0 && (q == 0 || q == 3)) ? 3 - q : q;  // swap 0 <-> 3 when negative
+            h = gh[v_][a];
+            l = gl[v_][a];
+        },
+        g, W, lane, W, lane, error, fp64_route);
 }
 
 enum PairClass : int { P_NO = 0, P_TET_INSIDE = 1, P_CELL_INSIDE = 2, P_PARTIAL = 3 };
@@ -537,18 +593,23 @@ __device__ __noinline__ void deposit_tet_fp64_warp(const float3 v[4], const int 
 
 // FP64 evaluation of the four plane bounds for a cell whose FP32 test was
 // inside the error band: exact decision for the FP32-rounded tet.
+template <class Table>
 ADECO_HD
 #ifdef __CUDA_ARCH__
 __noinline__
 #endif
-int classify_fp64(const WarpTets &W, const GridDesc &g, int s, int a, int b, int c)
+int classify_fp64(const Table &W, const GridDesc &g, int s, int a, int b, int c)
 {
     const double ca = a * g.rcell[0], cb = b * g.rcell[1], cc = c * g.rcell[2];
     double q[4][3];
 #pragma unroll
     for (int v = 0; v < 4; ++v)
 #pragma unroll
-        for (int x = 0; x < 3; ++x) q[v][x] = (double)W.q[3 * v + x][s] + (double)W.qlo[3 * v + x][s];
+        for (int x = 0; x < 3; ++x) {
+            float hi, lo;
+            tet_coord(W, g, s, v, x, hi, lo);
+            q[v][x] = (double)hi + (double)lo;
+        }
     const int fa[4] = {0, 0, 0, 1}, fb[4] = {2, 3, 1, 2}, fc[4] = {1, 2, 3, 3};
     bool all_in = true;
     for (int f = 0; f < 4; ++f) {
@@ -567,7 +628,8 @@ int classify_fp64(const WarpTets &W, const GridDesc &g, int s, int a, int b, int
 // cross: the one tet face plane the cell straddles when the cell is certainly
 // inside the other three (then cell ∩ tet = cell ∩ that face's half-space),
 // else -1.
-ADECO_HD inline int classify_pair(const WarpTets &W, const GridDesc &g, int s, int a, int b, int c, bool &used_fp64,
+template <class Table>
+ADECO_HD inline int classify_pair(const Table &W, const GridDesc &g, int s, int a, int b, int c, bool &used_fp64,
                                   int &cross)
 {
     cross = -1;
@@ -613,12 +675,12 @@ ADECO_HD inline int classify_pair(const WarpTets &W, const GridDesc &g, int s, i
 // n . origin - (d + dlo) cancels terms as large as the tet is wide in cells:
 // it is formed exactly in double-float (TwoProd of n with the integer cell
 // offsets) and kept as a pair for the corner values.
-template <bool kExactD = true>
-ADECO_HD inline F2 face_value_at_cell(const WarpTets &W, const GridDesc &g, int s, int a, int b, int c, int f)
+template <bool kExactD = true, class Table>
+ADECO_HD inline F2 face_value_at_cell(const Table &W, const GridDesc &g, int s, int a, int b, int c, int f)
 {
     const int cc[3] = {a, b, c};
     F2 G;
-    if (kExactD) {
+    if constexpr (kExactD) {
         G = {-W.d[f][s], -W.dlo[f][s]};
     } else {  // the exact offset setup_tet<true> would have stored
         const int fa = f == 3 ? 1 : 0, fb = f == 0 ? 2 : (f == 1 ? 3 : (f == 2 ? 1 : 2)),
@@ -626,12 +688,9 @@ ADECO_HD inline F2 face_value_at_cell(const WarpTets &W, const GridDesc &g, int 
         float q[3][3], l[3][3];
 #pragma unroll
         for (int x = 0; x < 3; ++x) {
-            q[0][x] = W.q[3 * fa + x][s];
-            l[0][x] = W.qlo[3 * fa + x][s];
-            q[1][x] = W.q[3 * fb + x][s];
-            l[1][x] = W.qlo[3 * fb + x][s];
-            q[2][x] = W.q[3 * fc + x][s];
-            l[2][x] = W.qlo[3 * fc + x][s];
+            tet_coord(W, g, s, fa, x, q[0][x], l[0][x]);
+            tet_coord(W, g, s, fb, x, q[1][x], l[1][x]);
+            tet_coord(W, g, s, fc, x, q[2][x], l[2][x]);
         }
         const float n[3] = {W.n[f][0][s], W.n[f][1][s], W.n[f][2][s]};
         const F2 d = plane_offset(q[0], l[0], q[1], l[1], q[2], l[2], n);
@@ -649,13 +708,13 @@ ADECO_HD inline F2 face_value_at_cell(const WarpTets &W, const GridDesc &g, int 
 
 // 6x volume of cell (a, b, c) ∩ slot s's tet when the cell straddles only
 // face f: the cube's part on its inside.
-template <bool kExactD = true>
+template <bool kExactD = true, class Table>
 #ifdef __CUDA_ARCH__
 __device__ __noinline__
 #else
 inline
 #endif
-float halfspace_pair_vol6(const WarpTets &W, const GridDesc &g, int s, int a, int b, int c, int f)
+float halfspace_pair_vol6(const Table &W, const GridDesc &g, int s, int a, int b, int c, int f)
 {
     return halfspace_cube_vol6(face_value_at_cell<kExactD>(W, g, s, a, b, c, f), W.n[f][0][s], W.n[f][1][s],
                                W.n[f][2][s]);
@@ -665,7 +724,7 @@ float halfspace_pair_vol6(const WarpTets &W, const GridDesc &g, int s, int a, in
 // 64-bit fixed-point accumulator, with integer operations only.  Inlined: as
 // a call it made the pair loop save and restore its live registers in local
 // memory around every scatter (C2: 16% of the kernel time).
-__device__ __forceinline__ void scatter(const DepositParams &P, const GridDesc &g, const WarpTets &W, int s, int a,
+__device__ __forceinline__ void scatter(const DepositParams &P, const GridDesc &g, const WaveTets &W, int s, int a,
                                         int b, int c, float m)
 {
     const unsigned long long fx = to_fixed(m, g.shift);
@@ -696,7 +755,8 @@ ADECO_HD inline float pair_mass(long long vacc, float f6)
 // vertex (up to 5e-5 of such a cell's mass on a 256^3 lattice; 5e-7
 // mirrored).  An odd number of reflections is undone by swapping vertices 0
 // and 1 (the engine wants a positively oriented tet).
-ADECO_HD inline void piece_coords(const WarpTets &W, const GridDesc &g, int s, int a, int b, int c, float p[12])
+template <class Table>
+ADECO_HD inline void piece_coords(const Table &W, const GridDesc &g, int s, int a, int b, int c, float p[12])
 {
     const int cc[3] = {a, b, c};
     int nflip = 0;
@@ -705,57 +765,36 @@ ADECO_HD inline void piece_coords(const WarpTets &W, const GridDesc &g, int s, i
         const bool flip = W.bmin[x][s] > (float)cc[x];
         nflip += flip;
 #pragma unroll
-        for (int v = 0; v < 4; ++v)
-            p[3 * v + x] = cell_coord_fast(W.q[3 * v + x][s], W.qlo[3 * v + x][s], cc[x], g.drcell[x], flip);
-    }
-    if (nflip & 1) {
-#pragma unroll
-        for (int x = 0; x < 3; ++x) {
-            const float t = p[x];
-            p[x] = p[3 + x];
-            p[3 + x] = t;
+        for (int v = 0; v < 4; ++v) {
+            float hi, lo;
+            tet_coord(W, g, s, v, x, hi, lo);
+            p[3 * v + x] = cell_coord_fast(hi, lo, cc[x], g.drcell[x], flip);
         }
+    }
+    const unsigned odd = bit_mask(nflip & 1);
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        const float t = p[x];
+        p[x] = bit_sel(odd, p[3 + x], t);
+        p[3 + x] = bit_sel(odd, t, p[3 + x]);
     }
 }
 
 #ifdef __CUDACC__
-// piece of pair `entry` (slot << 27 | local pair index) in its cell's frame
-__device__ __forceinline__ void pair_piece(const GridDesc &g, const WarpTets &W, uint32_t entry, float p[12], int &s,
-                                           int &a, int &b, int &c)
+// The cell of a candidate pair as PairList holds it: its offsets in the tet's
+// candidate box, a | b << 10 | c << 20; in a wave with a box of more than 1024
+// cells along an axis, the flattened offset.
+__device__ __forceinline__ int3 flat_cell(const WaveTets &W, int s, int local)
 {
-    s = entry >> 27;
-    const int local = entry & ((1u << 27) - 1);
-    const int ex0 = W.ex[0][s], ex1 = W.ex[1][s];
-    a = local % ex0;
-    const int r = local / ex0;
-    b = r % ex1;
-    c = r / ex1;
-    piece_coords(W, g, s, a, b, c, p);
+    const int ex0 = W.ex[0][s], ex1 = W.ex[1][s], r = local / ex0, c = r / ex1;
+    return make_int3(local - r * ex0, r - c * ex1, c);
+}
+__device__ __forceinline__ int3 pair_cell(const WaveTets &W, int s, uint32_t e, bool wide)
+{
+    if (wide) return flat_cell(W, s, (int)e);
+    return make_int3((int)(e & 1023u), (int)((e >> 10) & 1023u), (int)(e >> 20));
 }
 #endif
-
-// clip the warp's listed partial pairs Q[0..np), then scatter them
-__device__ __forceinline__ void clip_list(const DepositParams &P, const GridDesc &g, const WarpTets &W,
-                                          WarpPool &pool, const uint32_t *Q, int np, unsigned &fallbacks)
-{
-    clip_pairs(
-        pool, np,
-        [&](int j, float *p) {
-            int s, a, b, c;
-            pair_piece(g, W, Q[j], p, s, a, b, c);
-        },
-        fallbacks);
-    for (int j = threadIdx.x & 31; j < np; j += 32) {
-        const uint32_t e = Q[j];
-        const int s = e >> 27;
-        const int local = e & ((1u << 27) - 1);
-        const int ex0 = W.ex[0][s], ex1 = W.ex[1][s];
-        const int a = local % ex0, r = local / ex0, b = r % ex1, c = r / ex1;
-        const long long v = pool.vacc[j];
-        if (v > 0) scatter(P, g, W, s, a, b, c, pair_mass(v, W.f6[s]));
-    }
-    __syncwarp();
-}
 
 // -------------------------------------------------- mixed batched kernel
 // per-thread pair counters
@@ -763,34 +802,69 @@ struct PairStats {
     unsigned tets = 0, cand = 0, bbox = 0, in = 0, cin = 0, part = 0, fp64 = 0, fb = 0;
 };
 
-// Sets up group grp (tets 32 grp .. 32 grp + 31 of the item's live cubes) in
-// the warp's table W and returns its candidate pairs.  route64: this lane's
-// tet is ill-conditioned (listed by group_route, no pairs here).
-template <bool kShare>
-__device__ __forceinline__ int group_setup(const DepositParams &P, const SharedMixed &S, WarpTets &W,
-                                           const GridDesc &g, int grp, int ntet, int vx, int vy, int cvx, int cvy,
-                                           int lane, PairStats &st, bool &route64, int &tid)
+// Ill-conditioned tets are listed for route_fp64_kernel: calling their
+// (large) routine from the pair loop made the whole loop spill.
+__device__ __forceinline__ void route_append(const DepositParams &P, const SharedMixed &S, int tid, int vx, int vy)
 {
-    tid = grp * 32 + lane;
+    const unsigned long long n = atomicAdd(P.route_count, 1ull);
+    const int v0 = S.cubes[tid / 6], r = small_div(v0, vx), i = v0 - r * vx, k = small_div(r, vy), j = r - k * vy;
+    if (n < P.route_cap)
+        P.route[n] = ((unsigned long long)S.item << 16) |
+                     (unsigned long long)((i + (vx - 1) * (j + (vy - 1) * k)) * 6 + tid % 6);
+    else
+        atomicOr(P.error, 4);
+}
+
+// Set-up phase: this warp's 32 tets of the wave that starts at tet `first` of
+// the item's live cubes.
+__device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &S, const Item &it, int first, int ntet,
+                                           int vx, int vy, unsigned &n_tets)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slot = threadIdx.x, tid = first + slot;
     int cnt = 0;
-    route64 = false;
+    bool route64 = false;
     if (tid < ntet) {
-        float3 v[4];
-        int vid[4];
-        load_tet(S.vert, vx, vy, S.cubes[tid / 6], tid % 6, P.order, cvx, cvy, v, vid);
-        float gh[4][3], gl[4][3];
+        const int t = tid % 6, v0 = S.cubes[tid / 6];
+        const ushort4 off = *reinterpret_cast<const ushort4 *>(S.vert_off[t]);
+        ushort4 vid = make_ushort4(v0 + off.x, v0 + off.y, v0 + off.z, v0 + off.w);
+        uint2 mn = S.range[vid.x], mx = mn;
+        uint32_t flags = mn.y;
+        const int more[3] = {vid.y, vid.z, vid.w};
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                gh[q][a] = S.gh[a][vid[q]];
-                gl[q][a] = S.gl[a][vid[q]];
-            }
-        cnt = setup_tet<kShare>(v, gh, gl, g, W, lane, P.error, &route64);
+        for (int q = 0; q < 3; ++q) {
+            const uint2 w = S.range[more[q]];
+            flags |= w.y;
+            mn.x = __vminu2(mn.x, w.x);
+            mx.x = __vmaxu2(mx.x, w.x);
+            mn.y = __vminu2(mn.y, w.y);
+            mx.y = __vmaxu2(mx.y, w.y);
+        }
+        // the orientation rule needs the positions themselves (L1 hits: the block was just staged)
+        const int r = small_div(v0, vx), i = v0 - r * vx, k = small_div(r, vy), j = r - k * vy;
+        const long long gi = it.base + i + P.stride_y * j + P.stride_z * k;
+        const int4 so = *reinterpret_cast<const int4 *>(S.src_off[t]);
+        const int sgn = vol6_sign_ref(vol6_exact(load_vertex(P, gi + so.x), load_vertex(P, gi + so.y),
+                                                 load_vertex(P, gi + so.z), load_vertex(P, gi + so.w)));
+        if (sgn < 0) vid = make_ushort4(vid.w, vid.y, vid.z, vid.x);
+        S.wt.vid[slot] = vid;
+        // the tet's AABB strictly overlaps the grid box, and its volume is not zero
+        if ((flags & (kBelowMax | kAboveMin)) == (kBelowMax | kAboveMin) && sgn != 0)
+            cnt = setup_frame<false>(
+                mn, mx,
+                [&](int q, int a, float &h, float &l) {
+                    const int v = q == 0 ? vid.x : (q == 1 ? vid.y : (q == 2 ? vid.z : vid.w));
+                    h = S.wt.gh[a][v];
+                    l = S.wt.gl[a][v];
+                },
+                S.g, reinterpret_cast<TetVertices &>(S.pool[warp]), lane, S.wt, slot, P.error, &route64);
+        if (cnt > 0 && (S.wt.ex[0][slot] > 1024 || S.wt.ex[1][slot] > 1024 || S.wt.ex[2][slot] > 1024)) S.wide = 1;
     }
-    st.tets += (cnt > 0);
-    route64 = route64 && cnt > 0;
-    if (route64) cnt = 0;  // deposited by route_fp64_kernel
+    n_tets += (cnt > 0);
+    if (route64 && cnt > 0) {  // deposited by route_fp64_kernel
+        cnt = 0;
+        route_append(P, S, tid, vx, vy);
+    }
+    __syncwarp();
     // exclusive scan of the pair counts across the warp
     int incl = cnt;
 #pragma unroll
@@ -798,113 +872,101 @@ __device__ __forceinline__ int group_setup(const DepositParams &P, const SharedM
         const int y = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += y;
     }
-    W.scan[lane] = incl - cnt;
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    if (lane == 31) W.scan[32] = total;
-    __syncwarp();
-    return total;
+    S.scan[slot] = incl - cnt;
+    if (lane == 31) S.warp_pairs[warp] = incl;
 }
 
-// Ill-conditioned tets are listed for route_fp64_kernel: calling their
-// (large) routine from the pair loop made the whole loop spill.
-__device__ __forceinline__ void group_route(const DepositParams &P, const SharedMixed &S, int item, bool route64,
-                                            int tid)
+// Classify phase: the warps take the wave's candidate pairs 32 at a time and
+// classify them; inside cells and one-face cells are deposited at once,
+// partial cells listed, until no pair is left or the list might not hold the
+// 32 pairs each warp may have in hand (`room` of it are used).  Returns
+// whether pairs are left.
+template <bool kStats>
+__device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixed &S, int total, int room, PairStats &st)
 {
-    if (route64) {
-        const unsigned long long k = atomicAdd(P.route_count, 1ull);
-        if (k < P.route_cap)
-            P.route[k] = ((unsigned long long)item << 16) | (unsigned long long)(S.cubes[tid / 6] * 6 + tid % 6);
-        else
-            atomicOr(P.error, 4);
-    }
-}
-
-// Candidate pairs [c0, c1) of the group in table Wc, flattened across the
-// warp: classified, inside cells and one-face cells deposited at once,
-// partial cells listed in Q and clipped by the engine (one call site keeps a
-// single copy of it).
-template <bool kShare>
-__device__ __forceinline__ void pair_range(const DepositParams &P, const GridDesc &g, const WarpTets &Wc,
-                                           WarpPool &pool, uint32_t *Q, int c0, int c1, int lane, PairStats &st)
-{
-    int np = 0;  // partial pairs listed in Q
-    // clip once more than `flush` pairs are listed (then np + 32 <= kQueue)
-    const int flush = min(max(P.clip_batch, 64), kQueue) - 32;
-    for (int pb = c0;; pb += 32) {
-        if (np > flush || (pb >= c1 && np)) {
-            clip_list(P, g, Wc, pool, Q, np, st.fb);
-            np = 0;
-        }
-        if (pb >= c1) break;
-        const int pidx = pb + lane;
-        bool part = false;
-        uint32_t entry = 0;
-        if (pidx < c1) {
-            int s = 0;
+    const int lane = threadIdx.x & 31;
+    const WaveTets &W = S.wt;
+    const GridDesc &g = S.g;
+    const bool wide = S.wide != 0;
+    // pairs of the warps' tets before warp `lane`'s
+    int pre = lane < kWarps ? S.warp_pairs[lane] : 0;
+    {
+        const int own = pre;
 #pragma unroll
-            for (int step = 16; step > 0; step >>= 1)
-                if (Wc.scan[s + step] <= pidx) s += step;
-            const int local = pidx - Wc.scan[s];
-            const int ex0 = Wc.ex[0][s], ex1 = Wc.ex[1][s];
-            const int a = local % ex0, r = local / ex0, b = r % ex1, c = r / ex1;
-            ++st.cand;
-            bool f64 = false;
-            int cross = -1;
-            const int cls = classify_pair(Wc, g, s, a, b, c, f64, cross);
-            st.fp64 += f64;
-            if (cls == P_TET_INSIDE) {
-                ++st.in;
-                ++st.bbox;
-                scatter(P, g, Wc, s, a, b, c, g.tet_mass);
-            } else if (cls == P_CELL_INSIDE) {
-                ++st.cin;
-                ++st.bbox;
-                scatter(P, g, Wc, s, a, b, c, 6.f * Wc.f6[s]);
-            } else if (cls == P_PARTIAL) {
-                ++st.part;
-                ++st.bbox;
-                if (cross >= 0) {  // one face cuts the cell: closed form, no clipping
-                    const float dm = halfspace_pair_vol6<kShare>(Wc, g, s, a, b, c, cross) * Wc.f6[s];
-                    if (dm > 0.f) scatter(P, g, Wc, s, a, b, c, dm);
-                } else {
-                    part = true;
-                    entry = ((uint32_t)s << 27) | (uint32_t)local;
-                }
+        for (int o = 1; o < kWarps; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, pre, o);
+            if (lane >= o) pre += y;
+        }
+        pre -= own;
+    }
+    for (;;) {
+        int c0 = 0;
+        if (lane == 0) c0 = *(volatile int *)&S.list.n > room - kThreads ? total : atomicAdd(&S.cursor, 32);
+        c0 = __shfl_sync(0xffffffffu, c0, 0);
+        if (c0 >= total) break;
+        const int pidx = c0 + lane;
+        // the pair's tet: by warps, then in the warp's scan
+        int s = 0, before = 0;
+#pragma unroll
+        for (int step = kWarps / 2; step > 0; step >>= 1) {
+            const int y = __shfl_sync(0xffffffffu, pre, s + step);
+            if (y <= pidx) {
+                s += step;
+                before = y;
             }
         }
+        const int in_warp = pidx - before;
+        s *= 32;
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+            if (S.scan[s + step] <= in_warp) s += step;
+        bool part = false;
+        uint32_t entry = 0;
+        if (pidx < total) {
+            const int local = in_warp - S.scan[s];
+            const int3 c = flat_cell(W, s, local);
+            entry = wide ? (uint32_t)local : ((uint32_t)c.x | ((uint32_t)c.y << 10) | ((uint32_t)c.z << 20));
+            if (kStats) ++st.cand;
+            bool f64 = false;
+            int cross = -1;
+            const int cls = classify_pair(W, g, s, c.x, c.y, c.z, f64, cross);
+            if (kStats) {
+                st.fp64 += f64;
+                st.in += cls == P_TET_INSIDE;
+                st.cin += cls == P_CELL_INSIDE;
+                st.part += cls == P_PARTIAL;
+                st.bbox += cls != P_NO;
+            }
+            part = cls == P_PARTIAL && cross < 0;
+            float m = cls == P_TET_INSIDE ? g.tet_mass : (cls == P_CELL_INSIDE ? 6.f * W.f6[s] : 0.f);
+            // one face cuts the cell: closed form, no clipping
+            if (cross >= 0) m = halfspace_pair_vol6<false>(W, g, s, c.x, c.y, c.z, cross) * W.f6[s];
+            if (m > 0.f) scatter(P, g, W, s, c.x, c.y, c.z, m);
+        }
         const unsigned bal = __ballot_sync(0xffffffffu, part);
-        if (part) Q[np + __popc(bal & ((1u << lane) - 1))] = entry;
-        np += __popc(bal);
-        __syncwarp();
+        int at = 0;
+        if (lane == 0 && bal) at = atomicAdd(&S.list.n, __popc(bal));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1));
+        if (part) {
+            S.list.cell[at] = entry;
+            S.list.tet[at] = (uint8_t)s;
+        }
     }
 }
 
 // Persistent: CTAs take work items (grid x vertex block) from a global
-// counter; inside an item the warps take groups of 32 tets from a shared
-// counter, so no warp waits for another until the item is done.
-// kShare (zoom batches): a group with more than one chunk of pairs is
-// published in its warp's slot, and warps whose groups are done take chunks
-// of P.share_chunk pairs from open slots instead of waiting for the slowest warp at
-// the end of the item.  On fine grids an item holds few tets with thousands
-// of cells each, and one warp carried most of it (zoom batch 8.19 s without,
-// 6.2 s with).  On coarse grids every group is a single chunk: kShare false
-// keeps the plain loop there, whose registers the slot state would crowd
-// (octree leaves 12% slower with it).
-template <bool kShare>
+// counter and deposit an item's tets in waves of kWave (see the top of the
+// file).  A wave whose partial pairs do not fit the list is clipped in parts.
+// kStats: count the pairs (collect_stats); a separate instantiation, so that
+// the other carries no counters.
+template <bool kStats>
 __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParams P)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SharedMixed &S = *reinterpret_cast<SharedMixed *>(smem_raw);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    WarpTets &W = S.wt[warp];
-    uint32_t *Q = S.queue[warp];
-    WarpPool &pool = S.pool[warp];
+    const int warp = threadIdx.x >> 5;
     PairStats st;
-    const int chunk = P.share_chunk > 0 ? P.share_chunk : kChunk;  // pairs per shared chunk (> 0)
-    if (kShare && threadIdx.x < kWarps) {
-        S.slot_busy[threadIdx.x] = 0;
-        S.slot_open[threadIdx.x] = 0;
-    }
+    const int room = min(max(P.clip_batch, 64), kQueue) * kWarps;
 
     for (int taken = 0;; ++taken) {
         // one-item CTAs (serving): a CTA exits after its items, so that the
@@ -913,8 +975,8 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
         if (threadIdx.x == 0) {
             S.item = atomicAdd(P.counter, 1);
             S.n_cubes = 0;
-            S.next_group = 0;
-            S.groups_set = 0;
+            S.list.n = 0;
+            S.list.next = 0;
         }
         __syncthreads();
         const int item = S.item;
@@ -922,126 +984,59 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
         const Item it = P.items[item];
         if (threadIdx.x == 0) S.g = P.grids[it.grid];
         const int vx = it.nv & 0xff, vy = (it.nv >> 8) & 0xff, vz = (it.nv >> 16) & 0xff;
-        stage_block(P, it, S.vert, vx, vy, vz, S.gh, S.gl);
+        stage_block(P, it, P.grids[it.grid], S, vx, vy, vz);
         __syncthreads();
-        const GridDesc &g = S.g;
         const int cvx = vx - 1, cvy = vy - 1, cvz = vz - 1;
         const int ncube = (cvx > 0 && cvy > 0 && cvz > 0) ? cvx * cvy * cvz : 0;
         for (int c = threadIdx.x; c < ncube; c += blockDim.x) {
-            const int ci = c % cvx, r = c / cvx, cj = r % cvy, ck = r / cvy;
-            if (cube_alive(S.vert, vx, vy, ci, cj, ck, g)) S.cubes[atomicAdd(&S.n_cubes, 1)] = (uint16_t)c;
+            const int r = small_div(c, cvx), k = small_div(r, cvy);
+            const int v0 = c - r * cvx + vx * (r - k * cvy + vy * k);
+            if (cube_alive(S, v0, vx, vy)) S.cubes[atomicAdd(&S.n_cubes, 1)] = (uint16_t)v0;
         }
         __syncthreads();
         const int ntet = 6 * S.n_cubes;
-        const int ngroups = (ntet + 31) / 32;
-        if (!kShare) {
-            for (;;) {
-                int grp = 0;
-                if (lane == 0) grp = atomicAdd(&S.next_group, 1);
-                grp = __shfl_sync(0xffffffffu, grp, 0);
-                if (grp >= ngroups) break;
-                bool route64;
-                int tid;
-                const int total = group_setup<kShare>(P, S, W, g, grp, ntet, vx, vy, cvx, cvy, lane, st, route64, tid);
-                pair_range<kShare>(P, g, W, pool, Q, 0, total, lane, st);
-                group_route(P, S, item, route64, tid);
-                __syncwarp();
+        for (int first = 0; first < ntet; first += kWave) {
+            if (threadIdx.x == 0) {
+                S.cursor = 0;
+                S.wide = 0;
             }
-        } else {
-            int cur = -1;      // slot whose pairs this warp takes (its own: cur == warp)
-            int total = 0;     // pairs of slot cur
-            int own_next = 0;  // own group: next pair if kept private, -1 if published
-            for (;;) {
-                if (cur < 0) {
-                    int grp = 0;
-                    if (lane == 0) grp = atomicAdd(&S.next_group, 1);
-                    grp = __shfl_sync(0xffffffffu, grp, 0);
-                    if (grp < ngroups) {
-                        bool route64;
-                        int tid;
-                        total = group_setup<kShare>(P, S, W, g, grp, ntet, vx, vy, cvx, cvy, lane, st, route64, tid);
-                        group_route(P, S, item, route64, tid);
-                        // a group of one chunk or less is kept private
-                        const bool pub = total > chunk;
-                        if (lane == 0) {
-                            if (pub) {
-                                S.slot_total[warp] = total;
-                                S.slot_next[warp] = 0;
-                                __threadfence_block();
-                                *(volatile int *)&S.slot_open[warp] = 1;
-                            }
-                            atomicAdd(&S.groups_set, 1);
-                        }
-                        __syncwarp();
-                        cur = warp;
-                        own_next = pub ? -1 : 0;
-                    } else {
-                        // help: join an open slot with pairs left; leave once every
-                        // group is set up and none has pairs left (bounded wait)
-                        int h = -1, ht = 0;
-                        for (unsigned spin = 0;; ++spin) {
-                            int set = 0;
-                            if (lane == 0) {
-                                // read before the scan: if every group was set up by
-                                // then, the scan sees every slot that still has pairs
-                                set = *(volatile int *)&S.groups_set;
-                                __threadfence_block();
-                                for (int d = 1; d < kWarps && h < 0; ++d) {
-                                    const int w = (warp + d) % kWarps;
-                                    if (*(volatile int *)&S.slot_open[w] &&
-                                        *(volatile int *)&S.slot_next[w] < *(volatile int *)&S.slot_total[w]) {
-                                        atomicAdd(&S.slot_busy[w], 1);
-                                        __threadfence_block();
-                                        if (*(volatile int *)&S.slot_open[w]) {
-                                            __threadfence_block();  // then the owner's table is visible
-                                            h = w;
-                                            ht = *(volatile int *)&S.slot_total[w];
-                                        } else {
-                                            atomicSub(&S.slot_busy[w], 1);
-                                        }
-                                    }
-                                }
-                            }
-                            h = __shfl_sync(0xffffffffu, h, 0);
-                            set = __shfl_sync(0xffffffffu, set, 0);
-                            if (h >= 0 || set >= ngroups || spin > P.help_spins) break;
-                            __nanosleep(256);
-                        }
-                        if (h < 0) break;
-                        cur = h;
-                        total = __shfl_sync(0xffffffffu, ht, 0);
-                        own_next = -1;
-                    }
+            __syncthreads();
+            wave_setup(P, S, it, first, ntet, vx, vy, st.tets);
+            __syncthreads();
+            int total = 0;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) total += S.warp_pairs[w];
+            bool left = total > 0;
+            while (left) {
+                wave_classify<kStats>(P, S, total, room, st);
+                __syncthreads();
+                left = S.cursor < total;
+                const int np = S.list.n;
+                clip_pairs(
+                    S.pool[warp], S.list, np,
+                    [&](int j, float *p) {
+                        const int s = S.list.tet[j];
+                        const int3 c = pair_cell(S.wt, s, S.list.cell[j], S.wide != 0);
+                        piece_coords(S.wt, S.g, s, c.x, c.y, c.z, p);
+                    },
+                    st.fb);
+                __syncthreads();
+                for (int j = threadIdx.x; j < np; j += kThreads) {
+                    const int s = S.list.tet[j];
+                    const int3 c = pair_cell(S.wt, s, S.list.cell[j], S.wide != 0);
+                    const long long v = S.list.volume(j);
+                    if (v > 0) scatter(P, S.g, S.wt, s, c.x, c.y, c.z, pair_mass(v, S.wt.f6[s]));
                 }
-                // next chunk of slot cur
-                int c0 = own_next;
-                if (own_next >= 0) {
-                    own_next = total;
-                } else {
-                    if (lane == 0) c0 = atomicAdd(&S.slot_next[cur], chunk);
-                    c0 = __shfl_sync(0xffffffffu, c0, 0);
+                if (threadIdx.x == 0) {
+                    S.list.n = 0;
+                    S.list.next = 0;
                 }
-                if (c0 >= total) {
-                    if (lane == 0) {
-                        if (cur != warp) {
-                            atomicSub(&S.slot_busy[cur], 1);
-                        } else if (*(volatile int *)&S.slot_open[warp]) {
-                            // close the slot, then wait for the helpers still reading W
-                            *(volatile int *)&S.slot_open[warp] = 0;
-                            __threadfence_block();
-                            if (!wait_zero_bounded(&S.slot_busy[warp], P.close_spins, 32)) atomicOr(P.error, 8);
-                        }
-                    }
-                    __syncwarp();
-                    cur = -1;
-                    continue;
-                }
-                pair_range<kShare>(P, g, S.wt[cur], pool, Q, c0, min(total, c0 + chunk), lane, st);
+                __syncthreads();
             }
         }
         __syncthreads();
     }
-    if (P.stats) {
+    if (kStats) {
         warp_stat(P.stats, ST_TETS, st.tets);
         warp_stat(P.stats, ST_CAND, st.cand);
         warp_stat(P.stats, ST_BBOX, st.bbox);

@@ -172,7 +172,7 @@ int mixed_setup(int device, DeviceProps &dp)
 // Launch-shape and batching parameters (adeco_tuning), per session.
 struct Tuning {
     int zoom_tile = 64;                       // cells per tile edge of a zoom grid
-    int share_chunk = kChunk;                 // work sharing: pairs per chunk
+    int share_chunk = 512;                    // accepted for callers that set it; pairs are shared 32 at a time
     int clip_batch = kQueue;                  // partial pairs listed per warp before clipping
     int ctas_per_sm = 0;                      // persistent launches: CTAs per SM (0: occupancy)
     unsigned long long route_capacity = 0;    // 0: route_capacity(items)
@@ -186,10 +186,7 @@ DepositParams base_params(const Tuning &t)
     DepositParams P;
     std::memset(&P, 0, sizeof P);
     P.per_cta_items = 0;
-    P.share_chunk = t.share_chunk;
     P.clip_batch = t.clip_batch;
-    P.help_spins = kHelpSpins;
-    P.close_spins = kCloseSpins;
     return P;
 }
 
@@ -218,17 +215,15 @@ static int deposit_error(int err, const char *where)
 }
 
 // One persistent launch of the mixed kernel over `n_items` items, then the
-// launch that deposits the ill-conditioned tets it listed.  share: warps of
-// an item share the pairs of large tet groups (zoom grids, whose cells are
-// much smaller than the tets).
-int launch_mixed(const DeviceProps &dp, DepositParams P, bool share, cudaStream_t st, int ctas_per_sm = 0)
+// launch that deposits the ill-conditioned tets it listed.
+int launch_mixed(const DeviceProps &dp, DepositParams P, cudaStream_t st, int ctas_per_sm = 0)
 {
     if (P.n_items <= 0) return ADECO_OK;
     CUDA_TRY(cudaMemsetAsync(P.counter, 0, sizeof(int), st));
     CUDA_TRY(cudaMemsetAsync(P.route_count, 0, sizeof(unsigned long long), st));
     const int per_sm = ctas_per_sm > 0 ? std::min(ctas_per_sm, dp.mixed_blocks_per_sm) : dp.mixed_blocks_per_sm;
     const int grid = std::max(1, std::min(P.n_items, dp.sms * per_sm));
-    if (share)
+    if (P.stats)
         deposit_mixed_kernel<true><<<grid, kThreads, dp.mixed_smem, st>>>(P);
     else
         deposit_mixed_kernel<false><<<grid, kThreads, dp.mixed_smem, st>>>(P);
@@ -432,7 +427,7 @@ static int deposit_device_core(int dev, const float *d_pos, size_t patch_offset,
                                  cudaMemcpyHostToDevice, st));
         rc = launch_plain(dp, P, d_cube_off.p, 0, cube_off.back(), st);
     } else {
-        rc = launch_mixed(dp, P, false, st);
+        rc = launch_mixed(dp, P, st);
     }
     if (rc) return rc;
     int err = 0;
@@ -1124,7 +1119,7 @@ static int enqueue_leaves_mixed(adeco_session *s, bool stats)
 {
     const size_t nv = s->out_values;
     CUDA_TRY(cudaMemsetAsync(s->d_fixed.p, 0, nv * sizeof(unsigned long long), s->stream));
-    int rc = launch_mixed(s->dp, session_params(s, stats), false, s->stream, s->tuning.ctas_per_sm);
+    int rc = launch_mixed(s->dp, session_params(s, stats), s->stream, s->tuning.ctas_per_sm);
     if (rc) return rc;
     const long long cells = (long long)s->leaf_dims * s->leaf_dims * s->leaf_dims;
     fixed_to_f64_grids_kernel<<<s->dp.sms * 4, 256, 0, s->stream>>>(s->d_fixed.p, s->d_out.p, s->d_grids.p,
@@ -1172,7 +1167,7 @@ extern "C" int adeco_session_deposit_leaves(adeco_session *s, int precision, dou
     } else {
         CUDA_TRY(cudaMemsetAsync(s->d_fixed.p, 0, s->out_values * sizeof(unsigned long long), s->stream));
         CUDA_TRY(cudaEventRecord(e0, s->stream));
-        rc = launch_mixed(s->dp, session_params(s, collect_stats != 0), false, s->stream, s->tuning.ctas_per_sm);
+        rc = launch_mixed(s->dp, session_params(s, collect_stats != 0), s->stream, s->tuning.ctas_per_sm);
         launches = 2;  // the mixed kernel and the ill-conditioned-tet launch
         CUDA_TRY(cudaEventRecord(e1, s->stream));
         const long long cells = (long long)s->leaf_dims * s->leaf_dims * s->leaf_dims;

@@ -368,7 +368,7 @@ static int launch_job(Server &S, ServeJob &j)
     P.per_cta_items = 1;
     if (j.t0) CUDA_TRY(cudaEventRecord(j.t0, st));
     if (P.n_items > 0) {
-        deposit_mixed_kernel<true><<<P.n_items, kThreads, s->dp.mixed_smem, st>>>(P);
+        deposit_mixed_kernel<false><<<P.n_items, kThreads, s->dp.mixed_smem, st>>>(P);
         CUDA_TRY(cudaGetLastError());
         route_fp64_kernel<<<s->dp.sms * 2, kThreads, kRouteSmem, st>>>(P);
         CUDA_TRY(cudaGetLastError());
