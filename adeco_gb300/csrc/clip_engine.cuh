@@ -571,9 +571,9 @@ long long clip_piece_serial(const float p0[12], int done0)
 }
 
 #ifdef __CUDACC__
-constexpr int kPool = 72;    // pieces per warp pool (2 CTAs of 8 warps fit in an SM's shared memory)
+constexpr int kPool = 78;    // pieces per warp pool (2 CTAs of 8 warps fit in an SM's shared memory)
 constexpr int kLast = 88;    // pieces at their last crossed face per warp
-constexpr int kPairs = 1024;  // partial pairs a CTA lists
+constexpr int kPairs = 1280;  // partial pairs a CTA lists
 
 static_assert(kPool >= 32 + 3 && kLast >= 32 + 3, "one split step fits a full pool and list");
 

@@ -40,7 +40,7 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kMaxVerts = 512;   // 8^3
 constexpr int kMaxCubes = 343;   // 7^3
 constexpr int kWave = kThreads;       // tets set up together
-constexpr int kQueue = kPairs / kWarps;  // partial pairs listed per warp before clipping, at the most
+constexpr int kQueue = 128;            // largest clip_batch: the whole pair list
 
 struct Item {
     long long base;  // vertex index of the block origin (lattice) or of the patch origin + offset
@@ -71,8 +71,9 @@ struct DepositParams {
     unsigned long long *route_count;
     unsigned long long route_cap;
     // launch-shape and batching parameters (set by the host, tunable)
+    int parts;           // CTAs that share an item, each with every parts-th cube (>= 1)
     int per_cta_items;   // items a CTA takes before it exits (0: persistent, until the queue is empty)
-    int clip_batch;      // partial pairs listed per warp before they are clipped (64..kQueue)
+    int clip_batch;      // share of the pair list used, in kQueue-ths (64..kQueue)
 };
 
 enum Stat : int {
@@ -161,7 +162,7 @@ struct SharedMixed {
     alignas(8) uint16_t vert_off[6][4];  //   and among the staged vertices
     uint16_t cubes[kMaxCubes + 1];  // the live cubes' first staged vertices
     int n_cubes;
-    int item;
+    int item, part;
     GridDesc g;
     int scan[kWave];     // pairs of the warp's tets before this one
     int warp_pairs[kWarps];
@@ -311,7 +312,7 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
     long long cnt0 = 1;
     unsigned cnt = 1;
     float R = 0.f;
-#pragma unroll 1
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
         const int top = g.dims - 1;
         const int wlo = (int)((a == 2 ? mn.y : (mn.x >> (16 * a))) & 0xffffu),
@@ -364,7 +365,7 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
     // tet's volume normaliser): edge vectors from vertex 3, then the triple
     // product with TwoProd / TwoSum, a cofactor of the first edge at a time
     F2 w6 = {0.f, 0.f};
-#pragma unroll 1
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
         const int b = a == 2 ? 0 : a + 1, c = a == 0 ? 2 : a - 1;
         auto edge = [&](int q, int x) {
@@ -382,7 +383,7 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
     // only turns the plane about the centroid (the one-face closed form
     // relies on it)
     float tolmax = 0.f, L2 = 0.f;
-#pragma unroll 1
+#pragma unroll
     for (int f = 0; f < 4; ++f) {
         const int fa = f == 3, fb = (0x2312 >> (12 - 4 * f)) & 3, fc = (0x1233 >> (12 - 4 * f)) & 3;
         float A[3], B[3], C[3], e1[3], e2[3];
@@ -815,15 +816,15 @@ __device__ __forceinline__ void route_append(const DepositParams &P, const Share
         atomicOr(P.error, 4);
 }
 
-// Set-up phase: this warp's 32 tets of the wave that starts at tet `first` of
-// the item's live cubes.
-__device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &S, const Item &it, int first, int ntet,
+// Set-up phase: this warp's tets of the wave [first, end) of the tets of the
+// item's live cubes.
+__device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &S, const Item &it, int first, int end,
                                            int vx, int vy, unsigned &n_tets)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slot = threadIdx.x, tid = first + slot;
     int cnt = 0;
     bool route64 = false;
-    if (tid < ntet) {
+    if (tid < end) {
         const int t = tid % 6, v0 = S.cubes[tid / 6];
         const ushort4 off = *reinterpret_cast<const ushort4 *>(S.vert_off[t]);
         ushort4 vid = make_ushort4(v0 + off.x, v0 + off.y, v0 + off.z, v0 + off.w);
@@ -966,42 +967,47 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
     SharedMixed &S = *reinterpret_cast<SharedMixed *>(smem_raw);
     const int warp = threadIdx.x >> 5;
     PairStats st;
-    const int room = min(max(P.clip_batch, 64), kQueue) * kWarps;
+    const int room = kPairs / kQueue * min(max(P.clip_batch, 64), kQueue);
 
     for (int taken = 0;; ++taken) {
         // one-item CTAs (serving): a CTA exits after its items, so that the
         // CTAs of other requests' launches get SMs as these finish
         if (P.per_cta_items > 0 && taken >= P.per_cta_items) break;
         if (threadIdx.x == 0) {
-            S.item = atomicAdd(P.counter, 1);
+            const int unit = atomicAdd(P.counter, 1);
+            S.item = unit / P.parts;
+            S.part = unit - S.item * P.parts;
             S.n_cubes = 0;
             S.list.n = 0;
             S.list.next = 0;
         }
         __syncthreads();
-        const int item = S.item;
-        if (item >= P.n_items) break;
-        const Item it = P.items[item];
+        if (S.item >= P.n_items) break;
+        const Item it = P.items[S.item];
         if (threadIdx.x == 0) S.g = P.grids[it.grid];
         const int vx = it.nv & 0xff, vy = (it.nv >> 8) & 0xff, vz = (it.nv >> 16) & 0xff;
         stage_block(P, it, P.grids[it.grid], S, vx, vy, vz);
         __syncthreads();
         const int cvx = vx - 1, cvy = vy - 1, cvz = vz - 1;
         const int ncube = (cvx > 0 && cvy > 0 && cvz > 0) ? cvx * cvy * cvz : 0;
-        for (int c = threadIdx.x; c < ncube; c += blockDim.x) {
+        // the live ones of this CTA's cubes (every parts-th)
+        for (int c = S.part + threadIdx.x * P.parts; c < ncube; c += blockDim.x * P.parts) {
             const int r = small_div(c, cvx), k = small_div(r, cvy);
             const int v0 = c - r * cvx + vx * (r - k * cvy + vy * k);
             if (cube_alive(S, v0, vx, vy)) S.cubes[atomicAdd(&S.n_cubes, 1)] = (uint16_t)v0;
         }
         __syncthreads();
+        // waves of equal size: a whole meta-cell's 2058 tets are 9 of 229, not
+        // 8 of 256 and one of 10
         const int ntet = 6 * S.n_cubes;
-        for (int first = 0; first < ntet; first += kWave) {
+        const int nwave = (ntet + kWave - 1) / kWave, wave = nwave ? (ntet + nwave - 1) / nwave : 0;
+        for (int first = 0; first < ntet; first += wave) {
             if (threadIdx.x == 0) {
                 S.cursor = 0;
                 S.wide = 0;
             }
             __syncthreads();
-            wave_setup(P, S, it, first, ntet, vx, vy, st.tets);
+            wave_setup(P, S, it, first, min(first + wave, ntet), vx, vy, st.tets);
             __syncthreads();
             int total = 0;
 #pragma unroll

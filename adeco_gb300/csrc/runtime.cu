@@ -185,6 +185,7 @@ DepositParams base_params(const Tuning &t)
 {
     DepositParams P;
     std::memset(&P, 0, sizeof P);
+    P.parts = 1;
     P.per_cta_items = 0;
     P.clip_batch = t.clip_batch;
     return P;
@@ -214,6 +215,15 @@ static int deposit_error(int err, const char *where)
     return fail(ADECO_ERR_LIMIT, "a tet spans more than 2^25 candidate cells of %s", where);
 }
 
+// CTAs that share an item, for n_items items on `slots` CTA slots: with few
+// items most slots would idle, or wait at the end for the last ones.  Two
+// units of work a slot; more gave nothing (a unit repeats the staging of its
+// item's block).  A block has at most 343 cubes.
+int item_parts(int n_items, int slots)
+{
+    return std::max(1, std::min((2 * slots + n_items - 1) / n_items, kMaxCubes));
+}
+
 // One persistent launch of the mixed kernel over `n_items` items, then the
 // launch that deposits the ill-conditioned tets it listed.
 int launch_mixed(const DeviceProps &dp, DepositParams P, cudaStream_t st, int ctas_per_sm = 0)
@@ -222,7 +232,8 @@ int launch_mixed(const DeviceProps &dp, DepositParams P, cudaStream_t st, int ct
     CUDA_TRY(cudaMemsetAsync(P.counter, 0, sizeof(int), st));
     CUDA_TRY(cudaMemsetAsync(P.route_count, 0, sizeof(unsigned long long), st));
     const int per_sm = ctas_per_sm > 0 ? std::min(ctas_per_sm, dp.mixed_blocks_per_sm) : dp.mixed_blocks_per_sm;
-    const int grid = std::max(1, std::min(P.n_items, dp.sms * per_sm));
+    P.parts = item_parts(P.n_items, dp.sms * per_sm);
+    const int grid = (int)std::min<long long>((long long)P.n_items * P.parts, (long long)dp.sms * per_sm);
     if (P.stats)
         deposit_mixed_kernel<true><<<grid, kThreads, dp.mixed_smem, st>>>(P);
     else
@@ -1527,7 +1538,9 @@ extern "C" int adeco_deposit_tets_device_noalloc(const float *d_positions, size_
     P.counter = counter;
     P.error = counter + 1;
     set_route(P, route, route_capacity(n_items));  // <= kNoAllocRouteCap, the allocating path's rule
-    const int blocks = (int)std::max(1LL, std::min(n_items, (long long)nd.sms * nd.blocks_per_sm));
+    const int slots = nd.sms * nd.blocks_per_sm;
+    P.parts = item_parts(P.n_items, slots);
+    const int blocks = (int)std::min<long long>(n_items * P.parts, slots);
     deposit_mixed_kernel<false><<<blocks, kThreads, sizeof(SharedMixed), st>>>(P);
     CUDA_TRY(cudaGetLastError());
     route_fp64_kernel<<<nd.sms * 2, kThreads, kRouteSmem, st>>>(P);  // the resident CTAs
