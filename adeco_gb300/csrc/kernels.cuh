@@ -456,142 +456,6 @@ ADECO_HD inline int setup_tet(const float3 v[4], const float gh[4][3], const flo
 
 enum PairClass : int { P_NO = 0, P_TET_INSIDE = 1, P_CELL_INSIDE = 2, P_PARTIAL = 3 };
 
-#ifdef __CUDACC__
-// One positively oriented tet, candidate range [lo, hi], deposited by the
-// whole warp in FP64 (the plain baseline): lanes stride over the candidate
-// cells, each classified with FP64 face planes and, when partial, clipped in
-// FP64; FP64 atomics.  Counts the (candidate, partial) pairs seen by this lane.
-__device__ __noinline__ void deposit_tet_fp64_warp(const float3 v[4], const int lo[3], const int hi[3], const GridDesc &g,
-                                                   double *out_d, unsigned &n_cand, unsigned &n_part)
-{
-    const int lane = threadIdx.x & 31;
-    double qd[4][3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const double anchor = fma((double)lo[a], g.delta_d[a], g.gmin_d[a]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const double x = (a == 0) ? (double)v[q].x : ((a == 1) ? (double)v[q].y : (double)v[q].z);
-            qd[q][a] = (x - anchor) * g.scale_d[a];
-        }
-    }
-    const double vq6 = fabs(vol6_fast<double>(qd[0], qd[1], qd[2], qd[3]));
-    const double f6 = g.mass_factor / vq6;
-    double bmin[3], bmax[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        bmin[a] = fmin(fmin(qd[0][a], qd[1][a]), fmin(qd[2][a], qd[3][a]));
-        bmax[a] = fmax(fmax(qd[0][a], qd[1][a]), fmax(qd[2][a], qd[3][a]));
-    }
-    // inward face planes: faces (0,2,1) (0,3,2) (0,1,3) (1,2,3)
-    double pn[4][3], pd[4], pp[4], pm[4];
-    {
-        const int fa[4] = {0, 0, 0, 1}, fb[4] = {2, 3, 1, 2}, fc[4] = {1, 2, 3, 3};
-#pragma unroll
-        for (int f = 0; f < 4; ++f) {
-            const double e1x = qd[fb[f]][0] - qd[fa[f]][0], e1y = qd[fb[f]][1] - qd[fa[f]][1],
-                         e1z = qd[fb[f]][2] - qd[fa[f]][2];
-            const double e2x = qd[fc[f]][0] - qd[fa[f]][0], e2y = qd[fc[f]][1] - qd[fa[f]][1],
-                         e2z = qd[fc[f]][2] - qd[fa[f]][2];
-            pn[f][0] = e1y * e2z - e1z * e2y;
-            pn[f][1] = e1z * e2x - e1x * e2z;
-            pn[f][2] = e1x * e2y - e1y * e2x;
-            pd[f] = pn[f][0] * qd[fa[f]][0] + pn[f][1] * qd[fa[f]][1] + pn[f][2] * qd[fa[f]][2];
-            pp[f] = fmax(pn[f][0], 0.0) + fmax(pn[f][1], 0.0) + fmax(pn[f][2], 0.0);
-            pm[f] = fmin(pn[f][0], 0.0) + fmin(pn[f][1], 0.0) + fmin(pn[f][2], 0.0);
-        }
-    }
-    const int ex0 = hi[0] - lo[0] + 1, ex1 = hi[1] - lo[1] + 1, ex2 = hi[2] - lo[2] + 1;
-    auto put = [&](long long idx, double dm) { atomicAdd(out_d + idx, dm); };
-    // one cell, decided exactly in FP64 (bbox, plane bounds, clipping)
-    auto cell = [&](int a, int b, int k) {
-        ++n_cand;
-        // cell origin in the anchor frame (the cell extends 1 along each axis)
-        const double oa = a * g.rcell[0], ob = b * g.rcell[1], ok = k * g.rcell[2];
-        if (!(bmin[0] < oa + 1.0 && oa < bmax[0] && bmin[1] < ob + 1.0 && ob < bmax[1] && bmin[2] < ok + 1.0 &&
-              ok < bmax[2]))
-            return;
-        bool outside = false, all_in = true;
-#pragma unroll
-        for (int f = 0; f < 4; ++f) {
-            const double base = pn[f][0] * oa + pn[f][1] * ob + pn[f][2] * ok - pd[f];
-            if (base + pp[f] <= 0.0) outside = true;
-            if (!(base + pm[f] > 0.0)) all_in = false;
-        }
-        if (outside) return;
-        double dm;
-        if (bmin[0] >= oa && bmax[0] <= oa + 1.0 && bmin[1] >= ob && bmax[1] <= ob + 1.0 && bmin[2] >= ok &&
-            bmax[2] <= ok + 1.0) {
-            dm = (double)g.tet_mass;
-        } else if (all_in) {
-            dm = 6.0 * f6;
-        } else {
-            double p[4][3];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                p[q][0] = qd[q][0] - oa;
-                p[q][1] = qd[q][1] - ob;
-                p[q][2] = qd[q][2] - ok;
-            }
-            ++n_part;
-            dm = clip_volume6<double, double>(p) * f6;
-        }
-        if (!(dm > 0.0)) return;
-        put(g.out_offset + (lo[0] + a) + (long long)g.dims * ((lo[1] + b) + (long long)g.dims * (lo[2] + k)), dm);
-    };
-    if (ex0 < 8) {  // short rows: one lane per cell
-        const long long ncell = (long long)ex0 * ex1 * ex2;
-        for (long long cc = lane; cc < ncell; cc += 32) {
-            const long long rr = cc / ex0;
-            cell((int)(cc % ex0), (int)(rr % ex1), (int)(rr / ex1));
-        }
-        return;
-    }
-    // Long rows along x, one per lane.  The plane bounds are linear in the
-    // cell index a, so each plane bounds a; widened / narrowed by a cell
-    // against rounding, cells outside [c0, c1] cannot meet the tet and cells
-    // inside [i0, i1] lie inside it (CELL_INSIDE_TET: the mass the per-cell
-    // test gives them); only the cells in between are tested one by one.
-    const long long nrows = (long long)ex1 * ex2;
-    for (long long rr = lane; rr < nrows; rr += 32) {
-        const int b = (int)(rr % ex1), k = (int)(rr / ex1);
-        const double ob = b * g.rcell[1], ok = k * g.rcell[2];
-        double c0 = 0.0, c1 = ex0 - 1, i0 = 0.0, i1 = ex0 - 1;
-        bool none = false, no_in = false;
-#pragma unroll
-        for (int f = 0; f < 4; ++f) {
-            const double nx = pn[f][0] * g.rcell[0];
-            const double K = pn[f][1] * ob + pn[f][2] * ok - pd[f];
-            if (nx > 0.0) {
-                c0 = fmax(c0, floor(-(K + pp[f]) / nx) - 1.0);
-                i0 = fmax(i0, floor(-(K + pm[f]) / nx) + 2.0);
-            } else if (nx < 0.0) {
-                c1 = fmin(c1, ceil(-(K + pp[f]) / nx) + 1.0);
-                i1 = fmin(i1, ceil(-(K + pm[f]) / nx) - 2.0);
-            } else {
-                none = none || !(K + pp[f] > 0.0);
-                no_in = no_in || !(K + pm[f] > 0.0);
-            }
-        }
-        if (none) continue;
-        const int lc = (int)fmax(c0, 0.0), hc = (int)fmin(c1, (double)(ex0 - 1));
-        int li = (int)fmax(i0, (double)lc), hi_ = (int)fmin(i1, (double)hc);
-        if (no_in || li > hi_) {
-            li = hc + 1;
-            hi_ = hc;
-        }
-        for (int a = lc; a < li; ++a) cell(a, b, k);
-        if (li <= hi_) {
-            n_cand += hi_ - li + 1;
-            const long long row =
-                g.out_offset + lo[0] + (long long)g.dims * ((lo[1] + b) + (long long)g.dims * (lo[2] + k));
-            for (int a = li; a <= hi_; ++a) put(row + a, 6.0 * f6);
-        }
-        for (int a = hi_ + 1; a <= hc; ++a) cell(a, b, k);
-    }
-}
-#endif
-
 // FP64 evaluation of the four plane bounds for a cell whose FP32 test was
 // inside the error band: exact decision for the FP32-rounded tet.
 template <class Table>
@@ -1055,64 +919,9 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
 }
 
 // ------------------------------------------------------ plain FP64 kernel
-// The baseline the batched kernel is measured against: one warp per cube,
-// every tet classified and clipped in FP64 lane-per-cell, FP64 atomics into
-// the output grid; one launch per request.
-__global__ void __launch_bounds__(kThreads) deposit_plain_fp64_kernel(DepositParams P, long long cube_begin,
-                                                                      long long cube_end,
-                                                                      const long long *item_cube_offset)
-{
-    const int lane = threadIdx.x & 31;
-    const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long cube = cube_begin + gw; cube < cube_end; cube += nw) {
-        // item owning this cube (binary search over the cube offsets)
-        int lo_i = 0, hi_i = P.n_items - 1;
-        while (lo_i < hi_i) {
-            const int mid = (lo_i + hi_i + 1) >> 1;
-            if (item_cube_offset[mid] <= cube) lo_i = mid; else hi_i = mid - 1;
-        }
-        const Item it = P.items[lo_i];
-        const GridDesc g = P.grids[it.grid];
-        const int vx = it.nv & 0xff, vy = (it.nv >> 8) & 0xff;
-        const int cvx = vx - 1, cvy = vy - 1;
-        const int c = (int)(cube - item_cube_offset[lo_i]);
-        const int ci = c % cvx, r = c / cvx, cj = r % cvy, ck = r / cvy;
-        float3 corner[8];
-        bool pad = false;
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-            const int3 o = corner_offset(P.order, s);
-            const long long gi = it.base + (ci + o.x) + P.stride_y * (cj + o.y) + P.stride_z * (ck + o.z);
-            if (P.src_kind == SRC_LATTICE_F4) {
-                const float4 p = __ldg(reinterpret_cast<const float4 *>(P.src) + gi);
-                corner[s] = make_float3(p.x, p.y, p.z);
-            } else {
-                const float *q = reinterpret_cast<const float *>(P.src) + 3 * gi;
-                corner[s] = make_float3(__ldg(q), __ldg(q + 1), __ldg(q + 2));
-                if (P.pad_check) {
-                    const float sum = __fadd_rn(__fadd_rn(fabsf(__fsub_rn(corner[s].x, 666.f)),
-                                                          fabsf(__fsub_rn(corner[s].y, 666.f))),
-                                                fabsf(__fsub_rn(corner[s].z, 666.f)));
-                    pad |= ((double)sum < 1.E-03);
-                }
-            }
-        }
-        if (pad) continue;
-        for (int t = 0; t < 6; ++t) {
-            float3 v[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) v[q] = corner[tet_conn(t, q)];
-            const float v6 = vol6_exact(v[0], v[1], v[2], v[3]);
-            const int sgn = vol6_sign_ref(v6);
-            int lo[3], hi[3];
-            if (!candidate_range(v, g, lo, hi) || sgn == 0 || !tile_clamp(g, lo, hi)) continue;
-            if (sgn < 0) { const float3 tt = v[0]; v[0] = v[3]; v[3] = tt; }
-            unsigned nc = 0, np = 0;
-            deposit_tet_fp64_warp(v, lo, hi, g, P.out_d, nc, np);
-        }
-    }
-}
+}  // namespace adeco
+#include "plain_fp64.cuh"
+namespace adeco {
 
 // -------------------------------------------------- ill-conditioned tets
 // Per-warp state of the tet being routed (shared memory, written by lane 0):

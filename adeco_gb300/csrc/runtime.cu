@@ -162,6 +162,7 @@ int mixed_setup(int device, DeviceProps &dp)
     CUDA_TRY(cudaFuncSetAttribute(deposit_mixed_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)dp.mixed_smem));
     CUDA_TRY(cudaFuncSetAttribute(route_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRouteSmem));
+    CUDA_TRY(cudaFuncSetAttribute(deposit_plain_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlainSmem));
     int nb = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, deposit_mixed_kernel<false>, kThreads, dp.mixed_smem));
     dp.mixed_blocks_per_sm = std::max(1, nb);
@@ -250,10 +251,12 @@ int launch_plain(const DeviceProps &dp, DepositParams P, const long long *d_cube
                  cudaStream_t st)
 {
     if (P.n_items <= 0 || c1 <= c0) return ADECO_OK;
-    const long long warps = c1 - c0;
-    const long long want = (warps * 32 + kThreads - 1) / kThreads;
-    const int grid = (int)std::max(1LL, std::min(want, (long long)dp.sms * 8));
-    deposit_plain_fp64_kernel<<<grid, kThreads, 0, st>>>(P, c0, c1, d_cube_off);
+    // fewer cubes a warp where that leaves SMs idle: 8 warps an SM are resident
+    const long long n = c1 - c0;
+    const int warp_cubes = (int)std::max(1LL, std::min<long long>(kPlainCubes, n / (dp.sms * 16LL)));
+    const long long per_cta = (long long)warp_cubes * kPlainWarps;
+    const int grid = (int)std::max(1LL, std::min((n + per_cta - 1) / per_cta, dp.sms * 24LL));
+    deposit_plain_fp64_kernel<<<grid, kPlainThreads, kPlainSmem, st>>>(P, c0, c1, d_cube_off, warp_cubes);
     CUDA_TRY(cudaGetLastError());
     return ADECO_OK;
 }
