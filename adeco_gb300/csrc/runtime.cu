@@ -9,6 +9,7 @@
 // batched persistent launch (mixed precision) or as one FP64 launch per leaf
 // (the plain baseline).
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -139,6 +140,7 @@ GridDesc make_grid(const float bbox[6], int dims, double tet_mass, int shift, lo
 
 struct DeviceProps {
     int sms = 0;
+    bool host_tables = false;  // kernels reach pageable host memory, through the host's page tables
     int mixed_blocks_per_sm = 0;
     size_t mixed_smem = 0;
 };
@@ -156,6 +158,9 @@ int mixed_setup(int device, DeviceProps &dp)
     cudaDeviceProp prop;
     CUDA_TRY(cudaGetDeviceProperties(&prop, device));
     dp.sms = prop.multiProcessorCount;
+    int pageable = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device));
+    dp.host_tables = pageable != 0;
     dp.mixed_smem = sizeof(SharedMixed);
     CUDA_TRY(cudaFuncSetAttribute(deposit_mixed_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)dp.mixed_smem));
@@ -226,12 +231,11 @@ int item_parts(int n_items, int slots)
 }
 
 // One persistent launch of the mixed kernel over `n_items` items, then the
-// launch that deposits the ill-conditioned tets it listed.
+// launch that deposits the ill-conditioned tets it listed.  The work counter
+// and the route count are 0 when it starts.
 int launch_mixed(const DeviceProps &dp, DepositParams P, cudaStream_t st, int ctas_per_sm = 0)
 {
     if (P.n_items <= 0) return ADECO_OK;
-    CUDA_TRY(cudaMemsetAsync(P.counter, 0, sizeof(int), st));
-    CUDA_TRY(cudaMemsetAsync(P.route_count, 0, sizeof(unsigned long long), st));
     const int per_sm = ctas_per_sm > 0 ? std::min(ctas_per_sm, dp.mixed_blocks_per_sm) : dp.mixed_blocks_per_sm;
     P.parts = item_parts(P.n_items, dp.sms * per_sm);
     const int grid = (int)std::min<long long>((long long)P.n_items * P.parts, (long long)dp.sms * per_sm);
@@ -272,35 +276,6 @@ int select_device(int use_specific_gpu, size_t device_id, int &dev)
     dev = use_specific_gpu ? (int)device_id : 0;
     CUDA_TRY(cudaSetDevice(dev));
     return ADECO_OK;
-}
-
-// Work items for patches [p0, p0+np) of (m+1)^3-vertex patches: sub-blocks of
-// at most 7^3 cubes each.
-void patch_items(size_t p0, size_t np, int m, int grid, std::vector<Item> &items, std::vector<long long> *cube_off)
-{
-    const long long n1 = m + 1, n2 = n1 * n1;
-    const int nsb = MetaGrid::ceil_div(m, kMetaCubes);
-    long long cubes = cube_off && !cube_off->empty() ? cube_off->back() : 0;
-    for (size_t p = p0; p < p0 + np; ++p) {
-        const long long pbase = (long long)p * n1 * n2;
-        for (int sz = 0; sz < nsb; ++sz)
-            for (int sy = 0; sy < nsb; ++sy)
-                for (int sx = 0; sx < nsb; ++sx) {
-                    const int ox = sx * kMetaCubes, oy = sy * kMetaCubes, oz = sz * kMetaCubes;
-                    const int vx = std::min(kMetaCubes + 1, m + 1 - ox), vy = std::min(kMetaCubes + 1, m + 1 - oy),
-                              vz = std::min(kMetaCubes + 1, m + 1 - oz);
-                    Item it;
-                    it.base = pbase + ox + n1 * oy + n2 * oz;
-                    it.grid = grid;
-                    it.nv = vx | (vy << 8) | (vz << 16);
-                    items.push_back(it);
-                    if (cube_off) {
-                        cube_off->push_back(cubes);
-                        cubes += (long long)(vx - 1) * (vy - 1) * (vz - 1);
-                    }
-                }
-    }
-    if (cube_off) cube_off->push_back(cubes);
 }
 
 int validate_boundary(size_t patch_offset, size_t num_patches, const float *positions, size_t positions_size, int m,
@@ -348,19 +323,24 @@ struct BoundaryWork {
     DevBuf<unsigned long long> route, fixed;
     DevBuf<double> f64, packed;
     DevBuf<float> pos, part;
+    DevBuf<CallBox> box;
     double *pinned = nullptr;  // D2H staging of the grid
     size_t pinned_n = 0;
-    float *pin_part = nullptr;  // D2H staging of the vertex-box partials
+    struct Status {  // what a call reads back at its end
+        int error;
+        CallBox box;
+    } *status = nullptr;
     ~BoundaryWork() { drop(); }
     void drop()
     {
         items.release(); grid.release(); counter.release(); cube_off.release();
         route.release(); fixed.release(); f64.release(); packed.release(); pos.release(); part.release();
+        box.release();
         if (pinned) cudaFreeHost(pinned);
         pinned = nullptr;
         pinned_n = 0;
-        if (pin_part) cudaFreeHost(pin_part);
-        pin_part = nullptr;
+        if (status) cudaFreeHost(status);
+        status = nullptr;
         if (stream) cudaStreamDestroy(stream);
         stream = nullptr;
     }
@@ -373,11 +353,9 @@ struct BoundaryWork {
         CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         return ADECO_OK;
     }
-    int box_staging()
+    int status_block()
     {
-        if (pin_part) return ADECO_OK;
-        if (int rc = part.reserve(kBoxBlocks * 7)) return rc;
-        CUDA_TRY(cudaHostAlloc((void **)&pin_part, kBoxBlocks * 7 * sizeof(float), cudaHostAllocDefault));
+        if (!status) CUDA_TRY(cudaHostAlloc((void **)&status, sizeof(Status), cudaHostAllocDefault));
         return ADECO_OK;
     }
     static constexpr int kBoxBlocks = 256;
@@ -395,36 +373,35 @@ struct BoundaryWork {
 thread_local BoundaryWork t_work;
 }  // namespace
 
-// Deposit patches [patch_offset, +num_patches) of device-resident patch data
-// into d_fixed (mixed, fixed point 2^shift) or d_f64 (plain FP64).
-static int deposit_device_core(int dev, const float *d_pos, size_t patch_offset, size_t num_patches, int m,
-                               const float *bbox, int dims, int precision, int order, double tet_mass,
-                               unsigned long long *d_fixed, double *d_f64, int shift, cudaStream_t st)
+// Enqueues the deposit of patches [patch_offset, +num_patches) of
+// device-resident patch data into d_fixed (mixed, fixed point 2^shift) or
+// d_f64 (plain FP64).  The device error flag is t_work.counter's second word,
+// cleared by the call's first pass; with_box: t_work.box is kept too.
+static int enqueue_deposit(int dev, const DeviceProps &dp, const float *d_pos, size_t patch_offset, size_t num_patches,
+                           int m, const float *bbox, int dims, int precision, int order, double tet_mass,
+                           unsigned long long *d_fixed, double *d_f64, int shift, bool first, bool with_box,
+                           cudaStream_t st)
 {
-    DeviceProps dp;
-    int rc = mixed_setup(dev, dp);
+    int rc = t_work.bind(dev);
     if (rc) return rc;
-    std::vector<Item> items;
-    std::vector<long long> cube_off;
-    patch_items(patch_offset, num_patches, m, 0, items, precision == ADECO_PREC_FP64 ? &cube_off : nullptr);
-    GridDesc g = make_grid(bbox, dims, tet_mass, shift, 0);
-    if ((rc = t_work.bind(dev))) return rc;
-    DevBuf<Item> &d_items = t_work.items;
-    DevBuf<GridDesc> &d_grid = t_work.grid;
-    DevBuf<int> &d_counter = t_work.counter;
-    DevBuf<long long> &d_cube_off = t_work.cube_off;
-    DevBuf<unsigned long long> &d_route = t_work.route;
-    const unsigned long long rcap = route_capacity((long long)items.size());
-    if ((rc = d_items.reserve(items.size())) || (rc = d_grid.reserve(1)) || (rc = d_counter.reserve(2))) return rc;
-    if (precision != ADECO_PREC_FP64 && (rc = d_route.reserve(rcap + 1))) return rc;
-    CUDA_TRY(cudaMemsetAsync(d_counter.p, 0, 2 * sizeof(int), st));
-    CUDA_TRY(cudaMemcpyAsync(d_items.p, items.data(), items.size() * sizeof(Item), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(d_grid.p, &g, sizeof g, cudaMemcpyHostToDevice, st));
+    const int nsb = MetaGrid::ceil_div(m, kMetaCubes);
+    const size_t n_items = num_patches * nsb * nsb * nsb;
+    const bool plain = precision == ADECO_PREC_FP64;
+    const unsigned long long rcap = route_capacity((long long)n_items);
+    if ((rc = t_work.items.reserve(n_items)) || (rc = t_work.grid.reserve(1)) || (rc = t_work.counter.reserve(2)) ||
+        (with_box && (rc = t_work.box.reserve(1))))
+        return rc;
+    if (plain ? (rc = t_work.cube_off.reserve(n_items + 1)) : (rc = t_work.route.reserve(rcap + 1))) return rc;
+    patch_items_kernel<<<(unsigned)((n_items + 127) / 128), 128, 0, st>>>(
+        t_work.items.p, plain ? t_work.cube_off.p : nullptr, (long long)patch_offset, (int)n_items, m, nsb, t_work.grid.p,
+        make_grid(bbox, dims, tet_mass, shift, 0), t_work.counter.p, plain ? nullptr : t_work.route.p,
+        with_box ? t_work.box.p : nullptr, first);
+    CUDA_TRY(cudaGetLastError());
     DepositParams P = base_params(Tuning());
-    P.items = d_items.p;
-    P.n_items = (int)items.size();
+    P.items = t_work.items.p;
+    P.n_items = (int)n_items;
     P.src_kind = SRC_PATCH_F3;
-    P.grids = d_grid.p;
+    P.grids = t_work.grid.p;
     P.src = d_pos;
     P.stride_y = m + 1;
     P.stride_z = (long long)(m + 1) * (m + 1);
@@ -432,23 +409,34 @@ static int deposit_device_core(int dev, const float *d_pos, size_t patch_offset,
     P.pad_check = 1;
     P.out = d_fixed;
     P.out_d = d_f64;
-    P.counter = d_counter.p;
-    P.error = d_counter.p + 1;
-    if (precision != ADECO_PREC_FP64) set_route(P, d_route.p, rcap);
-    if (precision == ADECO_PREC_FP64) {
-        if ((rc = d_cube_off.reserve(cube_off.size()))) return rc;
-        CUDA_TRY(cudaMemcpyAsync(d_cube_off.p, cube_off.data(), cube_off.size() * sizeof(long long),
-                                 cudaMemcpyHostToDevice, st));
-        rc = launch_plain(dp, P, d_cube_off.p, 0, cube_off.back(), st);
-    } else {
-        rc = launch_mixed(dp, P, st);
+    P.counter = t_work.counter.p;
+    P.error = t_work.counter.p + 1;
+    if (plain) return launch_plain(dp, P, t_work.cube_off.p, 0, (long long)num_patches * m * m * m, st);
+    set_route(P, t_work.route.p, rcap);
+    return launch_mixed(dp, P, st);
+}
+
+// Makes the pages of rows [lo, lo + ext) of a dims^3 grid of `size`-byte cells
+// present and writable, by writing a cell of each back to itself: a kernel's
+// first write to a page that the host never touched takes tens of microseconds.
+static void touch_rows(void *grid, size_t size, int dims, const int lo[3], const int ext[3])
+{
+    static const size_t page = (size_t)std::max(4096L, sysconf(_SC_PAGESIZE));
+    char *base = static_cast<char *>(grid), *next = base;
+    const size_t d = (size_t)dims;
+    const bool whole = (size_t)ext[0] == d && (size_t)ext[1] == d;
+    const size_t rows = whole ? 1 : (size_t)ext[1] * ext[2];
+    const size_t len = size * (whole ? d * d * (size_t)ext[2] : (size_t)ext[0]);
+    for (size_t r = 0; r < rows; ++r) {
+        const size_t y = lo[1] + r % ext[1], z = lo[2] + r / ext[1];
+        char *a = base + size * ((size_t)lo[0] + d * (y + d * z)), *end = a + len;
+        for (char *p = std::max(a, next); p < end;) {
+            volatile char *v = p;
+            *v = *v;
+            p = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) / page + 1) * page);
+            next = p;
+        }
     }
-    if (rc) return rc;
-    int err = 0;
-    CUDA_TRY(cudaMemcpyAsync(&err, d_counter.p + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    if (err) return deposit_error(err, "the grid");
-    return ADECO_OK;
 }
 
 extern "C" int adeco_deposit_tets_ex(const adeco_deposit_args *a)
@@ -481,122 +469,114 @@ extern "C" int adeco_deposit_tets_ex(const adeco_deposit_args *a)
     size_t per_pass = (size_t)((budget - (double)grid_bytes) / (double)patch_bytes);
     per_pass = std::max<size_t>(1, std::min(per_pass, a->num_patches));
 
-    if ((rc = t_work.bind(dev))) return rc;
+    DeviceProps dp;
+    if ((rc = mixed_setup(dev, dp)) || (rc = t_work.bind(dev)) || (rc = t_work.status_block())) return rc;
     cudaStream_t st = t_work.stream;
+    const bool plain = a->precision == ADECO_PREC_FP64;
     DevBuf<float> &d_pos = t_work.pos;
     DevBuf<unsigned long long> &d_fixed = t_work.fixed;
     DevBuf<double> &d_f64 = t_work.f64;
-    rc = d_pos.reserve(per_pass * fpp);
-    if (!rc) rc = (a->precision == ADECO_PREC_FP64) ? d_f64.reserve(ncell) : d_fixed.reserve(ncell);
-    if (!rc && a->precision == ADECO_PREC_FP64) {
-        if (cudaMemsetAsync(d_f64.p, 0, ncell * sizeof(double), st) != cudaSuccess) rc = fail(ADECO_ERR_CUDA, "memset");
-    } else if (!rc) {
-        if (cudaMemsetAsync(d_fixed.p, 0, ncell * sizeof(unsigned long long), st) != cudaSuccess)
-            rc = fail(ADECO_ERR_CUDA, "memset");
-    }
+    if ((rc = d_pos.reserve(per_pass * fpp)) || (rc = t_work.part.reserve(BoundaryWork::kBoxBlocks * 7)) ||
+        (rc = plain ? d_f64.reserve(ncell) : d_fixed.reserve(ncell)))
+        return rc;
+    void *const sums = plain ? (void *)d_f64.p : (void *)d_fixed.p;
     // the fixed-point scale is fixed for the whole call
     const int call_shift = choose_shift(6.0 * (double)a->num_patches * (double)m * m * m, a->tet_mass);
-    // the box of the deposited vertices (padding left out), over all passes:
-    // only the grid cells in its range can receive mass, so only those are
-    // brought back and added (an image box of a periodic volume touches a
-    // thin slab of the grid)
-    float vmin[3] = {INFINITY, INFINITY, INFINITY}, vmax[3] = {-INFINITY, -INFINITY, -INFINITY};
-    bool vnan = false;
-    if (!rc) rc = t_work.box_staging();
-    for (size_t done = 0; !rc && done < a->num_patches; done += per_pass) {
-        const size_t np = std::min(per_pass, a->num_patches - done);
-        const float *src = a->positions + (a->patch_offset + done) * fpp;
-        if (cudaMemcpyAsync(d_pos.p, src, np * fpp * sizeof(float), cudaMemcpyHostToDevice, st) != cudaSuccess) {
-            rc = fail(ADECO_ERR_CUDA, "H2D positions");
-            break;
+    const double scale = std::ldexp(1.0, -call_shift);
+    // Everything of the call is enqueued, and the host waits once: positions,
+    // the deposit, the box of the deposited vertices (padding left out) over
+    // all passes.  Only the grid cells in its range can receive mass, so only
+    // those are added (an image box of a periodic volume touches a thin slab
+    // of the grid).  On an error the stream is drained before the buffers are
+    // used again.
+    rc = [&]() -> int {
+        CUDA_TRY(cudaMemsetAsync(sums, 0, ncell * 8, st));
+        for (size_t done = 0; done < a->num_patches; done += per_pass) {
+            const size_t np = std::min(per_pass, a->num_patches - done);
+            const float *src = a->positions + (a->patch_offset + done) * fpp;
+            CUDA_TRY(cudaMemcpyAsync(d_pos.p, src, np * fpp * sizeof(float), cudaMemcpyHostToDevice, st));
+            const long long nvert = (long long)(np * fpp / 3);
+            const int bb_blocks =
+                (int)std::min<long long>(BoundaryWork::kBoxBlocks, (nvert + kBoxThreads - 1) / kBoxThreads);
+            patch_bbox_kernel<<<bb_blocks, kBoxThreads, 0, st>>>(d_pos.p, nvert, t_work.part.p);
+            CUDA_TRY(cudaGetLastError());
+            // every pass uses the call's shift: deposit patches [0, np) of the slice
+            if (int e = enqueue_deposit(dev, dp, d_pos.p, 0, np, m, a->bbox, a->dims, a->precision, a->tet_order,
+                                        a->tet_mass, d_fixed.p, d_f64.p, call_shift, done == 0, true, st))
+                return e;
+            call_box_kernel<<<1, 7 * 32, 0, st>>>(t_work.part.p, bb_blocks, t_work.grid.p, t_work.box.p);
+            CUDA_TRY(cudaGetLastError());
         }
-        const long long nvert = (long long)(np * fpp / 3);
-        const int bb_blocks = (int)std::min<long long>(BoundaryWork::kBoxBlocks, (nvert + kBoxThreads - 1) / kBoxThreads);
-        patch_bbox_kernel<<<bb_blocks, kBoxThreads, 0, st>>>(d_pos.p, nvert, t_work.part.p);
-        if (cudaGetLastError() != cudaSuccess ||
-            cudaMemcpyAsync(t_work.pin_part, t_work.part.p, (size_t)bb_blocks * 7 * sizeof(float), cudaMemcpyDeviceToHost,
-                            st) != cudaSuccess) {
-            rc = fail(ADECO_ERR_CUDA, "vertex box");
-            break;
+        const int *d_error = t_work.counter.p + 1;
+        const size_t cell = a->out_type == ADECO_OUT_F64 ? sizeof(double) : sizeof(float);
+        const auto read_status = [&]() -> int {
+            CUDA_TRY(cudaMemcpyAsync(&t_work.status->error, d_error, sizeof(int), cudaMemcpyDeviceToHost, st));
+            CUDA_TRY(cudaMemcpyAsync(&t_work.status->box, t_work.box.p, sizeof(CallBox), cudaMemcpyDeviceToHost, st));
+            CUDA_TRY(cudaStreamSynchronize(st));
+            return ADECO_OK;
+        };
+        const auto add_on_device = [&]() -> int {
+            const unsigned blocks = (unsigned)std::min<size_t>((size_t)dp.sms * 4, (ncell + 255) / 256);
+            if (a->out_type == ADECO_OUT_F64)
+                host_accumulate_kernel<double><<<blocks, 256, 0, st>>>(plain ? nullptr : d_fixed.p, d_f64.p,
+                                                                       (double *)a->data, a->dims, t_work.box.p, d_error, scale);
+            else
+                host_accumulate_kernel<float><<<blocks, 256, 0, st>>>(plain ? nullptr : d_fixed.p, d_f64.p,
+                                                                      (float *)a->data, a->dims, t_work.box.p, d_error, scale);
+            CUDA_TRY(cudaGetLastError());
+            return ADECO_OK;
+        };
+        const CallBox &box = t_work.status->box;
+        // Grids of up to 64 MB: all their pages are touched while the device
+        // works and the sums added behind the deposit.  Larger ones wait for
+        // the box, and only its rows are touched.
+        const bool small = ncell * cell <= ((size_t)64 << 20);
+        if (dp.host_tables && small) {
+            const int lo[3] = {0, 0, 0}, ext[3] = {a->dims, a->dims, a->dims};
+            touch_rows(a->data, cell, a->dims, lo, ext);
+            if (int e = add_on_device()) return e;
         }
-        // every pass uses the call's shift: deposit patches [0, np) of the slice
-        rc = deposit_device_core(dev, d_pos.p, 0, np, m, a->bbox, a->dims, a->precision, a->tet_order, a->tet_mass,
-                                 d_fixed.p, d_f64.p, call_shift, st);
-        if (rc) break;  // deposit_device_core synchronised the stream: the partials are in
-        for (int b = 0; b < bb_blocks; ++b) {
-            const float *q = t_work.pin_part + 7 * b;
-            for (int x = 0; x < 3; ++x) {
-                vmin[x] = std::fmin(vmin[x], q[x]);
-                vmax[x] = std::fmax(vmax[x], q[3 + x]);
+        if (int e = read_status()) return e;
+        if (t_work.status->error) return deposit_error(t_work.status->error, "the grid");
+        if (box.empty || (dp.host_tables && small)) return ADECO_OK;
+        if (dp.host_tables) {
+            touch_rows(a->data, cell, a->dims, box.lo, box.ext);
+            if (int e = add_on_device()) return e;
+            CUDA_TRY(cudaStreamSynchronize(st));
+            return ADECO_OK;
+        }
+        // convert the box's cells to FP64 packed, bring them back, add them
+        // into the caller's grid
+        const size_t nbox = (size_t)box.ext[0] * box.ext[1] * box.ext[2];
+        const double *dsrc = d_f64.p;  // the plain FP64 path accumulates in FP64: the whole grid is the grid itself
+        if (!plain || nbox != ncell) {
+            DevBuf<double> &dst = plain ? t_work.packed : d_f64;
+            if (int e = dst.reserve(nbox)) return e;
+            const unsigned blocks = (unsigned)std::min<size_t>(1024, (nbox + 255) / 256);
+            grid_box_kernel<<<blocks, 256, 0, st>>>(plain ? nullptr : d_fixed.p, d_f64.p, dst.p, a->dims, box.lo[0],
+                                                    box.lo[1], box.lo[2], box.ext[0], box.ext[1], box.ext[2], scale);
+            CUDA_TRY(cudaGetLastError());
+            dsrc = dst.p;
+        }
+        if (int e = t_work.staging(nbox)) return e;
+        CUDA_TRY(cudaMemcpyAsync(t_work.pinned, dsrc, nbox * sizeof(double), cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaStreamSynchronize(st));
+        const size_t d = (size_t)a->dims;
+        for (int z = 0; z < box.ext[2]; ++z)
+            for (int y = 0; y < box.ext[1]; ++y) {
+                const double *row = t_work.pinned + (size_t)box.ext[0] * (y + (size_t)box.ext[1] * z);
+                const size_t c0 = (size_t)box.lo[0] + d * ((size_t)(box.lo[1] + y) + d * (size_t)(box.lo[2] + z));
+                if (a->out_type == ADECO_OUT_F64) {
+                    double *out = (double *)a->data + c0;
+                    for (int x = 0; x < box.ext[0]; ++x) out[x] += row[x];
+                } else {
+                    float *out = (float *)a->data + c0;
+                    for (int x = 0; x < box.ext[0]; ++x) out[x] += (float)row[x];
+                }
             }
-            vnan = vnan || q[6] != 0.f;
-        }
-    }
-    // the cell range of the vertex box (one cell of margin against the
-    // rounding of the kernels' FP32 range arithmetic); a NaN coordinate
-    // falls back to the whole grid
-    int lo[3] = {0, 0, 0}, ext[3] = {a->dims, a->dims, a->dims};
-    bool empty = false;
-    if (!rc && !vnan) {
-        for (int x = 0; x < 3; ++x) {
-            const double gmin = a->bbox[2 * x], gmax = a->bbox[2 * x + 1];
-            const double delta = (double)((a->bbox[2 * x + 1] - a->bbox[2 * x]) / (float)a->dims);
-            if (!(vmin[x] <= vmax[x]) || (double)vmax[x] < gmin || (double)vmin[x] > gmax || !(delta > 0.0)) {
-                empty = true;
-                break;
-            }
-            const double flo = std::floor((std::fmax((double)vmin[x], gmin) - gmin) / delta) - 1.0;
-            const double fhi = std::ceil((std::fmin((double)vmax[x], gmax) - gmin) / delta) + 1.0;
-            const int l = (int)std::fmin(std::fmax(flo, 0.0), (double)(a->dims - 1));
-            const int h = (int)std::fmin(std::fmax(fhi, 0.0), (double)(a->dims - 1));
-            lo[x] = l;
-            ext[x] = h - l + 1;
-        }
-    }
-    // convert the box's cells to FP64 packed, bring them back, add them into
-    // the caller's grid
-    if (!rc && !empty) {
-        const size_t nbox = (size_t)ext[0] * ext[1] * ext[2];
-        const bool whole = nbox == ncell;
-        const double *dsrc = nullptr;  // device FP64 of the box, packed
-        if (a->precision == ADECO_PREC_FP64 && whole) {
-            dsrc = d_f64.p;  // the plain FP64 path accumulates in FP64: the grid itself
-        } else {
-            DevBuf<double> &dst = (a->precision == ADECO_PREC_FP64) ? t_work.packed : d_f64;
-            if ((rc = dst.reserve(nbox)) == ADECO_OK) {
-                const unsigned blocks = (unsigned)std::min<size_t>(1024, (nbox + 255) / 256);
-                grid_box_kernel<<<blocks, 256, 0, st>>>(a->precision == ADECO_PREC_FP64 ? nullptr : d_fixed.p, d_f64.p,
-                                                        dst.p, a->dims, lo[0], lo[1], lo[2], ext[0], ext[1], ext[2],
-                                                        std::ldexp(1.0, -call_shift));
-                dsrc = dst.p;
-            }
-        }
-        if (!rc) rc = t_work.staging(nbox);
-        if (!rc) {
-            const double *host = t_work.pinned;
-            if (cudaGetLastError() != cudaSuccess ||
-                cudaMemcpyAsync(t_work.pinned, dsrc, nbox * sizeof(double), cudaMemcpyDeviceToHost, st) !=
-                    cudaSuccess ||
-                cudaStreamSynchronize(st) != cudaSuccess) {
-                rc = fail(ADECO_ERR_CUDA, "D2H grid: %s", cudaGetErrorString(cudaGetLastError()));
-            } else {
-                const size_t d = (size_t)a->dims;
-                for (int z = 0; z < ext[2]; ++z)
-                    for (int y = 0; y < ext[1]; ++y) {
-                        const double *row = host + (size_t)ext[0] * (y + (size_t)ext[1] * z);
-                        const size_t c0 = (size_t)lo[0] + d * ((size_t)(lo[1] + y) + d * (size_t)(lo[2] + z));
-                        if (a->out_type == ADECO_OUT_F64) {
-                            double *out = (double *)a->data + c0;
-                            for (int x = 0; x < ext[0]; ++x) out[x] += row[x];
-                        } else {
-                            float *out = (float *)a->data + c0;
-                            for (int x = 0; x < ext[0]; ++x) out[x] += (float)row[x];
-                        }
-                    }
-            }
-        }
-    }
-    cudaStreamSynchronize(st);
+        return ADECO_OK;
+    }();
+    if (rc) cudaStreamSynchronize(st);
     return rc;
 }
 
@@ -635,21 +615,31 @@ extern "C" int adeco_deposit_tets_device(const float *d_positions, size_t positi
     cudaStream_t st = (cudaStream_t)stream;
     const size_t ncell = (size_t)dims * dims * dims;
     const int shift = choose_shift(6.0 * (double)num_patches * (double)m * m * m, tet_mass);
-    if (precision == ADECO_PREC_FP64) {
-        return deposit_device_core(dev, d_positions, patch_offset, num_patches, m, bbox, dims, precision, tet_order,
-                                   tet_mass, nullptr, d_out, shift, st);
-    }
-    if ((rc = t_work.bind(dev))) return rc;
-    DevBuf<unsigned long long> &d_fixed = t_work.fixed;
-    if ((rc = d_fixed.reserve(ncell))) return rc;
-    CUDA_TRY(cudaMemsetAsync(d_fixed.p, 0, ncell * sizeof(unsigned long long), st));
-    rc = deposit_device_core(dev, d_positions, patch_offset, num_patches, m, bbox, dims, precision, tet_order,
-                             tet_mass, d_fixed.p, nullptr, shift, st);
-    if (rc) return rc;
-    fixed_accumulate_f64_kernel<<<1024, 256, 0, st>>>(d_fixed.p, d_out, (long long)ncell, std::ldexp(1.0, -shift));
-    CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaStreamSynchronize(st));
-    return ADECO_OK;
+    DeviceProps dp;
+    if ((rc = mixed_setup(dev, dp)) || (rc = t_work.bind(dev)) || (rc = t_work.status_block())) return rc;
+    rc = [&]() -> int {
+        if (precision == ADECO_PREC_FP64) {
+            if (int e = enqueue_deposit(dev, dp, d_positions, patch_offset, num_patches, m, bbox, dims, precision, tet_order,
+                                        tet_mass, nullptr, d_out, shift, true, false, st))
+                return e;
+        } else {
+            DevBuf<unsigned long long> &d_fixed = t_work.fixed;
+            if (int e = d_fixed.reserve(ncell)) return e;
+            CUDA_TRY(cudaMemsetAsync(d_fixed.p, 0, ncell * sizeof(unsigned long long), st));
+            if (int e = enqueue_deposit(dev, dp, d_positions, patch_offset, num_patches, m, bbox, dims, precision, tet_order,
+                                        tet_mass, d_fixed.p, nullptr, shift, true, false, st))
+                return e;
+            fixed_accumulate_f64_kernel<<<1024, 256, 0, st>>>(d_fixed.p, d_out, (long long)ncell, std::ldexp(1.0, -shift),
+                                                              t_work.counter.p + 1);
+            CUDA_TRY(cudaGetLastError());
+        }
+        CUDA_TRY(cudaMemcpyAsync(&t_work.status->error, t_work.counter.p + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaStreamSynchronize(st));
+        if (t_work.status->error) return deposit_error(t_work.status->error, "the grid");
+        return ADECO_OK;
+    }();
+    if (rc) cudaStreamSynchronize(st);
+    return rc;
 }
 
 // ============================================================ sessions
@@ -1133,6 +1123,8 @@ static int enqueue_leaves_mixed(adeco_session *s, bool stats)
 {
     const size_t nv = s->out_values;
     CUDA_TRY(cudaMemsetAsync(s->d_fixed.p, 0, nv * sizeof(unsigned long long), s->stream));
+    CUDA_TRY(cudaMemsetAsync(s->d_counter.p, 0, sizeof(int), s->stream));
+    CUDA_TRY(cudaMemsetAsync(s->d_route.p, 0, sizeof(unsigned long long), s->stream));
     int rc = launch_mixed(s->dp, session_params(s, stats), s->stream, s->tuning.ctas_per_sm);
     if (rc) return rc;
     const long long cells = (long long)s->leaf_dims * s->leaf_dims * s->leaf_dims;
@@ -1180,6 +1172,8 @@ extern "C" int adeco_session_deposit_leaves(adeco_session *s, int precision, dou
         CUDA_TRY(cudaEventRecord(e2, s->stream));
     } else {
         CUDA_TRY(cudaMemsetAsync(s->d_fixed.p, 0, s->out_values * sizeof(unsigned long long), s->stream));
+        CUDA_TRY(cudaMemsetAsync(s->d_counter.p, 0, sizeof(int), s->stream));
+        CUDA_TRY(cudaMemsetAsync(s->d_route.p, 0, sizeof(unsigned long long), s->stream));
         CUDA_TRY(cudaEventRecord(e0, s->stream));
         rc = launch_mixed(s->dp, session_params(s, collect_stats != 0), s->stream, s->tuning.ctas_per_sm);
         launches = 2;  // the mixed kernel and the ill-conditioned-tet launch
@@ -1466,28 +1460,6 @@ int noalloc_setup(int dev, NoAllocDevice &out)
 }
 }  // namespace
 
-// the grid descriptor, passed by value, into the scratch
-__global__ void noalloc_grid_kernel(GridDesc *dst, GridDesc g) { *dst = g; }
-
-// work items of patches [p0, p0 + np): sub-blocks of <= 7^3 cubes, as patch_items()
-__global__ void noalloc_items_kernel(Item *items, long long p0, int n_items, int m, int nsb)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_items) return;
-    const long long n1 = m + 1, n2 = n1 * n1;
-    const int per = nsb * nsb * nsb;
-    const long long p = p0 + i / per;
-    const int sb = i % per, sx = sb % nsb, sy = (sb / nsb) % nsb, sz = sb / (nsb * nsb);
-    const int ox = sx * kMetaCubes, oy = sy * kMetaCubes, oz = sz * kMetaCubes;
-    const int vx = min(kMetaCubes + 1, m + 1 - ox), vy = min(kMetaCubes + 1, m + 1 - oy),
-              vz = min(kMetaCubes + 1, m + 1 - oz);
-    Item it;
-    it.base = p * n1 * n2 + ox + n1 * oy + n2 * oz;
-    it.grid = 0;
-    it.nv = vx | (vy << 8) | (vz << 16);
-    items[i] = it;
-}
-
 extern "C" int adeco_deposit_tets_device_noalloc(const float *d_positions, size_t positions_size, size_t patch_offset,
                                                  size_t num_patches, int meta_cells_per_patch, const float bbox[6],
                                                  int dims, double *d_out, int tet_order, double tet_mass, void *stream)
@@ -1520,12 +1492,10 @@ extern "C" int adeco_deposit_tets_device_noalloc(const float *d_positions, size_
         reinterpret_cast<unsigned long long *>(nd.scratch + kNoAllocHeader + (size_t)kNoAllocMaxItems * sizeof(Item));
     unsigned long long *route = fixed + kNoAllocMaxCells;  // count word, then the entries
     const int shift = choose_shift(6.0 * (double)num_patches * (double)m * m * m, tet_mass);
-    CUDA_TRY(cudaMemsetAsync(counter, 0, 2 * sizeof(int), st));
-    CUDA_TRY(cudaMemsetAsync(route, 0, sizeof(unsigned long long), st));
     CUDA_TRY(cudaMemsetAsync(fixed, 0, (size_t)ncell * sizeof(unsigned long long), st));
-    noalloc_grid_kernel<<<1, 1, 0, st>>>(grid, make_grid(bbox, dims, tet_mass, shift, 0));
-    noalloc_items_kernel<<<(unsigned)((n_items + 127) / 128), 128, 0, st>>>(items, (long long)patch_offset,
-                                                                           (int)n_items, m, nsb);
+    patch_items_kernel<<<(unsigned)((n_items + 127) / 128), 128, 0, st>>>(
+        items, nullptr, (long long)patch_offset, (int)n_items, m, nsb, grid, make_grid(bbox, dims, tet_mass, shift, 0),
+        counter, route, nullptr, 1);
     CUDA_TRY(cudaGetLastError());
     DepositParams P = base_params(Tuning());
     P.items = items;
@@ -1548,7 +1518,7 @@ extern "C" int adeco_deposit_tets_device_noalloc(const float *d_positions, size_
     CUDA_TRY(cudaGetLastError());
     route_fp64_kernel<<<nd.sms * 2, kThreads, kRouteSmem, st>>>(P);  // the resident CTAs
     CUDA_TRY(cudaGetLastError());
-    fixed_accumulate_f64_kernel<<<1024, 256, 0, st>>>(fixed, d_out, ncell, std::ldexp(1.0, -shift));
+    fixed_accumulate_f64_kernel<<<1024, 256, 0, st>>>(fixed, d_out, ncell, std::ldexp(1.0, -shift), counter + 1);
     CUDA_TRY(cudaGetLastError());
     int err = 0;
     CUDA_TRY(cudaMemcpyAsync(&err, counter + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
