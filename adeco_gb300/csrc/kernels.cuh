@@ -112,6 +112,7 @@ struct TetVertices {
 // (d + dlo: ~44 bits), which setup_tet<true> stores.  The kernels form the
 // vertices and the exact offsets again for the pairs that need them.
 struct WarpTets : TetPlanes<32>, TetVertices {
+    static constexpr bool kHasRest = true;
     float dlo[4][32];
 };
 
@@ -141,6 +142,7 @@ __device__ __forceinline__ bool wait_zero_bounded(const int *count, unsigned lim
 
 // The staged vertex block and the wave's tets.
 struct WaveTets : TetPlanes<kWave> {
+    static constexpr bool kHasRest = false;
     float gh[3][kMaxVerts];  // grid-frame coordinates of the staged vertices, hi
     float gl[3][kMaxVerts];  //   and lo parts
     ushort4 vid[kWave];      // the tets' vertices, ordered by the orientation rule
@@ -300,11 +302,13 @@ ADECO_HD inline F2 plane_offset(const float qa[3], const float la[3], const floa
 // instruction cache holds about 32 KB: a loop of that size issues at 0.87 of
 // the peak, one of 48 KB at 0.5).
 //
-// kExactD: store each face's exact plane offset (d, dlo: the one-face closed
-// form reads them).  Otherwise only an FP32 d for the classification, whose
-// error band covers its rounding; the closed form then forms the exact
-// offset itself (plane_offset from the stored vertices) for the pairs that
-// take it: the double-float offsets had been ~40% of the set-up.
+// kExactD: each face's plane offset in double-float, rounded once (d; its
+// remainder too where the table has room for it, dlo).  Otherwise an FP32 d,
+// whose rounding the classification's error band covers.  The double-float
+// offsets had been ~40% of the set-up: octree leaves and boundary grids do
+// without, zoom grids, whose tets have thousands of pairs each, use them.
+// The one-face closed form takes exact offsets either way (it forms them from
+// the stored vertices).
 template <bool kExactD, class Table, class Frame>
 ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc &g, TetVertices &Q, int lane, Table &W,
                                 int t, int *error, bool *fp64_route)
@@ -414,7 +418,7 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
             }
             const F2 d = plane_offset(A, la, B, lb, C, lc, nn);
             W.d[f][t] = d.hi;
-            W.dlo[f][t] = d.lo;
+            if constexpr (Table::kHasRest) W.dlo[f][t] = d.lo;
         } else {
             constexpr float kThird = 1.f / 3.f;
             W.d[f][t] = (nn[0] * (A[0] + B[0] + C[0]) + nn[1] * (A[1] + B[1] + C[1]) + nn[2] * (A[2] + B[2] + C[2])) * kThird;
@@ -682,6 +686,7 @@ __device__ __forceinline__ void route_append(const DepositParams &P, const Share
 
 // Set-up phase: this warp's tets of the wave [first, end) of the tets of the
 // item's live cubes.
+template <bool kExactD>
 __device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &S, const Item &it, int first, int end,
                                            int vx, int vy, unsigned &n_tets)
 {
@@ -714,7 +719,7 @@ __device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &
         S.wt.vid[slot] = vid;
         // the tet's AABB strictly overlaps the grid box, and its volume is not zero
         if ((flags & (kBelowMax | kAboveMin)) == (kBelowMax | kAboveMin) && sgn != 0)
-            cnt = setup_frame<false>(
+            cnt = setup_frame<kExactD>(
                 mn, mx,
                 [&](int q, int a, float &h, float &l) {
                     const int v = q == 0 ? vid.x : (q == 1 ? vid.y : (q == 2 ? vid.z : vid.w));
@@ -823,8 +828,8 @@ __device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixe
 // counter and deposit an item's tets in waves of kWave (see the top of the
 // file).  A wave whose partial pairs do not fit the list is clipped in parts.
 // kStats: count the pairs (collect_stats); a separate instantiation, so that
-// the other carries no counters.
-template <bool kStats>
+// the others carry no counters.  kExactD: see setup_frame.
+template <bool kStats, bool kExactD = false>
 __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParams P)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -871,7 +876,7 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
                 S.wide = 0;
             }
             __syncthreads();
-            wave_setup(P, S, it, first, min(first + wave, ntet), vx, vy, st.tets);
+            wave_setup<kExactD>(P, S, it, first, min(first + wave, ntet), vx, vy, st.tets);
             __syncthreads();
             int total = 0;
 #pragma unroll

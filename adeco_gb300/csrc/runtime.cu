@@ -166,6 +166,8 @@ int mixed_setup(int device, DeviceProps &dp)
                                   (int)dp.mixed_smem));
     CUDA_TRY(cudaFuncSetAttribute(deposit_mixed_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)dp.mixed_smem));
+    CUDA_TRY(cudaFuncSetAttribute(deposit_mixed_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)dp.mixed_smem));
     CUDA_TRY(cudaFuncSetAttribute(route_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRouteSmem));
     CUDA_TRY(cudaFuncSetAttribute(deposit_plain_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlainSmem));
     int nb = 0;
