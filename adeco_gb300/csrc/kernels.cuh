@@ -1423,7 +1423,6 @@ __global__ void patch_items_kernel(Item *items, long long *cube_off, long long p
         // whole slabs, then whole rows of this slab, then blocks of this row
         const long long before = p * m * m * m + (long long)oz * m * m + (long long)(vz - 1) * ((long long)oy * m + (long long)(vy - 1) * ox);
         cube_off[i] = before;
-        if (i == n_items - 1) cube_off[n_items] = before + (long long)(vx - 1) * (vy - 1) * (vz - 1);
     }
 }
 

@@ -22,7 +22,7 @@
 
 namespace adeco {
 
-constexpr int kTreeChunk = 2048;   // pairs of one parent per block
+constexpr int kTreeChunk = 512;    // pairs of one parent per block (2048: 25 blocks at the root of 256^3, fill 33 us)
 constexpr int kTreeThreads = 256;  // 8 warps
 constexpr size_t kTreeMaxNodes = (size_t)1 << 24;
 
@@ -246,6 +246,101 @@ __global__ void __launch_bounds__(kTreeThreads) tree_fill_kernel(TreeMeta md, co
     if (threadIdx.x < 8 && est[threadIdx.x]) atomicAdd(&child_est[(size_t)ch.parent * 8 + threadIdx.x], est[threadIdx.x]);
 }
 
+// A leaf's meta-cell list on the device.
+struct LeafList {
+    const unsigned *ids;
+    long long off;  // its first work item
+    int len;
+    int pad;
+};
+
+// A leaf's work items (leaf x meta-cell) from its list, a block per leaf; the
+// lists back to back (ids_out), the items' cube offsets within their leaf and
+// the leaf's cubes.
+__global__ void __launch_bounds__(kTreeThreads) leaf_items_kernel(const LeafList *__restrict__ leaves, TreeMeta md,
+                                                                  Item *__restrict__ items, unsigned *__restrict__ ids_out,
+                                                                  long long *__restrict__ cube_off,
+                                                                  unsigned *__restrict__ leaf_cubes)
+{
+    __shared__ int wsum[kTreeThreads / 32];
+    const LeafList leaf = leaves[blockIdx.x];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned nb = (unsigned)md.cd[0], nb2 = nb * (unsigned)md.cd[1];
+    const int n[3] = {md.nx, md.ny, md.nz};
+    long long before = 0;
+    for (int r0 = 0; r0 < leaf.len; r0 += kTreeThreads) {
+        const int i = r0 + threadIdx.x;
+        int cubes = 0;
+        if (i < leaf.len) {
+            const unsigned id = leaf.ids[i];
+            const int c[3] = {(int)(id % nb), (int)((id % nb2) / nb), (int)(id / nb2)};
+            int org[3], nv[3];
+            cubes = 1;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                org[a] = c[a] * kMetaCubes;
+                nv[a] = (c[a] + 1 == md.cd[a]) ? (n[a] - org[a]) : kMetaCubes + 1;
+                cubes *= nv[a] - 1;
+            }
+            Item it;
+            it.base = org[0] + (long long)md.nx * (org[1] + (long long)md.ny * org[2]);
+            it.grid = (int)blockIdx.x;
+            it.nv = nv[0] | (nv[1] << 8) | (nv[2] << 16);
+            items[leaf.off + i] = it;
+            ids_out[leaf.off + i] = id;
+        }
+        int incl = cubes;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        int base = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < kTreeThreads / 32; ++w) {
+            base += w < warp ? wsum[w] : 0;
+            all += wsum[w];
+        }
+        if (i < leaf.len) cube_off[leaf.off + i] = before + base + incl - cubes;
+        before += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) leaf_cubes[blockIdx.x] = (unsigned)before;
+}
+
+// Device memory of a session's octree builds, kept between them: the levels'
+// id lists from a few large blocks, and the levels' small arrays.
+struct TreeWork {
+    std::vector<std::unique_ptr<DevBuf<unsigned>>> blocks;
+    size_t block = 0, used = 0;  // the block in use and its entries taken
+    DevBuf<unsigned char> lvl;
+    std::vector<unsigned char> h_lvl;
+
+    void reset() { block = used = 0; }
+    // room for n entries (give_back() returns what a list did not need)
+    int take(size_t n, size_t first_block, unsigned **p)
+    {
+        while (block < blocks.size() && used + n > blocks[block]->n) {
+            ++block;
+            used = 0;
+        }
+        if (block == blocks.size()) {
+            blocks.emplace_back(new DevBuf<unsigned>());
+            if (int rc = blocks.back()->reserve(std::max(n, first_block))) {
+                blocks.pop_back();
+                return rc;
+            }
+            used = 0;
+        }
+        *p = blocks[block]->p + used;
+        used += n;
+        return ADECO_OK;
+    }
+    void give_back(size_t n) { used -= n; }
+};
+
 namespace tree_host {
 
 inline bool meets(const float *a, const float *b)
@@ -269,10 +364,13 @@ struct BfsNode {
 
 }  // namespace tree_host
 
-// Builds `tree` as Octree::build(mg, box6, roi6, max_tets, max_level) does.
+// Builds `tree` as Octree::build(mg, box6, roi6, max_tets, max_level) does, but
+// for the leaves' meta-cell lists, which stay on the device: `lists`, in leaf
+// order, valid until `work` is used again.
 // d_mbb: the meta-cells' AABBs on the device (6 floats each, min xyz, max xyz).
 static int build_octree_device(const MetaGrid &mg, const float *d_mbb, const float box6[6], const float *roi6,
-                               uint64_t max_tets, int max_level, cudaStream_t st, Octree &tree)
+                               uint64_t max_tets, int max_level, cudaStream_t st, TreeWork &work, Octree &tree,
+                               std::vector<LeafList> &lists)
 {
     using namespace tree_host;
     tree.nodes.clear();
@@ -290,13 +388,14 @@ static int build_octree_device(const MetaGrid &mg, const float *d_mbb, const flo
     md.nx = mg.nx; md.ny = mg.ny; md.nz = mg.nz;
     for (int a = 0; a < 3; ++a) md.cd[a] = mg.cd[a];
 
-    std::vector<std::unique_ptr<DevBuf<unsigned>>> lv_ids;
+    std::vector<unsigned *> lv_ids;  // the levels' lists
     // A level's small arrays share one device block and one host block, so
     // a level costs one copy each way and the block is reallocated only when
     // it grows (by 2x at least): est | off (brought back), chunks | pfc | cbox
     // (sent), cnt | base (device only).
-    DevBuf<unsigned char> d_lvl;
-    std::vector<unsigned char> h_lvl;
+    DevBuf<unsigned char> &d_lvl = work.lvl;
+    std::vector<unsigned char> &h_lvl = work.h_lvl;
+    work.reset();
     int rc;
 
     std::vector<BfsNode> bfs(1);
@@ -316,15 +415,18 @@ static int build_octree_device(const MetaGrid &mg, const float *d_mbb, const flo
         bfs[0].len = (int)nmc;
     }
     int levels = 1;
-    lv_ids.emplace_back(new DevBuf<unsigned>());
-    if ((rc = lv_ids[0]->reserve(nmc)) || (rc = d_lvl.reserve(4096))) return rc;
+    // lists grow by a little from level to level, but a level's need is known
+    // only when it is filled: room for 8 times the last
+    const size_t first_block = (size_t)nmc * 20;
+    lv_ids.push_back(nullptr);
+    if ((rc = work.take(nmc, first_block, &lv_ids[0])) || (rc = d_lvl.reserve((size_t)1 << 16))) return rc;
     {
         unsigned long long *d_est = reinterpret_cast<unsigned long long *>(d_lvl.p);
         CUDA_TRY(cudaMemsetAsync(d_est, 0, sizeof(unsigned long long), st));
         TreeBox rb;
         node_box(bfs[0].n, rb.v);
         const unsigned blocks = std::min<unsigned>((nmc + 255) / 256, 4096u);
-        tree_root_kernel<<<blocks, 256, 0, st>>>(md, d_mbb, nmc, rb, lv_ids[0]->p, d_est);
+        tree_root_kernel<<<blocks, 256, 0, st>>>(md, d_mbb, nmc, rb, lv_ids[0], d_est);
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaMemcpyAsync(&bfs[0].n.estimate, d_est, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
@@ -390,7 +492,7 @@ static int build_octree_device(const MetaGrid &mg, const float *d_mbb, const flo
         const size_t nc = 8 * refined.size();
         const size_t cap = 8 * pairs;
         if (cap >= (1ull << 31)) return fail(ADECO_ERR_LIMIT, "octree level lists exceed 2^31 entries");
-        lv_ids.emplace_back(new DevBuf<unsigned>());
+        lv_ids.push_back(nullptr);
         const int nch = (int)chunks.size();
         // byte offsets in the level block, each 16-byte aligned
         const auto up = [](size_t b) { return (b + 15) & ~(size_t)15; };
@@ -401,7 +503,7 @@ static int build_octree_device(const MetaGrid &mg, const float *d_mbb, const flo
         const size_t o_cnt = up(o_cbox + cbox.size() * sizeof(float));
         const size_t o_base = up(o_cnt + (size_t)nch * 8 * sizeof(int));
         const size_t bytes = up(o_base + (size_t)nch * 8 * sizeof(int));
-        if ((rc = lv_ids[lv + 1]->reserve(cap))) return rc;
+        if ((rc = work.take(cap, first_block, &lv_ids[lv + 1]))) return rc;
         if (bytes > d_lvl.n && (rc = d_lvl.reserve(std::max(bytes, 2 * d_lvl.n)))) return rc;
         h_lvl.resize(std::max(h_lvl.size(), bytes));
         std::memcpy(h_lvl.data() + o_chunks, chunks.data(), (size_t)nch * sizeof(TreeChunk));
@@ -417,12 +519,12 @@ static int build_octree_device(const MetaGrid &mg, const float *d_mbb, const flo
         int *d_base = reinterpret_cast<int *>(blk + o_base);
         CUDA_TRY(cudaMemcpyAsync(blk + o_chunks, h_lvl.data() + o_chunks, o_cnt - o_chunks, cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemsetAsync(d_est, 0, nc * sizeof(unsigned long long), st));
-        tree_count_kernel<<<nch, kTreeThreads, 0, st>>>(d_mbb, lv_ids[lv]->p, d_chunks, d_cbox, d_cnt);
+        tree_count_kernel<<<nch, kTreeThreads, 0, st>>>(d_mbb, lv_ids[lv], d_chunks, d_cbox, d_cnt);
         CUDA_TRY(cudaGetLastError());
         tree_scan_kernel<<<1, 1024, 0, st>>>(d_chunks, nch, d_pfc, (int)refined.size(), d_cnt, d_base, d_off);
         CUDA_TRY(cudaGetLastError());
-        tree_fill_kernel<<<nch, kTreeThreads, 0, st>>>(md, d_mbb, lv_ids[lv]->p, d_chunks, d_cbox, d_base,
-                                                        lv_ids[lv + 1]->p, d_est);
+        tree_fill_kernel<<<nch, kTreeThreads, 0, st>>>(md, d_mbb, lv_ids[lv], d_chunks, d_cbox, d_base,
+                                                        lv_ids[lv + 1], d_est);
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaMemcpyAsync(h_lvl.data(), blk, o_chunks, cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
@@ -437,6 +539,7 @@ static int build_octree_device(const MetaGrid &mg, const float *d_mbb, const flo
             b.off = o0;
             b.len = o1 - o0;
         }
+        work.give_back(cap - (size_t)(bfs.back().off + bfs.back().len));
         lv_begin = first_child;
         lv_end = bfs.size();
     }
@@ -476,27 +579,14 @@ static int build_octree_device(const MetaGrid &mg, const float *d_mbb, const flo
             tree.leaves.push_back(cur);
         }
     }
-    // leaf lists: bring the levels' id lists back once, then copy per leaf
-    std::vector<std::vector<unsigned>> h_ids(lv_ids.size());
-    std::vector<size_t> lv_len(lv_ids.size(), 0);
-    for (const BfsNode &b : bfs) lv_len[b.lv] = std::max(lv_len[b.lv], (size_t)b.off + (size_t)b.len);
-    for (size_t l = 0; l < lv_ids.size(); ++l) {
-        h_ids[l].resize(lv_len[l]);
-        if (lv_len[l])
-            CUDA_TRY(cudaMemcpyAsync(h_ids[l].data(), lv_ids[l]->p, lv_len[l] * sizeof(unsigned), cudaMemcpyDeviceToHost,
-                                     st));
-    }
-    CUDA_TRY(cudaStreamSynchronize(st));
+    lists.clear();
+    lists.reserve(tree.leaves.size());
     tree.leaf_meta_off.reserve(tree.leaves.size() + 1);
-    size_t total = 0;
-    for (int32_t l : tree.leaves) total += (size_t)bfs[bfs_of[l]].len;
-    tree.leaf_meta_ids.reserve(total);
     int64_t off = 0;
     for (int32_t l : tree.leaves) {
         const BfsNode &b = bfs[bfs_of[l]];
         tree.leaf_meta_off.push_back(off);
-        const unsigned *src = h_ids[b.lv].data() + b.off;
-        tree.leaf_meta_ids.insert(tree.leaf_meta_ids.end(), src, src + b.len);
+        lists.push_back(LeafList{lv_ids[b.lv] + b.off, off, b.len, 0});
         off += b.len;
     }
     tree.leaf_meta_off.push_back(off);

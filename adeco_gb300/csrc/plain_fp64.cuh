@@ -293,7 +293,7 @@ __device__ __forceinline__ void plain_clip(PlainWarp &W, const GridDesc &g, int 
     }
 }
 
-// item_cube_offset: n_items + 1 offsets of the items' cubes; the launch
+// item_cube_offset: the offsets of the items' cubes; the launch
 // deposits cubes [cube_begin, cube_end), warp_cubes (at most kPlainCubes) a
 // warp at a time.  All items have the same grid.
 __global__ void __launch_bounds__(kPlainThreads) deposit_plain_fp64_kernel(DepositParams P, long long cube_begin,

@@ -252,7 +252,7 @@ int launch_mixed(const DeviceProps &dp, DepositParams P, cudaStream_t st, int ct
 }
 
 // Plain FP64 launch over the cubes of `n_items` items.
-// d_cube_off: n_items+1 cube offsets of the items (device), [c0, c1) their range.
+// d_cube_off: cube offsets of the items (device), [c0, c1) their range.
 int launch_plain(const DeviceProps &dp, DepositParams P, const long long *d_cube_off, long long c0, long long c1,
                  cudaStream_t st)
 {
@@ -645,6 +645,8 @@ extern "C" int adeco_deposit_tets_device(const float *d_positions, size_t positi
 }
 
 // ============================================================ sessions
+#include "octree_device.cuh"
+
 struct adeco_session {
     int device = 0;
     int order = ORDER_REF;
@@ -665,8 +667,8 @@ struct adeco_session {
     bool has_tree = false;
     int leaf_dims = 16;
     std::vector<GridDesc> leaf_grids;
-    std::vector<Item> leaf_items;
-    std::vector<std::vector<int>> leaf_item_ranges;
+    size_t n_items = 0;                 // work items: (leaf, meta-cell), in leaf order
+    std::vector<unsigned> leaf_back;    // the leaves' meta-cell ids, then their cubes, as they come from the device
     DevBuf<Item> d_items;
     DevBuf<GridDesc> d_grids;
     DevBuf<unsigned long long> d_fixed;
@@ -675,8 +677,10 @@ struct adeco_session {
     DevBuf<unsigned long long> d_stats;
     DevBuf<unsigned long long> d_route;  // ill-conditioned tets of a leaf deposit
     unsigned long long route_cap = 0;
-    DevBuf<long long> d_cube_off;
-    std::vector<long long> cube_off;
+    DevBuf<long long> d_cube_off;       // the items' cube offsets within their leaf
+    DevBuf<unsigned> d_leaf_back;
+    DevBuf<unsigned char> d_leaf_lists;
+    std::unique_ptr<TreeWork> tree_work;
     size_t out_values = 0;
     cudaGraphExec_t graph_exec = nullptr;
     cudaGraph_t graph = nullptr;
@@ -765,7 +769,6 @@ static int session_finish(adeco_session &S)
 }
 
 #include "readers.cuh"
-#include "octree_device.cuh"
 
 // Reads `path` into the session's lattice (see readers.cuh).
 static int read_particle_file(adeco_session &S, const char *path, int format, int stride, int periodic, float bbox_out[6])
@@ -981,53 +984,59 @@ extern "C" int adeco_session_build_octree(adeco_session *s, const float *box6, c
     // max_tets_per_node = min(global tets / ranks, parameter) (src/AdDepositWorkFlow.h:169), one rank
     const uint64_t total_tets = 6ull * (uint64_t)(s->nx - 1) * (uint64_t)(s->ny - 1) * (uint64_t)(s->nz - 1);
     const uint64_t max_tets = std::min(total_tets, max_tets_per_node);
+    CUDA_TRY(cudaSetDevice(s->device));
+    int rc;
+    std::vector<LeafList> lists;
     if (s->octree_builder == ADECO_OCTREE_DEVICE) {
-        CUDA_TRY(cudaSetDevice(s->device));
-        const int rc = build_octree_device(s->meta, s->d_meta_bbox.p, box, roi6, max_tets, max_level, s->stream, s->tree);
-        if (rc) return rc;
+        if (!s->tree_work) s->tree_work.reset(new TreeWork());
+        if ((rc = build_octree_device(s->meta, s->d_meta_bbox.p, box, roi6, max_tets, max_level, s->stream, *s->tree_work,
+                                      s->tree, lists)))
+            return rc;
     } else if (!s->tree.build(s->meta, box, roi6, max_tets, max_level)) {
         return fail(ADECO_ERR_LIMIT, "octree generation did not terminate");
     }
     s->leaf_dims = leaf_dims;
-    // per-leaf grids and work items (leaf x meta-cell)
     const size_t nl = s->tree.leaves.size();
     const long long cells = (long long)leaf_dims * leaf_dims * leaf_dims;
+    s->n_items = (size_t)s->tree.leaf_meta_off[nl];
+    s->out_values = nl * (size_t)cells;
+    s->route_cap = route_capacity((long long)s->n_items);
+    if ((rc = s->d_items.reserve(s->n_items)) || (rc = s->d_grids.reserve(nl)) || (rc = s->d_fixed.reserve(s->out_values)) ||
+        (rc = s->d_out.reserve(s->out_values)) || (rc = s->d_cube_off.reserve(s->n_items)) ||
+        (rc = s->d_route.reserve(s->route_cap + 1)) || (rc = s->d_leaf_back.reserve(s->n_items + nl)) ||
+        (rc = s->d_leaf_lists.reserve(nl * sizeof(LeafList))))
+        return rc;
+    if (s->octree_builder != ADECO_OCTREE_DEVICE) {
+        // the host builder's lists go to where the items kernel writes them
+        s->leaf_back.assign(s->tree.leaf_meta_ids.begin(), s->tree.leaf_meta_ids.end());
+        CUDA_TRY(cudaMemcpyAsync(s->d_leaf_back.p, s->leaf_back.data(), s->n_items * sizeof(unsigned), cudaMemcpyHostToDevice,
+                                 s->stream));
+        for (size_t q = 0; q < nl; ++q) {
+            const int64_t m0 = s->tree.leaf_meta_off[q];
+            lists.push_back(LeafList{s->d_leaf_back.p + m0, m0, (int)(s->tree.leaf_meta_off[q + 1] - m0), 0});
+        }
+    }
+    // per-leaf grids here, the work items (leaf x meta-cell) on the device
+    CUDA_TRY(cudaMemcpyAsync(s->d_leaf_lists.p, lists.data(), nl * sizeof(LeafList), cudaMemcpyHostToDevice, s->stream));
+    TreeMeta md;
+    md.nx = s->nx; md.ny = s->ny; md.nz = s->nz;
+    for (int a = 0; a < 3; ++a) md.cd[a] = s->meta.cd[a];
+    leaf_items_kernel<<<(unsigned)nl, kTreeThreads, 0, s->stream>>>(reinterpret_cast<const LeafList *>(s->d_leaf_lists.p), md,
+                                                                    s->d_items.p, s->d_leaf_back.p, s->d_cube_off.p,
+                                                                    s->d_leaf_back.p + s->n_items);
+    CUDA_TRY(cudaGetLastError());
     s->leaf_grids.resize(nl);
-    const size_t n_items = (size_t)s->tree.leaf_meta_off[nl];
-    s->leaf_items.resize(n_items);
-    s->cube_off.resize(n_items + 1);
-    long long cubes = 0;
     for (size_t q = 0; q < nl; ++q) {
         const OctNode &nd = s->tree.nodes[s->tree.leaves[q]];
         const float bb[6] = {nd.min[0], nd.min[0] + nd.ext, nd.min[1], nd.min[1] + nd.ext, nd.min[2], nd.min[2] + nd.ext};
-        const int64_t m0 = s->tree.leaf_meta_off[q], m1 = s->tree.leaf_meta_off[q + 1];
-        const int shift = choose_shift(2058.0 * (double)std::max<int64_t>(1, m1 - m0), s->tet_mass);
+        const int shift = choose_shift(2058.0 * (double)std::max(1, lists[q].len), s->tet_mass);
         s->leaf_grids[q] = make_grid(bb, leaf_dims, s->tet_mass, shift, (long long)q * cells);
-        for (int64_t k = m0; k < m1; ++k) {
-            int org[3], nv[3];
-            s->meta.range(s->tree.leaf_meta_ids[k], org, nv);
-            Item &it = s->leaf_items[k];
-            it.base = org[0] + (long long)s->nx * (org[1] + (long long)s->ny * org[2]);
-            it.grid = (int)q;
-            it.nv = nv[0] | (nv[1] << 8) | (nv[2] << 16);
-            s->cube_off[k] = cubes;
-            cubes += (long long)(nv[0] - 1) * (nv[1] - 1) * (nv[2] - 1);
-        }
     }
-    s->cube_off[n_items] = cubes;
-    int rc;
-    s->out_values = nl * (size_t)cells;
-    s->route_cap = route_capacity((long long)s->leaf_items.size());
-    if ((rc = s->d_items.reserve(s->leaf_items.size())) || (rc = s->d_grids.reserve(nl)) ||
-        (rc = s->d_fixed.reserve(s->out_values)) || (rc = s->d_out.reserve(s->out_values)) ||
-        (rc = s->d_cube_off.reserve(s->cube_off.size())) || (rc = s->d_route.reserve(s->route_cap + 1)))
-        return rc;
-    CUDA_TRY(cudaMemcpyAsync(s->d_items.p, s->leaf_items.data(), s->leaf_items.size() * sizeof(Item),
-                             cudaMemcpyHostToDevice, s->stream));
     CUDA_TRY(cudaMemcpyAsync(s->d_grids.p, s->leaf_grids.data(), nl * sizeof(GridDesc), cudaMemcpyHostToDevice,
                              s->stream));
-    CUDA_TRY(cudaMemcpyAsync(s->d_cube_off.p, s->cube_off.data(), s->cube_off.size() * sizeof(long long),
-                             cudaMemcpyHostToDevice, s->stream));
+    s->leaf_back.resize(s->n_items + nl);
+    CUDA_TRY(cudaMemcpyAsync(s->leaf_back.data(), s->d_leaf_back.p, (s->n_items + nl) * sizeof(unsigned),
+                             cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     s->has_tree = true;
     return ADECO_OK;
@@ -1093,7 +1102,7 @@ extern "C" int adeco_session_leaf_meta(adeco_session *s, int leaf_index, uint64_
     *count = (int)(b - a);
     if (ids) {
         if (capacity < *count) return fail(ADECO_ERR_ARGUMENT, "capacity too small");
-        std::copy(s->tree.leaf_meta_ids.begin() + a, s->tree.leaf_meta_ids.begin() + b, ids);
+        std::copy(s->leaf_back.begin() + a, s->leaf_back.begin() + b, ids);
     }
     return ADECO_OK;
 }
@@ -1102,7 +1111,7 @@ static DepositParams session_params(adeco_session *s, bool stats)
 {
     DepositParams P = base_params(s->tuning);
     P.items = s->d_items.p;
-    P.n_items = (int)s->leaf_items.size();
+    P.n_items = (int)s->n_items;
     P.src_kind = SRC_LATTICE_F4;
     P.grids = s->d_grids.p;
     P.src = s->lattice.p;
@@ -1156,19 +1165,16 @@ extern "C" int adeco_session_deposit_leaves(adeco_session *s, int precision, dou
         CUDA_TRY(cudaEventRecord(e0, s->stream));
         // one launch per leaf (one request per launch)
         DepositParams P = session_params(s, false);
-        size_t item0 = 0;
         for (size_t q = 0; q < s->leaf_grids.size() && !rc; ++q) {
-            size_t item1 = item0;
-            while (item1 < s->leaf_items.size() && s->leaf_items[item1].grid == (int)q) ++item1;
+            const int64_t item0 = s->tree.leaf_meta_off[q];
             DepositParams Q = P;
             Q.items = s->d_items.p + item0;
-            Q.n_items = (int)(item1 - item0);
-            const long long c0 = s->cube_off[item0], c1 = s->cube_off[item1];
-            if (Q.n_items > 0 && c1 > c0) {
-                rc = launch_plain(s->dp, Q, s->d_cube_off.p + item0, c0, c1, s->stream);
+            Q.n_items = (int)(s->tree.leaf_meta_off[q + 1] - item0);
+            const long long cubes = s->leaf_back[s->n_items + q];
+            if (Q.n_items > 0 && cubes > 0) {
+                rc = launch_plain(s->dp, Q, s->d_cube_off.p + item0, 0, cubes, s->stream);
                 ++launches;
             }
-            item0 = item1;
         }
         CUDA_TRY(cudaEventRecord(e1, s->stream));
         CUDA_TRY(cudaEventRecord(e2, s->stream));
@@ -1209,7 +1215,7 @@ extern "C" int adeco_session_deposit_leaves(adeco_session *s, int precision, dou
         timing->kernel_ms = k_ms;
         timing->total_ms = t_ms;
         timing->launches = launches;
-        timing->items = s->leaf_items.size();
+        timing->items = s->n_items;
         timing->routed_tets = routed;
         if (collect_stats) {
             unsigned long long st[kNumStats];
@@ -1272,7 +1278,7 @@ extern "C" int adeco_session_replay_leaves(adeco_session *s, int reps, adeco_tim
         timing->kernel_ms = ms / reps;
         timing->total_ms = ms / reps;
         timing->launches = 3ull * reps;
-        timing->items = s->leaf_items.size();
+        timing->items = s->n_items;
     }
     return ADECO_OK;
 }
