@@ -573,7 +573,7 @@ long long clip_piece_serial(const float p0[12], int done0)
 #ifdef __CUDACC__
 constexpr int kPool = 78;    // pieces per warp pool (2 CTAs of 8 warps fit in an SM's shared memory)
 constexpr int kLast = 88;    // pieces at their last crossed face per warp
-constexpr int kPairs = 1280;  // partial pairs a CTA lists
+constexpr int kPairs = 1152;  // partial pairs a CTA lists
 
 static_assert(kPool >= 32 + 3 && kLast >= 32 + 3, "one split step fits a full pool and list");
 
@@ -588,8 +588,8 @@ struct WarpPool {
 
 // The partial pairs a CTA has listed and their 6x volumes.
 struct PairList {
-    int n;      // pairs listed
-    int next;   // first pair no warp has taken
+    int n[2];     // pairs listed, and the first pair no warp has taken: a list's counters are cleared
+    int next[2];  // while the one before it is clipped, so lists alternate between two sets
     uint32_t cell[kPairs];  // the pair's cell (the caller's encoding)
     uint8_t tet[kPairs];    //   and its tet
     uint32_t vlo[kPairs], vhi[kPairs];  // fixed point 2^kVolShift
@@ -624,14 +624,19 @@ __device__ __forceinline__ void put_last(WarpPool &pool, int slot, const float p
 }
 
 // Clip the CTA's np listed pairs (build(j, p) writes pair j's tet in cell
-// coordinates); every warp takes pairs from the list until none is left.  When
-// all warps are through, list.volume(j) of j < np are the pairs' 6x volumes.
+// coordinates); every warp takes pairs from the list, 32 at a time, until none
+// is left.  A pair's pieces stay with the warp that took it: on return
+// list.volume(j) of this warp's pairs are their 6x volumes.  Returns the 32s
+// it took, a bit each.
 template <typename Build>
-__device__ __forceinline__ void clip_pairs(WarpPool &pool, PairList &list, int np, Build build, unsigned &fallbacks)
+__device__ __forceinline__ uint64_t clip_pairs(WarpPool &pool, PairList &list, int *next, int np, Build build,
+                                               unsigned &fallbacks)
 {
+    static_assert(kPairs <= 64 * 32 && kPool >= 63 && kLast >= 63, "a build step has room for 32 pairs");
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1;
     int top = 0, nlast = 0;
+    uint64_t taken = 0;
     bool more_pairs = np > 0;
     for (;;) {
         if (nlast >= 32 || (nlast && !top && !more_pairs)) {
@@ -649,11 +654,13 @@ __device__ __forceinline__ void clip_pairs(WarpPool &pool, PairList &list, int n
         }
         if (top < 32 && more_pairs) {
             // build step
-            int nb = min(32, min(kPool - top, kLast - nlast)), j = 0;
-            if (lane == 0) j = atomicAdd(&list.next, nb);
+            int j = 0;
+            if (lane == 0) j = atomicAdd(next, 32);
             j = __shfl_sync(0xffffffffu, j, 0);
-            more_pairs = j + nb < np;
-            nb = min(nb, np - j);  // may be <= 0
+            more_pairs = j + 32 < np;
+            if (j >= np) continue;
+            taken |= 1ull << (j >> 5);
+            const int nb = min(32, np - j);
             j += lane;
             bool push = false, last = false;
             float p[12];
@@ -685,7 +692,7 @@ __device__ __forceinline__ void clip_pairs(WarpPool &pool, PairList &list, int n
             __syncwarp();
             continue;
         }
-        if (!top) break;
+        if (!top) return taken;
         // split step: lane l takes slot top - 1 - l
         const int n = min(top, 32), idx = top - 1 - lane;
         int owner = 0;

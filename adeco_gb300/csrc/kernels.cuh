@@ -88,18 +88,17 @@ enum Stat : int {
     kNumStats = 8
 };
 
-// What the classification needs of N tets (structure of arrays in shared
-// memory, the fields as narrow as their ranges allow).
+// What the classification needs of N tets, in 16-byte words of shared memory:
+// it reads 24 numbers of a pair's tet, and a load instruction each had been a
+// tenth of its instructions.
 template <int N>
 struct TetPlanes {
-    float n[4][3][N];   // inward face normals
-    float d[4][N];      // plane offsets n . (face centroid): inside <=> n.x - d > 0
-    float tol[N];       // FP32 error bound of the plane tests (largest face)
-    float bmin[3][N];   // tet AABB in the anchor frame
-    float bmax[3][N];
-    float f6[N];        // mass per unit of 6x clipped volume (tet mass / |6V| in cell units)
-    uint16_t lo[3][N];  // anchor cell (first candidate cell) in grid indices (dims <= 4096)
-    uint16_t ex[3][N];  // candidate extents (cells per axis)
+    float4 plane[4][N];  // inward face normals and plane offsets n . (face centroid): inside <=> n.x - d > 0
+    float4 lower[N];     // tet AABB in the anchor frame, minimum; FP32 error bound of the plane tests (largest face)
+    float4 upper[N];     //   maximum; candidate extents of axes 0 | 1 << 16, as bits
+    float f6[N];         // mass per unit of 6x clipped volume (tet mass / |6V| in cell units)
+    uint16_t lo[3][N];   // anchor cell (first candidate cell) in grid indices (dims <= 4096)
+    uint16_t ex[3][N];   // candidate extents (cells per axis)
 };
 
 // The vertices of up to 32 tets in their anchor cells' frames (cell units).
@@ -166,10 +165,13 @@ struct SharedMixed {
     int n_cubes;
     int item, part;
     GridDesc g;
-    int scan[kWave];     // pairs of the warp's tets before this one
+    // per warp, its tets that have pairs, in order: the tet, and the warp's
+    // pairs before it (INT_MAX past the last)
+    int start[kWave];
+    uint8_t tet[kWave];
     int warp_pairs[kWarps];
     int cursor;          // first candidate pair of the wave not yet taken
-    int wide;            // a tet of the wave has more than 1024 candidate cells along an axis
+    int wide[2];         // a tet of the wave (even, odd) has more than 1024 candidate cells along an axis
     PairList list;
     WarpPool pool[kWarps];  // the set-up's TetVertices use the same memory
 };
@@ -315,7 +317,8 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
 {
     long long cnt0 = 1;
     unsigned cnt = 1;
-    float R = 0.f;
+    float R = 0.f, bmin[3], bmax[3];
+    uint32_t ext01 = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const int top = g.dims - 1;
@@ -351,8 +354,9 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
             R = fmaxf(R, fabsf(qf[q]));
         }
         R = fmaxf(R, (float)(ex - 1) + 1.f);
-        W.bmin[a][t] = fminf(fminf(qf[0], qf[1]), fminf(qf[2], qf[3]));
-        W.bmax[a][t] = fmaxf(fmaxf(qf[0], qf[1]), fmaxf(qf[2], qf[3]));
+        bmin[a] = fminf(fminf(qf[0], qf[1]), fminf(qf[2], qf[3]));
+        bmax[a] = fmaxf(fmaxf(qf[0], qf[1]), fmaxf(qf[2], qf[3]));
+        if (a < 2) ext01 |= (uint32_t)(ex & 0xffff) << (16 * a);
         W.lo[a][t] = (uint16_t)c0;
         W.ex[a][t] = (uint16_t)ex;
     }
@@ -407,8 +411,7 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
         L2 = fmaxf(L2, fmaxf(s1, fmaxf(s2, s3)));
         // n_in = (vb - va) x (vc - va) with the outward order reversed
         const float nn[3] = {e1[1] * e2[2] - e1[2] * e2[1], e1[2] * e2[0] - e1[0] * e2[2], e1[0] * e2[1] - e1[1] * e2[0]};
-#pragma unroll
-        for (int x = 0; x < 3; ++x) W.n[f][x][t] = nn[x];
+        float offset;
         if constexpr (kExactD) {
             float la[3], lb[3], lc[3];
             for (int x = 0; x < 3; ++x) {
@@ -417,18 +420,20 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
                 lc[x] = Q.qlo[3 * fc + x][lane];
             }
             const F2 d = plane_offset(A, la, B, lb, C, lc, nn);
-            W.d[f][t] = d.hi;
+            offset = d.hi;
             if constexpr (Table::kHasRest) W.dlo[f][t] = d.lo;
         } else {
             constexpr float kThird = 1.f / 3.f;
-            W.d[f][t] = (nn[0] * (A[0] + B[0] + C[0]) + nn[1] * (A[1] + B[1] + C[1]) + nn[2] * (A[2] + B[2] + C[2])) * kThird;
+            offset = (nn[0] * (A[0] + B[0] + C[0]) + nn[1] * (A[1] + B[1] + C[1]) + nn[2] * (A[2] + B[2] + C[2])) * kThird;
         }
+        W.plane[f][t] = make_float4(nn[0], nn[1], nn[2], offset);
         const float L1 = fmaxf(fmaxf(fabsf(e1[0]), fabsf(e1[1])), fabsf(e1[2]));
         const float M1 = fmaxf(fmaxf(fabsf(e2[0]), fabsf(e2[1])), fabsf(e2[2]));
         // generous bound on the FP32 rounding of n.x - d (|x| <= R + 1)
         tolmax = fmaxf(tolmax, 1.0e-5f * L1 * M1 * (R + 1.f));
     }
-    W.tol[t] = tolmax;
+    W.lower[t] = make_float4(bmin[0], bmin[1], bmin[2], tolmax);
+    W.upper[t] = make_float4(bmax[0], bmax[1], bmax[2], u2f(ext01));
     // conditioning: longest edge cubed over |6V|, both in cell units.  L^3 <=
     // kappa |6V| squared (both sides non-negative): no square root; NaN or an
     // overflow routes the tet
@@ -503,23 +508,21 @@ ADECO_HD inline int classify_pair(const Table &W, const GridDesc &g, int s, int 
 {
     cross = -1;
     const float fa = (float)a, fb = (float)b, fc = (float)c;
+    const float4 mn = W.lower[s], mx = W.upper[s];
     // strict AABB overlap with the cell [a,a+1] x [b,b+1] x [c,c+1]
-    if (!(W.bmin[0][s] < fa + 1.f && fa < W.bmax[0][s] && W.bmin[1][s] < fb + 1.f && fb < W.bmax[1][s] &&
-          W.bmin[2][s] < fc + 1.f && fc < W.bmax[2][s]))
-        return P_NO;
-    if (W.bmin[0][s] >= fa && W.bmax[0][s] <= fa + 1.f && W.bmin[1][s] >= fb && W.bmax[1][s] <= fb + 1.f &&
-        W.bmin[2][s] >= fc && W.bmax[2][s] <= fc + 1.f)
+    if (!(mn.x < fa + 1.f && fa < mx.x && mn.y < fb + 1.f && fb < mx.y && mn.z < fc + 1.f && fc < mx.z)) return P_NO;
+    if (mn.x >= fa && mx.x <= fa + 1.f && mn.y >= fb && mx.y <= fb + 1.f && mn.z >= fc && mx.z <= fc + 1.f)
         return P_TET_INSIDE;
     bool all_in = true, unsure = false;
     int ncross = 0, fcross = 0;
-    const float t = W.tol[s];
+    const float t = mn.w;
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
-        const float nx = W.n[f][0][s], ny = W.n[f][1][s], nz = W.n[f][2][s];
-        const float base = fmaf(nx, fa, fmaf(ny, fb, fmaf(nz, fc, -W.d[f][s])));
-        const float pos = fmaxf(nx, 0.f) + fmaxf(ny, 0.f) + fmaxf(nz, 0.f);
+        const float4 n = W.plane[f][s];
+        const float base = fmaf(n.x, fa, fmaf(n.y, fb, fmaf(n.z, fc, -n.w)));
+        const float pos = fmaxf(n.x, 0.f) + fmaxf(n.y, 0.f) + fmaxf(n.z, 0.f);
         const float mx = base + pos;
-        const float mn = base + ((nx + ny + nz) - pos);
+        const float mn = base + ((n.x + n.y + n.z) - pos);
         if (mx < -t) return P_NO;
         if (mx <= t) unsure = true;
         if (mn > t) continue;
@@ -548,9 +551,11 @@ template <bool kExactD = true, class Table>
 ADECO_HD inline F2 face_value_at_cell(const Table &W, const GridDesc &g, int s, int a, int b, int c, int f)
 {
     const int cc[3] = {a, b, c};
+    const float4 pl = W.plane[f][s];
+    const float n[3] = {pl.x, pl.y, pl.z};
     F2 G;
     if constexpr (kExactD) {
-        G = {-W.d[f][s], -W.dlo[f][s]};
+        G = {-pl.w, -W.dlo[f][s]};
     } else {  // the exact offset setup_tet<true> would have stored
         const int fa = f == 3 ? 1 : 0, fb = f == 0 ? 2 : (f == 1 ? 3 : (f == 2 ? 1 : 2)),
                   fc = f == 0 ? 1 : (f == 1 ? 2 : 3);
@@ -561,16 +566,15 @@ ADECO_HD inline F2 face_value_at_cell(const Table &W, const GridDesc &g, int s, 
             tet_coord(W, g, s, fb, x, q[1][x], l[1][x]);
             tet_coord(W, g, s, fc, x, q[2][x], l[2][x]);
         }
-        const float n[3] = {W.n[f][0][s], W.n[f][1][s], W.n[f][2][s]};
         const F2 d = plane_offset(q[0], l[0], q[1], l[1], q[2], l[2], n);
         G = {-d.hi, -d.lo};
     }
     float small = 0.f;  // the cells' deviation from unit size: n_x c_x dr_x, tiny
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
-        const float nx = W.n[f][x][s], fc = (float)cc[x];
-        G = f2_add(G, f2_two_prod(nx, fc));
-        small = fmaf(nx * fc, g.drcell[x], small);
+        const float fc = (float)cc[x];
+        G = f2_add(G, f2_two_prod(n[x], fc));
+        small = fmaf(n[x] * fc, g.drcell[x], small);
     }
     return f2_norm(G.hi, G.lo + small);
 }
@@ -585,8 +589,8 @@ inline
 #endif
 float halfspace_pair_vol6(const Table &W, const GridDesc &g, int s, int a, int b, int c, int f)
 {
-    return halfspace_cube_vol6(face_value_at_cell<kExactD>(W, g, s, a, b, c, f), W.n[f][0][s], W.n[f][1][s],
-                               W.n[f][2][s]);
+    const float4 n = W.plane[f][s];
+    return halfspace_cube_vol6(face_value_at_cell<kExactD>(W, g, s, a, b, c, f), n.x, n.y, n.z);
 }
 
 // Non-negative mass of a pair (FP32, about 1e-7 relative) -> the cell's
@@ -628,10 +632,12 @@ template <class Table>
 ADECO_HD inline void piece_coords(const Table &W, const GridDesc &g, int s, int a, int b, int c, float p[12])
 {
     const int cc[3] = {a, b, c};
+    const float4 mn = W.lower[s];
+    const float lower[3] = {mn.x, mn.y, mn.z};
     int nflip = 0;
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
-        const bool flip = W.bmin[x][s] > (float)cc[x];
+        const bool flip = lower[x] > (float)cc[x];
         nflip += flip;
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -655,7 +661,19 @@ ADECO_HD inline void piece_coords(const Table &W, const GridDesc &g, int s, int 
 // cells along an axis, the flattened offset.
 __device__ __forceinline__ int3 flat_cell(const WaveTets &W, int s, int local)
 {
-    const int ex0 = W.ex[0][s], ex1 = W.ex[1][s], r = local / ex0, c = r / ex1;
+    const uint32_t e = __float_as_uint(W.upper[s].w);
+    const int ex0 = (int)(e & 0xffffu), ex1 = (int)(e >> 16);
+    int r, c;
+    if (local < (1 << 20)) {
+        // The quotient of n + 1/2 is at least 1 / (2 ex) away from a whole
+        // number, the product with the approximate reciprocal closer than
+        // n / ex 2^-22 to it: rounding down is exact.
+        r = (int)(((float)local + 0.5f) * rcp_approx((float)ex0));
+        c = (int)(((float)r + 0.5f) * rcp_approx((float)ex1));
+    } else {
+        r = local / ex0;
+        c = r / ex1;
+    }
     return make_int3(local - r * ex0, r - c * ex1, c);
 }
 __device__ __forceinline__ int3 pair_cell(const WaveTets &W, int s, uint32_t e, bool wide)
@@ -688,7 +706,7 @@ __device__ __forceinline__ void route_append(const DepositParams &P, const Share
 // item's live cubes.
 template <bool kExactD>
 __device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &S, const Item &it, int first, int end,
-                                           int vx, int vy, unsigned &n_tets)
+                                           int vx, int vy, int odd, unsigned &n_tets)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slot = threadIdx.x, tid = first + slot;
     int cnt = 0;
@@ -727,7 +745,7 @@ __device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &
                     l = S.wt.gl[a][v];
                 },
                 S.g, reinterpret_cast<TetVertices &>(S.pool[warp]), lane, S.wt, slot, P.error, &route64);
-        if (cnt > 0 && (S.wt.ex[0][slot] > 1024 || S.wt.ex[1][slot] > 1024 || S.wt.ex[2][slot] > 1024)) S.wide = 1;
+        if (cnt > 0 && (S.wt.ex[0][slot] > 1024 || S.wt.ex[1][slot] > 1024 || S.wt.ex[2][slot] > 1024)) S.wide[odd] = 1;
     }
     n_tets += (cnt > 0);
     if (route64 && cnt > 0) {  // deposited by route_fp64_kernel
@@ -742,58 +760,65 @@ __device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &
         const int y = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += y;
     }
-    S.scan[slot] = incl - cnt;
+    const unsigned some = __ballot_sync(0xffffffffu, cnt > 0);
+    if (cnt > 0) {
+        const int k = 32 * warp + __popc(some & ((1u << lane) - 1));
+        S.start[k] = incl - cnt;
+        S.tet[k] = (uint8_t)slot;
+    }
+    if (lane >= __popc(some)) S.start[slot] = INT_MAX;
     if (lane == 31) S.warp_pairs[warp] = incl;
 }
 
 // Classify phase: the warps take the wave's candidate pairs 32 at a time and
 // classify them; inside cells and one-face cells are deposited at once,
 // partial cells listed, until no pair is left or the list might not hold the
-// 32 pairs each warp may have in hand (`room` of it are used).  Returns
-// whether pairs are left.
+// 32 pairs each warp may have in hand (`room` of it are used).
 template <bool kStats>
-__device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixed &S, int total, int room, PairStats &st)
+__device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixed &S, int *list_n, int room, bool wide, PairStats &st)
 {
     const int lane = threadIdx.x & 31;
+    const unsigned le = 0xffffffffu >> (31 - lane);
     const WaveTets &W = S.wt;
     const GridDesc &g = S.g;
-    const bool wide = S.wide != 0;
-    // pairs of the warps' tets before warp `lane`'s
-    int pre = lane < kWarps ? S.warp_pairs[lane] : 0;
-    {
-        const int own = pre;
+    // lane w: warp w's pairs, and the pairs of the warps before it
+    const int own = lane < kWarps ? S.warp_pairs[lane] : 0;
+    int pre = own;
 #pragma unroll
-        for (int o = 1; o < kWarps; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, pre, o);
-            if (lane >= o) pre += y;
-        }
-        pre -= own;
+    for (int o = 1; o < kWarps; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, pre, o);
+        if (lane >= o) pre += y;
     }
+    const int total = __shfl_sync(0xffffffffu, pre, kWarps - 1);
+    pre -= own;
     for (;;) {
         int c0 = 0;
-        if (lane == 0) c0 = *(volatile int *)&S.list.n > room - kThreads ? total : atomicAdd(&S.cursor, 32);
+        if (lane == 0) c0 = *(volatile int *)list_n > room - kThreads ? INT_MAX : atomicAdd(&S.cursor, 32);
         c0 = __shfl_sync(0xffffffffu, c0, 0);
         if (c0 >= total) break;
+        // The pair's tet, without a search per lane: lane k holds the start of
+        // a warp's k-th tet; the last start at or before the first pair, and
+        // the starts among the 32 as a bit mask.  Pairs q0.. of one warp's
+        // tets at a time: most 32s need one round.
         const int pidx = c0 + lane;
-        // the pair's tet: by warps, then in the warp's scan
-        int s = 0, before = 0;
-#pragma unroll
-        for (int step = kWarps / 2; step > 0; step >>= 1) {
-            const int y = __shfl_sync(0xffffffffu, pre, s + step);
-            if (y <= pidx) {
-                s += step;
-                before = y;
+        int s = 0, local = 0;
+        for (int q0 = c0;;) {
+            const int w = __popc(__ballot_sync(0xffffffffu, lane < kWarps && pre <= q0)) - 1;
+            const int before = __shfl_sync(0xffffffffu, pre, w), end = before + __shfl_sync(0xffffffffu, own, w);
+            const int start = S.start[32 * w + lane], rel = q0 - before, at = start - rel + (q0 - c0);
+            const int first = __popc(__ballot_sync(0xffffffffu, start <= rel)) - 1;
+            const unsigned starts = __reduce_or_sync(0xffffffffu, (start > rel && at < 32) ? 1u << at : 0u);
+            const int k = first + __popc(starts & le), from = __shfl_sync(0xffffffffu, start, k);
+            if (pidx >= q0 && pidx < end) {
+                s = S.tet[32 * w + k];
+                local = pidx - before - from;
             }
+            q0 = end;
+            if (q0 >= min(c0 + 32, total)) break;
         }
-        const int in_warp = pidx - before;
-        s *= 32;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1)
-            if (S.scan[s + step] <= in_warp) s += step;
         bool part = false;
         uint32_t entry = 0;
         if (pidx < total) {
-            const int local = in_warp - S.scan[s];
             const int3 c = flat_cell(W, s, local);
             entry = wide ? (uint32_t)local : ((uint32_t)c.x | ((uint32_t)c.y << 10) | ((uint32_t)c.z << 20));
             if (kStats) ++st.cand;
@@ -815,7 +840,7 @@ __device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixe
         }
         const unsigned bal = __ballot_sync(0xffffffffu, part);
         int at = 0;
-        if (lane == 0 && bal) at = atomicAdd(&S.list.n, __popc(bal));
+        if (lane == 0 && bal) at = atomicAdd(list_n, __popc(bal));
         at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1));
         if (part) {
             S.list.cell[at] = entry;
@@ -836,6 +861,8 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
     SharedMixed &S = *reinterpret_cast<SharedMixed *>(smem_raw);
     const int warp = threadIdx.x >> 5;
     PairStats st;
+    int turn = 0, odd = 0;  // the pair list's counters and the wave's flag in use
+    if (threadIdx.x == 0) S.wide[0] = S.list.n[0] = S.list.next[0] = 0;
     const int room = kPairs / kQueue * min(max(P.clip_batch, 64), kQueue);
 
     for (int taken = 0;; ++taken) {
@@ -847,8 +874,6 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
             S.item = unit / P.parts;
             S.part = unit - S.item * P.parts;
             S.n_cubes = 0;
-            S.list.n = 0;
-            S.list.next = 0;
         }
         __syncthreads();
         if (S.item >= P.n_items) break;
@@ -871,43 +896,48 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
         const int ntet = 6 * S.n_cubes;
         const int nwave = (ntet + kWave - 1) / kWave, wave = nwave ? (ntet + nwave - 1) / nwave : 0;
         for (int first = 0; first < ntet; first += wave) {
-            if (threadIdx.x == 0) {
-                S.cursor = 0;
-                S.wide = 0;
-            }
+            // every warp is through with the wave before
+            if (threadIdx.x == 0) S.cursor = S.wide[odd ^ 1] = 0;
+            wave_setup<kExactD>(P, S, it, first, min(first + wave, ntet), vx, vy, odd, st.tets);
             __syncthreads();
-            wave_setup<kExactD>(P, S, it, first, min(first + wave, ntet), vx, vy, st.tets);
-            __syncthreads();
+            const bool wide = S.wide[odd] != 0;
             int total = 0;
 #pragma unroll
             for (int w = 0; w < kWarps; ++w) total += S.warp_pairs[w];
             bool left = total > 0;
+            if (!left) __syncthreads();  // the next wave's set-up writes what this one's warps read above
             while (left) {
-                wave_classify<kStats>(P, S, total, room, st);
+                wave_classify<kStats>(P, S, &S.list.n[turn], room, wide, st);
                 __syncthreads();
                 left = S.cursor < total;
-                const int np = S.list.n;
-                clip_pairs(
-                    S.pool[warp], S.list, np,
+                const int np = S.list.n[turn];
+                if (threadIdx.x == 0) {  // the next list's
+                    S.list.n[turn ^ 1] = 0;
+                    S.list.next[turn ^ 1] = 0;
+                }
+                uint64_t mine = clip_pairs(
+                    S.pool[warp], S.list, &S.list.next[turn], np,
                     [&](int j, float *p) {
                         const int s = S.list.tet[j];
-                        const int3 c = pair_cell(S.wt, s, S.list.cell[j], S.wide != 0);
+                        const int3 c = pair_cell(S.wt, s, S.list.cell[j], wide);
                         piece_coords(S.wt, S.g, s, c.x, c.y, c.z, p);
                     },
                     st.fb);
-                __syncthreads();
-                for (int j = threadIdx.x; j < np; j += kThreads) {
-                    const int s = S.list.tet[j];
-                    const int3 c = pair_cell(S.wt, s, S.list.cell[j], S.wide != 0);
-                    const long long v = S.list.volume(j);
-                    if (v > 0) scatter(P, S.g, S.wt, s, c.x, c.y, c.z, pair_mass(v, S.wt.f6[s]));
+                // the masses of this warp's pairs
+                while (mine) {
+                    const int j = 32 * (__ffsll((long long)mine) - 1) + (threadIdx.x & 31);
+                    mine &= mine - 1;
+                    if (j < np) {
+                        const int s = S.list.tet[j];
+                        const int3 c = pair_cell(S.wt, s, S.list.cell[j], wide);
+                        const long long v = S.list.volume(j);
+                        if (v > 0) scatter(P, S.g, S.wt, s, c.x, c.y, c.z, pair_mass(v, S.wt.f6[s]));
+                    }
                 }
-                if (threadIdx.x == 0) {
-                    S.list.n = 0;
-                    S.list.next = 0;
-                }
+                turn ^= 1;
                 __syncthreads();
             }
+            odd ^= 1;
         }
         __syncthreads();
     }
