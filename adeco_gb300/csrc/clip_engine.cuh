@@ -117,17 +117,20 @@ ADECO_HD inline int face_bits(float x, float y, float z)
 // The cut of a piece by face f, its vertices permuted to A B C D, the k
 // inside ones first by an even permutation (the orientation is kept): the cut
 // points E0..E3 of the four cut edges -- k=1: AB AC AD AD; k=2: AC AD BC BD;
-// k=3: AD BD CD CD -- snapped onto the face.
-ADECO_HD inline void cut_points(const float A[3], const float B[3], const float C[3], const float D[3], int k, int f,
-                                float E[4][3])
+// k=3: AD BD CD CD -- snapped onto the face.  A vertex has N values, its
+// coordinates last; the others (N = 6: barycentric weights) are interpolated
+// with the coordinates' edge parameter.
+template <int N>
+ADECO_HD inline void cut_points(const float *A, const float *B, const float *C, const float *D, int k, int f,
+                                float E[4][N])
 {
     const int axis = f >> 1;
     const float plane = (f & 1) ? 1.f : 0.f;
     const unsigned k1 = bit_mask(k == 1), k2 = bit_mask(k == 2), k3 = bit_mask(k == 3);
     const unsigned a[3] = {bit_mask(axis == 0), bit_mask(axis == 1), bit_mask(axis == 2)};
-    float in[4][3], out[4][3];
+    float in[4][N], out[4][N];
 #pragma unroll
-    for (int x = 0; x < 3; ++x) {
+    for (int x = 0; x < N; ++x) {
         in[0][x] = A[x];
         out[0][x] = bit_sel(k1, B[x], bit_sel(k2, C[x], D[x]));
         in[1][x] = bit_sel(k3, B[x], A[x]);
@@ -139,11 +142,14 @@ ADECO_HD inline void cut_points(const float A[3], const float B[3], const float 
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        const float din = bit_sel(a[0], in[e][0], bit_sel(a[1], in[e][1], in[e][2]));
-        const float dout = bit_sel(a[0], out[e][0], bit_sel(a[1], out[e][1], out[e][2]));
+        const float din = bit_sel(a[0], in[e][N - 3], bit_sel(a[1], in[e][N - 2], in[e][N - 1]));
+        const float dout = bit_sel(a[0], out[e][N - 3], bit_sel(a[1], out[e][N - 2], out[e][N - 1]));
         const float t = sat01((plane - din) * rcp_nr(dout - din));  // |dout - din| > 0 on a crossing edge
 #pragma unroll
-        for (int x = 0; x < 3; ++x) E[e][x] = bit_sel(a[x], plane, fmaf(t, out[e][x] - in[e][x], in[e][x]));
+        for (int x = 0; x < N; ++x) {
+            const float cut = fmaf(t, out[e][x] - in[e][x], in[e][x]);
+            E[e][x] = x < N - 3 ? cut : bit_sel(a[x < N - 3 ? 0 : x - (N - 3)], plane, cut);
+        }
     }
 }
 
@@ -162,15 +168,16 @@ ADECO_HD inline float child_vertex(int child, int v, unsigned k1, unsigned k2, f
     return v == 1 ? bit_sel(k2, E[0], E[1]) : (v == 2 ? bit_sel(k2, E[1], E[2]) : bit_sel(k2, E[3], E[0]));
 }
 
-ADECO_HD inline void split_child(int child, unsigned k1, unsigned k2, const float A[3], const float B[3],
-                                 const float C[3], const float E[4][3], float p[12])
+template <int N>
+ADECO_HD inline void split_child(int child, unsigned k1, unsigned k2, const float *A, const float *B, const float *C,
+                                 const float E[4][N], float *p)
 {
 #pragma unroll
-    for (int x = 0; x < 3; ++x) {
+    for (int x = 0; x < N; ++x) {
         const float e[4] = {E[0][x], E[1][x], E[2][x], E[3][x]};
         p[x] = A[x];
 #pragma unroll
-        for (int v = 1; v < 4; ++v) p[3 * v + x] = child_vertex(child, v, k1, k2, B[x], C[x], e);
+        for (int v = 1; v < 4; ++v) p[N * v + x] = child_vertex(child, v, k1, k2, B[x], C[x], e);
     }
 }
 
@@ -369,7 +376,7 @@ ADECO_HD inline int bary_idx(int v, int i) { return i < 3 ? 3 * v + i : 12 + 3 *
 // vertex is a select between at most three candidates, no lookup.  Returns
 // the number of children (1 or 3).
 template <typename Put>
-ADECO_HD inline int bary_split(const float *r, int f, int mask, Put put)
+inline int bary_split(const float *r, int f, int mask, Put put)
 {
     const int axis = f >> 1;
     const float plane = (f & 1) ? 1.f : 0.f;
@@ -419,16 +426,10 @@ ADECO_HD inline int bary_split(const float *r, int f, int mask, Put put)
     return k1 ? 1 : 3;
 }
 
-
 // The share inside the unit cube of one barycentric piece rec0 whose faces
-// in done0 are already done, clipped serially with a stack.
-ADECO_HD
-#ifdef __CUDA_ARCH__
-__noinline__
-#else
-inline
-#endif
-F2 clip_bary_serial(const float *rec0, int done0)
+// in done0 are already done, clipped serially with a stack: the warp engine's
+// steps, faces, cut points and children, for checks on the host.
+inline F2 clip_bary_serial(const float *rec0, int done0)
 {
     constexpr int kDepth = 16;
     constexpr int kRec = kBaryRec;
@@ -555,14 +556,14 @@ long long clip_piece_serial(const float p0[12], int done0)
         for (int q = 0; q < 4; ++q)
 #pragma unroll
             for (int x = 0; x < 3; ++x) V[q][x] = sel4((pm >> (2 * q)) & 3, p[x], p[3 + x], p[6 + x], p[9 + x]);
-        cut_points(V[0], V[1], V[2], V[3], k, face, E);
+        cut_points<3>(V[0], V[1], V[2], V[3], k, face, E);
         const int n = k == 1 ? 1 : 3;
         if (sp + 3 > kDepth) continue;  // cannot happen (depth <= 2*5 + 3)
         const int d = sdone[sp] | (1 << face);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             if (c >= n) continue;
-            split_child(c, bit_mask(k == 1), bit_mask(k == 2), V[0], V[1], V[2], E, stk[sp]);
+            split_child<3>(c, bit_mask(k == 1), bit_mask(k == 2), V[0], V[1], V[2], E, stk[sp]);
             sdone[sp] = d;
             ++sp;
         }
@@ -587,12 +588,13 @@ struct WarpPool {
 };
 
 // The partial pairs a CTA has listed and their 6x volumes.
-struct PairList {
+template <int kCap>
+struct PairListOf {
     int n[2];     // pairs listed, and the first pair no warp has taken: a list's counters are cleared
     int next[2];  // while the one before it is clipped, so lists alternate between two sets
-    uint32_t cell[kPairs];  // the pair's cell (the caller's encoding)
-    uint8_t tet[kPairs];    //   and its tet
-    uint32_t vlo[kPairs], vhi[kPairs];  // fixed point 2^kVolShift
+    uint32_t cell[kCap];  // the pair's cell (the caller's encoding)
+    uint8_t tet[kCap];    //   and its tet
+    uint32_t vlo[kCap], vhi[kCap];  // fixed point 2^kVolShift
 
     __device__ __forceinline__ long long volume(int j) const
     {
@@ -613,6 +615,7 @@ struct PairList {
         vhi[j] = (uint32_t)((unsigned long long)v >> 32);
     }
 };
+using PairList = PairListOf<kPairs>;
 
 __device__ __forceinline__ void put_last(WarpPool &pool, int slot, const float p[12], float v6, int f, int mask, int owner)
 {
@@ -720,7 +723,7 @@ __device__ __forceinline__ uint64_t clip_pairs(WarpPool &pool, PairList &list, i
                 C[x] = pool.v[3 * ic + x][idx];
                 D[x] = pool.v[3 * id + x][idx];
             }
-            cut_points(A, B, C, D, k, f, E);
+            cut_points<3>(A, B, C, D, k, f, E);
             k1 = bit_mask(k == 1);
             k2 = bit_mask(k == 2);
             const int keep = 63 & ~(done | (1 << f));
@@ -791,7 +794,7 @@ __device__ __forceinline__ uint64_t clip_pairs(WarpPool &pool, PairList &list, i
         for (int c = 0; c < 3; ++c) {
             if (lane < commit && code[c]) {
                 float ch[12];
-                split_child(c, k1, k2, A, B, C, E, ch);
+                split_child<3>(c, k1, k2, A, B, C, E, ch);
                 if (code[c] == 3) {
                     const int slot = top + __popc(sm[c] & lt);
 #pragma unroll
@@ -819,36 +822,39 @@ __device__ __forceinline__ uint64_t clip_pairs(WarpPool &pool, PairList &list, i
 }
 
 // ------------------------------------------- barycentric warp engine
-// clip_pairs for barycentric pieces (kBaryRec floats each): the partial cells
-// of the ill-conditioned tets are listed per warp and clipped with every lane
-// busy, a lane per piece, instead of a lane per cell.  Steps, faces, cut
-// points, children and last-face fractions are clip_bary_serial's; a lane's
-// piece stays in registers (the vertex permutation and the child patterns
-// are selects, not indexed loads).
-constexpr int kBaryPool = 128;  // pieces per warp pool
-constexpr int kBaryList = 64;  // partial cells per warp list
+// clip_pairs for pieces that carry barycentric weights: a vertex has 6 values
+// (3 weights, 3 coordinates), and a piece inside every face is listed like
+// one at its last face, since its share of the tet (bary_share, a
+// double-float determinant) costs as much as a split and would run three
+// times, for a few lanes each, in the split step.
+constexpr int kBaryPool = 66;    // pieces per warp pool
+constexpr int kBaryLast = 66;    // pieces whose share is to be added, per warp
+constexpr int kBaryPairs = 640;  // partial pairs a CTA lists
+
+constexpr int kBaryRoom = kBaryPool - 8;  // what steps of several lanes may fill (see the split step)
+
+static_assert(kBaryRoom >= 32 && kBaryLast >= 31 + 32, "a build step fits");
 
 struct BaryPool {
-    float v[kBaryRec][kBaryPool];
-    uint32_t meta[kBaryPool];  // owner | faces done << 8
-    long long acc[kBaryList];  // share of each listed cell, fixed point 2^kVolShift
-    uint32_t cell[kBaryList];  // the listed cells (the caller's encoding)
+    float v[24][kBaryPool];         // row 6 q + i: vertex q's weights (i = 0..2) and coordinates (3..5)
+    uint32_t flags[kBaryPool];      // the vertices' inside flags, 6 bits each
+    float last[16][kBaryLast];      // weights 3 q + i, then the vertices' coordinate along the last face's axis
+    uint32_t last_meta[kBaryLast];  // inside mask (15: the whole piece) | upper face << 4 | owner << 8
+    uint16_t owner[kBaryPool];      // the piece's pair
 };
 
+using BaryList = PairListOf<kBaryPairs>;
 
-// next_face of a barycentric piece whose faces in `done` are done
-__device__ __forceinline__ int bary_step(const float *r, int done, int &face, int &mask, bool &last)
+__device__ __forceinline__ void put_share(BaryPool &pool, int slot, const float p[24], int f, int mask, int owner)
 {
-    return next_face(face_bits(r[12], r[13], r[14]), face_bits(r[15], r[16], r[17]), face_bits(r[18], r[19], r[20]),
-                     face_bits(r[21], r[22], r[23]), done, face, mask, last);
-}
-
-__device__ __forceinline__ float bary_last_fraction(const float *r, int f, int mask)
-{
-    const int axis = f >> 1;
-    const float plane = (f & 1) ? 1.f : 0.f;
-    return side_fraction(sel3(axis, r[12], r[13], r[14]), sel3(axis, r[15], r[16], r[17]),
-                         sel3(axis, r[18], r[19], r[20]), sel3(axis, r[21], r[22], r[23]), mask, plane);
+    const unsigned ax = bit_mask(f < 2), ay = bit_mask(f < 4);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) pool.last[3 * q + i][slot] = p[6 * q + i];
+        pool.last[12 + q][slot] = bit_sel(ax, p[6 * q + 3], bit_sel(ay, p[6 * q + 4], p[6 * q + 5]));
+    }
+    pool.last_meta[slot] = (uint32_t)(mask | ((f & 1) << 4) | (owner << 8));
 }
 
 __device__ __forceinline__ long long share_fixed(F2 c)
@@ -856,100 +862,186 @@ __device__ __forceinline__ long long share_fixed(F2 c)
     return vol_fixed(c.hi) + vol_fixed(c.lo);
 }
 
-// Clip the warp's np listed cells: build(j, r) writes cell j's piece (the
-// tet in the cell's frame with identity weights).  On return pool.acc[0..np)
-// hold the cells' shares of the tet in fixed point 2^kVolShift.
+// As clip_pairs: build(j, x) writes the coordinates (3 per vertex) of pair
+// j's tet; on return list.volume(j) of this warp's pairs are the cells'
+// shares of the tet in fixed point 2^kVolShift.
 template <typename Build>
-__device__ __forceinline__ void clip_bary_pairs(BaryPool &pool, int np, Build build, unsigned &fallbacks)
+__device__ __forceinline__ uint64_t clip_bary_pairs(BaryPool &pool, BaryList &list, int *next, int np, Build build)
 {
+    static_assert(kBaryPairs <= 64 * 32, "a bit per 32 pairs");
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1;
-    for (int j = lane; j < np; j += 32) pool.acc[j] = 0;
-    __syncwarp();
-    bool valid = false;
-    float r[kBaryRec];
-    int owner = 0, done = 0;  // the piece's cell and its faces done (one bit per face)
-    int top = 0, next = 0;
+    int top = 0, nlast = 0;
+    uint64_t taken = 0;
+    bool more_pairs = np > 0;
     for (;;) {
-        // refill idle lanes: pool first (last in, first out), then the list
-        const unsigned need = __ballot_sync(0xffffffffu, !valid);
-        const int rank = __popc(need & lt), nneed = __popc(need);
-        if (!valid) {
-            if (rank < top) {
-                const int idx = top - 1 - rank;
+        if (nlast >= 32 || (nlast && !top && !more_pairs)) {
+            // the shares of up to 32 pieces, or of their inside parts
+            const int n = min(nlast, 32), idx = nlast - 1 - lane;
+            if (lane < n) {
+                const uint32_t m = pool.last_meta[idx];
+                float w[12];
 #pragma unroll
-                for (int x = 0; x < kBaryRec; ++x) r[x] = pool.v[x][idx];
-                const uint32_t m = pool.meta[idx];
-                owner = (int)(m & 0xff);
-                done = (int)(m >> 8);
-                valid = true;
-            } else {
-                const int j = next + rank - top;
-                if (j < np) {
-                    build(j, r);
-                    owner = j;
-                    done = 0;
-                    valid = true;
-                }
+                for (int i = 0; i < 12; ++i) w[i] = pool.last[i][idx];
+                const F2 c = bary_share(w);
+                const float frac = side_fraction(pool.last[12][idx], pool.last[13][idx], pool.last[14][idx],
+                                                 pool.last[15][idx], m & 15, (m & 16) ? 1.f : 0.f);
+                const F2 cut = f2_mul_f(c, frac);
+                const bool whole = (m & 15) == 15;
+                list.add((int)(m >> 8), share_fixed({whole ? c.hi : cut.hi, whole ? c.lo : cut.lo}));
+            }
+            nlast -= n;
+            __syncwarp();
+            continue;
+        }
+        if (top <= kBaryRoom - 32 && more_pairs) {
+            // build step
+            int j = 0;
+            if (lane == 0) j = atomicAdd(next, 32);
+            j = __shfl_sync(0xffffffffu, j, 0);
+            more_pairs = j + 32 < np;
+            if (j >= np) continue;
+            taken |= 1ull << (j >> 5);
+            const int nb = min(32, np - j);
+            j += lane;
+            float p[24];
+            uint32_t flags = 0;
+            int code = 0, f = 0, mask = 0;
+            bool last = false;
+            if (lane < nb) {
+                float x[12];
+                build(j, x);
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        p[6 * q + i] = q == i + 1 ? 1.f : 0.f;  // the tet itself (bary_identity)
+                        p[6 * q + 3 + i] = x[3 * q + i];
+                    }
+                const int b0 = face_bits(x[0], x[1], x[2]), b1 = face_bits(x[3], x[4], x[5]),
+                          b2 = face_bits(x[6], x[7], x[8]), b3 = face_bits(x[9], x[10], x[11]);
+                flags = (uint32_t)(b0 | (b1 << 6) | (b2 << 12) | (b3 << 18));
+                code = next_face(b0, b1, b2, b3, 0, f, mask, last);
+                list.set(j, 0);
+            }
+            const bool push = code == 2 && !last, share = code == 1 || (code == 2 && last);
+            const unsigned pushing = __ballot_sync(0xffffffffu, push), lasts = __ballot_sync(0xffffffffu, share);
+            if (push) {
+                const int slot = top + __popc(pushing & lt);
+#pragma unroll
+                for (int x = 0; x < 24; ++x) pool.v[x][slot] = p[x];
+                pool.flags[slot] = flags;
+                pool.owner[slot] = (uint16_t)j;
+            }
+            if (share) put_share(pool, nlast + __popc(lasts & lt), p, f, code == 1 ? 15 : mask, j);
+            top += __popc(pushing);
+            nlast += __popc(lasts);
+            __syncwarp();
+            continue;
+        }
+        if (!top) return taken;
+        // split step: lane l takes slot top - 1 - l
+        const int n = min(top, 32), idx = top - 1 - lane;
+        int owner = 0;
+        int code[3] = {0, 0, 0};  // per child: 0 dropped, 1 inside, 2 at its last face, 3 to split further
+        uint32_t cflags[3];
+        int cnext[3];
+        float A[6], B[6], C[6], E[4][6];
+        unsigned k1 = 0, k2 = 0;
+        if (lane < n) {
+            const uint32_t m = pool.flags[idx];
+            owner = pool.owner[idx];
+            const int done = 63 & ~(int)(m | (m >> 6) | (m >> 12) | (m >> 18));
+            int f, mask;
+            bool last;
+            next_face(m & 63, (m >> 6) & 63, (m >> 12) & 63, (m >> 18) & 63, done, f, mask, last);
+            const int pm = split_perm(mask), k = split_kin(mask);
+            const int ia = pm & 3, ib = (pm >> 2) & 3, ic = (pm >> 4) & 3, id = (pm >> 6) & 3;
+            float D[6];
+#pragma unroll
+            for (int x = 0; x < 6; ++x) {
+                A[x] = pool.v[6 * ia + x][idx];
+                B[x] = pool.v[6 * ib + x][idx];
+                C[x] = pool.v[6 * ic + x][idx];
+                D[x] = pool.v[6 * id + x][idx];
+            }
+            cut_points<6>(A, B, C, D, k, f, E);
+            k1 = bit_mask(k == 1);
+            k2 = bit_mask(k == 2);
+            const int keep = 63 & ~(done | (1 << f));
+            const int bA = (int)(m >> (6 * ia)) & keep;
+            const float bB = __int_as_float((int)(m >> (6 * ib)) & keep), bC = __int_as_float((int)(m >> (6 * ic)) & keep);
+            float bE[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) bE[e] = __int_as_float(face_bits(E[e][3], E[e][4], E[e][5]) & keep);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const int b1 = __float_as_int(child_vertex(c, 1, k1, k2, bB, bC, bE)),
+                          b2 = __float_as_int(child_vertex(c, 2, k1, k2, bB, bC, bE)),
+                          b3 = __float_as_int(child_vertex(c, 3, k1, k2, bB, bC, bE));
+                cflags[c] = (uint32_t)(bA | (b1 << 6) | (b2 << 12) | (b3 << 18));
+                cnext[c] = keep & ~(bA & b1 & b2 & b3);  // crossed, or entirely outside
+                const bool out = (keep & ~(bA | b1 | b2 | b3)) != 0 || (c > 0 && k1);
+                code[c] = out ? 0 : (cnext[c] == 0 ? 1 : ((cnext[c] & (cnext[c] - 1)) == 0 ? 2 : 3));
             }
         }
-        const int from_pool = nneed < top ? nneed : top;
-        top -= from_pool;
-        next = min(np, next + (nneed - from_pool));
-        const unsigned held = __ballot_sync(0xffffffffu, valid);
-        if (!held) break;
-        __syncwarp();  // the pool slots just read may be written by this step's pushes
-        // one step, with the main engine's pool reservation: a lane whose two
-        // extra children do not fit keeps its piece for the next round; one
-        // lane clips serially only when every lane holds a piece and none can
-        // move
-        int f = 0, mask = 0, code = 0;
-        bool last = false;
-        if (valid) code = bary_step(r, done, f, mask, last);
-        const bool want_split = valid && code == 2 && !last;
-        const bool push = want_split && split_kin(mask) != 1;
-        const unsigned pushing = __ballot_sync(0xffffffffu, push);
-        const int fit = (kBaryPool - top) >> 1;
-        const int prank = __popc(pushing & lt);
-        const bool defer = push && prank >= fit;
-        const int nfit = min(__popc(pushing), fit);
-        const bool stuck = held == 0xffffffffu && pushing == 0xffffffffu && fit == 0;
-        if (valid && !defer) {
-            F2 c = {0.f, 0.f};
-            if (want_split) {
-                // the children of r: the first replaces r, the others go to
-                // the pool (written after every entry of r has been read)
-                const int base = top + 2 * prank;
-                bary_split(r, f, mask, [&](int ch, int x, float val) {
-                    if (ch == 0) r[x] = val;  // after bary_split's last read of r
-                    else if (push) pool.v[x][base + ch - 1] = val;
-                });
-                done |= 1 << f;
-                if (push) {
-                    const uint32_t m = (uint32_t)owner | ((uint32_t)done << 8);
-                    pool.meta[base] = m;
-                    pool.meta[base + 1] = m;
-                }
-            } else {
-                if (code == 1) c = bary_share(r);
-                if (code == 2) c = f2_mul_f(bary_share(r), bary_last_fraction(r, f, mask));
-                valid = false;
-            }
-            const long long v = share_fixed(c);
-            if (v) atomicAdd(reinterpret_cast<unsigned long long *>(&pool.acc[owner]), (unsigned long long)v);
-        } else if (stuck && lane == 0) {
-            float q[kBaryRec];  // a copy, so that r itself never needs an address (see clip_pairs)
+        unsigned sm[3], lm[3];  // the lanes whose child c goes to the pool / to the share list
+        int ns = 0, nl = 0;
 #pragma unroll
-            for (int x = 0; x < kBaryRec; ++x) q[x] = r[x];
-            atomicAdd(reinterpret_cast<unsigned long long *>(&pool.acc[owner]),
-                      (unsigned long long)share_fixed(clip_bary_serial(q, done)));
-            valid = false;
-            ++fallbacks;
+        for (int c = 0; c < 3; ++c) {
+            sm[c] = __ballot_sync(0xffffffffu, code[c] == 3);
+            lm[c] = __ballot_sync(0xffffffffu, code[c] == 1 || code[c] == 2);
+            ns += __popc(sm[c]);
+            nl += __popc(lm[c]);
         }
-        top += 2 * nfit;
+        // The first lanes whose children fit commit their step, as in
+        // clip_pairs; several lanes fill kBaryRoom of the pool at most.  A
+        // step by one lane always fits: a piece crossing 6 faces leaves at most
+        // 2 pieces pending at each of the 4 splits before its last two, so
+        // clipping it and then its children, last in first out, takes 8 more.
+        int commit = n;
+        if (top - n + ns > kBaryRoom || nlast + nl > kBaryLast) {
+            int s_incl = 0, l_incl = 0;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                s_incl += __popc(sm[c] & (lt << 1 | 1));
+                l_incl += __popc(lm[c] & (lt << 1 | 1));
+            }
+            const unsigned bad = __ballot_sync(0xffffffffu, lane > 0 && lane < n && (top - (lane + 1) + s_incl > kBaryRoom ||
+                                                                                     nlast + l_incl > kBaryLast));
+            if (bad) commit = __ffs(bad) - 1;
+            const unsigned cm = commit < 32 ? (1u << commit) - 1 : 0xffffffffu;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                sm[c] &= cm;
+                lm[c] &= cm;
+            }
+        }
+        top -= commit;
+        __syncwarp();  // every lane has read its slot
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if (lane < commit && code[c]) {
+                float ch[24];
+                split_child<6>(c, k1, k2, A, B, C, E, ch);
+                if (code[c] == 3) {
+                    const int slot = top + __popc(sm[c] & lt);
+#pragma unroll
+                    for (int x = 0; x < 24; ++x) pool.v[x][slot] = ch[x];
+                    pool.flags[slot] = cflags[c];
+                    pool.owner[slot] = (uint16_t)owner;
+                } else {
+                    const int f = 31 - __clz(cnext[c] | 1);
+                    const uint32_t t = cflags[c] >> f;
+                    const int mask = (int)((t & 1) | ((t >> 5) & 2) | ((t >> 10) & 4) | ((t >> 15) & 8));
+                    put_share(pool, nlast + __popc(lm[c] & lt), ch, f, code[c] == 1 ? 15 : mask, owner);
+                }
+            }
+            top += __popc(sm[c]);
+            nlast += __popc(lm[c]);
+        }
         __syncwarp();
     }
-    __syncwarp();
 }
 #endif
 
