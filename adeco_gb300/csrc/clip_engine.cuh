@@ -572,6 +572,47 @@ long long clip_piece_serial(const float p0[12], int done0)
 }
 
 #ifdef __CUDACC__
+// The warp engines hold a piece's inside flags as a byte per vertex (6 bits
+// each): what holds for all or any of the vertices comes from two steps over
+// the word, a vertex order is one byte permutation, and so are the flags of a
+// child, whose vertices are picked from two words by its case.
+__device__ __forceinline__ unsigned pack_flags(int b0, int b1, int b2, int b3)
+{
+    return (unsigned)(b0 + 256 * b1) + 65536u * (unsigned)(b2 + 256 * b3);
+}
+__device__ __forceinline__ int flags_all(unsigned m)  // in bits 0..5
+{
+    const unsigned a = m & (m >> 16);
+    return (int)(a & (a >> 8));
+}
+__device__ __forceinline__ int flags_any(unsigned m)
+{
+    const unsigned o = m | (m >> 16);
+    return (int)(o | (o >> 8));
+}
+// The vertices' flags of face f as a 4-bit mask: bits 0, 8, 16, 24 of m >> f
+// moved to 28..31 (no two products of the multiplication meet below).
+__device__ __forceinline__ int flags_mask(unsigned m, int f)
+{
+    return (int)((((m >> f) & 0x01010101u) * 0x10204080u) >> 28);
+}
+// next_face's choice for a piece of which the faces in `next` (not 0) are crossed
+__device__ __forceinline__ int flags_face(unsigned m, int next)
+{
+    const unsigned a = m & (m >> 16), o = m | (m >> 16), x = m ^ (m >> 16);
+    const int odd = (int)(x ^ (x >> 8));
+    const int two = (int)(a | (a >> 8) | (o & (o >> 8)));
+    const int one_in = next & odd & ~two, two_in = next & ~odd;
+    const int pick = one_in ? one_in : (two_in ? two_in : next);
+    return 31 - __clz(pick & -pick);
+}
+// child_vertex as byte selectors: bytes 0..2 are A B C, bytes 4..7 E0..E3
+__device__ __forceinline__ unsigned child_bytes(int child, unsigned k1, unsigned k2)
+{
+    if (child == 0) return k1 ? 0x6540u : (k2 ? 0x7610u : 0x6210u);
+    return child == 1 ? (k2 ? 0x7460u : 0x5610u) : (k2 ? 0x7540u : 0x4650u);
+}
+
 constexpr int kPool = 78;    // pieces per warp pool (2 CTAs of 8 warps fit in an SM's shared memory)
 constexpr int kLast = 88;    // pieces at their last crossed face per warp
 constexpr int kPairs = 1152;  // partial pairs a CTA lists
@@ -581,7 +622,7 @@ static_assert(kPool >= 32 + 3 && kLast >= 32 + 3, "one split step fits a full po
 struct WarpPool {
     float v[12][kPool];         // the pieces' coordinates, a row per coordinate: a lane's four vertices come in
                                 // any order by their addresses, without a bank conflict
-    uint32_t flags[kPool];      // the vertices' inside flags, 6 bits each
+    uint32_t flags[kPool];      // the vertices' inside flags, a byte each
     uint16_t owner[kPool];      // the piece's pair
     float last[5][kLast];       // pieces at their last face: 6x volume, the vertices' coordinate along its axis
     uint32_t last_meta[kLast];  // inside mask | upper face << 4 | owner << 8
@@ -674,11 +715,17 @@ __device__ __forceinline__ uint64_t clip_pairs(WarpPool &pool, PairList &list, i
                 build(j, p);
                 const int b0 = face_bits(p[0], p[1], p[2]), b1 = face_bits(p[3], p[4], p[5]),
                           b2 = face_bits(p[6], p[7], p[8]), b3 = face_bits(p[9], p[10], p[11]);
-                flags = (uint32_t)(b0 | (b1 << 6) | (b2 << 12) | (b3 << 18));
-                const int code = next_face(b0, b1, b2, b3, 0, f, mask, last);
-                push = code == 2 && !last;
-                last = code == 2 && last;
-                if (code == 1) v = vol_fixed(piece_vol6(p));
+                flags = pack_flags(b0, b1, b2, b3);
+                const int next = 63 & ~flags_all(flags);  // crossed, or entirely outside
+                if ((63 & ~flags_any(flags)) == 0) {
+                    push = (next & (next - 1)) != 0;
+                    last = next && !push;
+                    if (last) {
+                        f = 31 - __clz(next);
+                        mask = flags_mask(flags, f);
+                    }
+                    if (next == 0) v = vol_fixed(piece_vol6(p));
+                }
                 list.set(j, v);
             }
             const unsigned pushing = __ballot_sync(0xffffffffu, push), lasts = __ballot_sync(0xffffffffu, last);
@@ -709,10 +756,8 @@ __device__ __forceinline__ uint64_t clip_pairs(WarpPool &pool, PairList &list, i
             // piece can have (the piece would lie outside it): no done set is kept.
             const uint32_t m = pool.flags[idx];
             owner = pool.owner[idx];
-            const int done = 63 & ~(int)(m | (m >> 6) | (m >> 12) | (m >> 18));
-            int f, mask;
-            bool last;
-            next_face(m & 63, (m >> 6) & 63, (m >> 12) & 63, (m >> 18) & 63, done, f, mask, last);
+            const int left = 63 & flags_any(m);
+            const int f = flags_face(m, left & ~flags_all(m)), mask = flags_mask(m, f);
             const int pm = split_perm(mask), k = split_kin(mask);
             const int ia = pm & 3, ib = (pm >> 2) & 3, ic = (pm >> 4) & 3, id = (pm >> 6) & 3;
             float D[3];
@@ -726,20 +771,18 @@ __device__ __forceinline__ uint64_t clip_pairs(WarpPool &pool, PairList &list, i
             cut_points<3>(A, B, C, D, k, f, E);
             k1 = bit_mask(k == 1);
             k2 = bit_mask(k == 2);
-            const int keep = 63 & ~(done | (1 << f));
-            const int bA = (int)(m >> (6 * ia)) & keep;
-            const float bB = __int_as_float((int)(m >> (6 * ib)) & keep), bC = __int_as_float((int)(m >> (6 * ic)) & keep);
-            float bE[4];
+            const int keep = left & ~(1 << f);
+            const unsigned keep4 = 0x01010101u * (unsigned)keep;
+            const unsigned wV = __byte_perm(m & keep4, 0, ia + 16 * ib + 256 * ic);  // bytes A B C
+            unsigned bE[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) bE[e] = __int_as_float(face_bits(E[e][0], E[e][1], E[e][2]) & keep);
+            for (int e = 0; e < 4; ++e) bE[e] = (unsigned)face_bits(E[e][0], E[e][1], E[e][2]);
+            const unsigned wE = pack_flags(bE[0], bE[1], bE[2], bE[3]) & keep4;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const int b1 = __float_as_int(child_vertex(c, 1, k1, k2, bB, bC, bE)),
-                          b2 = __float_as_int(child_vertex(c, 2, k1, k2, bB, bC, bE)),
-                          b3 = __float_as_int(child_vertex(c, 3, k1, k2, bB, bC, bE));
-                cflags[c] = (uint32_t)(bA | (b1 << 6) | (b2 << 12) | (b3 << 18));
-                cnext[c] = keep & ~(bA & b1 & b2 & b3);  // crossed, or entirely outside
-                const bool out = (keep & ~(bA | b1 | b2 | b3)) != 0 || (c > 0 && k1);
+                cflags[c] = __byte_perm(wV, wE, child_bytes(c, k1, k2));
+                cnext[c] = keep & ~flags_all(cflags[c]);  // crossed, or entirely outside
+                const bool out = (keep & ~flags_any(cflags[c])) != 0 || (c > 0 && k1);
                 code[c] = out ? 0 : (cnext[c] == 0 ? 1 : ((cnext[c] & (cnext[c] - 1)) == 0 ? 2 : 3));
             }
         }
@@ -779,7 +822,7 @@ __device__ __forceinline__ uint64_t clip_pairs(WarpPool &pool, PairList &list, i
 #pragma unroll
                     for (int x = 0; x < 12; ++x) q[x] = pool.v[x][idx];
                     const uint32_t m = pool.flags[idx];
-                    list.add(owner, clip_piece_serial(q, 63 & ~(int)(m | (m >> 6) | (m >> 12) | (m >> 18))));
+                    list.add(owner, clip_piece_serial(q, 63 & ~flags_any(m)));
                     ++fallbacks;
                 }
                 --top;
@@ -807,9 +850,7 @@ __device__ __forceinline__ uint64_t clip_pairs(WarpPool &pool, PairList &list, i
                         v += vol_fixed(v6);
                     } else {
                         const int f = 31 - __clz(cnext[c]);
-                        const uint32_t t = cflags[c] >> f;
-                        const int mask = (int)((t & 1) | ((t >> 5) & 2) | ((t >> 10) & 4) | ((t >> 15) & 8));
-                        put_last(pool, nlast + __popc(lm[c] & lt), ch, v6, f, mask, owner);
+                        put_last(pool, nlast + __popc(lm[c] & lt), ch, v6, f, flags_mask(cflags[c], f), owner);
                     }
                 }
             }
@@ -837,7 +878,7 @@ static_assert(kBaryRoom >= 32 && kBaryLast >= 31 + 32, "a build step fits");
 
 struct BaryPool {
     float v[24][kBaryPool];         // row 6 q + i: vertex q's weights (i = 0..2) and coordinates (3..5)
-    uint32_t flags[kBaryPool];      // the vertices' inside flags, 6 bits each
+    uint32_t flags[kBaryPool];      // the vertices' inside flags, a byte each
     float last[16][kBaryLast];      // weights 3 q + i, then the vertices' coordinate along the last face's axis
     uint32_t last_meta[kBaryLast];  // inside mask (15: the whole piece) | upper face << 4 | owner << 8
     uint16_t owner[kBaryPool];      // the piece's pair
@@ -906,8 +947,8 @@ __device__ __forceinline__ uint64_t clip_bary_pairs(BaryPool &pool, BaryList &li
             j += lane;
             float p[24];
             uint32_t flags = 0;
-            int code = 0, f = 0, mask = 0;
-            bool last = false;
+            int f = 0, mask = 0;
+            bool push = false, share = false;
             if (lane < nb) {
                 float x[12];
                 build(j, x);
@@ -920,11 +961,16 @@ __device__ __forceinline__ uint64_t clip_bary_pairs(BaryPool &pool, BaryList &li
                     }
                 const int b0 = face_bits(x[0], x[1], x[2]), b1 = face_bits(x[3], x[4], x[5]),
                           b2 = face_bits(x[6], x[7], x[8]), b3 = face_bits(x[9], x[10], x[11]);
-                flags = (uint32_t)(b0 | (b1 << 6) | (b2 << 12) | (b3 << 18));
-                code = next_face(b0, b1, b2, b3, 0, f, mask, last);
+                flags = pack_flags(b0, b1, b2, b3);
+                const int next = 63 & ~flags_all(flags);  // crossed, or entirely outside
+                if ((63 & ~flags_any(flags)) == 0) {
+                    push = (next & (next - 1)) != 0;
+                    share = !push;
+                    f = 31 - __clz(next | 1);
+                    mask = next ? flags_mask(flags, f) : 15;
+                }
                 list.set(j, 0);
             }
-            const bool push = code == 2 && !last, share = code == 1 || (code == 2 && last);
             const unsigned pushing = __ballot_sync(0xffffffffu, push), lasts = __ballot_sync(0xffffffffu, share);
             if (push) {
                 const int slot = top + __popc(pushing & lt);
@@ -933,7 +979,7 @@ __device__ __forceinline__ uint64_t clip_bary_pairs(BaryPool &pool, BaryList &li
                 pool.flags[slot] = flags;
                 pool.owner[slot] = (uint16_t)j;
             }
-            if (share) put_share(pool, nlast + __popc(lasts & lt), p, f, code == 1 ? 15 : mask, j);
+            if (share) put_share(pool, nlast + __popc(lasts & lt), p, f, mask, j);
             top += __popc(pushing);
             nlast += __popc(lasts);
             __syncwarp();
@@ -951,10 +997,8 @@ __device__ __forceinline__ uint64_t clip_bary_pairs(BaryPool &pool, BaryList &li
         if (lane < n) {
             const uint32_t m = pool.flags[idx];
             owner = pool.owner[idx];
-            const int done = 63 & ~(int)(m | (m >> 6) | (m >> 12) | (m >> 18));
-            int f, mask;
-            bool last;
-            next_face(m & 63, (m >> 6) & 63, (m >> 12) & 63, (m >> 18) & 63, done, f, mask, last);
+            const int left = 63 & flags_any(m);
+            const int f = flags_face(m, left & ~flags_all(m)), mask = flags_mask(m, f);
             const int pm = split_perm(mask), k = split_kin(mask);
             const int ia = pm & 3, ib = (pm >> 2) & 3, ic = (pm >> 4) & 3, id = (pm >> 6) & 3;
             float D[6];
@@ -968,20 +1012,18 @@ __device__ __forceinline__ uint64_t clip_bary_pairs(BaryPool &pool, BaryList &li
             cut_points<6>(A, B, C, D, k, f, E);
             k1 = bit_mask(k == 1);
             k2 = bit_mask(k == 2);
-            const int keep = 63 & ~(done | (1 << f));
-            const int bA = (int)(m >> (6 * ia)) & keep;
-            const float bB = __int_as_float((int)(m >> (6 * ib)) & keep), bC = __int_as_float((int)(m >> (6 * ic)) & keep);
-            float bE[4];
+            const int keep = left & ~(1 << f);
+            const unsigned keep4 = 0x01010101u * (unsigned)keep;
+            const unsigned wV = __byte_perm(m & keep4, 0, ia + 16 * ib + 256 * ic);  // bytes A B C
+            unsigned bE[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) bE[e] = __int_as_float(face_bits(E[e][3], E[e][4], E[e][5]) & keep);
+            for (int e = 0; e < 4; ++e) bE[e] = (unsigned)face_bits(E[e][3], E[e][4], E[e][5]);
+            const unsigned wE = pack_flags(bE[0], bE[1], bE[2], bE[3]) & keep4;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const int b1 = __float_as_int(child_vertex(c, 1, k1, k2, bB, bC, bE)),
-                          b2 = __float_as_int(child_vertex(c, 2, k1, k2, bB, bC, bE)),
-                          b3 = __float_as_int(child_vertex(c, 3, k1, k2, bB, bC, bE));
-                cflags[c] = (uint32_t)(bA | (b1 << 6) | (b2 << 12) | (b3 << 18));
-                cnext[c] = keep & ~(bA & b1 & b2 & b3);  // crossed, or entirely outside
-                const bool out = (keep & ~(bA | b1 | b2 | b3)) != 0 || (c > 0 && k1);
+                cflags[c] = __byte_perm(wV, wE, child_bytes(c, k1, k2));
+                cnext[c] = keep & ~flags_all(cflags[c]);  // crossed, or entirely outside
+                const bool out = (keep & ~flags_any(cflags[c])) != 0 || (c > 0 && k1);
                 code[c] = out ? 0 : (cnext[c] == 0 ? 1 : ((cnext[c] & (cnext[c] - 1)) == 0 ? 2 : 3));
             }
         }
@@ -1032,9 +1074,7 @@ __device__ __forceinline__ uint64_t clip_bary_pairs(BaryPool &pool, BaryList &li
                     pool.owner[slot] = (uint16_t)owner;
                 } else {
                     const int f = 31 - __clz(cnext[c] | 1);
-                    const uint32_t t = cflags[c] >> f;
-                    const int mask = (int)((t & 1) | ((t >> 5) & 2) | ((t >> 10) & 4) | ((t >> 15) & 8));
-                    put_share(pool, nlast + __popc(lm[c] & lt), ch, f, code[c] == 1 ? 15 : mask, owner);
+                    put_share(pool, nlast + __popc(lm[c] & lt), ch, f, code[c] == 1 ? 15 : flags_mask(cflags[c], f), owner);
                 }
             }
             top += __popc(sm[c]);
