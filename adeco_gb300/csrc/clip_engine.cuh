@@ -140,6 +140,29 @@ ADECO_HD inline void cut_points(const float *A, const float *B, const float *C, 
         in[3][x] = bit_sel(k2, B[x], bit_sel(k3, C[x], A[x]));
         out[3][x] = D[x];
     }
+#ifdef __CUDA_ARCH__
+    // two edges at a time; with r the approximate reciprocal of din - dout, that is
+    // minus the one of dout - din, the same steps as below: t = (din - plane) (r + r (1 + (dout - din) r))
+#pragma unroll
+    for (int e = 0; e < 4; e += 2) {
+        float2 din, dout;
+        din.x = bit_sel(a[0], in[e][N - 3], bit_sel(a[1], in[e][N - 2], in[e][N - 1]));
+        din.y = bit_sel(a[0], in[e + 1][N - 3], bit_sel(a[1], in[e + 1][N - 2], in[e + 1][N - 1]));
+        dout.x = bit_sel(a[0], out[e][N - 3], bit_sel(a[1], out[e][N - 2], out[e][N - 1]));
+        dout.y = bit_sel(a[0], out[e + 1][N - 3], bit_sel(a[1], out[e + 1][N - 2], out[e + 1][N - 1]));
+        const float2 d = sub2(dout, din);
+        const float2 r = make_float2(rcp_approx(-d.x), rcp_approx(-d.y));
+        const float2 q = fma2(r, fma2(d, r, both(1.f)), r), num = add2(din, both(-plane));
+        const float2 t = make_float2(sat01(num.x * q.x), sat01(num.y * q.y));
+#pragma unroll
+        for (int x = 0; x < N; ++x) {
+            const float2 i = make_float2(in[e][x], in[e + 1][x]);
+            const float2 cut = fma2(t, sub2(make_float2(out[e][x], out[e + 1][x]), i), i);
+            E[e][x] = x < N - 3 ? cut.x : bit_sel(a[x < N - 3 ? 0 : x - (N - 3)], plane, cut.x);
+            E[e + 1][x] = x < N - 3 ? cut.y : bit_sel(a[x < N - 3 ? 0 : x - (N - 3)], plane, cut.y);
+        }
+    }
+#else
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const float din = bit_sel(a[0], in[e][N - 3], bit_sel(a[1], in[e][N - 2], in[e][N - 1]));
@@ -151,6 +174,7 @@ ADECO_HD inline void cut_points(const float *A, const float *B, const float *C, 
             E[e][x] = x < N - 3 ? cut : bit_sel(a[x < N - 3 ? 0 : x - (N - 3)], plane, cut);
         }
     }
+#endif
 }
 
 // Inside part of a cut piece as 1 or 3 positively oriented pieces, child
@@ -580,6 +604,29 @@ __device__ __forceinline__ unsigned pack_flags(int b0, int b1, int b2, int b3)
 {
     return (unsigned)(b0 + 256 * b1) + 65536u * (unsigned)(b2 + 256 * b3);
 }
+// face_bits of two points
+__device__ __forceinline__ void face_bits2(const float *p, const float *q, int &bp, int &bq)
+{
+    unsigned b = 0, c = 0;
+#pragma unroll
+    for (int a = 2; a >= 0; --a) {
+        const float2 x = make_float2(p[a], q[a]), m1 = both(-1.f);
+        const float2 up = add2(x, m1), lo = fma2(x, m1, both(0.f));
+        b = __funnelshift_l(__float_as_uint(up.x), b, 1);
+        b = __funnelshift_l(__float_as_uint(lo.x), b, 1);
+        c = __funnelshift_l(__float_as_uint(up.y), c, 1);
+        c = __funnelshift_l(__float_as_uint(lo.y), c, 1);
+    }
+    bp = (int)b;
+    bq = (int)c;
+}
+__device__ __forceinline__ unsigned face_flags(const float *p0, const float *p1, const float *p2, const float *p3)
+{
+    int b0, b1, b2, b3;
+    face_bits2(p0, p1, b0, b1);
+    face_bits2(p2, p3, b2, b3);
+    return pack_flags(b0, b1, b2, b3);
+}
 __device__ __forceinline__ int flags_all(unsigned m)  // in bits 0..5
 {
     const unsigned a = m & (m >> 16);
@@ -713,9 +760,7 @@ __device__ __forceinline__ uint64_t clip_pairs(WarpPool &pool, PairList &list, i
             long long v = 0;
             if (lane < nb) {
                 build(j, p);
-                const int b0 = face_bits(p[0], p[1], p[2]), b1 = face_bits(p[3], p[4], p[5]),
-                          b2 = face_bits(p[6], p[7], p[8]), b3 = face_bits(p[9], p[10], p[11]);
-                flags = pack_flags(b0, b1, b2, b3);
+                flags = face_flags(p, p + 3, p + 6, p + 9);
                 const int next = 63 & ~flags_all(flags);  // crossed, or entirely outside
                 if ((63 & ~flags_any(flags)) == 0) {
                     push = (next & (next - 1)) != 0;
@@ -774,10 +819,7 @@ __device__ __forceinline__ uint64_t clip_pairs(WarpPool &pool, PairList &list, i
             const int keep = left & ~(1 << f);
             const unsigned keep4 = 0x01010101u * (unsigned)keep;
             const unsigned wV = __byte_perm(m & keep4, 0, ia + 16 * ib + 256 * ic);  // bytes A B C
-            unsigned bE[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) bE[e] = (unsigned)face_bits(E[e][0], E[e][1], E[e][2]);
-            const unsigned wE = pack_flags(bE[0], bE[1], bE[2], bE[3]) & keep4;
+            const unsigned wE = face_flags(E[0], E[1], E[2], E[3]) & keep4;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 cflags[c] = __byte_perm(wV, wE, child_bytes(c, k1, k2));
@@ -959,9 +1001,7 @@ __device__ __forceinline__ uint64_t clip_bary_pairs(BaryPool &pool, BaryList &li
                         p[6 * q + i] = q == i + 1 ? 1.f : 0.f;  // the tet itself (bary_identity)
                         p[6 * q + 3 + i] = x[3 * q + i];
                     }
-                const int b0 = face_bits(x[0], x[1], x[2]), b1 = face_bits(x[3], x[4], x[5]),
-                          b2 = face_bits(x[6], x[7], x[8]), b3 = face_bits(x[9], x[10], x[11]);
-                flags = pack_flags(b0, b1, b2, b3);
+                flags = face_flags(x, x + 3, x + 6, x + 9);
                 const int next = 63 & ~flags_all(flags);  // crossed, or entirely outside
                 if ((63 & ~flags_any(flags)) == 0) {
                     push = (next & (next - 1)) != 0;
@@ -1015,10 +1055,7 @@ __device__ __forceinline__ uint64_t clip_bary_pairs(BaryPool &pool, BaryList &li
             const int keep = left & ~(1 << f);
             const unsigned keep4 = 0x01010101u * (unsigned)keep;
             const unsigned wV = __byte_perm(m & keep4, 0, ia + 16 * ib + 256 * ic);  // bytes A B C
-            unsigned bE[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) bE[e] = (unsigned)face_bits(E[e][3], E[e][4], E[e][5]);
-            const unsigned wE = pack_flags(bE[0], bE[1], bE[2], bE[3]) & keep4;
+            const unsigned wE = face_flags(E[0] + 3, E[1] + 3, E[2] + 3, E[3] + 3) & keep4;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 cflags[c] = __byte_perm(wV, wE, child_bytes(c, k1, k2));

@@ -156,6 +156,15 @@ __device__ __forceinline__ void tet_coord(const WaveTets &W, const GridDesc &g, 
     shift_frame(W.gh[x][i], W.gl[x][i], W.lo[x][s], g.drcell[x], hi, lo);
 }
 
+// the same of vertices v and v + 1
+__device__ __forceinline__ void tet_coord2(const WaveTets &W, const GridDesc &g, int s, int v, int x, float2 &hi, float2 &lo)
+{
+    const ushort4 id = W.vid[s];
+    const int i = v == 0 ? id.x : id.z, j = v == 0 ? id.y : id.w;
+    shift_frame2(make_float2(W.gh[x][i], W.gh[x][j]), make_float2(W.gl[x][i], W.gl[x][j]), (float)W.lo[x][s], g.drcell[x],
+                 hi, lo);
+}
+
 struct SharedMixed {
     WaveTets wt;
     uint2 range[kMaxVerts];   // the staged vertices' candidate cells and box flags (vertex_range)
@@ -639,6 +648,19 @@ ADECO_HD inline void piece_coords(const Table &W, const GridDesc &g, int s, int 
     for (int x = 0; x < 3; ++x) {
         const bool flip = lower[x] > (float)cc[x];
         nflip += flip;
+#ifdef __CUDA_ARCH__
+        if constexpr (!Table::kHasRest) {  // two vertices at a time
+            float2 hi, lo;
+#pragma unroll
+            for (int v = 0; v < 4; v += 2) {
+                tet_coord2(W, g, s, v, x, hi, lo);
+                const float2 c2 = cell_coord_fast2(hi, lo, cc[x], g.drcell[x], flip);
+                p[3 * v + x] = c2.x;
+                p[3 * v + 3 + x] = c2.y;
+            }
+            continue;
+        }
+#endif
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
             float hi, lo;
