@@ -93,7 +93,10 @@ enum Stat : int {
 // tenth of its instructions.
 template <int N>
 struct TetPlanes {
-    float4 plane[4][N];  // inward face normals and plane offsets n . (face centroid): inside <=> n.x - d > 0
+    // inward face normals n and plane offsets d = n . (face centroid): inside
+    // <=> n.x - d > 0.  Two faces at a time: (nx ny) of faces 0 and 1, (nz -d) of
+    // them, then faces 2 and 3
+    float4 plane[4][N];
     float4 lower[N];     // tet AABB in the anchor frame, minimum; FP32 error bound of the plane tests (largest face)
     float4 upper[N];     //   maximum; candidate extents of axes 0 | 1 << 16, as bits
     float f6[N];         // mass per unit of 6x clipped volume (tet mass / |6V| in cell units)
@@ -182,9 +185,8 @@ struct SharedMixed {
     int cursor;          // first candidate pair of the wave not yet taken
     int wide[2];         // a tet of the wave (even, odd) has more than 1024 candidate cells along an axis
     PairList list;
-    WarpPool pool[kWarps];  // the set-up's TetVertices use the same memory
+    WarpPool pool[kWarps];
 };
-static_assert(sizeof(TetVertices) <= sizeof(WarpPool), "the set-up's vertices share the pool");
 
 __device__ __forceinline__ void stat_add(unsigned long long *stats, int which, unsigned long long v)
 {
@@ -306,12 +308,8 @@ ADECO_HD inline F2 plane_offset(const float qa[3], const float la[3], const floa
 // Entry t of table W from the grid-frame coordinates of a tet's vertices,
 // ordered by the orientation rule (frame(q, a, hi, lo): vertex q, axis a), and
 // its candidate cells as vertex_range words (mn / mx: the least and the
-// greatest of its vertices); its vertices in the anchor frame go to Q's entry
-// `lane`.  Returns the candidate pair count (0 if the tet is skipped).
-//
-// The loops over axes, cofactors and faces are not unrolled: code size (the
-// instruction cache holds about 32 KB: a loop of that size issues at 0.87 of
-// the peak, one of 48 KB at 0.5).
+// greatest of its vertices).  Returns the candidate pair count (0 if the tet
+// is skipped).
 //
 // kExactD: each face's plane offset in double-float, rounded once (d; its
 // remainder too where the table has room for it, dlo).  Otherwise an FP32 d,
@@ -321,12 +319,13 @@ ADECO_HD inline F2 plane_offset(const float qa[3], const float la[3], const floa
 // The one-face closed form takes exact offsets either way (it forms them from
 // the stored vertices).
 template <bool kExactD, class Table, class Frame>
-ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc &g, TetVertices &Q, int lane, Table &W,
-                                int t, int *error, bool *fp64_route)
+ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc &g, Table &W, int t, int *error,
+                                bool *fp64_route)
 {
     long long cnt0 = 1;
     unsigned cnt = 1;
     float R = 0.f, bmin[3], bmax[3];
+    float V[4][3], L[4][3];  // the vertices in the anchor frame, hi and lo
     uint32_t ext01 = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -353,18 +352,26 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
         const int c0 = lo > u0 ? lo : u0, c1 = hi < u1 ? hi : u1;
         const int ex = c1 - c0 + 1;
         cnt = ex > 0 ? cnt * (unsigned)ex : 0u;
-        float qf[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            float lq;
-            shift_frame(h[q], l[q], c0, g.drcell[a], qf[q], lq);
-            Q.q[3 * q + a][lane] = qf[q];
-            Q.qlo[3 * q + a][lane] = lq;
-            R = fmaxf(R, fabsf(qf[q]));
+        for (int q = 0; q < 4; q += 2) {
+            float2 hi, lo2;
+            shift_frame2(make_float2(h[q], h[q + 1]), make_float2(l[q], l[q + 1]), (float)c0, g.drcell[a], hi, lo2);
+            V[q][a] = hi.x;
+            V[q + 1][a] = hi.y;
+            L[q][a] = lo2.x;
+            L[q + 1][a] = lo2.y;
         }
         R = fmaxf(R, (float)(ex - 1) + 1.f);
-        bmin[a] = fminf(fminf(qf[0], qf[1]), fminf(qf[2], qf[3]));
-        bmax[a] = fmaxf(fmaxf(qf[0], qf[1]), fmaxf(qf[2], qf[3]));
+        bmin[a] = fminf(fminf(V[0][a], V[1][a]), fminf(V[2][a], V[3][a]));
+        bmax[a] = fmaxf(fmaxf(V[0][a], V[1][a]), fmaxf(V[2][a], V[3][a]));
+        R = fmaxf(R, fmaxf(fabsf(bmin[a]), fabsf(bmax[a])));
+        if constexpr (Table::kHasRest) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                W.q[3 * q + a][t] = V[q][a];
+                W.qlo[3 * q + a][t] = L[q][a];
+            }
+        }
         if (a < 2) ext01 |= (uint32_t)(ex & 0xffff) << (16 * a);
         W.lo[a][t] = (uint16_t)c0;
         W.ex[a][t] = (uint16_t)ex;
@@ -386,7 +393,7 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
     for (int a = 0; a < 3; ++a) {
         const int b = a == 2 ? 0 : a + 1, c = a == 0 ? 2 : a - 1;
         auto edge = [&](int q, int x) {
-            return f2_add(F2{Q.q[3 * q + x][lane], Q.qlo[3 * q + x][lane]}, F2{-Q.q[9 + x][lane], -Q.qlo[9 + x][lane]});
+            return f2_add(F2{V[q][x], L[q][x]}, F2{-V[3][x], -L[3][x]});
         };
         const F2 cof = f2_add(f2_mul(edge(1, b), edge(2, c)), f2_neg(f2_mul(edge(1, c), edge(2, b))));
         w6 = f2_add(w6, f2_mul(edge(0, a), cof));
@@ -399,47 +406,48 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
     // through the face's centroid, so that the FP32 rounding of the normal
     // only turns the plane about the centroid (the one-face closed form
     // relies on it)
-    float tolmax = 0.f, L2 = 0.f;
+    // edges v1 - v0, v2 - v0, v3 - v0, v2 - v1, v3 - v1 and the largest of their components
+    constexpr int kFrom[6] = {0, 0, 0, 1, 1, 2}, kTo[6] = {1, 2, 3, 2, 3, 3};
+    float e[5][3], big[5], normal[4][4], tolmax = 0.f, L2 = 0.f;
 #pragma unroll
-    for (int f = 0; f < 4; ++f) {
-        const int fa = f == 3, fb = (0x2312 >> (12 - 4 * f)) & 3, fc = (0x1233 >> (12 - 4 * f)) & 3;
-        float A[3], B[3], C[3], e1[3], e2[3];
-        float s1 = 0.f, s2 = 0.f, s3 = 0.f;
+    for (int k = 0; k < 6; ++k) {
+        float d[3], sq = 0.f;
 #pragma unroll
         for (int x = 0; x < 3; ++x) {
-            A[x] = Q.q[3 * fa + x][lane];
-            B[x] = Q.q[3 * fb + x][lane];
-            C[x] = Q.q[3 * fc + x][lane];
-            e1[x] = B[x] - A[x];
-            e2[x] = C[x] - A[x];
-            const float e3 = C[x] - B[x];
-            s1 = fmaf(e1[x], e1[x], s1);
-            s2 = fmaf(e2[x], e2[x], s2);
-            s3 = fmaf(e3, e3, s3);
+            d[x] = V[kTo[k]][x] - V[kFrom[k]][x];
+            sq = fmaf(d[x], d[x], sq);
+            if (k < 5) e[k][x] = d[x];
         }
-        L2 = fmaxf(L2, fmaxf(s1, fmaxf(s2, s3)));
-        // n_in = (vb - va) x (vc - va) with the outward order reversed
+        if (k < 5) big[k] = fmaxf(fmaxf(fabsf(d[0]), fabsf(d[1])), fabsf(d[2]));
+        L2 = fmaxf(L2, sq);
+    }
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+        // n_in = (vb - va) x (vc - va) with the outward order reversed: faces (0,2,1) (0,3,2) (0,1,3) (1,2,3)
+        constexpr int kA[4] = {0, 0, 0, 1}, kB[4] = {2, 3, 1, 2}, kC[4] = {1, 2, 3, 3};
+        constexpr int kE1[4] = {1, 2, 0, 3}, kE2[4] = {0, 1, 2, 4};
+        const float *A = V[kA[f]], *B = V[kB[f]], *C = V[kC[f]], *e1 = e[kE1[f]], *e2 = e[kE2[f]];
         const float nn[3] = {e1[1] * e2[2] - e1[2] * e2[1], e1[2] * e2[0] - e1[0] * e2[2], e1[0] * e2[1] - e1[1] * e2[0]};
         float offset;
         if constexpr (kExactD) {
-            float la[3], lb[3], lc[3];
-            for (int x = 0; x < 3; ++x) {
-                la[x] = Q.qlo[3 * fa + x][lane];
-                lb[x] = Q.qlo[3 * fb + x][lane];
-                lc[x] = Q.qlo[3 * fc + x][lane];
-            }
-            const F2 d = plane_offset(A, la, B, lb, C, lc, nn);
+            const F2 d = plane_offset(A, L[kA[f]], B, L[kB[f]], C, L[kC[f]], nn);
             offset = d.hi;
             if constexpr (Table::kHasRest) W.dlo[f][t] = d.lo;
         } else {
             constexpr float kThird = 1.f / 3.f;
             offset = (nn[0] * (A[0] + B[0] + C[0]) + nn[1] * (A[1] + B[1] + C[1]) + nn[2] * (A[2] + B[2] + C[2])) * kThird;
         }
-        W.plane[f][t] = make_float4(nn[0], nn[1], nn[2], offset);
-        const float L1 = fmaxf(fmaxf(fabsf(e1[0]), fabsf(e1[1])), fabsf(e1[2]));
-        const float M1 = fmaxf(fmaxf(fabsf(e2[0]), fabsf(e2[1])), fabsf(e2[2]));
+        normal[f][0] = nn[0];
+        normal[f][1] = nn[1];
+        normal[f][2] = nn[2];
+        normal[f][3] = -offset;
         // generous bound on the FP32 rounding of n.x - d (|x| <= R + 1)
-        tolmax = fmaxf(tolmax, 1.0e-5f * L1 * M1 * (R + 1.f));
+        tolmax = fmaxf(tolmax, 1.0e-5f * big[kE1[f]] * big[kE2[f]] * (R + 1.f));
+    }
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+        const int k = f & 2, i = 2 * (f & 1);
+        W.plane[f][t] = make_float4(normal[k][i], normal[k + 1][i], normal[k][i + 1], normal[k + 1][i + 1]);
     }
     W.lower[t] = make_float4(bmin[0], bmin[1], bmin[2], tolmax);
     W.upper[t] = make_float4(bmax[0], bmax[1], bmax[2], u2f(ext01));
@@ -469,7 +477,15 @@ ADECO_HD inline int setup_tet(const float3 v[4], const float gh[4][3], const flo
             h = gh[v_][a];
             l = gl[v_][a];
         },
-        g, W, lane, W, lane, error, fp64_route);
+        g, W, lane, error, fp64_route);
+}
+
+// face f's normal and -d
+template <class Table>
+ADECO_HD inline float4 face_plane(const Table &W, int f, int s)
+{
+    const float *p = &W.plane[f & 2][s].x + (f & 1), *q = &W.plane[(f & 2) + 1][s].x + (f & 1);
+    return make_float4(p[0], p[2], q[0], q[2]);
 }
 
 enum PairClass : int { P_NO = 0, P_TET_INSIDE = 1, P_CELL_INSIDE = 2, P_PARTIAL = 3 };
@@ -526,19 +542,25 @@ ADECO_HD inline int classify_pair(const Table &W, const GridDesc &g, int s, int 
     int ncross = 0, fcross = 0;
     const float t = mn.w;
 #pragma unroll
-    for (int f = 0; f < 4; ++f) {
-        const float4 n = W.plane[f][s];
-        const float base = fmaf(n.x, fa, fmaf(n.y, fb, fmaf(n.z, fc, -n.w)));
-        const float pos = fmaxf(n.x, 0.f) + fmaxf(n.y, 0.f) + fmaxf(n.z, 0.f);
-        const float mx = base + pos;
-        const float mn = base + ((n.x + n.y + n.z) - pos);
-        if (mx < -t) return P_NO;
-        if (mx <= t) unsure = true;
-        if (mn > t) continue;
-        all_in = false;
-        ++ncross;
-        fcross = f;
-        if (mn > -t) unsure = true;
+    for (int f = 0; f < 4; f += 2) {
+        const float4 p = W.plane[f][s], q = W.plane[f + 1][s];
+        const float2 nx = make_float2(p.x, p.y), ny = make_float2(p.z, p.w), nz = make_float2(q.x, q.y);
+        const float2 base = fma2(nx, both(fa), fma2(ny, both(fb), fma2(nz, both(fc), make_float2(q.z, q.w))));
+        const float2 pos = add2(add2(make_float2(fmaxf(nx.x, 0.f), fmaxf(nx.y, 0.f)),
+                                     make_float2(fmaxf(ny.x, 0.f), fmaxf(ny.y, 0.f))),
+                                make_float2(fmaxf(nz.x, 0.f), fmaxf(nz.y, 0.f)));
+        const float2 mx2 = add2(base, pos), mn2 = add2(base, sub2(add2(add2(nx, ny), nz), pos));
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float mx = i ? mx2.y : mx2.x, mn = i ? mn2.y : mn2.x;
+            if (mx < -t) return P_NO;
+            if (mx <= t) unsure = true;
+            if (mn > t) continue;
+            all_in = false;
+            ++ncross;
+            fcross = f + i;
+            if (mn > -t) unsure = true;
+        }
     }
     if (unsure) {
         used_fp64 = true;
@@ -560,11 +582,11 @@ template <bool kExactD = true, class Table>
 ADECO_HD inline F2 face_value_at_cell(const Table &W, const GridDesc &g, int s, int a, int b, int c, int f)
 {
     const int cc[3] = {a, b, c};
-    const float4 pl = W.plane[f][s];
+    const float4 pl = face_plane(W, f, s);
     const float n[3] = {pl.x, pl.y, pl.z};
     F2 G;
     if constexpr (kExactD) {
-        G = {-pl.w, -W.dlo[f][s]};
+        G = {pl.w, -W.dlo[f][s]};
     } else {  // the exact offset setup_tet<true> would have stored
         const int fa = f == 3 ? 1 : 0, fb = f == 0 ? 2 : (f == 1 ? 3 : (f == 2 ? 1 : 2)),
                   fc = f == 0 ? 1 : (f == 1 ? 2 : 3);
@@ -598,7 +620,7 @@ inline
 #endif
 float halfspace_pair_vol6(const Table &W, const GridDesc &g, int s, int a, int b, int c, int f)
 {
-    const float4 n = W.plane[f][s];
+    const float4 n = face_plane(W, f, s);
     return halfspace_cube_vol6(face_value_at_cell<kExactD>(W, g, s, a, b, c, f), n.x, n.y, n.z);
 }
 
@@ -771,7 +793,7 @@ __device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &
                     h = S.wt.gh[a][v];
                     l = S.wt.gl[a][v];
                 },
-                S.g, reinterpret_cast<TetVertices &>(S.pool[warp]), lane, S.wt, slot, P.error, &route64);
+                S.g, S.wt, slot, P.error, &route64);
         if (cnt > 0 && (S.wt.ex[0][slot] > 1024 || S.wt.ex[1][slot] > 1024 || S.wt.ex[2][slot] > 1024)) S.wide[odd] = 1;
     }
     n_tets += (cnt > 0);
