@@ -660,9 +660,9 @@ __device__ __forceinline__ unsigned child_bytes(int child, unsigned k1, unsigned
     return child == 1 ? (k2 ? 0x7460u : 0x5610u) : (k2 ? 0x7540u : 0x4650u);
 }
 
-constexpr int kPool = 78;    // pieces per warp pool (2 CTAs of 8 warps fit in an SM's shared memory)
-constexpr int kLast = 88;    // pieces at their last crossed face per warp
-constexpr int kPairs = 1152;  // partial pairs a CTA lists
+constexpr int kPool = 80;    // pieces per warp pool (2 CTAs of 8 warps fit in an SM's shared memory)
+constexpr int kLast = 84;    // pieces at their last crossed face per warp
+constexpr int kPairs = 1280;  // partial pairs a CTA lists
 
 static_assert(kPool >= 32 + 3 && kLast >= 32 + 3, "one split step fits a full pool and list");
 

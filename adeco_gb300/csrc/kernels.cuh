@@ -101,7 +101,6 @@ struct TetPlanes {
     float4 upper[N];     //   maximum; candidate extents of axes 0 | 1 << 16, as bits
     float f6[N];         // mass per unit of 6x clipped volume (tet mass / |6V| in cell units)
     uint16_t lo[3][N];   // anchor cell (first candidate cell) in grid indices (dims <= 4096)
-    uint16_t ex[3][N];   // candidate extents (cells per axis)
 };
 
 // The vertices of up to 32 tets in their anchor cells' frames (cell units).
@@ -116,6 +115,7 @@ struct TetVertices {
 struct WarpTets : TetPlanes<32>, TetVertices {
     static constexpr bool kHasRest = true;
     float dlo[4][32];
+    uint16_t ex[3][32];  // candidate extents (cells per axis)
 };
 
 ADECO_HD inline void tet_coord(const WarpTets &W, const GridDesc &, int s, int v, int x, float &hi, float &lo)
@@ -309,7 +309,7 @@ ADECO_HD inline F2 plane_offset(const float qa[3], const float la[3], const floa
 // ordered by the orientation rule (frame(q, a, hi, lo): vertex q, axis a), and
 // its candidate cells as vertex_range words (mn / mx: the least and the
 // greatest of its vertices).  Returns the candidate pair count (0 if the tet
-// is skipped).
+// is skipped); *wide: more than 1024 of them along an axis.
 //
 // kExactD: each face's plane offset in double-float, rounded once (d; its
 // remainder too where the table has room for it, dlo).  Otherwise an FP32 d,
@@ -320,13 +320,14 @@ ADECO_HD inline F2 plane_offset(const float qa[3], const float la[3], const floa
 // the stored vertices).
 template <bool kExactD, class Table, class Frame>
 ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc &g, Table &W, int t, int *error,
-                                bool *fp64_route)
+                                bool *fp64_route, bool *wide)
 {
     long long cnt0 = 1;
     unsigned cnt = 1;
     float R = 0.f, bmin[3], bmax[3];
     float V[4][3], L[4][3];  // the vertices in the anchor frame, hi and lo
     uint32_t ext01 = 0;
+    int big_ex = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const int top = g.dims - 1;
@@ -374,7 +375,8 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
         }
         if (a < 2) ext01 |= (uint32_t)(ex & 0xffff) << (16 * a);
         W.lo[a][t] = (uint16_t)c0;
-        W.ex[a][t] = (uint16_t)ex;
+        big_ex = big_ex > ex ? big_ex : ex;
+        if constexpr (Table::kHasRest) W.ex[a][t] = (uint16_t)ex;
     }
     if (cnt0 > kMaxPairsPerTet) {
 #ifdef __CUDA_ARCH__
@@ -454,6 +456,7 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
     // conditioning: longest edge cubed over |6V|, both in cell units.  L^3 <=
     // kappa |6V| squared (both sides non-negative): no square root; NaN or an
     // overflow routes the tet
+    *wide = big_ex > 1024;
     *fp64_route = !(L2 * L2 * L2 <= (kKappaFp64 * kKappaFp64) * (vq6 * vq6));
     return (int)cnt;
 }
@@ -465,6 +468,7 @@ ADECO_HD inline int setup_tet(const float3 v[4], const float gh[4][3], const flo
                               Table &W, int lane, int *error, bool *fp64_route)
 {
     *fp64_route = false;
+    bool wide;
     const int sgn = vol6_sign_ref(vol6_exact(v[0], v[1], v[2], v[3]));
     int lo[3], hi[3];
     if (!candidate_range(v, g, lo, hi) || sgn == 0) return 0;
@@ -477,7 +481,7 @@ ADECO_HD inline int setup_tet(const float3 v[4], const float gh[4][3], const flo
             h = gh[v_][a];
             l = gl[v_][a];
         },
-        g, W, lane, error, fp64_route);
+        g, W, lane, error, fp64_route, &wide);
 }
 
 // face f's normal and -d
@@ -759,7 +763,7 @@ __device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slot = threadIdx.x, tid = first + slot;
     int cnt = 0;
-    bool route64 = false;
+    bool route64 = false, wide = false;
     if (tid < end) {
         const int t = tid % 6, v0 = S.cubes[tid / 6];
         const ushort4 off = *reinterpret_cast<const ushort4 *>(S.vert_off[t]);
@@ -793,8 +797,8 @@ __device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &
                     h = S.wt.gh[a][v];
                     l = S.wt.gl[a][v];
                 },
-                S.g, S.wt, slot, P.error, &route64);
-        if (cnt > 0 && (S.wt.ex[0][slot] > 1024 || S.wt.ex[1][slot] > 1024 || S.wt.ex[2][slot] > 1024)) S.wide[odd] = 1;
+                S.g, S.wt, slot, P.error, &route64, &wide);
+        if (cnt > 0 && wide) S.wide[odd] = 1;
     }
     n_tets += (cnt > 0);
     if (route64 && cnt > 0) {  // deposited by route_fp64_kernel
