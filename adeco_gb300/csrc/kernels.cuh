@@ -183,6 +183,8 @@ struct SharedMixed {
     uint8_t tet[kWave];
     int warp_pairs[kWarps];
     int cursor;          // first candidate pair of the wave not yet taken
+    int cut[2];          // one-face pairs at the list's end (alternating as list.n),
+    int cut_next[2];     //   and the first not taken
     int wide[2];         // a tet of the wave (even, odd) has more than 1024 candidate cells along an axis
     PairList list;
     WarpPool pool[kWarps];
@@ -824,11 +826,14 @@ __device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &
 }
 
 // Classify phase: the warps take the wave's candidate pairs 32 at a time and
-// classify them; inside cells and one-face cells are deposited at once,
-// partial cells listed, until no pair is left or the list might not hold the
-// 32 pairs each warp may have in hand (`room` of it are used).
+// classify them; inside cells are deposited at once, partial cells listed, and
+// those that one face cuts at the list's end (with the face in the top bits):
+// their closed form, for a few lanes of nearly every 32, had taken more than
+// the classification itself.  Until no pair is left or the list might not hold
+// the 32 pairs each warp may have in hand (`room` of it are used).
 template <bool kStats>
-__device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixed &S, int *list_n, int room, bool wide, PairStats &st)
+__device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixed &S, int *list_n, int *cut_n, int room, bool wide,
+                                              PairStats &st)
 {
     const int lane = threadIdx.x & 31;
     const unsigned le = 0xffffffffu >> (31 - lane);
@@ -846,7 +851,8 @@ __device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixe
     pre -= own;
     for (;;) {
         int c0 = 0;
-        if (lane == 0) c0 = *(volatile int *)list_n > room - kThreads ? INT_MAX : atomicAdd(&S.cursor, 32);
+        if (lane == 0)
+            c0 = *(volatile int *)list_n + *(volatile int *)cut_n > room - kThreads ? INT_MAX : atomicAdd(&S.cursor, 32);
         c0 = __shfl_sync(0xffffffffu, c0, 0);
         if (c0 >= total) break;
         // The pair's tet, without a search per lane: lane k holds the start of
@@ -870,13 +876,13 @@ __device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixe
             if (q0 >= min(c0 + 32, total)) break;
         }
         bool part = false;
+        int cross = -1;
         uint32_t entry = 0;
         if (pidx < total) {
             const int3 c = flat_cell(W, s, local);
             entry = wide ? (uint32_t)local : ((uint32_t)c.x | ((uint32_t)c.y << 10) | ((uint32_t)c.z << 20));
             if (kStats) ++st.cand;
             bool f64 = false;
-            int cross = -1;
             const int cls = classify_pair(W, g, s, c.x, c.y, c.z, f64, cross);
             if (kStats) {
                 st.fp64 += f64;
@@ -886,16 +892,21 @@ __device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixe
                 st.bbox += cls != P_NO;
             }
             part = cls == P_PARTIAL && cross < 0;
-            float m = cls == P_TET_INSIDE ? g.tet_mass : (cls == P_CELL_INSIDE ? 6.f * W.f6[s] : 0.f);
-            // one face cuts the cell: closed form, no clipping
-            if (cross >= 0) m = halfspace_pair_vol6<false>(W, g, s, c.x, c.y, c.z, cross) * W.f6[s];
+            const float m = cls == P_TET_INSIDE ? g.tet_mass : (cls == P_CELL_INSIDE ? 6.f * W.f6[s] : 0.f);
             if (m > 0.f) scatter(P, g, W, s, c.x, c.y, c.z, m);
         }
-        const unsigned bal = __ballot_sync(0xffffffffu, part);
+        const unsigned bal = __ballot_sync(0xffffffffu, part), cut = __ballot_sync(0xffffffffu, cross >= 0);
+        const unsigned lt = le >> 1;
         int at = 0;
         if (lane == 0 && bal) at = atomicAdd(list_n, __popc(bal));
-        at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1));
-        if (part) {
+        if (lane == 1 && cut) at = atomicAdd(cut_n, __popc(cut));
+        const int cut_at = kPairs - 1 - (__shfl_sync(0xffffffffu, at, 1) + __popc(cut & lt));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & lt);
+        if (cross >= 0) {
+            at = cut_at;
+            entry |= (uint32_t)cross << 30;
+        }
+        if (part || cross >= 0) {
             S.list.cell[at] = entry;
             S.list.tet[at] = (uint8_t)s;
         }
@@ -915,7 +926,7 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
     const int warp = threadIdx.x >> 5;
     PairStats st;
     int turn = 0, odd = 0;  // the pair list's counters and the wave's flag in use
-    if (threadIdx.x == 0) S.wide[0] = S.list.n[0] = S.list.next[0] = 0;
+    if (threadIdx.x == 0) S.wide[0] = S.list.n[0] = S.list.next[0] = S.cut[0] = S.cut_next[0] = 0;
     const int room = kPairs / kQueue * min(max(P.clip_batch, 64), kQueue);
 
     for (int taken = 0;; ++taken) {
@@ -960,13 +971,15 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
             bool left = total > 0;
             if (!left) __syncthreads();  // the next wave's set-up writes what this one's warps read above
             while (left) {
-                wave_classify<kStats>(P, S, &S.list.n[turn], room, wide, st);
+                wave_classify<kStats>(P, S, &S.list.n[turn], &S.cut[turn], room, wide, st);
                 __syncthreads();
                 left = S.cursor < total;
                 const int np = S.list.n[turn];
                 if (threadIdx.x == 0) {  // the next list's
                     S.list.n[turn ^ 1] = 0;
                     S.list.next[turn ^ 1] = 0;
+                    S.cut[turn ^ 1] = 0;
+                    S.cut_next[turn ^ 1] = 0;
                 }
                 uint64_t mine = clip_pairs(
                     S.pool[warp], S.list, &S.list.next[turn], np,
@@ -986,6 +999,23 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
                         const long long v = S.list.volume(j);
                         if (v > 0) scatter(P, S.g, S.wt, s, c.x, c.y, c.z, pair_mass(v, S.wt.f6[s]));
                     }
+                }
+                // one face cuts the cell: closed form, no clipping; taken by the
+                // warps that are through with their pairs first
+                for (const int ncut = S.cut[turn];;) {
+                    int j = 0;
+                    if ((threadIdx.x & 31) == 0) j = ncut ? atomicAdd(&S.cut_next[turn], 32) : 0;
+                    j = __shfl_sync(0xffffffffu, j, 0);
+                    if (j >= ncut) break;
+                    j += threadIdx.x & 31;
+                    if (j < ncut) {
+                        const uint32_t e = S.list.cell[kPairs - 1 - j];
+                        const int s = S.list.tet[kPairs - 1 - j];
+                        const int3 c = pair_cell(S.wt, s, e & 0x3fffffffu, wide);
+                        const float m = halfspace_pair_vol6<false>(S.wt, S.g, s, c.x, c.y, c.z, (int)(e >> 30)) * S.wt.f6[s];
+                        if (m > 0.f) scatter(P, S.g, S.wt, s, c.x, c.y, c.z, m);
+                    }
+                    __syncwarp();
                 }
                 turn ^= 1;
                 __syncthreads();
