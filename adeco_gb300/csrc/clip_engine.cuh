@@ -267,12 +267,13 @@ ADECO_HD inline float halfspace_cube_vol6(F2 G0, float nx, float ny, float nz)
     nx = fabsf(nx);
     ny = fabsf(ny);
     nz = fabsf(nz);
-    const F2 e1 = f2_add(G0, F2{nx, 0.f}), e2 = f2_add(G0, F2{ny, 0.f}), e4 = f2_add(G0, F2{nz, 0.f});
-    const F2 e3 = f2_add(e1, F2{ny, 0.f}), e5 = f2_add(e1, F2{nz, 0.f}), e6 = f2_add(e2, F2{nz, 0.f});
-    const F2 e7 = f2_add(e3, F2{nz, 0.f});
+    const F2x2 e12 = f2x2_add({both(G0.hi), both(G0.lo)}, make_float2(nx, ny));
+    const F2x2 e45 = f2x2_add({make_float2(G0.hi, e12.hi.x), make_float2(G0.lo, e12.lo.x)}, both(nz));
+    const F2x2 e36 = f2x2_add(e12, make_float2(ny, nz));
+    const F2 e7 = f2_add(F2{e36.hi.x, e36.lo.x}, F2{nz, 0.f});
     const float g0 = G0.hi + G0.lo, g7 = e7.hi;
-    const float ga[3] = {e1.hi, e2.hi, e4.hi};  // a = 1, 2, 4
-    const float gb[3] = {e3.hi, e5.hi, e6.hi};  // b = 3, 5, 6
+    const float ga[3] = {e12.hi.x, e12.hi.y, e45.hi.x};   // a = 1, 2, 4
+    const float gb[3] = {e36.hi.x, e45.hi.y, e36.hi.y};   // b = 3, 5, 6
     if (!(g7 > 0.f)) return 0.f;
     if (g0 > 0.f) return 6.f;
     const float r70 = rcp_nr(g7 - g0);
@@ -280,26 +281,30 @@ ADECO_HD inline float halfspace_cube_vol6(F2 G0, float nx, float ny, float nz)
     float ta0[3], ua0[3], t7a[3], tb0[3], ub0[3], t7b[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        const float ra0 = rcp_nr(ga[i] - g0), rb0 = rcp_nr(gb[i] - g0);
-        ta0[i] = ga[i] * ra0;
-        ua0[i] = -g0 * ra0;
-        tb0[i] = gb[i] * rb0;
-        ub0[i] = -g0 * rb0;
-        t7a[i] = g7 * rcp_nr(g7 - ga[i]);
-        t7b[i] = g7 * rcp_nr(g7 - gb[i]);
+        const float2 gab = make_float2(ga[i], gb[i]);
+        const float2 r0 = rcp_nr2(sub2(both(g0), gab)), r7 = rcp_nr2(sub2(gab, both(g7)));
+        const float2 t0 = mul2(gab, r0), u0 = mul2(both(-g0), r0), t7 = mul2(both(g7), r7);
+        ta0[i] = t0.x;
+        tb0[i] = t0.y;
+        ua0[i] = u0.x;
+        ub0[i] = u0.y;
+        t7a[i] = t7.x;
+        t7b[i] = t7.y;
     }
     // tets (a, b) by index into ga / gb: (1,3) (1,5) (2,3) (2,6) (4,5) (4,6)
     const int ia[6] = {0, 0, 1, 1, 2, 2}, ib[6] = {0, 1, 0, 2, 1, 2};
     float v = 0.f;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) {
-        const int i = ia[q], j = ib[q];
-        const float rba = rcp_nr(gb[j] - ga[i]);
-        const float tba = gb[j] * rba, uba = -ga[i] * rba;
-        const float k1 = t70 * t7a[i] * t7b[j];
-        const float k2 = fmaf(tb0[j], tba, t70 * fmaf(tba, ub0[j], t7a[i] * uba));
-        const float k3 = fmaf(ua0[i], fmaf(ub0[j], t70, tb0[j]), ta0[i]);
-        v += (gb[j] <= 0.f) ? k1 : ((ga[i] <= 0.f) ? k2 : k3);
+    for (int q = 0; q < 6; q += 2) {  // two tets of the same a
+        const int i = ia[q], j = ib[q], k = ib[q + 1];
+        const float2 g = make_float2(gb[j], gb[k]), tb = make_float2(tb0[j], tb0[k]), ub = make_float2(ub0[j], ub0[k]);
+        const float2 rba = rcp_nr2(sub2(both(ga[i]), g));
+        const float2 tba = mul2(g, rba), uba = mul2(both(-ga[i]), rba);
+        const float2 k1 = mul2(both(t70 * t7a[i]), make_float2(t7b[j], t7b[k]));
+        const float2 k2 = fma2(tb, tba, mul2(both(t70), fma2(tba, ub, mul2(both(t7a[i]), uba))));
+        const float2 k3 = fma2(both(ua0[i]), fma2(ub, both(t70), tb), both(ta0[i]));
+        v += (g.x <= 0.f) ? k1.x : ((ga[i] <= 0.f) ? k2.x : k3.x);
+        v += (g.y <= 0.f) ? k1.y : ((ga[i] <= 0.f) ? k2.y : k3.y);
     }
     return v;
 }

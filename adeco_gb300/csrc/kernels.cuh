@@ -159,11 +159,13 @@ __device__ __forceinline__ void tet_coord(const WaveTets &W, const GridDesc &g, 
     shift_frame(W.gh[x][i], W.gl[x][i], W.lo[x][s], g.drcell[x], hi, lo);
 }
 
-// the same of vertices v and v + 1
-__device__ __forceinline__ void tet_coord2(const WaveTets &W, const GridDesc &g, int s, int v, int x, float2 &hi, float2 &lo)
+// the same of vertices v and w
+__device__ __forceinline__ void tet_coord2(const WaveTets &W, const GridDesc &g, int s, int v, int w, int x, float2 &hi,
+                                           float2 &lo)
 {
     const ushort4 id = W.vid[s];
-    const int i = v == 0 ? id.x : id.z, j = v == 0 ? id.y : id.w;
+    const int i = v == 0 ? id.x : (v == 1 ? id.y : (v == 2 ? id.z : id.w));
+    const int j = w == 0 ? id.x : (w == 1 ? id.y : (w == 2 ? id.z : id.w));
     shift_frame2(make_float2(W.gh[x][i], W.gh[x][j]), make_float2(W.gl[x][i], W.gl[x][j]), (float)W.lo[x][s], g.drcell[x],
                  hi, lo);
 }
@@ -599,6 +601,18 @@ ADECO_HD inline F2 face_value_at_cell(const Table &W, const GridDesc &g, int s, 
         float q[3][3], l[3][3];
 #pragma unroll
         for (int x = 0; x < 3; ++x) {
+#ifdef __CUDA_ARCH__
+            if constexpr (!Table::kHasRest) {  // two vertices at a time
+                float2 hi, lo;
+                tet_coord2(W, g, s, fa, fb, x, hi, lo);
+                q[0][x] = hi.x;
+                q[1][x] = hi.y;
+                l[0][x] = lo.x;
+                l[1][x] = lo.y;
+                tet_coord(W, g, s, fc, x, q[2][x], l[2][x]);
+                continue;
+            }
+#endif
             tet_coord(W, g, s, fa, x, q[0][x], l[0][x]);
             tet_coord(W, g, s, fb, x, q[1][x], l[1][x]);
             tet_coord(W, g, s, fc, x, q[2][x], l[2][x]);
@@ -681,7 +695,7 @@ ADECO_HD inline void piece_coords(const Table &W, const GridDesc &g, int s, int 
             float2 hi, lo;
 #pragma unroll
             for (int v = 0; v < 4; v += 2) {
-                tet_coord2(W, g, s, v, x, hi, lo);
+                tet_coord2(W, g, s, v, v + 1, x, hi, lo);
                 const float2 c2 = cell_coord_fast2(hi, lo, cc[x], g.drcell[x], flip);
                 p[3 * v + x] = c2.x;
                 p[3 * v + 3 + x] = c2.y;
@@ -1199,26 +1213,30 @@ __global__ void __launch_bounds__(7 * 32) call_box_kernel(const float *part, int
         else if (r != 0.f) box->nan = 1;
     }
     __syncthreads();
-    if (threadIdx.x) return;
+    if (q) return;  // a lane per axis
     const GridDesc &g = *gp;
-    int empty = 0;
-    for (int a = 0; a < 3; ++a) {
-        box->lo[a] = 0;
-        box->ext[a] = g.dims;
-        if (box->nan) continue;
-        const double gmin = g.gmin[a], gmax = g.gmax[a], delta = g.delta[a];
-        const float vmin = box->vmin[a], vmax = box->vmax[a];
-        if (!(vmin <= vmax) || (double)vmax < gmin || (double)vmin > gmax || !(delta > 0.0)) {
-            empty = 1;
-            continue;
+    const int a = lane;
+    bool empty = false;
+    if (a < 3) {
+        int lo = 0, ext = g.dims;
+        if (!box->nan) {
+            const double gmin = g.gmin[a], gmax = g.gmax[a], delta = g.delta[a];
+            const float vmin = box->vmin[a], vmax = box->vmax[a];
+            if (!(vmin <= vmax) || (double)vmax < gmin || (double)vmin > gmax || !(delta > 0.0)) {
+                empty = true;
+            } else {
+                const double flo = floor((fmax((double)vmin, gmin) - gmin) / delta) - 1.0;
+                const double fhi = ceil((fmin((double)vmax, gmax) - gmin) / delta) + 1.0;
+                const int l = (int)fmin(fmax(flo, 0.0), (double)(g.dims - 1)), h = (int)fmin(fmax(fhi, 0.0), (double)(g.dims - 1));
+                lo = l;
+                ext = h - l + 1;
+            }
         }
-        const double flo = floor((fmax((double)vmin, gmin) - gmin) / delta) - 1.0;
-        const double fhi = ceil((fmin((double)vmax, gmax) - gmin) / delta) + 1.0;
-        const int l = (int)fmin(fmax(flo, 0.0), (double)(g.dims - 1)), h = (int)fmin(fmax(fhi, 0.0), (double)(g.dims - 1));
-        box->lo[a] = l;
-        box->ext[a] = h - l + 1;
+        box->lo[a] = lo;
+        box->ext[a] = ext;
     }
-    box->empty = empty;
+    empty = __any_sync(0xffffffffu, empty);
+    if (lane == 0) box->empty = empty;
 }
 
 // A pass's sums of the box's cells, from the fixed point grid (times scale)
