@@ -116,65 +116,58 @@ ADECO_HD inline int face_bits(float x, float y, float z)
 
 // The cut of a piece by face f, its vertices permuted to A B C D, the k
 // inside ones first by an even permutation (the orientation is kept): the cut
-// points E0..E3 of the four cut edges -- k=1: AB AC AD AD; k=2: AC AD BC BD;
-// k=3: AD BD CD CD -- snapped onto the face.  A vertex has N values, its
+// points E0..E3 of the cut edges -- k=1: AB AC AD; k=2: AC AD BC BD; k=3: AD
+// BD CD -- snapped onto the face.  A vertex has N values, its
 // coordinates last; the others (N = 6: barycentric weights) are interpolated
 // with the coordinates' edge parameter.
+// E3 is made for k = 2 only (BD; the other cases do not use it).  da..dd: the
+// vertices' coordinate along f's axis.
 template <int N>
-ADECO_HD inline void cut_points(const float *A, const float *B, const float *C, const float *D, int k, int f,
-                                float E[4][N])
+ADECO_HD inline void cut_points(const float *A, const float *B, const float *C, const float *D, float da, float db,
+                                float dc, float dd, int k, int f, float E[4][N])
 {
     const int axis = f >> 1;
     const float plane = (f & 1) ? 1.f : 0.f;
     const unsigned k1 = bit_mask(k == 1), k2 = bit_mask(k == 2), k3 = bit_mask(k == 3);
-    const unsigned a[3] = {bit_mask(axis == 0), bit_mask(axis == 1), bit_mask(axis == 2)};
-    float in[4][N], out[4][N];
+    const unsigned ax[3] = {bit_mask(axis == 0), bit_mask(axis == 1), bit_mask(axis == 2)};
+    // the ends of edges 0 and 1, 2 and 3
+    const auto ends = [&](float a, float b, float c, float d, float2 in[2], float2 out[2]) {
+        in[0] = make_float2(a, bit_sel(k3, b, a));
+        out[0] = make_float2(bit_sel(k1, b, bit_sel(k2, c, d)), bit_sel(k1, c, d));
+        in[1] = make_float2(bit_sel(k1, a, bit_sel(k2, b, c)), b);
+        out[1] = make_float2(bit_sel(k2, c, d), d);
+    };
+    // two edges at a time; |dout - din| > 0 on a crossing edge
+    float2 din[2], dout[2], t[2];
+    ends(da, db, dc, dd, din, dout);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        // t = (plane - din) / (dout - din) as (din - plane) times minus the reciprocal
+#ifdef __CUDA_ARCH__
+        const float2 d = sub2(dout[e], din[e]);
+        const float2 r = make_float2(rcp_approx(-d.x), rcp_approx(-d.y));
+        const float2 q = fma2(r, fma2(d, r, both(1.f)), r);
+#else
+        const float2 q = make_float2(rcp_nr(din[e].x - dout[e].x), rcp_nr(din[e].y - dout[e].y));
+#endif
+        const float2 num = add2(din[e], both(-plane));
+        t[e] = make_float2(sat01(num.x * q.x), sat01(num.y * q.y));
+    }
 #pragma unroll
     for (int x = 0; x < N; ++x) {
-        in[0][x] = A[x];
-        out[0][x] = bit_sel(k1, B[x], bit_sel(k2, C[x], D[x]));
-        in[1][x] = bit_sel(k3, B[x], A[x]);
-        out[1][x] = bit_sel(k1, C[x], D[x]);
-        in[2][x] = bit_sel(k1, A[x], bit_sel(k2, B[x], C[x]));
-        out[2][x] = bit_sel(k2, C[x], D[x]);
-        in[3][x] = bit_sel(k2, B[x], bit_sel(k3, C[x], A[x]));
-        out[3][x] = D[x];
-    }
-#ifdef __CUDA_ARCH__
-    // two edges at a time; with r the approximate reciprocal of din - dout, that is
-    // minus the one of dout - din, the same steps as below: t = (din - plane) (r + r (1 + (dout - din) r))
+        float2 in[2], out[2];
+        ends(A[x], B[x], C[x], D[x], in, out);
 #pragma unroll
-    for (int e = 0; e < 4; e += 2) {
-        float2 din, dout;
-        din.x = bit_sel(a[0], in[e][N - 3], bit_sel(a[1], in[e][N - 2], in[e][N - 1]));
-        din.y = bit_sel(a[0], in[e + 1][N - 3], bit_sel(a[1], in[e + 1][N - 2], in[e + 1][N - 1]));
-        dout.x = bit_sel(a[0], out[e][N - 3], bit_sel(a[1], out[e][N - 2], out[e][N - 1]));
-        dout.y = bit_sel(a[0], out[e + 1][N - 3], bit_sel(a[1], out[e + 1][N - 2], out[e + 1][N - 1]));
-        const float2 d = sub2(dout, din);
-        const float2 r = make_float2(rcp_approx(-d.x), rcp_approx(-d.y));
-        const float2 q = fma2(r, fma2(d, r, both(1.f)), r), num = add2(din, both(-plane));
-        const float2 t = make_float2(sat01(num.x * q.x), sat01(num.y * q.y));
-#pragma unroll
-        for (int x = 0; x < N; ++x) {
-            const float2 i = make_float2(in[e][x], in[e + 1][x]);
-            const float2 cut = fma2(t, sub2(make_float2(out[e][x], out[e + 1][x]), i), i);
-            E[e][x] = x < N - 3 ? cut.x : bit_sel(a[x < N - 3 ? 0 : x - (N - 3)], plane, cut.x);
-            E[e + 1][x] = x < N - 3 ? cut.y : bit_sel(a[x < N - 3 ? 0 : x - (N - 3)], plane, cut.y);
+        for (int e = 0; e < 2; ++e) {
+            float2 cut = fma2(t[e], sub2(out[e], in[e]), in[e]);
+            if (x >= N - 3) {
+                const unsigned m = ax[x < N - 3 ? 0 : x - (N - 3)];
+                cut = make_float2(bit_sel(m, plane, cut.x), bit_sel(m, plane, cut.y));
+            }
+            E[2 * e][x] = cut.x;
+            E[2 * e + 1][x] = cut.y;
         }
     }
-#else
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const float din = bit_sel(a[0], in[e][N - 3], bit_sel(a[1], in[e][N - 2], in[e][N - 1]));
-        const float dout = bit_sel(a[0], out[e][N - 3], bit_sel(a[1], out[e][N - 2], out[e][N - 1]));
-        const float t = sat01((plane - din) * rcp_nr(dout - din));  // |dout - din| > 0 on a crossing edge
-#pragma unroll
-        for (int x = 0; x < N; ++x) {
-            const float cut = fmaf(t, out[e][x] - in[e][x], in[e][x]);
-            E[e][x] = x < N - 3 ? cut : bit_sel(a[x < N - 3 ? 0 : x - (N - 3)], plane, cut);
-        }
-    }
-#endif
 }
 
 // Inside part of a cut piece as 1 or 3 positively oriented pieces, child
@@ -585,7 +578,9 @@ long long clip_piece_serial(const float p0[12], int done0)
         for (int q = 0; q < 4; ++q)
 #pragma unroll
             for (int x = 0; x < 3; ++x) V[q][x] = sel4((pm >> (2 * q)) & 3, p[x], p[3 + x], p[6 + x], p[9 + x]);
-        cut_points<3>(V[0], V[1], V[2], V[3], k, face, E);
+        const int ax = face >> 1;
+        cut_points<3>(V[0], V[1], V[2], V[3], sel3(ax, V[0][0], V[0][1], V[0][2]), sel3(ax, V[1][0], V[1][1], V[1][2]),
+                      sel3(ax, V[2][0], V[2][1], V[2][2]), sel3(ax, V[3][0], V[3][1], V[3][2]), k, face, E);
         const int n = k == 1 ? 1 : 3;
         if (sp + 3 > kDepth) continue;  // cannot happen (depth <= 2*5 + 3)
         const int d = sdone[sp] | (1 << face);
@@ -818,7 +813,9 @@ __device__ __forceinline__ uint64_t clip_pairs(WarpPool &pool, PairList &list, i
                 C[x] = pool.v[3 * ic + x][idx];
                 D[x] = pool.v[3 * id + x][idx];
             }
-            cut_points<3>(A, B, C, D, k, f, E);
+            const int ax = f >> 1;
+            cut_points<3>(A, B, C, D, pool.v[3 * ia + ax][idx], pool.v[3 * ib + ax][idx], pool.v[3 * ic + ax][idx],
+                          pool.v[3 * id + ax][idx], k, f, E);
             k1 = bit_mask(k == 1);
             k2 = bit_mask(k == 2);
             const int keep = left & ~(1 << f);
@@ -1054,7 +1051,9 @@ __device__ __forceinline__ uint64_t clip_bary_pairs(BaryPool &pool, BaryList &li
                 C[x] = pool.v[6 * ic + x][idx];
                 D[x] = pool.v[6 * id + x][idx];
             }
-            cut_points<6>(A, B, C, D, k, f, E);
+            const int ax = 3 + (f >> 1);
+            cut_points<6>(A, B, C, D, pool.v[6 * ia + ax][idx], pool.v[6 * ib + ax][idx], pool.v[6 * ic + ax][idx],
+                          pool.v[6 * id + ax][idx], k, f, E);
             k1 = bit_mask(k == 1);
             k2 = bit_mask(k == 2);
             const int keep = left & ~(1 << f);
