@@ -16,12 +16,14 @@
 //     volumes times the inside fractions (from the edge parameters alone, no
 //     cut points).
 // A pair whose tet crosses several faces (up to 3^6 pieces) so spreads over
-// the warp instead of serialising one lane.  No per-thread stack: nothing
-// spills to local memory.  One loop whose step did all of it, each lane in its
-// own branch, had run ~640 instructions a step; the three kinds run ~290, 800
-// and 110, the 800 once for the pieces of 2.6 such steps.  With the selects
-// free of branches (bit_sel), octree leaves of a 192^3 lattice: 1.78e10 ->
-// 1.43e10 warp instructions with 21.9 -> 26.0 of 32 lanes.
+// the warp instead of serialising one lane.  What bounds it is issue, the ALU
+// pipe (selects, flags) first.  One loop whose step did all of it, each lane
+// in its own branch, had run ~640 instructions a step.  Octree leaves of a
+// 192^3 lattice, the whole kernel, warp instructions and time: that loop
+// 1.78e10, 25.4 ms; three kinds of steps, with selects free of branches
+// (bit_sel), 1.43e10; flags as a byte per vertex 1.33e10, 17.7 ms; two FP32
+// operations an instruction (fma2) 1.24e10, 17.1 ms; with the set-up's and
+// the classification's share 1.20e10, 16.3 ms.
 //
 // The split keeps every piece positively oriented: the vertices are permuted
 // (an even permutation) so that the k inside vertices come first, then the
@@ -660,7 +662,12 @@ __device__ __forceinline__ unsigned child_bytes(int child, unsigned k1, unsigned
     return child == 1 ? (k2 ? 0x7460u : 0x5610u) : (k2 ? 0x7540u : 0x4650u);
 }
 
-constexpr int kPool = 80;    // pieces per warp pool (2 CTAs of 8 warps fit in an SM's shared memory)
+// Two CTAs of 8 warps fill an SM's shared memory.  Every list's end costs a
+// drain with few lanes and a wait, so a longer list gains, until the pools,
+// which fine grids fill, get too small: no-allocation 96^3 / octree leaves
+// 256^3 / one zoom grid in ms with a list of 896 2.73 / 31.0 / 3.41, 1152 2.47 /
+// 29.8 / 3.22, 1280 2.44 / 29.8 / 3.16, 1408 (pool 71) 2.43 / 29.9 / 3.53.
+constexpr int kPool = 80;    // pieces per warp pool
 constexpr int kLast = 84;    // pieces at their last crossed face per warp
 constexpr int kPairs = 1280;  // partial pairs a CTA lists
 
@@ -668,7 +675,8 @@ static_assert(kPool >= 32 + 3 && kLast >= 32 + 3, "one split step fits a full po
 
 struct WarpPool {
     float v[12][kPool];         // the pieces' coordinates, a row per coordinate: a lane's four vertices come in
-                                // any order by their addresses, without a bank conflict
+                                // any order by their addresses (rows of a multiple of 32, free of bank
+                                // conflicts, were no faster)
     uint32_t flags[kPool];      // the vertices' inside flags, a byte each
     uint16_t owner[kPool];      // the piece's pair
     float last[5][kLast];       // pieces at their last face: 6x volume, the vertices' coordinate along its axis
@@ -911,7 +919,10 @@ __device__ __forceinline__ uint64_t clip_pairs(WarpPool &pool, PairList &list, i
 // (3 weights, 3 coordinates), and a piece inside every face is listed like
 // one at its last face, since its share of the tet (bary_share, a
 // double-float determinant) costs as much as a split and would run three
-// times, for a few lanes each, in the split step.
+// times, for a few lanes each, in the split step.  The pool's last 8 places are
+// for steps of one lane, so that none ever has to clip a piece by itself (in a
+// pool of 66 that had happened 5386 times on a clustered 128^3 lattice, with
+// a stack in local memory: 2.7 -> 2.2 ms of the kernel).
 constexpr int kBaryPool = 66;    // pieces per warp pool
 constexpr int kBaryLast = 66;    // pieces whose share is to be added, per warp
 constexpr int kBaryPairs = 640;  // partial pairs a CTA lists

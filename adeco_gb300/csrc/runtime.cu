@@ -1325,7 +1325,7 @@ extern "C" int adeco_debug_tet_records(const float *positions, size_t positions_
 // ============================================================ bounded waits
 // One warp waits, through wait_zero_bounded (the wait every spin of the
 // deposit kernels uses), on a count that nothing decrements; when the limit
-// runs out it sets error bit 3, as the work-sharing wait does, and returns.
+// runs out it sets error bit 3 and returns.
 __global__ void bounded_wait_kernel(int *error, unsigned spins)
 {
     __shared__ int busy;

@@ -8,16 +8,16 @@ the per-cell bar):
 * ``zoom_tile``   -- cells per tile edge of a zoom grid: one work item per
   (tile, meta-cell); smaller tiles balance fine grids better but stage and
   cull each meta-cell's vertex block more often;
-* ``share_chunk`` -- candidate pairs per chunk when the warps of an item share
-  a large tet group (zoom grids);
-* ``clip_batch``  -- the staging depth of the clip engine: partial pairs a
-  warp lists before it clips them together (deeper lists keep more lanes
-  busy, shallower ones clip sooner);
+* ``share_chunk`` -- accepted, without effect: a CTA's warps take pairs 32 at
+  a time from the whole wave;
+* ``clip_batch``  -- the staging depth of the clip engine: the share, in
+  128ths, of a CTA's list of partial pairs that is filled before it is clipped
+  (deeper lists keep more lanes busy, shallower ones clip sooner);
 * ``ctas_per_sm`` -- CTAs per SM of the persistent leaf launch;
 * ``item_pairs``  -- the expected candidate pairs above which a zoom
   request's tile edge is halved (fine grids: smaller items, shorter tails).
 
-The number of tets a warp sets up at once is the warp width (32, one per
+The number of tets a CTA sets up at once is its thread count (256, one per
 lane); it is not a parameter.  The reference has no tuner: its launch shape
 is the compile-time pair AMD_CUDA_GRID_DIM / AMD_CUDA_BLOCK_DIM
 (src/AdDeposit2Grid.h:51-52, <<<512, 64>>>).

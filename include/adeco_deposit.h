@@ -204,7 +204,7 @@ typedef struct {
     uint64_t routed_tets;   /* ill-conditioned tets (longest edge^3 > 32 |6V|) that the
                                barycentric route deposited                          */
     uint64_t serial_pieces; /* pieces a lane clipped alone because its warp's piece
-                               pool was full and no lane could move (collect_stats) */
+                               pool was full (collect_stats)                        */
 } adeco_timing;
 
 /* Deposit every leaf (leaf_dims^3 cells over the leaf's cube) in one batched
@@ -226,8 +226,8 @@ int adeco_session_replay_leaves(adeco_session *s, int reps, adeco_timing *timing
  * change fields, set them back; out-of-range values return ADECO_ERR_ARGUMENT. */
 typedef struct {
     int zoom_tile;           /* cells per tile edge of zoom grids, 16..256 (default 64)              */
-    int share_chunk;         /* zoom grids: candidate pairs per work-sharing chunk, 64..8192 (512)  */
-    int clip_batch;          /* partial pairs a warp lists before clipping them, 64..128 (128)      */
+    int share_chunk;         /* 64..8192 (512); kept for callers that set it, without effect        */
+    int clip_batch;          /* 128ths of a CTA's pair list filled before clipping, 64..128 (128)   */
     int ctas_per_sm;         /* CTAs per SM of the persistent leaf launch, 1..2 (2)                 */
     uint64_t route_capacity; /* ill-conditioned tets one launch may list; more set ADECO_ERR_LIMIT
                                 (0: automatic, max(65536, 256 x work items))                         */
