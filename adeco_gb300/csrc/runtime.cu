@@ -224,12 +224,16 @@ static int deposit_error(int err, const char *where)
 }
 
 // CTAs that share an item, for n_items items on `slots` CTA slots: with few
-// items most slots would idle, or wait at the end for the last ones.  Two
-// units of work a slot; more gave nothing (a unit repeats the staging of its
-// item's block).  A block has at most 343 cubes.
+// items most slots would idle, or wait at the end for the last ones.  Six
+// units of work a slot, since a unit repeats the staging of its item's block:
+// with 2 / 6 / 12 / 24 the smallest boundary call takes 159 / 151 / 158 / 156 us,
+// ragged patches 1.74 / 1.55 / 1.48 / 1.52 ms, a periodic 64^3 lattice 9.06 / 8.77 /
+// 9.17 / 9.86, 64^3 leaves 0.758 / 0.749 / 0.785 / 0.854.  A block has at most 343
+// cubes.
 int item_parts(int n_items, int slots)
 {
-    return std::max(1, std::min((2 * slots + n_items - 1) / n_items, kMaxCubes));
+    constexpr int kUnits = 6;
+    return std::max(1, std::min((kUnits * slots + n_items - 1) / n_items, kMaxCubes));
 }
 
 // One persistent launch of the mixed kernel over `n_items` items, then the
