@@ -295,7 +295,9 @@ constexpr long long kMaxPairsPerTet = 1LL << 25;
 // its vertices as FP32 pairs (hi + lo) and the FP32 normal n: 3 d = n . (va
 // + vb + vc) in double-float, divided by 3 as a product with 1/3 whose
 // remainder (exact, fma) is carried into the low part, so that d_hi + d_lo
-// keeps ~44 bits.
+// keeps ~44 bits.  kStored: both products rounded, as if the offset had been
+// stored (else the compiler may contract them into the sums they go to).
+template <bool kStored = false>
 ADECO_HD inline F2 plane_offset(const float qa[3], const float la[3], const float qb[3], const float lb[3],
                                 const float qc[3], const float lc[3], const float n[3])
 {
@@ -306,6 +308,10 @@ ADECO_HD inline F2 plane_offset(const float qa[3], const float la[3], const floa
         dd = f2_add(dd, f2_mul_f(sum, n[a]));
     }
     constexpr float kThird = 1.f / 3.f;
+    if constexpr (kStored) {
+        const float d_hi = mul_rn(dd.hi, kThird);
+        return {d_hi, mul_rn(fmaf(-d_hi, 3.f, dd.hi) + dd.lo, kThird)};
+    }
     const float d_hi = dd.hi * kThird;
     return {d_hi, (fmaf(-d_hi, 3.f, dd.hi) + dd.lo) * kThird};
 }
@@ -587,7 +593,7 @@ ADECO_HD inline int classify_pair(const Table &W, const GridDesc &g, int s, int 
 // n . origin - (d + dlo) cancels terms as large as the tet is wide in cells:
 // it is formed exactly in double-float (TwoProd of n with the integer cell
 // offsets) and kept as a pair for the corner values.
-template <bool kExactD = true, class Table>
+template <bool kExactD = true, bool kStored = false, class Table>
 ADECO_HD inline F2 face_value_at_cell(const Table &W, const GridDesc &g, int s, int a, int b, int c, int f)
 {
     const int cc[3] = {a, b, c};
@@ -618,7 +624,7 @@ ADECO_HD inline F2 face_value_at_cell(const Table &W, const GridDesc &g, int s, 
             tet_coord(W, g, s, fb, x, q[1][x], l[1][x]);
             tet_coord(W, g, s, fc, x, q[2][x], l[2][x]);
         }
-        const F2 d = plane_offset(q[0], l[0], q[1], l[1], q[2], l[2], n);
+        const F2 d = plane_offset<kStored>(q[0], l[0], q[1], l[1], q[2], l[2], n);
         G = {-d.hi, -d.lo};
     }
     float small = 0.f;  // the cells' deviation from unit size: n_x c_x dr_x, tiny
@@ -633,7 +639,7 @@ ADECO_HD inline F2 face_value_at_cell(const Table &W, const GridDesc &g, int s, 
 
 // 6x volume of cell (a, b, c) ∩ slot s's tet when the cell straddles only
 // face f: the cube's part on its inside.
-template <bool kExactD = true, class Table>
+template <bool kExactD = true, bool kStored = false, class Table>
 #ifdef __CUDA_ARCH__
 __device__ __noinline__
 #else
@@ -642,7 +648,7 @@ inline
 float halfspace_pair_vol6(const Table &W, const GridDesc &g, int s, int a, int b, int c, int f)
 {
     const float4 n = face_plane(W, f, s);
-    return halfspace_cube_vol6(face_value_at_cell<kExactD>(W, g, s, a, b, c, f), n.x, n.y, n.z);
+    return halfspace_cube_vol6(face_value_at_cell<kExactD, kStored>(W, g, s, a, b, c, f), n.x, n.y, n.z);
 }
 
 // Non-negative mass of a pair (FP32, about 1e-7 relative) -> the cell's
@@ -1033,7 +1039,7 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
                         const uint32_t e = S.list.cell[kPairs - 1 - j];
                         const int s = S.list.tet[kPairs - 1 - j];
                         const int3 c = pair_cell(S.wt, s, e & 0x3fffffffu, wide);
-                        const float m = halfspace_pair_vol6<false>(S.wt, S.g, s, c.x, c.y, c.z, (int)(e >> 30)) * S.wt.f6[s];
+                        const float m = halfspace_pair_vol6<false, kExactD>(S.wt, S.g, s, c.x, c.y, c.z, (int)(e >> 30)) * S.wt.f6[s];
                         if (m > 0.f) scatter(P, S.g, S.wt, s, c.x, c.y, c.z, m);
                     }
                     __syncwarp();
