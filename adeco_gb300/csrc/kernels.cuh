@@ -185,7 +185,7 @@ struct SharedMixed {
     int start[kWave];
     uint8_t tet[kWave];
     int warp_pairs[kWarps];
-    int cursor;          // first candidate pair of the wave not yet taken
+    int cursor;          // first candidate pair of the wave's part not yet taken
     int cut[2];          // one-face pairs at the list's end (alternating as list.n),
     int cut_next[2];     //   and the first not taken
     int wide[2];         // a tet of the wave (even, odd) has more than 1024 candidate cells along an axis
@@ -286,10 +286,33 @@ __device__ __forceinline__ bool cube_alive(const SharedMixed &S, int v0, int vx,
 }
 
 // ------------------------------------------------------ per-tet set-up
-// Candidate pairs of one tet are limited to kMaxPairsPerTet so that the
-// per-warp flattened pair index fits 32 bits and a queue entry (5-bit slot,
-// 27-bit local index); a larger tet sets the error flag and is skipped.
+// Candidate pairs of one tet are limited to kMaxPairsPerTet, so that a pair's
+// number within its tet leaves the top bits of a list entry free and a warp's
+// 32 tets have at most 2^30 of them; a larger tet sets the error flag and is
+// skipped.
 constexpr long long kMaxPairsPerTet = 1LL << 25;
+
+// The pairs of a wave's tets are numbered through in an int, but those of its
+// 8 warps may be 2^33 (tets that each cover a grid of hundreds of cells an
+// axis).  They are taken in parts: the warps [first, end) whose pairs together
+// stay below 2^31, the 32 that each warp may add to the cursor past the end
+// among them.  Returns end > first; total: the part's pairs.  Nearly every
+// wave is one part.
+constexpr int kMaxPartPairs = INT_MAX - 32 * kWarps;
+static_assert(32 * kMaxPairsPerTet <= kMaxPartPairs, "a warp's pairs fit a part");
+
+ADECO_HD inline int wave_part(const int *warp_pairs, int first, int &total)
+{
+    int end = first;
+    total = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+        const bool take = w == end && warp_pairs[w] <= kMaxPartPairs - total;
+        total += take ? warp_pairs[w] : 0;
+        end += take;
+    }
+    return end;
+}
 
 // Offset of a tet face's plane n . x = d through the face's centroid, from
 // its vertices as FP32 pairs (hi + lo) and the FP32 normal n: 3 d = n . (va
@@ -846,22 +869,23 @@ __device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &
     if (lane == 31) S.warp_pairs[warp] = incl;
 }
 
-// Classify phase: the warps take the wave's candidate pairs 32 at a time and
-// classify them; inside cells are deposited at once, partial cells listed, and
-// those that one face cuts at the list's end (with the face in the top bits):
-// their closed form, for a few lanes of nearly every 32, had taken more than
-// the classification itself.  Until no pair is left or the list might not hold
-// the 32 pairs each warp may have in hand (`room` of it are used).
+// Classify phase: the warps take the candidate pairs of the wave's part, those
+// of the tets of warps [w0, w1), 32 at a time and classify them; inside cells
+// are deposited at once, partial cells listed, and those that one face cuts at
+// the list's end (with the face in the top bits): their closed form, for a few
+// lanes of nearly every 32, had taken more than the classification itself.
+// Until no pair is left or the list might not hold the 32 pairs each warp may
+// have in hand (`room` of it are used).
 template <bool kStats>
-__device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixed &S, int *list_n, int *cut_n, int room, bool wide,
-                                              PairStats &st)
+__device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixed &S, int w0, int w1, int *list_n,
+                                              int *cut_n, int room, bool wide, PairStats &st)
 {
     const int lane = threadIdx.x & 31;
     const unsigned le = 0xffffffffu >> (31 - lane);
     const WaveTets &W = S.wt;
     const GridDesc &g = S.g;
     // lane w: warp w's pairs, and the pairs of the warps before it
-    const int own = lane < kWarps ? S.warp_pairs[lane] : 0;
+    const int own = lane >= w0 && lane < w1 ? S.warp_pairs[lane] : 0;
     int pre = own;
 #pragma unroll
     for (int o = 1; o < kWarps; o <<= 1) {
@@ -992,13 +1016,11 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
             wave_setup<kExactD>(P, S, it, first, min(first + wave, ntet), vx, vy, odd, st.tets);
             __syncthreads();
             const bool wide = S.wide[odd] != 0;
-            int total = 0;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) total += S.warp_pairs[w];
+            int w0 = 0, total, w1 = wave_part(S.warp_pairs, 0, total);
             bool left = total > 0;
             if (!left) __syncthreads();  // the next wave's set-up writes what this one's warps read above
             while (left) {
-                wave_classify<kStats>(P, S, &S.list.n[turn], &S.cut[turn], room, wide, st);
+                wave_classify<kStats>(P, S, w0, w1, &S.list.n[turn], &S.cut[turn], room, wide, st);
                 __syncthreads();
                 left = S.cursor < total;
                 const int np = S.list.n[turn];
@@ -1046,6 +1068,13 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
                 }
                 turn ^= 1;
                 __syncthreads();
+                if (!left && w1 < kWarps) {  // the wave's next part
+                    w0 = w1;
+                    w1 = wave_part(S.warp_pairs, w0, total);
+                    left = true;
+                    if (threadIdx.x == 0) S.cursor = 0;
+                    __syncthreads();
+                }
             }
             odd ^= 1;
         }

@@ -1,0 +1,40 @@
+"""GPU: calls at the limits of the kernels' counts and of the caller's memory."""
+import numpy as np
+import pytest
+
+from test_deposit_gpu import adeco  # noqa: F401  (the fixture)
+
+pytestmark = pytest.mark.gpu
+
+
+def folded_patches(m, count):
+    """Patch 0 folds its cubes onto the unit cube (vertex i at i mod 2) and
+    leaves 11 of them, 66 tets, alive; the others are padding."""
+    v = m + 1
+    p = np.full((count, v, v, v, 3), 666.0, np.float32)
+    z, y, x = np.meshgrid(*[np.arange(v)] * 3, indexing="ij")
+    own = np.stack([x % 2, y % 2, z % 2], -1).astype(np.float32)
+    p[0, :2] = own[:2]            # the 9 cubes of the lowest layer
+    p[0, 2, :2, :3] = own[2, :2, :3]  # and 2 of the next
+    return p.reshape(-1)
+
+
+def test_wave_of_more_than_2_31_pairs(adeco):
+    """66 tets of one block that each cover a grid of 322^3 cells: 2.2e9
+    candidate pairs in one wave (2000 patches, so that each is one unit of
+    work), against the FP64 path.
+
+    A partial cell's share comes from FP32 coordinates of up to 644 cells,
+    rounded by 4e-5 of a cell (6e-8 relative): under 1e-3 of the mean cell.
+    Cells cut by a face are a few in a hundred, and a sum's quantum, 2^-43, is
+    5e-6 of a cube's mass in a cell, rounded the same way in most cells: the
+    total holds to 1e-5."""
+    m, count, dims = 3, 2000, 322
+    box = np.array([0.25, 0.75] * 3, np.float32)
+    pos = folded_patches(m, count)
+    got = adeco.deposit_tets_ex(pos, m, box, dims, num_patches=count)
+    want = adeco.deposit_tets_ex(pos, m, box, dims, num_patches=1, precision=1)  # the padding adds nothing
+    # the reference's corner order covers a cube once on average, not evenly
+    assert abs(want.mean() / (66.0 * (0.5 / dims) ** 3) - 1.0) < 1e-2
+    assert abs(got.sum() / want.sum() - 1.0) < 1e-5
+    assert np.abs(got - want).max() < 1e-3 * want.mean()
