@@ -143,6 +143,10 @@ __device__ __forceinline__ bool wait_zero_bounded(const int *count, unsigned lim
     return true;
 }
 
+// A tet of the wave has more than 1024 candidate cells along an axis; a warp
+// has more than kMaxPartPairs / kWarps candidate pairs.
+constexpr int kWideTet = 1, kManyPairs = 2;
+
 // The staged vertex block and the wave's tets.
 struct WaveTets : TetPlanes<kWave> {
     static constexpr bool kHasRest = false;
@@ -185,10 +189,11 @@ struct SharedMixed {
     int start[kWave];
     uint8_t tet[kWave];
     int warp_pairs[kWarps];
-    int cursor;          // first candidate pair of the wave's part not yet taken
+    int all_pairs[kWarps], part_end;  // of a wave taken in parts: its warps' pairs, the warps taken (wave_next_part)
+    int cursor;          // first candidate pair of the wave not yet taken
     int cut[2];          // one-face pairs at the list's end (alternating as list.n),
     int cut_next[2];     //   and the first not taken
-    int wide[2];         // a tet of the wave (even, odd) has more than 1024 candidate cells along an axis
+    int flags[2];        // of the wave (even, odd): kWideTet, kManyPairs
     PairList list;
     WarpPool pool[kWarps];
 };
@@ -296,8 +301,9 @@ constexpr long long kMaxPairsPerTet = 1LL << 25;
 // 8 warps may be 2^33 (tets that each cover a grid of hundreds of cells an
 // axis).  They are taken in parts: the warps [first, end) whose pairs together
 // stay below 2^31, the 32 that each warp may add to the cursor past the end
-// among them.  Returns end > first; total: the part's pairs.  Nearly every
-// wave is one part.
+// among them.  Returns end > first; total: the part's pairs.  A wave without
+// kManyPairs is one part and does not ask (asking took 0.6% of the time of
+// octree leaves).
 constexpr int kMaxPartPairs = INT_MAX - 32 * kWarps;
 static_assert(32 * kMaxPairsPerTet <= kMaxPartPairs, "a warp's pairs fit a part");
 
@@ -844,7 +850,7 @@ __device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &
                     l = S.wt.gl[a][v];
                 },
                 S.g, S.wt, slot, P.error, &route64, &wide);
-        if (cnt > 0 && wide) S.wide[odd] = 1;
+        if (cnt > 0 && wide) atomicOr(&S.flags[odd], kWideTet);
     }
     n_tets += (cnt > 0);
     if (route64 && cnt > 0) {  // deposited by route_fp64_kernel
@@ -866,26 +872,49 @@ __device__ __forceinline__ void wave_setup(const DepositParams &P, SharedMixed &
         S.tet[k] = (uint8_t)slot;
     }
     if (lane >= __popc(some)) S.start[slot] = INT_MAX;
-    if (lane == 31) S.warp_pairs[warp] = incl;
+    if (lane == 31) {
+        S.warp_pairs[warp] = incl;
+        if (incl > kMaxPartPairs / kWarps) atomicOr(&S.flags[odd], kManyPairs);
+    }
 }
 
-// Classify phase: the warps take the candidate pairs of the wave's part, those
-// of the tets of warps [w0, w1), 32 at a time and classify them; inside cells
-// are deposited at once, partial cells listed, and those that one face cuts at
-// the list's end (with the face in the top bits): their closed form, for a few
-// lanes of nearly every 32, had taken more than the classification itself.
-// Until no pair is left or the list might not hold the 32 pairs each warp may
-// have in hand (`room` of it are used).
+// The next part of a wave that has kManyPairs, from warp `first` on: the pairs
+// of the other warps are set to none.  Returns the part's pairs, 0 after the
+// last.  (The whole CTA.)
+__device__ __noinline__ int wave_next_part(SharedMixed &S, int first)
+{
+    if (first == 0) {
+        if (threadIdx.x < kWarps) S.all_pairs[threadIdx.x] = S.warp_pairs[threadIdx.x];
+        __syncthreads();
+    }
+    int total;
+    const int end = wave_part(S.all_pairs, first, total), w = threadIdx.x;
+    __syncthreads();
+    if (w < kWarps) S.warp_pairs[w] = w >= first && w < end ? S.all_pairs[w] : 0;
+    if (w == 0) {
+        S.cursor = 0;
+        S.part_end = end;
+    }
+    __syncthreads();
+    return total;
+}
+
+// Classify phase: the warps take the wave's candidate pairs 32 at a time and
+// classify them; inside cells are deposited at once, partial cells listed, and
+// those that one face cuts at the list's end (with the face in the top bits):
+// their closed form, for a few lanes of nearly every 32, had taken more than
+// the classification itself.  Until no pair is left or the list might not hold
+// the 32 pairs each warp may have in hand (`room` of it are used).
 template <bool kStats>
-__device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixed &S, int w0, int w1, int *list_n,
-                                              int *cut_n, int room, bool wide, PairStats &st)
+__device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixed &S, int *list_n, int *cut_n, int room, bool wide,
+                                              PairStats &st)
 {
     const int lane = threadIdx.x & 31;
     const unsigned le = 0xffffffffu >> (31 - lane);
     const WaveTets &W = S.wt;
     const GridDesc &g = S.g;
     // lane w: warp w's pairs, and the pairs of the warps before it
-    const int own = lane >= w0 && lane < w1 ? S.warp_pairs[lane] : 0;
+    const int own = lane < kWarps ? S.warp_pairs[lane] : 0;
     int pre = own;
 #pragma unroll
     for (int o = 1; o < kWarps; o <<= 1) {
@@ -977,7 +1006,7 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
     const int warp = threadIdx.x >> 5;
     PairStats st;
     int turn = 0, odd = 0;  // the pair list's counters and the wave's flag in use
-    if (threadIdx.x == 0) S.wide[0] = S.list.n[0] = S.list.next[0] = S.cut[0] = S.cut_next[0] = 0;
+    if (threadIdx.x == 0) S.flags[0] = S.list.n[0] = S.list.next[0] = S.cut[0] = S.cut_next[0] = 0;
     const int room = kPairs / kQueue * min(max(P.clip_batch, 64), kQueue);
 
     for (int taken = 0;; ++taken) {
@@ -1012,15 +1041,21 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
         const int nwave = (ntet + kWave - 1) / kWave, wave = nwave ? (ntet + nwave - 1) / nwave : 0;
         for (int first = 0; first < ntet; first += wave) {
             // every warp is through with the wave before
-            if (threadIdx.x == 0) S.cursor = S.wide[odd ^ 1] = 0;
+            if (threadIdx.x == 0) S.cursor = S.flags[odd ^ 1] = 0;
             wave_setup<kExactD>(P, S, it, first, min(first + wave, ntet), vx, vy, odd, st.tets);
             __syncthreads();
-            const bool wide = S.wide[odd] != 0;
-            int w0 = 0, total, w1 = wave_part(S.warp_pairs, 0, total);
+            const int flags = S.flags[odd];
+            const bool wide = (flags & kWideTet) != 0;
+            int total = 0;
+            if (flags & kManyPairs)
+                total = wave_next_part(S, 0);
+            else
+#pragma unroll
+                for (int w = 0; w < kWarps; ++w) total += S.warp_pairs[w];
             bool left = total > 0;
             if (!left) __syncthreads();  // the next wave's set-up writes what this one's warps read above
             while (left) {
-                wave_classify<kStats>(P, S, w0, w1, &S.list.n[turn], &S.cut[turn], room, wide, st);
+                wave_classify<kStats>(P, S, &S.list.n[turn], &S.cut[turn], room, wide, st);
                 __syncthreads();
                 left = S.cursor < total;
                 const int np = S.list.n[turn];
@@ -1068,12 +1103,9 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
                 }
                 turn ^= 1;
                 __syncthreads();
-                if (!left && w1 < kWarps) {  // the wave's next part
-                    w0 = w1;
-                    w1 = wave_part(S.warp_pairs, w0, total);
-                    left = true;
-                    if (threadIdx.x == 0) S.cursor = 0;
-                    __syncthreads();
+                if (!left && (flags & kManyPairs)) {
+                    total = wave_next_part(S, S.part_end);
+                    left = total > 0;
                 }
             }
             odd ^= 1;
