@@ -899,6 +899,15 @@ __device__ __noinline__ int wave_next_part(SharedMixed &S, int first)
     return total;
 }
 
+// Of 32 pairs, the bit of the one a tet starts at: its start and the pair
+// `skip` in the numbering of its warp (start: INT_MAX for none).  0 if it is at
+// or before that pair or past the 32.
+ADECO_HD inline unsigned start_bit(int start, int rel, int skip)
+{
+    const unsigned at = (unsigned)start - (unsigned)rel + (unsigned)skip;  // below 2^32: no wrap for a start past rel
+    return start > rel && at < 32u ? 1u << at : 0u;
+}
+
 // Classify phase: the warps take the wave's candidate pairs 32 at a time and
 // classify them; inside cells are deposited at once, partial cells listed, and
 // those that one face cuts at the list's end (with the face in the top bits):
@@ -938,9 +947,9 @@ __device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixe
         for (int q0 = c0;;) {
             const int w = __popc(__ballot_sync(0xffffffffu, lane < kWarps && pre <= q0)) - 1;
             const int before = __shfl_sync(0xffffffffu, pre, w), end = before + __shfl_sync(0xffffffffu, own, w);
-            const int start = S.start[32 * w + lane], rel = q0 - before, at = start - rel + (q0 - c0);
+            const int start = S.start[32 * w + lane], rel = q0 - before;
             const int first = __popc(__ballot_sync(0xffffffffu, start <= rel)) - 1;
-            const unsigned starts = __reduce_or_sync(0xffffffffu, (start > rel && at < 32) ? 1u << at : 0u);
+            const unsigned starts = __reduce_or_sync(0xffffffffu, start_bit(start, rel, q0 - c0));
             const int k = first + __popc(starts & le), from = __shfl_sync(0xffffffffu, start, k);
             if (pidx >= q0 && pidx < end) {
                 s = S.tet[32 * w + k];

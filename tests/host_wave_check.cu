@@ -1,7 +1,9 @@
 // Host check of the rule by which the mixed kernel takes a wave's candidate
 // pairs in parts (wave_part): the parts cover the warps in order, and a part's
 // pairs, with the 32 that each warp may add to the cursor past the end, fit an
-// int.  Built for the host only; no GPU.
+// int.  And of where a tet's pairs start among 32 (start_bit).  Built for the
+// host only, with the compiler's check for undefined behaviour where it has
+// one; no GPU.
 #include "../adeco_gb300/csrc/kernels.cuh"
 
 #include <climits>
@@ -52,6 +54,19 @@ int main()
         for (int w = 0; w < kWarps; ++w) pairs[w] = (int)(rng() % (unsigned)(most + 1)) >> (rng() % 31);
         parts_of(pairs);
     }
+    // a tet's start among the 32 pairs that a warp takes, against 64-bit arithmetic
+    const int rels[] = {0, 1, 31, 32, 1 << 20, (1 << 30) - 1, 1 << 30};
+    for (int rel : rels)
+        for (int skip = 0; skip < 32; ++skip) {
+            const long long starts[] = {0, 1, rel - 1LL, rel, rel + 1LL, rel + 31LL - skip, rel + 32LL - skip, rel + 33LL,
+                                        (1LL << 30) - 1, INT_MAX - 1LL, INT_MAX};
+            for (long long start : starts) {
+                if (start < 0) continue;
+                const long long at = start - rel + skip;
+                const unsigned want = start > rel && at < 32 ? 1u << at : 0u;
+                bad += start_bit((int)start, rel, skip) != want;
+            }
+        }
     std::printf("parts of a wave: %s (%ld)\n", bad ? "FAIL" : "ok", bad);
     return bad ? 1 : 0;
 }
