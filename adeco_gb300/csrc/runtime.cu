@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "../../include/adeco_deposit.h"
+#include "host_grid.h"
 #include "kernels.cuh"
 #include "octree.h"
 
@@ -536,16 +537,16 @@ extern "C" int adeco_deposit_tets_ex(const adeco_deposit_args *a)
         // Grids of up to 64 MB: all their pages are touched while the device
         // works and the sums added behind the deposit.  Larger ones wait for
         // the box, and only its rows are touched.
-        const bool small = ncell * cell <= ((size_t)64 << 20);
-        if (dp.host_tables && small) {
+        const bool small = ncell * cell <= ((size_t)64 << 20), on_device = device_adds(dp.host_tables, a->data, cell);
+        if (on_device && small) {
             const int lo[3] = {0, 0, 0}, ext[3] = {a->dims, a->dims, a->dims};
             touch_rows(a->data, cell, a->dims, lo, ext);
             if (int e = add_on_device()) return e;
         }
         if (int e = read_status()) return e;
         if (t_work.status->error) return deposit_error(t_work.status->error, "the grid");
-        if (box.empty || (dp.host_tables && small)) return ADECO_OK;
-        if (dp.host_tables) {
+        if (box.empty || (on_device && small)) return ADECO_OK;
+        if (on_device) {
             touch_rows(a->data, cell, a->dims, box.lo, box.ext);
             if (int e = add_on_device()) return e;
             CUDA_TRY(cudaStreamSynchronize(st));
@@ -567,19 +568,10 @@ extern "C" int adeco_deposit_tets_ex(const adeco_deposit_args *a)
         if (int e = t_work.staging(nbox)) return e;
         CUDA_TRY(cudaMemcpyAsync(t_work.pinned, dsrc, nbox * sizeof(double), cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
-        const size_t d = (size_t)a->dims;
-        for (int z = 0; z < box.ext[2]; ++z)
-            for (int y = 0; y < box.ext[1]; ++y) {
-                const double *row = t_work.pinned + (size_t)box.ext[0] * (y + (size_t)box.ext[1] * z);
-                const size_t c0 = (size_t)box.lo[0] + d * ((size_t)(box.lo[1] + y) + d * (size_t)(box.lo[2] + z));
-                if (a->out_type == ADECO_OUT_F64) {
-                    double *out = (double *)a->data + c0;
-                    for (int x = 0; x < box.ext[0]; ++x) out[x] += row[x];
-                } else {
-                    float *out = (float *)a->data + c0;
-                    for (int x = 0; x < box.ext[0]; ++x) out[x] += (float)row[x];
-                }
-            }
+        if (a->out_type == ADECO_OUT_F64)
+            add_box<double>(a->data, t_work.pinned, a->dims, box.lo, box.ext);
+        else
+            add_box<float>(a->data, t_work.pinned, a->dims, box.lo, box.ext);
         return ADECO_OK;
     }();
     if (rc) cudaStreamSynchronize(st);

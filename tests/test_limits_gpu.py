@@ -38,3 +38,30 @@ def test_wave_of_more_than_2_31_pairs(adeco):
     assert abs(want.mean() / (66.0 * (0.5 / dims) ** 3) - 1.0) < 1e-2
     assert abs(got.sum() / want.sum() - 1.0) < 1e-5
     assert np.abs(got - want).max() < 1e-3 * want.mean()
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["mixed", "plain_fp64"])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("box", [(0.5, 4.5), (-9.0, 3.0), (40.0, 44.0)], ids=["whole", "part", "empty"])
+def test_grid_off_its_cells_alignment(adeco, box, dtype, precision):
+    """A caller's grid that starts between two cells gains what an aligned one
+    does: the sums come back and are added by the host.  (Bit for bit; the FP64
+    path's atomic sums differ by their order, some 100 adds a cell: 1e-13.)"""
+    dims, m = 21, 5
+    rng = np.random.default_rng(5)
+    v = np.stack(np.meshgrid(*[np.arange(m + 1.0)] * 3, indexing="ij"), -1)[..., ::-1]
+    pos = (v + rng.uniform(-0.3, 0.3, v.shape)).astype(np.float32).reshape(-1)
+    bb = np.array(box * 3, np.float32)
+    n, size = dims ** 3, np.dtype(dtype).itemsize
+    pre = rng.uniform(0.5, 2.0, n).astype(dtype)
+    want = adeco.deposit_tets_ex(pos, m, bb, dims, data=pre.copy(), precision=precision)
+    for offset in (1, 2, size - 1, size + 2):
+        room = np.full(n * size + 32, 7, np.uint8)
+        room[offset:offset + n * size] = pre.view(np.uint8)
+        got = room[offset:offset + n * size].view(dtype)
+        assert not got.flags.aligned and got.flags.c_contiguous
+        adeco.deposit_tets_ex(pos, m, bb, dims, data=got, precision=precision)
+        got = np.array(got)
+        assert np.array_equal(got, want) if precision == 0 else np.allclose(got, want, rtol=1e-13 if size == 8 else 1e-6)
+        assert np.all(room[:offset] == 7) and np.all(room[offset + n * size:] == 7)
+    assert (want.sum() > pre.sum()) == (box[0] < 40.0)
