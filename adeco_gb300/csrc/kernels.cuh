@@ -1279,8 +1279,10 @@ __global__ void patch_items_kernel(Item *items, long long *cube_off, long long p
 
 // Adds a pass's block boxes (patch_bbox_kernel) to the call's box and forms its
 // cell range: one cell of margin against the rounding of the kernels' FP32
-// range arithmetic; a NaN coordinate takes the whole grid.
-__global__ void __launch_bounds__(7 * 32) call_box_kernel(const float *part, int nblocks, const GridDesc *gp, CallBox *box)
+// range arithmetic; a NaN coordinate takes the whole grid.  host: a copy for the
+// host, in page-locked memory, or null.
+__global__ void __launch_bounds__(7 * 32) call_box_kernel(const float *part, int nblocks, const GridDesc *gp, CallBox *box,
+                                                          CallBox *host)
 {
     const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;  // a warp per number of the box, the last for the NaN flag
     float r = q < 3 ? INFINITY : (q < 6 ? -INFINITY : 0.f);
@@ -1319,7 +1321,10 @@ __global__ void __launch_bounds__(7 * 32) call_box_kernel(const float *part, int
         box->ext[a] = ext;
     }
     empty = __any_sync(0xffffffffu, empty);
-    if (lane == 0) box->empty = empty;
+    if (lane == 0) {
+        box->empty = empty;
+        if (host) *host = *box;
+    }
 }
 
 // A pass's sums of the box's cells, from the fixed point grid (times scale)

@@ -333,10 +333,11 @@ struct BoundaryWork {
     DevBuf<CallBox> box;
     double *pinned = nullptr;  // D2H staging of the grid
     size_t pinned_n = 0;
-    struct Status {  // what a call reads back at its end
+    struct Status {  // what a call brings back besides its sums (page-locked)
         int error;
         CallBox box;
     } *status = nullptr;
+    cudaEvent_t box_ready = nullptr;  // status->box is written
     ~BoundaryWork() { drop(); }
     void drop()
     {
@@ -348,6 +349,8 @@ struct BoundaryWork {
         pinned_n = 0;
         if (status) cudaFreeHost(status);
         status = nullptr;
+        if (box_ready) cudaEventDestroy(box_ready);
+        box_ready = nullptr;
         if (stream) cudaStreamDestroy(stream);
         stream = nullptr;
     }
@@ -363,6 +366,7 @@ struct BoundaryWork {
     int status_block()
     {
         if (!status) CUDA_TRY(cudaHostAlloc((void **)&status, sizeof(Status), cudaHostAllocDefault));
+        if (!box_ready) CUDA_TRY(cudaEventCreateWithFlags(&box_ready, cudaEventDisableTiming));
         return ADECO_OK;
     }
     static constexpr int kBoxBlocks = 256;
@@ -383,11 +387,14 @@ thread_local BoundaryWork t_work;
 // Enqueues the deposit of patches [patch_offset, +num_patches) of
 // device-resident patch data into d_fixed (mixed, fixed point 2^shift) or
 // d_f64 (plain FP64).  The device error flag is t_work.counter's second word,
-// cleared by the call's first pass; with_box: t_work.box is kept too.
+// cleared by the call's first pass.  box_blocks: that many block boxes of the
+// pass's vertices (t_work.part) are added to the call's box before the deposit
+// starts, and the last pass's tells the host through status->box and box_ready
+// (0: the call keeps no box).
 static int enqueue_deposit(int dev, const DeviceProps &dp, const float *d_pos, size_t patch_offset, size_t num_patches,
                            int m, const float *bbox, int dims, int precision, int order, double tet_mass,
-                           unsigned long long *d_fixed, double *d_f64, int shift, bool first, bool with_box,
-                           cudaStream_t st)
+                           unsigned long long *d_fixed, double *d_f64, int shift, bool first, int box_blocks,
+                           bool last, cudaStream_t st)
 {
     int rc = t_work.bind(dev);
     if (rc) return rc;
@@ -396,14 +403,20 @@ static int enqueue_deposit(int dev, const DeviceProps &dp, const float *d_pos, s
     const bool plain = precision == ADECO_PREC_FP64;
     const unsigned long long rcap = route_capacity((long long)n_items);
     if ((rc = t_work.items.reserve(n_items)) || (rc = t_work.grid.reserve(1)) || (rc = t_work.counter.reserve(2)) ||
-        (with_box && (rc = t_work.box.reserve(1))))
+        (box_blocks && (rc = t_work.box.reserve(1))))
         return rc;
     if (plain ? (rc = t_work.cube_off.reserve(n_items + 1)) : (rc = t_work.route.reserve(rcap + 1))) return rc;
     patch_items_kernel<<<(unsigned)((n_items + 127) / 128), 128, 0, st>>>(
         t_work.items.p, plain ? t_work.cube_off.p : nullptr, (long long)patch_offset, (int)n_items, m, nsb, t_work.grid.p,
         make_grid(bbox, dims, tet_mass, shift, 0), t_work.counter.p, plain ? nullptr : t_work.route.p,
-        with_box ? t_work.box.p : nullptr, first);
+        box_blocks ? t_work.box.p : nullptr, first);
     CUDA_TRY(cudaGetLastError());
+    if (box_blocks) {
+        call_box_kernel<<<1, 7 * 32, 0, st>>>(t_work.part.p, box_blocks, t_work.grid.p, t_work.box.p,
+                                              last ? &t_work.status->box : nullptr);
+        CUDA_TRY(cudaGetLastError());
+        if (last) CUDA_TRY(cudaEventRecord(t_work.box_ready, st));
+    }
     DepositParams P = base_params(Tuning());
     P.items = t_work.items.p;
     P.n_items = (int)n_items;
@@ -421,29 +434,6 @@ static int enqueue_deposit(int dev, const DeviceProps &dp, const float *d_pos, s
     if (plain) return launch_plain(dp, P, t_work.cube_off.p, 0, (long long)num_patches * m * m * m, st);
     set_route(P, t_work.route.p, rcap);
     return launch_mixed(dp, P, st);
-}
-
-// Makes the pages of rows [lo, lo + ext) of a dims^3 grid of `size`-byte cells
-// present and writable, by writing a cell of each back to itself: a kernel's
-// first write to a page that the host never touched takes tens of microseconds.
-static void touch_rows(void *grid, size_t size, int dims, const int lo[3], const int ext[3])
-{
-    static const size_t page = (size_t)std::max(4096L, sysconf(_SC_PAGESIZE));
-    char *base = static_cast<char *>(grid), *next = base;
-    const size_t d = (size_t)dims;
-    const bool whole = (size_t)ext[0] == d && (size_t)ext[1] == d;
-    const size_t rows = whole ? 1 : (size_t)ext[1] * ext[2];
-    const size_t len = size * (whole ? d * d * (size_t)ext[2] : (size_t)ext[0]);
-    for (size_t r = 0; r < rows; ++r) {
-        const size_t y = lo[1] + r % ext[1], z = lo[2] + r / ext[1];
-        char *a = base + size * ((size_t)lo[0] + d * (y + d * z)), *end = a + len;
-        for (char *p = std::max(a, next); p < end;) {
-            volatile char *v = p;
-            *v = *v;
-            p = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) / page + 1) * page);
-            next = p;
-        }
-    }
 }
 
 extern "C" int adeco_deposit_tets_ex(const adeco_deposit_args *a)
@@ -490,12 +480,11 @@ extern "C" int adeco_deposit_tets_ex(const adeco_deposit_args *a)
     // the fixed-point scale is fixed for the whole call
     const int call_shift = choose_shift(6.0 * (double)a->num_patches * (double)m * m * m, a->tet_mass);
     const double scale = std::ldexp(1.0, -call_shift);
-    // Everything of the call is enqueued, and the host waits once: positions,
-    // the deposit, the box of the deposited vertices (padding left out) over
-    // all passes.  Only the grid cells in its range can receive mass, so only
-    // those are added (an image box of a periodic volume touches a thin slab
-    // of the grid).  On an error the stream is drained before the buffers are
-    // used again.
+    // Positions, the box of the deposited vertices (padding left out) over all
+    // passes and the deposit are enqueued at once.  Only the grid cells in the
+    // box's range can receive mass, so only those are added (an image box of a
+    // periodic volume touches a thin slab of the grid).  On an error the stream
+    // is drained before the buffers are used again.
     rc = [&]() -> int {
         CUDA_TRY(cudaMemsetAsync(sums, 0, ncell * 8, st));
         for (size_t done = 0; done < a->num_patches; done += per_pass) {
@@ -508,21 +497,22 @@ extern "C" int adeco_deposit_tets_ex(const adeco_deposit_args *a)
             patch_bbox_kernel<<<bb_blocks, kBoxThreads, 0, st>>>(d_pos.p, nvert, t_work.part.p);
             CUDA_TRY(cudaGetLastError());
             // every pass uses the call's shift: deposit patches [0, np) of the slice
+            const bool last = done + np == a->num_patches;
             if (int e = enqueue_deposit(dev, dp, d_pos.p, 0, np, m, a->bbox, a->dims, a->precision, a->tet_order,
-                                        a->tet_mass, d_fixed.p, d_f64.p, call_shift, done == 0, true, st))
+                                        a->tet_mass, d_fixed.p, d_f64.p, call_shift, done == 0, bb_blocks, last, st))
                 return e;
-            call_box_kernel<<<1, 7 * 32, 0, st>>>(t_work.part.p, bb_blocks, t_work.grid.p, t_work.box.p);
-            CUDA_TRY(cudaGetLastError());
         }
         const int *d_error = t_work.counter.p + 1;
         const size_t cell = a->out_type == ADECO_OUT_F64 ? sizeof(double) : sizeof(float);
-        const auto read_status = [&]() -> int {
-            CUDA_TRY(cudaMemcpyAsync(&t_work.status->error, d_error, sizeof(int), cudaMemcpyDeviceToHost, st));
-            CUDA_TRY(cudaMemcpyAsync(&t_work.status->box, t_work.box.p, sizeof(CallBox), cudaMemcpyDeviceToHost, st));
-            CUDA_TRY(cudaStreamSynchronize(st));
-            return ADECO_OK;
-        };
-        const auto add_on_device = [&]() -> int {
+        // The box is known before the last pass's deposit starts: while the
+        // device works, the host makes the pages of the box's rows present.
+        // (A device's first write to a page that the host never touched takes
+        // tens of microseconds.)
+        CUDA_TRY(cudaEventSynchronize(t_work.box_ready));
+        const CallBox &box = t_work.status->box;
+        const bool on_device = device_adds(dp.host_tables, a->data, cell);
+        if (on_device && !box.empty) {
+            touch_rows(a->data, cell, a->dims, box.lo, box.ext, (size_t)std::max(4096L, sysconf(_SC_PAGESIZE)));
             const unsigned blocks = (unsigned)std::min<size_t>((size_t)dp.sms * 4, (ncell + 255) / 256);
             if (a->out_type == ADECO_OUT_F64)
                 host_accumulate_kernel<double><<<blocks, 256, 0, st>>>(plain ? nullptr : d_fixed.p, d_f64.p,
@@ -531,27 +521,11 @@ extern "C" int adeco_deposit_tets_ex(const adeco_deposit_args *a)
                 host_accumulate_kernel<float><<<blocks, 256, 0, st>>>(plain ? nullptr : d_fixed.p, d_f64.p,
                                                                       (float *)a->data, a->dims, t_work.box.p, d_error, scale);
             CUDA_TRY(cudaGetLastError());
-            return ADECO_OK;
-        };
-        const CallBox &box = t_work.status->box;
-        // Grids of up to 64 MB: all their pages are touched while the device
-        // works and the sums added behind the deposit.  Larger ones wait for
-        // the box, and only its rows are touched.
-        const bool small = ncell * cell <= ((size_t)64 << 20), on_device = device_adds(dp.host_tables, a->data, cell);
-        if (on_device && small) {
-            const int lo[3] = {0, 0, 0}, ext[3] = {a->dims, a->dims, a->dims};
-            touch_rows(a->data, cell, a->dims, lo, ext);
-            if (int e = add_on_device()) return e;
         }
-        if (int e = read_status()) return e;
+        CUDA_TRY(cudaMemcpyAsync(&t_work.status->error, d_error, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaStreamSynchronize(st));
         if (t_work.status->error) return deposit_error(t_work.status->error, "the grid");
-        if (box.empty || (on_device && small)) return ADECO_OK;
-        if (on_device) {
-            touch_rows(a->data, cell, a->dims, box.lo, box.ext);
-            if (int e = add_on_device()) return e;
-            CUDA_TRY(cudaStreamSynchronize(st));
-            return ADECO_OK;
-        }
+        if (box.empty || on_device) return ADECO_OK;
         // convert the box's cells to FP64 packed, bring them back, add them
         // into the caller's grid
         const size_t nbox = (size_t)box.ext[0] * box.ext[1] * box.ext[2];
@@ -618,14 +592,14 @@ extern "C" int adeco_deposit_tets_device(const float *d_positions, size_t positi
     rc = [&]() -> int {
         if (precision == ADECO_PREC_FP64) {
             if (int e = enqueue_deposit(dev, dp, d_positions, patch_offset, num_patches, m, bbox, dims, precision, tet_order,
-                                        tet_mass, nullptr, d_out, shift, true, false, st))
+                                        tet_mass, nullptr, d_out, shift, true, 0, true, st))
                 return e;
         } else {
             DevBuf<unsigned long long> &d_fixed = t_work.fixed;
             if (int e = d_fixed.reserve(ncell)) return e;
             CUDA_TRY(cudaMemsetAsync(d_fixed.p, 0, ncell * sizeof(unsigned long long), st));
             if (int e = enqueue_deposit(dev, dp, d_positions, patch_offset, num_patches, m, bbox, dims, precision, tet_order,
-                                        tet_mass, d_fixed.p, nullptr, shift, true, false, st))
+                                        tet_mass, d_fixed.p, nullptr, shift, true, 0, true, st))
                 return e;
             fixed_accumulate_f64_kernel<<<1024, 256, 0, st>>>(d_fixed.p, d_out, (long long)ncell, std::ldexp(1.0, -shift),
                                                               t_work.counter.p + 1);

@@ -1,4 +1,7 @@
 """GPU: calls at the limits of the kernels' counts and of the caller's memory."""
+import ctypes
+import mmap
+
 import numpy as np
 import pytest
 
@@ -65,3 +68,30 @@ def test_grid_off_its_cells_alignment(adeco, box, dtype, precision):
         assert np.array_equal(got, want) if precision == 0 else np.allclose(got, want, rtol=1e-13 if size == 8 else 1e-6)
         assert np.all(room[:offset] == 7) and np.all(room[offset + n * size:] == 7)
     assert (want.sum() > pre.sum()) == (box[0] < 40.0)
+
+
+@pytest.mark.parametrize("shift,rows", [(0.0, (0, 3)), (50.0, (23, 28)), (-200.0, None)], ids=["corner", "slab", "outside"])
+def test_only_the_pages_of_the_box_become_resident(adeco, shift, rows):
+    """A 64 MB grid that the caller never touched: a call that meets some
+    layers of cells makes the pages of those resident, a call beside the grid
+    none."""
+    dims, m = 256, 4
+    page = mmap.PAGESIZE
+    rng = np.random.default_rng(3)
+    v = np.stack(np.meshgrid(*[np.arange(m + 1.0)] * 3, indexing="ij"), -1)[..., ::-1] + rng.uniform(-0.2, 0.2, (m + 1,) * 3 + (3,))
+    v[..., 2] += shift
+    box = np.array([0.5, 512.5] * 3, np.float32)  # cells of 2
+    mem = mmap.mmap(-1, 4 * dims ** 3, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+    mem.madvise(mmap.MADV_NOHUGEPAGE)
+    grid = np.frombuffer(mem, np.float32)
+    adeco.deposit_tets_ex(v.astype(np.float32).reshape(-1), m, box, dims, data=grid)
+    vec = (ctypes.c_ubyte * (len(mem) // page))()
+    libc = ctypes.CDLL(None, use_errno=True)
+    assert libc.mincore(ctypes.c_void_p(grid.ctypes.data), ctypes.c_size_t(len(mem)), vec) == 0
+    resident = np.flatnonzero(np.frombuffer(vec, np.uint8) & 1) * page // (4 * dims * dims)  # their layers
+    if rows is None:
+        assert resident.size == 0
+    else:
+        assert resident.size > 0 and resident.min() >= rows[0] and resident.max() <= rows[1]
+        assert grid.sum() > 0
+    assert (grid.sum() == 0) == (rows is None)
