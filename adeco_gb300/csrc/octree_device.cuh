@@ -255,10 +255,10 @@ struct LeafList {
 };
 
 // A leaf's work items (leaf x meta-cell) from its list, a block per leaf; the
-// lists back to back (ids_out), the items' cube offsets within their leaf and
-// the leaf's cubes.
+// lists back to back (ids_out, where a list may be already), the items' cube
+// offsets within their leaf and the leaf's cubes.
 __global__ void __launch_bounds__(kTreeThreads) leaf_items_kernel(const LeafList *__restrict__ leaves, TreeMeta md,
-                                                                  Item *__restrict__ items, unsigned *__restrict__ ids_out,
+                                                                  Item *__restrict__ items, unsigned *ids_out,
                                                                   long long *__restrict__ cube_off,
                                                                   unsigned *__restrict__ leaf_cubes)
 {

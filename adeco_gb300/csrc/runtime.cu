@@ -976,38 +976,49 @@ extern "C" int adeco_session_build_octree(adeco_session *s, const float *box6, c
         (rc = s->d_route.reserve(s->route_cap + 1)) || (rc = s->d_leaf_back.reserve(s->n_items + nl)) ||
         (rc = s->d_leaf_lists.reserve(nl * sizeof(LeafList))))
         return rc;
-    if (s->octree_builder != ADECO_OCTREE_DEVICE) {
-        // the host builder's lists go to where the items kernel writes them
-        s->leaf_back.assign(s->tree.leaf_meta_ids.begin(), s->tree.leaf_meta_ids.end());
-        CUDA_TRY(cudaMemcpyAsync(s->d_leaf_back.p, s->leaf_back.data(), s->n_items * sizeof(unsigned), cudaMemcpyHostToDevice,
-                                 s->stream));
-        for (size_t q = 0; q < nl; ++q) {
-            const int64_t m0 = s->tree.leaf_meta_off[q];
-            lists.push_back(LeafList{s->d_leaf_back.p + m0, m0, (int)(s->tree.leaf_meta_off[q + 1] - m0), 0});
+    // What the copies below read and write on the host lives until the stream
+    // has been waited for, also on an error: pageable memory may be read by the
+    // device itself, after the copy's call has returned.
+    std::vector<unsigned> host_ids;
+    rc = [&]() -> int {
+        if (s->octree_builder != ADECO_OCTREE_DEVICE) {
+            // the host builder's lists go to where the items kernel writes them
+            host_ids.assign(s->tree.leaf_meta_ids.begin(), s->tree.leaf_meta_ids.end());
+            CUDA_TRY(cudaMemcpyAsync(s->d_leaf_back.p, host_ids.data(), s->n_items * sizeof(unsigned), cudaMemcpyHostToDevice,
+                                     s->stream));
+            for (size_t q = 0; q < nl; ++q) {
+                const int64_t m0 = s->tree.leaf_meta_off[q];
+                lists.push_back(LeafList{s->d_leaf_back.p + m0, m0, (int)(s->tree.leaf_meta_off[q + 1] - m0), 0});
+            }
         }
+        // per-leaf grids here, the work items (leaf x meta-cell) on the device
+        CUDA_TRY(cudaMemcpyAsync(s->d_leaf_lists.p, lists.data(), nl * sizeof(LeafList), cudaMemcpyHostToDevice, s->stream));
+        TreeMeta md;
+        md.nx = s->nx; md.ny = s->ny; md.nz = s->nz;
+        for (int a = 0; a < 3; ++a) md.cd[a] = s->meta.cd[a];
+        leaf_items_kernel<<<(unsigned)nl, kTreeThreads, 0, s->stream>>>(reinterpret_cast<const LeafList *>(s->d_leaf_lists.p), md,
+                                                                        s->d_items.p, s->d_leaf_back.p, s->d_cube_off.p,
+                                                                        s->d_leaf_back.p + s->n_items);
+        CUDA_TRY(cudaGetLastError());
+        s->leaf_grids.resize(nl);
+        for (size_t q = 0; q < nl; ++q) {
+            const OctNode &nd = s->tree.nodes[s->tree.leaves[q]];
+            const float bb[6] = {nd.min[0], nd.min[0] + nd.ext, nd.min[1], nd.min[1] + nd.ext, nd.min[2], nd.min[2] + nd.ext};
+            const int shift = choose_shift(2058.0 * (double)std::max(1, lists[q].len), s->tet_mass);
+            s->leaf_grids[q] = make_grid(bb, leaf_dims, s->tet_mass, shift, (long long)q * cells);
+        }
+        CUDA_TRY(cudaMemcpyAsync(s->d_grids.p, s->leaf_grids.data(), nl * sizeof(GridDesc), cudaMemcpyHostToDevice,
+                                 s->stream));
+        s->leaf_back.resize(s->n_items + nl);
+        CUDA_TRY(cudaMemcpyAsync(s->leaf_back.data(), s->d_leaf_back.p, (s->n_items + nl) * sizeof(unsigned),
+                                 cudaMemcpyDeviceToHost, s->stream));
+        CUDA_TRY(cudaStreamSynchronize(s->stream));
+        return ADECO_OK;
+    }();
+    if (rc) {
+        cudaStreamSynchronize(s->stream);
+        return rc;
     }
-    // per-leaf grids here, the work items (leaf x meta-cell) on the device
-    CUDA_TRY(cudaMemcpyAsync(s->d_leaf_lists.p, lists.data(), nl * sizeof(LeafList), cudaMemcpyHostToDevice, s->stream));
-    TreeMeta md;
-    md.nx = s->nx; md.ny = s->ny; md.nz = s->nz;
-    for (int a = 0; a < 3; ++a) md.cd[a] = s->meta.cd[a];
-    leaf_items_kernel<<<(unsigned)nl, kTreeThreads, 0, s->stream>>>(reinterpret_cast<const LeafList *>(s->d_leaf_lists.p), md,
-                                                                    s->d_items.p, s->d_leaf_back.p, s->d_cube_off.p,
-                                                                    s->d_leaf_back.p + s->n_items);
-    CUDA_TRY(cudaGetLastError());
-    s->leaf_grids.resize(nl);
-    for (size_t q = 0; q < nl; ++q) {
-        const OctNode &nd = s->tree.nodes[s->tree.leaves[q]];
-        const float bb[6] = {nd.min[0], nd.min[0] + nd.ext, nd.min[1], nd.min[1] + nd.ext, nd.min[2], nd.min[2] + nd.ext};
-        const int shift = choose_shift(2058.0 * (double)std::max(1, lists[q].len), s->tet_mass);
-        s->leaf_grids[q] = make_grid(bb, leaf_dims, s->tet_mass, shift, (long long)q * cells);
-    }
-    CUDA_TRY(cudaMemcpyAsync(s->d_grids.p, s->leaf_grids.data(), nl * sizeof(GridDesc), cudaMemcpyHostToDevice,
-                             s->stream));
-    s->leaf_back.resize(s->n_items + nl);
-    CUDA_TRY(cudaMemcpyAsync(s->leaf_back.data(), s->d_leaf_back.p, (s->n_items + nl) * sizeof(unsigned),
-                             cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
     s->has_tree = true;
     return ADECO_OK;
 }

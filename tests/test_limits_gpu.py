@@ -95,3 +95,22 @@ def test_only_the_pages_of_the_box_become_resident(adeco, shift, rows):
         assert resident.size > 0 and resident.min() >= rows[0] and resident.max() <= rows[1]
         assert grid.sum() > 0
     assert (grid.sum() == 0) == (rows is None)
+
+
+def test_leaf_lists_of_repeated_builds(adeco):
+    """Builds of growing and shrinking size in one session: the leaves' lists
+    that come back from the device are the host builder's, whichever built
+    them, and so are the leaves' sums.  (The host builder's lists go to the
+    device and come back with the leaves' cubes behind them.)"""
+    from adeco_gb300.synthetic import zeldovich_lattice
+    pos = zeldovich_lattice(64, L=64.0, seed=12, rms_disp=2.0)
+    with adeco.Session(pos) as s:
+        for max_tets in (60000, 1500, 20000, 400, 1500):
+            lists, grids = [], []
+            for builder in ("device", "host"):
+                info = s.build_octree(max_tets, 8, leaf_dims=2, builder=builder)
+                lists.append([s.leaf_meta(q) for q in range(len(info.leaves))])
+                grids.append(s.deposit_leaves()[0])
+            assert len(lists[0]) == len(lists[1])
+            assert all(np.array_equal(a, b) for a, b in zip(*lists))
+            assert np.array_equal(*grids)
