@@ -13,6 +13,7 @@
 // The FP32 expressions keep the reference's operation order.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <vector>
 
@@ -67,6 +68,18 @@ struct MetaGrid {
             org[a] = c[a] * kMetaCubes;
             nv[a] = (c[a] + 1 == cd[a]) ? (n[a] - org[a]) : kMetaCubes + 1;
         }
+    }
+    // lattice cubes of the meta-cells ids[0..n) (a leaf's; 64 bits: a lattice of
+    // 1626^3 has 2^32)
+    uint64_t cubes(const uint32_t *ids, size_t n) const
+    {
+        uint64_t sum = 0;
+        for (size_t i = 0; i < n; ++i) {
+            int org[3], nv[3];
+            range(ids[i], org, nv);
+            sum += (uint64_t)(nv[0] - 1) * (uint64_t)(nv[1] - 1) * (uint64_t)(nv[2] - 1);
+        }
+        return sum;
     }
     uint64_t estimate(uint64_t id, const float box[6]) const;
 };

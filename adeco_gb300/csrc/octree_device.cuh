@@ -255,12 +255,11 @@ struct LeafList {
 };
 
 // A leaf's work items (leaf x meta-cell) from its list, a block per leaf; the
-// lists back to back (ids_out, where a list may be already), the items' cube
-// offsets within their leaf and the leaf's cubes.
+// lists back to back (ids_out, where a list may be already) and the items' cube
+// offsets within their leaf.
 __global__ void __launch_bounds__(kTreeThreads) leaf_items_kernel(const LeafList *__restrict__ leaves, TreeMeta md,
                                                                   Item *__restrict__ items, unsigned *ids_out,
-                                                                  long long *__restrict__ cube_off,
-                                                                  unsigned *__restrict__ leaf_cubes)
+                                                                  long long *__restrict__ cube_off)
 {
     __shared__ int wsum[kTreeThreads / 32];
     const LeafList leaf = leaves[blockIdx.x];
@@ -307,7 +306,6 @@ __global__ void __launch_bounds__(kTreeThreads) leaf_items_kernel(const LeafList
         before += all;
         __syncthreads();
     }
-    if (threadIdx.x == 0) leaf_cubes[blockIdx.x] = (unsigned)before;
 }
 
 // Device memory of a session's octree builds, kept between them: the levels'

@@ -638,7 +638,7 @@ struct adeco_session {
     int leaf_dims = 16;
     std::vector<GridDesc> leaf_grids;
     size_t n_items = 0;                 // work items: (leaf, meta-cell), in leaf order
-    std::vector<unsigned> leaf_back;    // the leaves' meta-cell ids, then their cubes, as they come from the device
+    std::vector<unsigned> leaf_back;    // the leaves' meta-cell ids as they come from the device
     DevBuf<Item> d_items;
     DevBuf<GridDesc> d_grids;
     DevBuf<unsigned long long> d_fixed;
@@ -973,7 +973,7 @@ extern "C" int adeco_session_build_octree(adeco_session *s, const float *box6, c
     s->route_cap = route_capacity((long long)s->n_items);
     if ((rc = s->d_items.reserve(s->n_items)) || (rc = s->d_grids.reserve(nl)) || (rc = s->d_fixed.reserve(s->out_values)) ||
         (rc = s->d_out.reserve(s->out_values)) || (rc = s->d_cube_off.reserve(s->n_items)) ||
-        (rc = s->d_route.reserve(s->route_cap + 1)) || (rc = s->d_leaf_back.reserve(s->n_items + nl)) ||
+        (rc = s->d_route.reserve(s->route_cap + 1)) || (rc = s->d_leaf_back.reserve(s->n_items)) ||
         (rc = s->d_leaf_lists.reserve(nl * sizeof(LeafList))))
         return rc;
     // What the copies below read and write on the host lives until the stream
@@ -997,8 +997,7 @@ extern "C" int adeco_session_build_octree(adeco_session *s, const float *box6, c
         md.nx = s->nx; md.ny = s->ny; md.nz = s->nz;
         for (int a = 0; a < 3; ++a) md.cd[a] = s->meta.cd[a];
         leaf_items_kernel<<<(unsigned)nl, kTreeThreads, 0, s->stream>>>(reinterpret_cast<const LeafList *>(s->d_leaf_lists.p), md,
-                                                                        s->d_items.p, s->d_leaf_back.p, s->d_cube_off.p,
-                                                                        s->d_leaf_back.p + s->n_items);
+                                                                        s->d_items.p, s->d_leaf_back.p, s->d_cube_off.p);
         CUDA_TRY(cudaGetLastError());
         s->leaf_grids.resize(nl);
         for (size_t q = 0; q < nl; ++q) {
@@ -1009,9 +1008,9 @@ extern "C" int adeco_session_build_octree(adeco_session *s, const float *box6, c
         }
         CUDA_TRY(cudaMemcpyAsync(s->d_grids.p, s->leaf_grids.data(), nl * sizeof(GridDesc), cudaMemcpyHostToDevice,
                                  s->stream));
-        s->leaf_back.resize(s->n_items + nl);
-        CUDA_TRY(cudaMemcpyAsync(s->leaf_back.data(), s->d_leaf_back.p, (s->n_items + nl) * sizeof(unsigned),
-                                 cudaMemcpyDeviceToHost, s->stream));
+        s->leaf_back.resize(s->n_items);
+        CUDA_TRY(cudaMemcpyAsync(s->leaf_back.data(), s->d_leaf_back.p, s->n_items * sizeof(unsigned), cudaMemcpyDeviceToHost,
+                                 s->stream));
         CUDA_TRY(cudaStreamSynchronize(s->stream));
         return ADECO_OK;
     }();
@@ -1151,7 +1150,7 @@ extern "C" int adeco_session_deposit_leaves(adeco_session *s, int precision, dou
             DepositParams Q = P;
             Q.items = s->d_items.p + item0;
             Q.n_items = (int)(s->tree.leaf_meta_off[q + 1] - item0);
-            const long long cubes = s->leaf_back[s->n_items + q];
+            const long long cubes = (long long)s->meta.cubes(s->leaf_back.data() + item0, (size_t)Q.n_items);
             if (Q.n_items > 0 && cubes > 0) {
                 rc = launch_plain(s->dp, Q, s->d_cube_off.p + item0, 0, cubes, s->stream);
                 ++launches;
