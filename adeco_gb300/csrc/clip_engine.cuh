@@ -384,122 +384,60 @@ ADECO_HD inline void bary_identity(float *r)
     for (int i = 0; i < 12; ++i) r[i] = (i & 3) == 3 ? 1.f : 0.f;  // entries 3, 7, 11
 }
 
-// record entry of vertex v's value i (0..2 weights, 3..5 coordinates)
-ADECO_HD inline int bary_idx(int v, int i) { return i < 3 ? 3 * v + i : 12 + 3 * v + (i - 3); }
-
-// Split of barycentric piece r by face f (mask: its vertices inside, k of
-// them), with split_cut's patterns over the 6 values of a vertex: the
-// vertices permuted to A B C D (inside first, even permutation), the cut
-// points E0..E3 of the edges k=1: AB AC AD AD; k=2: AC AD BC BD; k=3: AD BD CD
-// CD (weights interpolated with the coordinate's edge parameter, the
-// coordinate snapped onto the face), and the children
-//   c0 = (A, k1 ? E0 : B, k1 ? E1 : (k2 ? E2 : C), k1 ? E2 : (k2 ? E3 : E2))
-//   c1 = (A, k2 ? E2 : B, k2 ? E0 : E2, k2 ? E3 : E1)
-//   c2 = (A, k2 ? E0 : E1, k2 ? E1 : E2, k2 ? E3 : E0)
-// written entry by entry as put(child, record index, value): each child
-// vertex is a select between at most three candidates, no lookup.  Returns
-// the number of children (1 or 3).
-template <typename Put>
-inline int bary_split(const float *r, int f, int mask, Put put)
-{
-    const int axis = f >> 1;
-    const float plane = (f & 1) ? 1.f : 0.f;
-    const int pm = split_perm(mask), k = split_kin(mask);
-    const bool k1 = k == 1, k2 = k == 2, k3 = k == 3;
-    const int ia = pm & 3, ib = (pm >> 2) & 3, ic = (pm >> 4) & 3, id = (pm >> 6) & 3;
-    float A[6], B[6], C[6], D[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        const float a0 = r[bary_idx(0, i)], a1 = r[bary_idx(1, i)], a2 = r[bary_idx(2, i)], a3 = r[bary_idx(3, i)];
-        A[i] = sel4(ia, a0, a1, a2, a3);
-        B[i] = sel4(ib, a0, a1, a2, a3);
-        C[i] = sel4(ic, a0, a1, a2, a3);
-        D[i] = sel4(id, a0, a1, a2, a3);
-    }
-    float E[4][6];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        float in[6], out[6];
-#pragma unroll
-        for (int i = 0; i < 6; ++i) {
-            in[i] = e == 0 ? A[i] : (e == 1 ? (k3 ? B[i] : A[i]) : (e == 2 ? (k1 ? A[i] : (k2 ? B[i] : C[i]))
-                                                                             : (k2 ? B[i] : (k3 ? C[i] : A[i]))));
-            out[i] = e == 0 ? (k1 ? B[i] : (k2 ? C[i] : D[i])) : (e == 1 ? (k1 ? C[i] : D[i])
-                                                                          : (e == 2 ? (k2 ? C[i] : D[i]) : D[i]));
-        }
-        const float xin = sel3(axis, in[3], in[4], in[5]), xout = sel3(axis, out[3], out[4], out[5]);
-        const float t = fminf(fmaxf((plane - xin) * rcp_nr(xout - xin), 0.f), 1.f);
-#pragma unroll
-        for (int i = 0; i < 6; ++i) E[e][i] = (i == 3 + axis) ? plane : fmaf(t, out[i] - in[i], in[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        put(0, bary_idx(0, i), A[i]);
-        put(0, bary_idx(1, i), k1 ? E[0][i] : B[i]);
-        put(0, bary_idx(2, i), k1 ? E[1][i] : (k2 ? E[2][i] : C[i]));
-        put(0, bary_idx(3, i), k1 ? E[2][i] : (k2 ? E[3][i] : E[2][i]));
-        put(1, bary_idx(0, i), A[i]);
-        put(1, bary_idx(1, i), k2 ? E[2][i] : B[i]);
-        put(1, bary_idx(2, i), k2 ? E[0][i] : E[2][i]);
-        put(1, bary_idx(3, i), k2 ? E[3][i] : E[1][i]);
-        put(2, bary_idx(0, i), A[i]);
-        put(2, bary_idx(1, i), k2 ? E[0][i] : E[1][i]);
-        put(2, bary_idx(2, i), k2 ? E[1][i] : E[2][i]);
-        put(2, bary_idx(3, i), k2 ? E[3][i] : E[0][i]);
-    }
-    return k1 ? 1 : 3;
-}
-
 // The share inside the unit cube of one barycentric piece rec0 whose faces
-// in done0 are already done, clipped serially with a stack: the warp engine's
-// steps, faces, cut points and children, for checks on the host.
+// in done0 are already done, clipped serially with a stack, for checks on the
+// host: faces, cut points, children and shares by the warp engine's functions
+// (clip_bary_pairs).
 inline F2 clip_bary_serial(const float *rec0, int done0)
 {
     constexpr int kDepth = 16;
-    constexpr int kRec = kBaryRec;
-    float stk[kDepth][kRec];
+    float stk[kDepth][24];  // a vertex's 3 weights and 3 coordinates, as the engine's pool
     int sdone[kDepth];
-    for (int i = 0; i < kRec; ++i) stk[0][i] = rec0[i];
+    for (int q = 0; q < 4; ++q)
+        for (int i = 0; i < 3; ++i) {
+            stk[0][6 * q + i] = rec0[3 * q + i];
+            stk[0][6 * q + 3 + i] = rec0[12 + 3 * q + i];
+        }
     sdone[0] = done0;
     int sp = 1;
     F2 acc = {0.f, 0.f};
     while (sp > 0) {
         --sp;
-        float r[kRec];
-#pragma unroll
-        for (int i = 0; i < kRec; ++i) r[i] = stk[sp][i];
-        const float *w = r, *x = r + 12;
+        float V[4][6], w[12];
+        int bits[4];
+        for (int q = 0; q < 4; ++q) {
+            for (int i = 0; i < 6; ++i) V[q][i] = stk[sp][6 * q + i];
+            for (int i = 0; i < 3; ++i) w[3 * q + i] = V[q][i];
+            bits[q] = face_bits(V[q][3], V[q][4], V[q][5]);
+        }
         const int done = sdone[sp];
         int f = 0, mask = 0;
         bool last = false;
-        const int code = next_face(face_bits(x[0], x[1], x[2]), face_bits(x[3], x[4], x[5]),
-                                   face_bits(x[6], x[7], x[8]), face_bits(x[9], x[10], x[11]), done, f, mask, last);
+        const int code = next_face(bits[0], bits[1], bits[2], bits[3], done, f, mask, last);
         if (code == 0) continue;  // beyond a face
         if (code == 1) {
             acc = f2_add(acc, bary_share(w));
             continue;
         }
-        const int axis = f >> 1;
-        const float plane = (f & 1) ? 1.f : 0.f;
-        const float xa[4] = {x[axis], x[3 + axis], x[6 + axis], x[9 + axis]};
+        const int ax = 3 + (f >> 1);
         if (last) {  // last crossed face: the inside fraction of the piece
-            acc = f2_add(acc, f2_mul_f(bary_share(w), side_fraction(xa[0], xa[1], xa[2], xa[3], mask, plane)));
+            acc = f2_add(acc, f2_mul_f(bary_share(w), side_fraction(V[0][ax], V[1][ax], V[2][ax], V[3][ax], mask,
+                                                                    (f & 1) ? 1.f : 0.f)));
             continue;
         }
-        // split by face f into 1 or 3 pieces (bary_split, as the warp engine)
-        const int n = split_kin(mask) == 1 ? 1 : 3;
+        const int pm = split_perm(mask), k = split_kin(mask), n = k == 1 ? 1 : 3;
         if (sp + n > kDepth) continue;  // cannot happen: at most 2 pending pieces per face level
-        bary_split(r, f, mask, [&](int ch, int e, float val) {
-            if (ch < n) stk[sp + ch][e] = val;
-        });
+        const float *A = V[pm & 3], *B = V[(pm >> 2) & 3], *C = V[(pm >> 4) & 3], *D = V[(pm >> 6) & 3];
+        float E[4][6];
+        cut_points<6>(A, B, C, D, A[ax], B[ax], C[ax], D[ax], k, f, E);
         for (int c = 0; c < n; ++c) {
+            split_child<6>(c, bit_mask(k == 1), bit_mask(k == 2), A, B, C, E, stk[sp]);
             sdone[sp] = done | (1 << f);
             ++sp;
         }
     }
     return acc;
 }
-
 
 constexpr int kVolShift = 56;  // fixed point of 6x piece volumes (each <= 6)
 static_assert(kVolShift == 56, "vol_fixed scales by 0x1p56f");
