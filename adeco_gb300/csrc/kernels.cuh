@@ -223,7 +223,7 @@ __device__ __forceinline__ void warp_stat(unsigned long long *stats, int which, 
 constexpr uint32_t kBelowMax = 0x7u << 16, kAboveMin = 0x38u << 16;    // x < gmax, gmin < x, a bit per axis
 constexpr uint32_t kCullBox = 0xfc0u << 16, kPadVertex = 0x1000u << 16;  // the same two for the cull box; padding
 
-__device__ __forceinline__ uint2 vertex_range(const float p[3], const GridDesc &g, bool pad)
+ADECO_HD inline uint2 vertex_range(const float p[3], const GridDesc &g, bool pad)
 {
     uint32_t w[3], flags = pad ? kPadVertex : 0u;
 #pragma unroll
@@ -231,12 +231,26 @@ __device__ __forceinline__ uint2 vertex_range(const float p[3], const GridDesc &
         const float x = p[a];
         const float lim = (x < g.gmin[a]) ? g.gmin[a] : x;
         const float q = div_rn(sub_rn((lim < g.gmax[a]) ? lim : g.gmax[a], g.gmin[a]), g.delta[a]);
-        const int lo = (int)floorf(q), hi = (int)ceilf(q);
-        w[a] = (uint32_t)(2 * max(0, min(lo, 8191)) + (hi > lo));
+        int lo = (int)floorf(q);
+        const int more = (int)ceilf(q) > lo;
+        lo = lo < 0 ? 0 : (lo > 8191 ? 8191 : lo);
+        w[a] = (uint32_t)(2 * lo + more);
         flags |= ((x < g.gmax[a] ? 1u : 0u) | (g.gmin[a] < x ? 8u : 0u) | (x < g.cull_max[a] ? 64u : 0u) |
                   (g.cull_min[a] < x ? 512u : 0u)) << (16 + a);
     }
     return make_uint2(w[0] | (w[1] << 16), w[2] | flags);
+}
+
+// A tet's candidate cells [lo, hi] along axis a, in grid indices up to top, from
+// the least and the greatest words of its vertices.
+ADECO_HD inline void word_range(uint2 mn, uint2 mx, int a, int top, int &lo, int &hi)
+{
+    const int wlo = (int)((a == 2 ? mn.y : (mn.x >> (16 * a))) & 0xffffu),
+              whi = (int)((a == 2 ? mx.y : (mx.x >> (16 * a))) & 0xffffu);
+    lo = wlo >> 1;
+    hi = (whi + 1) >> 1;
+    lo = lo > top ? top : lo;
+    hi = hi > top ? top : hi;
 }
 
 // position of source vertex gi (the w of a lattice vertex is not used)
@@ -370,12 +384,8 @@ ADECO_HD inline int setup_frame(uint2 mn, uint2 mx, Frame frame, const GridDesc 
     int big_ex = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const int top = g.dims - 1;
-        const int wlo = (int)((a == 2 ? mn.y : (mn.x >> (16 * a))) & 0xffffu),
-                  whi = (int)((a == 2 ? mx.y : (mx.x >> (16 * a))) & 0xffffu);
-        int lo = wlo >> 1, hi = (whi + 1) >> 1;
-        lo = lo > top ? top : lo;
-        hi = hi > top ? top : hi;
+        int lo, hi;
+        word_range(mn, mx, a, g.dims - 1, lo, hi);
         lo = lo < g.tile_lo[a] ? g.tile_lo[a] : lo;
         hi = hi > g.tile_hi[a] ? g.tile_hi[a] : hi;
         cnt0 = hi < lo ? 0 : cnt0 * (hi - lo + 1);
