@@ -65,7 +65,7 @@ struct DepositParams {
     int *counter;                     // persistent work counter
     unsigned long long *stats;        // kNumStats counters or nullptr
     int *error;                       // device error flag (bit 0: tet too large, bit 2: route list full,
-                                      // bit 3: a bounded wait timed out)
+                                      // bit 3: a bounded wait timed out; no deposit kernel has one)
     // ill-conditioned tets, deposited by a second launch (route_fp64_kernel):
     // entries item << 16 | (cube slot * 6 + tet), count in *route_count
     unsigned long long *route;

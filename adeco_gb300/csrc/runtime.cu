@@ -182,7 +182,7 @@ int mixed_setup(int device, DeviceProps &dp)
 struct Tuning {
     int zoom_tile = 64;                       // cells per tile edge of a zoom grid
     int share_chunk = 512;                    // accepted for callers that set it; pairs are shared 32 at a time
-    int clip_batch = kQueue;                  // partial pairs listed per warp before clipping
+    int clip_batch = kQueue;                  // 128ths of a CTA's pair list filled before clipping
     int ctas_per_sm = 0;                      // persistent launches: CTAs per SM (0: occupancy)
     unsigned long long route_capacity = 0;    // 0: route_capacity(items)
     unsigned item_pairs = 1u << 18;           // zoom grids: expected candidate pairs per work item
@@ -220,7 +220,7 @@ static void set_route(DepositParams &P, unsigned long long *buf, unsigned long l
 static int deposit_error(int err, const char *where)
 {
     if (err & 4) return fail(ADECO_ERR_LIMIT, "more ill-conditioned tets in %s than the route list holds", where);
-    if (err & 8) return fail(ADECO_ERR_CUDA, "a warp of %s timed out waiting for the warps sharing its pairs", where);
+    if (err & 8) return fail(ADECO_ERR_CUDA, "a bounded wait of %s timed out", where);
     return fail(ADECO_ERR_LIMIT, "a tet spans more than 2^25 candidate cells of %s", where);
 }
 
@@ -1303,9 +1303,9 @@ extern "C" int adeco_debug_tet_records(const float *positions, size_t positions_
 #include "serving.cuh"
 
 // ============================================================ bounded waits
-// One warp waits, through wait_zero_bounded (the wait every spin of the
-// deposit kernels uses), on a count that nothing decrements; when the limit
-// runs out it sets error bit 3 and returns.
+// One warp waits, through wait_zero_bounded, on a count that nothing
+// decrements; when the limit runs out it sets error bit 3 and returns.  No
+// deposit kernel waits this way.
 __global__ void bounded_wait_kernel(int *error, unsigned spins)
 {
     __shared__ int busy;

@@ -8,8 +8,8 @@ the per-cell bar):
 * ``zoom_tile``   -- cells per tile edge of a zoom grid: one work item per
   (tile, meta-cell); smaller tiles balance fine grids better but stage and
   cull each meta-cell's vertex block more often;
-* ``share_chunk`` -- accepted, without effect: a CTA's warps take pairs 32 at
-  a time from the whole wave;
+* ``share_chunk`` -- accepted, without effect and not searched: a CTA's warps
+  take pairs 32 at a time from the whole wave;
 * ``clip_batch``  -- the staging depth of the clip engine: the share, in
   128ths, of a CTA's list of partial pairs that is filled before it is clipped
   (deeper lists keep more lanes busy, shallower ones clip sooner);
@@ -40,7 +40,7 @@ SPACES = {
     "leaf": {"clip_batch": [64, 96, 128], "ctas_per_sm": [1, 2]},
     # zoom grids (fine grids: cells much smaller than tets)
     "zoom": {"zoom_tile": [32, 64, 128], "item_pairs": [1 << 16, 1 << 17, 1 << 18, 1 << 20],
-             "share_chunk": [256, 512, 1024], "clip_batch": [96, 128]},
+             "clip_batch": [96, 128]},
 }
 DEFAULTS = {"zoom_tile": 64, "share_chunk": 512, "clip_batch": 128, "ctas_per_sm": 2, "item_pairs": 1 << 18}
 

@@ -282,7 +282,7 @@ typedef struct {
 int adeco_session_serving_stats(adeco_session *s, adeco_serving_stats *st);
 
 /* ------------------------------------------------------------------ */
-/* Parity diagnostics (same device functions as the deposit kernels)    */
+/* Parity diagnostics (the reference's rules on the device)             */
 
 /* 13 ints per tet of cubes [cube_begin,cube_end) of a patch sequence: the 4
  * corner slots after the orientation rule, volume sign, in-grid flag,
@@ -293,11 +293,11 @@ int adeco_debug_tet_records(const float *positions, size_t positions_size, int m
                             size_t cube_begin, size_t cube_end, const float bbox[6], int dims, int tet_order,
                             int32_t *records, uint32_t *cand);
 
-/* The bounded wait every spin-wait of the deposit kernels uses, run on a
- * count that nothing decrements, for at most `spins` sleeps of 32 ns: the
- * failure path of a wait that runs out, exercised without a fault.  Returns
- * ADECO_ERR_CUDA with the deposit's "timed out" message (device error bit 3)
- * when the wait ran out, as it must. */
+/* A bounded wait on a count that nothing decrements, for at most `spins`
+ * sleeps of 32 ns: the failure path of a wait that runs out, exercised without
+ * a fault.  Returns ADECO_ERR_CUDA with a "timed out" message (device error
+ * bit 3) when the wait ran out, as it must.  The deposit kernels themselves
+ * wait at barriers only. */
 int adeco_debug_bounded_wait(unsigned spins);
 
 /* Measured FP32 FMA throughput of `device` (TFLOP/s, 2 flops per FMA): the
