@@ -216,4 +216,11 @@ void MetaIndex::query(const MetaGrid &mg, const float box6[6], std::vector<uint3
     out.erase(std::unique(out.begin(), out.end()), out.end());
 }
 
+void MetaIndex::among(const MetaGrid &mg, const std::vector<uint32_t> &near, const float box6[6], std::vector<uint32_t> &out)
+{
+    out.clear();
+    for (const uint32_t id : near)
+        if (meets(&mg.bbox[6 * (size_t)id], box6)) out.push_back(id);
+}
+
 }  // namespace adeco

@@ -106,6 +106,8 @@ struct MetaIndex {
     void build(const MetaGrid &mg);
     // meta-cells whose AABB strictly meets box6 (min xyz, max xyz), ascending
     void query(const MetaGrid &mg, const float box6[6], std::vector<uint32_t> &out) const;
+    // the same from `near`, the answer for a box that holds box6
+    static void among(const MetaGrid &mg, const std::vector<uint32_t> &near, const float box6[6], std::vector<uint32_t> &out);
 };
 
 struct Octree {
