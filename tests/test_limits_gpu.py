@@ -114,3 +114,24 @@ def test_leaf_lists_of_repeated_builds(adeco):
             assert len(lists[0]) == len(lists[1])
             assert all(np.array_equal(a, b) for a, b in zip(*lists))
             assert np.array_equal(*grids)
+
+
+@pytest.mark.parametrize("dims", [79, 80, 81, 93, 94, 102])
+def test_results_copied_by_one_or_several_threads(adeco, dims):
+    """Results of 3.9 to 8.5 MB, around where the copy to the caller takes its
+    second, third and fourth thread: whole, the same each time, and the same
+    when they start at another place of the batch's block."""
+    from adeco_gb300.synthetic import zeldovich_lattice
+    pos = zeldovich_lattice(24, L=24.0, seed=5, rms_disp=1.0)
+    req = ((11.0, 12.0, 13.0), 18.0, dims)
+    with adeco.Session(pos) as s:
+        b = s.submit([req])
+        s.wait(b)
+        first, again = s.result(b, 0, dims), s.result(b, 0, dims)
+        s.release(b)
+        b = s.submit([((12.0, 12.0, 12.0), 5.0, 3), req])
+        s.wait(b)
+        third = s.result(b, 1, dims)
+        s.release(b)
+    assert np.array_equal(first, again) and np.array_equal(first, third)
+    assert (first.reshape(-1)[-dims:] > 0).any() and (first > 0).mean() > 0.9
