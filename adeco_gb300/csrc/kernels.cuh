@@ -1065,12 +1065,10 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
             __syncthreads();
             const int flags = S.flags[odd];
             const bool wide = (flags & kWideTet) != 0;
-            int total = 0;
-            if (flags & kManyPairs)
-                total = wave_next_part(S, 0);
-            else
+            unsigned sum = 0;
 #pragma unroll
-                for (int w = 0; w < kWarps; ++w) total += S.warp_pairs[w];
+            for (int w = 0; w < kWarps; ++w) sum += (unsigned)S.warp_pairs[w];
+            int total = (flags & kManyPairs) ? wave_next_part(S, 0) : (int)sum;
             bool left = total > 0;
             if (!left) __syncthreads();  // the next wave's set-up writes what this one's warps read above
             while (left) {
