@@ -155,6 +155,10 @@ struct Arena {
 inline void copy_result(void *dst, const void *src, size_t n)
 {
     constexpr size_t kPerThread = size_t(2) << 20;
+    if (n < 2 * kPerThread) {  // asking for the cores takes 4 us
+        std::memcpy(dst, src, n);
+        return;
+    }
     const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
     const size_t nt = std::max<size_t>(1, std::min<size_t>(std::min(8u, cores), n / kPerThread));
     const size_t part = round_up((n + nt - 1) / nt, 4096);
