@@ -704,6 +704,28 @@ __device__ __forceinline__ void scatter(const DepositParams &P, const GridDesc &
     atomicAdd(P.out + idx, fx);
 }
 
+#ifdef __CUDACC__
+// scatter of whole tets' mass by lanes `lanes` of the warp: of those that add
+// to the same cell, one adds for all (the same sum, in integers).  On grids
+// coarser than the tets nearly every pair is a whole tet, and the additions to
+// a few cells wait for one another: a 256^3 lattice onto 16^3 / 8^3 / 4^3 cells
+// 12.9 / 25.3 / 33.3 ms lane by lane, 6.5 / 6.3 / 5.5 so.  Fewer than 12 lanes
+// seldom share a cell and add by themselves.
+__device__ __forceinline__ void scatter_whole(const DepositParams &P, const GridDesc &g, const WaveTets &W, int s, int a,
+                                              int b, int c, unsigned lanes)
+{
+    unsigned long long fx = to_fixed(g.tet_mass, g.shift);
+    const long long i = W.lo[0][s] + a, j = W.lo[1][s] + b, k = W.lo[2][s] + c;
+    const long long idx = g.out_offset + i + (long long)g.dims * (j + (long long)g.dims * k);
+    if (__popc(lanes) >= 12) {
+        const unsigned same = __match_any_sync(lanes, idx);
+        if ((int)(threadIdx.x & 31) != __ffs(same) - 1) return;
+        fx *= (unsigned)__popc(same);
+    }
+    if (fx) atomicAdd(P.out + idx, fx);
+}
+#endif
+
 // A pair's 6x volume, summed in fixed point 2^kVolShift (0 <= vacc < 2^59),
 // times the tet's mass per unit of 6x volume.  The sum is converted to FP32
 // with one rounding from two exact 24-bit parts (bits 35..58 and 11..34): the
@@ -924,7 +946,9 @@ ADECO_HD inline unsigned start_bit(int start, int rel, int skip)
 // their closed form, for a few lanes of nearly every 32, had taken more than
 // the classification itself.  Until no pair is left or the list might not hold
 // the 32 pairs each warp may have in hand (`room` of it are used).
-template <bool kStats>
+// kExactD (zoom grids): whole tets are added where a lane finds them; octree
+// leaves of 256^3 take 0.6% longer so, fine zoom grids 3% the other way.
+template <bool kStats, bool kExactD>
 __device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixed &S, int *list_n, int *cut_n, int room, bool wide,
                                               PairStats &st)
 {
@@ -968,11 +992,12 @@ __device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixe
             q0 = end;
             if (q0 >= min(c0 + 32, total)) break;
         }
-        bool part = false;
+        bool part = false, holds = false;
         int cross = -1;
         uint32_t entry = 0;
+        int3 c = make_int3(0, 0, 0);
         if (pidx < total) {
-            const int3 c = flat_cell(W, s, local);
+            c = flat_cell(W, s, local);
             entry = wide ? (uint32_t)local : ((uint32_t)c.x | ((uint32_t)c.y << 10) | ((uint32_t)c.z << 20));
             if (kStats) ++st.cand;
             bool f64 = false;
@@ -985,8 +1010,14 @@ __device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixe
                 st.bbox += cls != P_NO;
             }
             part = cls == P_PARTIAL && cross < 0;
-            const float m = cls == P_TET_INSIDE ? g.tet_mass : (cls == P_CELL_INSIDE ? 6.f * W.f6[s] : 0.f);
+            holds = cls == P_TET_INSIDE;
+            if (kExactD && holds) scatter_whole(P, g, W, s, c.x, c.y, c.z, __activemask());
+            const float m = cls == P_CELL_INSIDE ? 6.f * W.f6[s] : 0.f;
             if (m > 0.f) scatter(P, g, W, s, c.x, c.y, c.z, m);
+        }
+        if (!kExactD) {
+            const unsigned lanes = __ballot_sync(0xffffffffu, holds);
+            if (holds) scatter_whole(P, g, W, s, c.x, c.y, c.z, lanes);
         }
         const unsigned bal = __ballot_sync(0xffffffffu, part), cut = __ballot_sync(0xffffffffu, cross >= 0);
         const unsigned lt = le >> 1;
@@ -1013,7 +1044,7 @@ __device__ __forceinline__ void wave_classify(const DepositParams &P, SharedMixe
 // lattice, ALU pipe 52% busy, DRAM idle); of the warps' cycles the clipping
 // takes 53%, the wait at its end 9, classification 13, set-up 9, staging 6,
 // masses 5.  256^3 octree leaves 43.1 ms with a warp in each phase for itself,
-// 29.7 now; one 128^3 zoom grid (whole call) 5.3 -> 2.7 ms; a 96^3 grid's
+// 29.0 now; one 128^3 zoom grid (whole call) 5.3 -> 2.7 ms; a 96^3 grid's
 // no-allocation call 4.9 -> 2.3 ms.
 // kStats: count the pairs (collect_stats); a separate instantiation, so that
 // the others carry no counters.  kExactD: see setup_frame.
@@ -1072,7 +1103,7 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
             bool left = total > 0;
             if (!left) __syncthreads();  // the next wave's set-up writes what this one's warps read above
             while (left) {
-                wave_classify<kStats>(P, S, &S.list.n[turn], &S.cut[turn], room, wide, st);
+                wave_classify<kStats, kExactD>(P, S, &S.list.n[turn], &S.cut[turn], room, wide, st);
                 __syncthreads();
                 left = S.cursor < total;
                 const int np = S.list.n[turn];

@@ -5,7 +5,7 @@ import mmap
 import numpy as np
 import pytest
 
-from test_deposit_gpu import adeco  # noqa: F401  (the fixture)
+from test_deposit_gpu import adeco, check_cells  # noqa: F401  (adeco: the fixture)
 
 pytestmark = pytest.mark.gpu
 
@@ -135,3 +135,34 @@ def test_results_copied_by_one_or_several_threads(adeco, dims):
         s.release(b)
     assert np.array_equal(first, again) and np.array_equal(first, third)
     assert (first.reshape(-1)[-dims:] > 0).any() and (first > 0).mean() > 0.9
+
+
+@pytest.mark.parametrize("order", [0, 1], ids=["ref", "conforming"])
+@pytest.mark.parametrize("dims", [1, 2, 3, 8])
+def test_whole_tets_on_coarse_grids(adeco, oracle, dims, order):
+    """Grids much coarser than the tets, where most lanes of a warp add a whole
+    tet to the same few cells: one cell that holds everything gains exactly a
+    mass per tet; others are within the mixed path's bar of the FP64 oracle.
+    The same through a session's zoom request and leaves."""
+    from adeco_gb300.synthetic import zeldovich_lattice
+    m = 14
+    pos = zeldovich_lattice(m + 1, L=15.0, seed=6, rms_disp=0.3)
+    lo, hi = float(pos.min()) - 0.25, float(pos.max()) + 0.25
+    box = np.array([lo, hi] * 3, np.float32)
+    n_tets = 6 * m ** 3
+    got = adeco.deposit_tets_ex(pos.reshape(-1), m, box, dims, tet_order=order)
+    ref = oracle.deposit_patches(pos.reshape(-1), m, box, dims, fp64=True, order=order)
+    check_cells(got, ref, n_tets=n_tets)
+    side, mid = float(box[1] - box[0]), 0.5 * float(box[0] + box[1])
+    with adeco.Session(pos, tet_order=order) as s:
+        b = s.submit([((mid, mid, mid), 1.02 * side, dims)])
+        s.wait(b)
+        zoom = s.result(b, 0, dims)
+        s.release(b)
+        s.build_octree(10 ** 9, 0, leaf_dims=dims)
+        leaf = s.deposit_leaves()[0]
+    # the request's box is not the grid's: its total, and that of the leaf (the particles' own box), only
+    tol = 1e-9 * n_tets + 3e-7 * np.sqrt(n_tets)
+    assert abs(zoom.sum() - n_tets) <= tol and abs(leaf.sum() - n_tets) <= tol
+    if dims == 1:
+        assert got.sum() == n_tets and zoom.sum() == n_tets
