@@ -638,7 +638,7 @@ struct adeco_session {
     int leaf_dims = 16;
     std::vector<GridDesc> leaf_grids;
     size_t n_items = 0;                 // work items: (leaf, meta-cell), in leaf order
-    std::vector<unsigned> leaf_back;    // the leaves' meta-cell ids as they come from the device
+    std::vector<unsigned> leaf_back;    // the leaves' meta-cell ids, back to back
     DevBuf<Item> d_items;
     DevBuf<GridDesc> d_grids;
     DevBuf<unsigned long long> d_fixed;
@@ -1008,10 +1008,13 @@ extern "C" int adeco_session_build_octree(adeco_session *s, const float *box6, c
         }
         CUDA_TRY(cudaMemcpyAsync(s->d_grids.p, s->leaf_grids.data(), nl * sizeof(GridDesc), cudaMemcpyHostToDevice,
                                  s->stream));
-        s->leaf_back.resize(s->n_items);
-        CUDA_TRY(cudaMemcpyAsync(s->leaf_back.data(), s->d_leaf_back.p, s->n_items * sizeof(unsigned), cudaMemcpyDeviceToHost,
-                                 s->stream));
+        if (s->octree_builder == ADECO_OCTREE_DEVICE) {
+            s->leaf_back.resize(s->n_items);
+            CUDA_TRY(cudaMemcpyAsync(s->leaf_back.data(), s->d_leaf_back.p, s->n_items * sizeof(unsigned),
+                                     cudaMemcpyDeviceToHost, s->stream));
+        }
         CUDA_TRY(cudaStreamSynchronize(s->stream));
+        if (s->octree_builder != ADECO_OCTREE_DEVICE) s->leaf_back.swap(host_ids);
         return ADECO_OK;
     }();
     if (rc) {
