@@ -148,19 +148,19 @@ struct Arena {
 // Copies n bytes from a pinned block to the caller's memory, large results by
 // several threads.  One Grace core copies at 13 to 25 GB/s, 8 at 62 GB/s, the
 // page faults of a fresh buffer among it (134 MB: 10.7 ms and 2.2 ms); a copy
-// by the device faults those pages in more slowly (24 ms).  A thread costs some
-// 20 us and faults contend: with 0.5 / 1 / 2 / 4 MB a thread, or one thread, a fresh
-// buffer of 2.1 MB takes 113 / 145 / 135 / 138 / 132 us, 4.3 MB 458 / 175 / 192 / 230 /
-// 225, 8.5 MB 500 / 485 / 283 / 368 / 511, 16.8 MB 570 / 624 / 618 / 501 / 1021.
+// by the device faults those pages in more slowly (24 ms).  Faults contend, and a
+// thread costs some 20 us: up to 4 threads of 1 MB or more, up to 8 of 4 MB or
+// more.  Into fresh buffers of 2.1 MB 1 / 2 threads take 158 / 145 us, 4.3 MB 1 / 2 /
+// 4 225 / 192 / 175, 8.5 MB 1 / 2 / 4 / 8 511 / 368 / 283 / 485, 16.8 MB 1 / 4 / 8
+// 1021 / 501 / 618.
 inline void copy_result(void *dst, const void *src, size_t n)
 {
-    constexpr size_t kPerThread = size_t(2) << 20;
-    if (n < 2 * kPerThread) {  // asking for the cores takes 4 us
+    if (n < size_t(2) << 20) {  // asking for the cores takes 4 us
         std::memcpy(dst, src, n);
         return;
     }
-    const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
-    const size_t nt = std::max<size_t>(1, std::min<size_t>(std::min(8u, cores), n / kPerThread));
+    const size_t cores = std::max(1u, std::thread::hardware_concurrency());
+    const size_t nt = std::min(cores, std::max(std::min<size_t>(4, n >> 20), std::min<size_t>(8, n >> 22)));
     const size_t part = round_up((n + nt - 1) / nt, 4096);
     const auto copy = [=](size_t k) {
         const size_t a = std::min(n, k * part), b = std::min(n, a + part);
