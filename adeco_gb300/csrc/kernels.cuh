@@ -64,6 +64,7 @@ struct DepositParams {
     double *out_d;                    // FP64 grids (plain path)
     int *counter;                     // persistent work counter
     unsigned long long *stats;        // kNumStats counters or nullptr
+    const int *nothing;               // null, or set when no tet can meet its grid: the launch ends at once
     int *error;                       // device error flag (bit 0: tet too large, bit 2: route list full,
                                       // bit 3: a bounded wait timed out; no deposit kernel has one)
     // ill-conditioned tets, deposited by a second launch (route_fp64_kernel):
@@ -1054,6 +1055,7 @@ __global__ void __launch_bounds__(kThreads, 2) deposit_mixed_kernel(DepositParam
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SharedMixed &S = *reinterpret_cast<SharedMixed *>(smem_raw);
     const int warp = threadIdx.x >> 5;
+    if (P.nothing && *P.nothing) return;
     PairStats st;
     int turn = 0, odd = 0;  // the pair list's counters and the wave's flag in use
     if (threadIdx.x == 0) S.flags[0] = S.list.n[0] = S.list.next[0] = S.cut[0] = S.cut_next[0] = 0;

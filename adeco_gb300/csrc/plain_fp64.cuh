@@ -313,6 +313,7 @@ __global__ void __launch_bounds__(kPlainThreads) deposit_plain_fp64_kernel(Depos
                                                                            const long long *item_cube_offset,
                                                                            int warp_cubes)
 {
+    if (P.nothing && *P.nothing) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PlainWarp &W = reinterpret_cast<PlainWarp *>(smem_raw)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;

@@ -431,6 +431,7 @@ static int enqueue_deposit(int dev, const DeviceProps &dp, const float *d_pos, s
     P.out_d = d_f64;
     P.counter = t_work.counter.p;
     P.error = t_work.counter.p + 1;
+    if (box_blocks) P.nothing = &t_work.box.p->empty;
     if (plain) return launch_plain(dp, P, t_work.cube_off.p, 0, (long long)num_patches * m * m * m, st);
     set_route(P, t_work.route.p, rcap);
     return launch_mixed(dp, P, st);

@@ -166,3 +166,26 @@ def test_whole_tets_on_coarse_grids(adeco, oracle, dims, order):
     assert abs(zoom.sum() - n_tets) <= tol and abs(leaf.sum() - n_tets) <= tol
     if dims == 1:
         assert got.sum() == n_tets and zoom.sum() == n_tets
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["mixed", "plain_fp64"])
+def test_calls_beside_and_inside_the_grid_in_turn(adeco, oracle, precision):
+    """A launch whose vertices cannot meet the grid ends at once: only that
+    one.  Boxes beside the patches, touching them by a face, holding one
+    corner, and a NaN vertex among patches that lie outside otherwise."""
+    m = 4
+    rng = np.random.default_rng(9)
+    v = np.stack(np.meshgrid(*[np.arange(m + 1.0)] * 3, indexing="ij"), -1)[..., ::-1] + rng.uniform(-0.2, 0.2, (m + 1,) * 3 + (3,))
+    v[0, 0, 0] = 0.0
+    v = np.maximum(v, 0.0).astype(np.float32)
+    tol = dict(rel=1e-5, abs_=1e-7) if precision == 0 else dict(rel=1e-10, abs_=1e-12)
+    for lo, hi, meets in ((9.0, 11.0, False), (1.0, 3.0, True), (-2.0, 0.0, False), (-2.0, 0.5, True), (50.0, 52.0, False)):
+        box = np.array([lo, hi] * 3, np.float32)
+        got = adeco.deposit_tets_ex(v.reshape(-1), m, box, 6, precision=precision)
+        check_cells(got, oracle.deposit_patches(v.reshape(-1), m, box, 6, fp64=True), n_tets=6 * m ** 3, **tol)
+        assert (got.sum() > 0) == meets
+    odd = v.copy()
+    odd[m, m, m, 1] = np.nan
+    got = adeco.deposit_tets_ex(odd.reshape(-1), m, np.array([1.0, 2.5] * 3, np.float32), 6, precision=precision)
+    want = adeco.deposit_tets_ex(v.reshape(-1), m, np.array([1.0, 2.5] * 3, np.float32), 6, precision=precision)
+    assert np.allclose(got, want, rtol=1e-13)  # the tets of that vertex lie outside this box
