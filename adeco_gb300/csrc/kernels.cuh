@@ -1362,10 +1362,9 @@ __global__ void __launch_bounds__(7 * 32) call_box_kernel(const float *part, int
         box->ext[a] = ext;
     }
     empty = __any_sync(0xffffffffu, empty);
-    if (lane == 0) {
-        box->empty = empty;
-        if (host) *host = *box;
-    }
+    if (lane == 0) box->empty = empty;
+    __syncwarp();  // the lanes' axes are written
+    if (lane == 0 && host) *host = *box;
 }
 
 // A pass's sums of the box's cells, from the fixed point grid (times scale)
