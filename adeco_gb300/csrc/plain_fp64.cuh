@@ -104,20 +104,23 @@ __device__ __forceinline__ double side_fraction_f64(double x0, double x1, double
     const double c = sel4_f64((pm >> 4) & 3, x0, x1, x2, x3), d = sel4_f64((pm >> 6) & 3, x0, x1, x2, x3);
     const double in[4] = {a, k3 ? b : a, k1 ? a : (k2 ? b : c), b};
     const double out[4] = {k1 ? b : (k2 ? c : d), k1 ? c : d, k2 ? c : d, d};
-    double t[4], u[4];
+    double t[4], w[4] = {1.0, 1.0, 1.0, 1.0}, r[4] = {1.0, 1.0, 1.0, 1.0};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         if (e == 3 && !k2) {  // only two inside vertices have a fourth edge
-            t[e] = u[e] = 0.0;
+            t[e] = 0.0;
             continue;
         }
-        const double d = out[e] - in[e], r = face_rcp(d);
-        t[e] = sat01_f64(quot_f64(plane - in[e], d, r));
-        u[e] = sat01_f64(quot_f64(out[e] - plane, d, r));
+        w[e] = out[e] - in[e];
+        r[e] = face_rcp(w[e]);
+        t[e] = sat01_f64(quot_f64(plane - in[e], w[e], r[e]));
     }
     if (k1) return t[0] * t[1] * t[2];
-    if (k2) return fma(t[2], t[3], t[0] * (t[3] * u[2] + t[1] * u[3]));
-    return fma(u[0], fma(u[1], t[2], t[1]), t[0]);
+    // u = 1 - t of the edges that have one: BC and BD (two inside), AD and BD (three)
+    const double ua = sat01_f64(quot_f64((k2 ? out[2] : out[0]) - plane, k2 ? w[2] : w[0], k2 ? r[2] : r[0]));
+    const double ub = sat01_f64(quot_f64((k2 ? out[3] : out[1]) - plane, k2 ? w[3] : w[1], k2 ? r[3] : r[1]));
+    if (k2) return fma(t[2], t[3], t[0] * (t[3] * ua + t[1] * ub));
+    return fma(ua, fma(ub, t[2], t[1]), t[0]);
 }
 
 __device__ __forceinline__ void plain_put_last(PlainWarp &W, int slot, const double p[12], int f, int mask, int owner)
